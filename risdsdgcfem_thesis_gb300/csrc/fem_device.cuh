@@ -49,7 +49,6 @@ struct StepScalars {
     uint32_t confirm;       // mixed: this iteration only measures the FP64 residual (exit test)
     float alpha_f;          // mixed: this iteration's alpha in FP32 (0 on a confirm iteration)
     uint32_t brk;           // mixed: this iteration breaks down (|d.q| < abs^2) and leaves the loop
-    uint32_t done_prev;     // MINRES: `done` as it was at the top of the current iteration
     uint32_t mr_pending;    // batch MINRES: 1 = this iteration's vector and iterate update is due,
                             // 2 = the start (or restart) residual is to be normalised
     // batch: the step's Newton level (QIE meshes make one pass of it)
@@ -68,7 +67,14 @@ struct StepScalars {
     // F^T F (FP64 MSVD in place of double-float), and with FP32 rotations an
     // MSVD branch near a tie or a failed sensitivity check
     uint32_t res_det_F, res_isotropic, res_tie, res_check;
-    uint32_t fin_ticket;    // FP64 solid: blocks of the running kernel done with their partial (0 between kernels)
+    // FP64 solid's step loops: the state after the running iteration. An
+    // iteration's kernels read either the committed fields above or these,
+    // never ones that another block of the same kernel writes: the last
+    // kernel of an iteration writes these, an early kernel of the next one
+    // commits them.
+    double delta_pend;
+    MinresScalars mr_pend;
+    uint32_t done_pend;
 };
 
 // One MINRES iteration's Givens rotation and update coefficients from
@@ -127,7 +133,16 @@ struct MeshView {
     const uint32_t* bsr_row = nullptr;
     const uint32_t* bsr_col = nullptr;
     const double* bsr_val = nullptr;
+    // FP64 solid, C_WRP: each element's fixed-point product matrix (fx.cuh),
+    // kFxGroups 16-byte groups of two entries, [kFxGroups][T], the last
+    // group's second half the scale; when set, eout holds fixed-point records
+    // of the product instead of doubles. fx_guard: log2 of the largest
+    // number of element corners at a node, rounded up.
+    int4* Kfx = nullptr;
+    uint32_t fx_guard = 0;
+    const float* grade = nullptr;  // [T] max|Dm| max|Dm^-1| of the rest shape
 };
+constexpr uint32_t kFxGroups = 23;
 
 struct StepConsts {
     double dt, inv_dt, mass, factor_M, factor_K;
@@ -146,6 +161,9 @@ void launch_begin_eval_fp64(const MeshView<double>& m, const double* x, double* 
 struct DapdParams;
 void launch_begin_eval_dapd_fp64(const MeshView<double>& m, const double* xprev, const double* x, uchar2* doc,
                                  const DapdParams& p, double* F_out, StepScalars* st, cudaStream_t s);
+// Bakes every element's fixed-point product matrix (m.Kfx) from its rotation,
+// shape gradients and material.
+void launch_elem_bake_fp64(const MeshView<double>& m, cudaStream_t s);
 void launch_elem_spmv_fp64(const MeshView<double>& m, const double* d, const StepScalars* st, int check_done,
                            cudaStream_t s);
 void launch_elem_force_fp64(const MeshView<double>& m, const double* x, int write_out, double* energy_partials,
@@ -156,17 +174,20 @@ void launch_knc_fp64(uint32_t N, uint32_t count, const uint32_t* nodes, const do
                      const StepConsts& c, double* b, double* y, cudaStream_t s);
 void launch_node_residual_fp64(const MeshView<double>& m, const StepConsts& c, const double* b, const double* y,
                                double* r, double* d, double* partials, cudaStream_t s);
-// The CG iteration's two reductions end in the kernel that makes their
-// partials: the block that finishes last adds them (slot order) and takes
-// the scalar step (alpha; beta and the loop test), and with set_cond sets
-// the step graph's WHILE condition.
-void launch_node_q_fp64(const MeshView<double>& m, const StepConsts& c, const double* d, double* q,
-                        double* partials, StepScalars* st, cudaStream_t s, cudaGraphConditionalHandle cond = 0,
-                        int set_cond = 0);
-void launch_node_xr_fp64(uint32_t N, double* y, double* r, const double* d, const double* q, double* partials,
-                         StepScalars* st, cudaStream_t s, cudaGraphConditionalHandle cond = 0, int set_cond = 0);
-void launch_node_d_fp64(uint32_t N, const uint8_t* fixed, double* d, const double* r, const StepScalars* st,
-                        cudaStream_t s);
+// The solvers' reductions are added where they are used: a kernel leaves one
+// partial per block, and every block of the next kernel adds them all (the
+// same sum in each) and takes the scalar step (alpha; beta and the loop
+// test). Against a last-block finish (fence, ticket, a second round trip)
+// that took 3.5 us off node_q and 3 us off node_xr at 20,480 tets. pq, pr:
+// the partials of d.q and |r|^2 (node_grid(N) and vec_grid(3 N) of them).
+// With set_cond the iteration's last kernel sets the step graph's WHILE
+// condition.
+void launch_node_q_fp64(const MeshView<double>& m, const StepConsts& c, const double* d, double* q, double* pq,
+                        const StepScalars* st, cudaStream_t s);
+void launch_node_xr_fp64(uint32_t N, double* y, double* r, const double* d, const double* q, const double* pq,
+                         double* pr, StepScalars* st, cudaStream_t s);
+void launch_node_d_fp64(uint32_t N, const uint8_t* fixed, double* d, const double* r, const double* pr,
+                        StepScalars* st, cudaStream_t s, cudaGraphConditionalHandle cond = 0, int set_cond = 0);
 void launch_integrate_fp64(uint32_t N, double dt, double* x, double* v, const double* y, cudaStream_t s);
 // Fully-implicit Euler (Newton on Delta x) pieces, FP64 solid path.
 void launch_node_b_fie_fp64(const MeshView<double>& m, const StepConsts& c, const double* x, const double* xn,
@@ -190,30 +211,31 @@ void launch_mr_start_fp64(uint32_t N, double* v1, double* v, double* p, double* 
                           cudaStream_t s);
 // v1 = S A w - beta v0 (w = v, eout of v) ; partial v1.v
 void launch_mr_q_fp64(const MeshView<double>& m, const StepConsts& c, const double* v, const double* v0,
-                      double* v1, double* partials, const StepScalars* st, cudaStream_t s);
-// v1 -= alpha v ; partial |v1|^2
-void launch_mr_v1_fp64(uint32_t N, double* v1, const double* v, double* partials, const StepScalars* st,
+                      double* v1, double* pq, StepScalars* st, cudaStream_t s);
+// alpha = v1.v ; v1 -= alpha v ; partial |v1|^2
+void launch_mr_v1_fp64(uint32_t N, double* v1, const double* v, const double* pq, double* pr, StepScalars* st,
                        cudaStream_t s);
+// |v1|^2, the Givens rotation and the loop test, then
 // v1 /= beta_new ; p0 <- (w - r2 p - r3 p0) / r1 (the new p, in p0's buffer) ; y += coef p_new
 void launch_mr_update_fp64(uint32_t N, double* v1, const double* v, const double* p, double* p0, double* y,
-                           const StepScalars* st, cudaStream_t s);
+                           const double* pr, StepScalars* st, cudaStream_t s, cudaGraphConditionalHandle cond = 0,
+                           int set_cond = 0);
 void launch_potential_fp64(const MeshView<double>& m, const StepConsts& c, const double* x, double* partials,
                            cudaStream_t s);
 void launch_apply_A_fp64(const MeshView<double>& m, double factor_M, double factor_K, double mass,
                          const double* d, double* q, cudaStream_t s);
-void launch_gather_sum_fp64(const MeshView<double>& m, double sign, double* f, cudaStream_t s);
+void launch_gather_sum_fp64(const MeshView<double>& m, double sign, double* f, bool records, cudaStream_t s);
 void launch_rebake_material_fp64(uint32_t T, const double* vol, double k0, double k1, double k2, double* mat,
                                  cudaStream_t s);
 
 // finalizers: one block, fixed-order sums of `count` block partials
 enum FinalizeKind {
-    FIN_INIT = 0, FIN_ALPHA = 1, FIN_BETA = 2, FIN_ENERGY_E = 3, FIN_ENERGY_P = 4, FIN_STATS = 5,
+    FIN_INIT = 0, FIN_ENERGY_E = 3, FIN_ENERGY_P = 4, FIN_STATS = 5,
     FIN_SUM = 6,  // host_sum = total
-    // MINRES: init (|r0|^2 = total, |b|^2 from host_sum), alpha, beta + Givens, stats
-    FIN_MR_INIT = 7, FIN_MR_ALPHA = 8, FIN_MR_BETA = 9, FIN_MR_STATS = 10
+    // MINRES: init (|r0|^2 = total, |b|^2 from host_sum), stats
+    FIN_MR_INIT = 7, FIN_MR_STATS = 8
 };
-// set_cond: the kinds that end a solver's loop test (init, alpha, beta and
-// their MINRES forms) also set the step graph's WHILE condition `cond` to
+// set_cond: the solvers' starts also set the step graph's WHILE condition `cond` to
 // "the loop goes on"
 void launch_finalize(int kind, const double* partials, uint32_t count, const StepConsts& c, StepScalars* st,
                      cudaStream_t s, cudaGraphConditionalHandle cond = 0, int set_cond = 0);
@@ -244,7 +266,22 @@ bool cg_cluster_fits(const CgClusterPlan& p);
 cudaError_t launch_cg_cluster_fp64(const MeshView<double>& m, const StepConsts& c, const CgClusterPlan& p,
                                    const uint32_t* ent, const double* b, double* y, StepScalars* st, cudaStream_t s);
 
-uint32_t grid_for(uint32_t n);    // grid size of the grid-stride kernels
+// Launch shapes of the grid-stride kernels. One FP64 instruction of a warp
+// holds its sub-partition for 64 clocks, so small launches spread one warp
+// per block until every sub-partition of the 152 SMs has one.
+constexpr uint32_t kSubPartitions = 608;
+inline uint32_t elem_block(uint32_t T) { return T <= 32 * kSubPartitions ? 32u : (T <= 64 * kSubPartitions ? 64u : 128u); }
+inline uint32_t capped(uint32_t g, uint32_t cap) { return g < 1 ? 1 : (g > cap ? cap : g); }
+inline uint32_t elem_grid(uint32_t T) { return capped((T + elem_block(T) - 1) / elem_block(T), 4096u); }
+// Node kernels (four lanes per node) and vector kernels (one per component):
+// 128 threads until every SM has two blocks, then 512; at most three blocks
+// per SM, so that the block that ends a reduction adds at most one partial
+// per thread.
+inline uint32_t row_block(uint32_t n) { return n <= 304u * 128u ? 128u : 512u; }
+inline uint32_t row_grid(uint32_t n) { return capped((n + row_block(n) - 1) / row_block(n), 456u); }
+inline uint32_t node_rows(uint32_t N) { return 4u * (N < (1u << 29) ? N : (1u << 29)); }
+inline uint32_t node_grid(uint32_t N) { return row_grid(node_rows(N)); }
+inline uint32_t vec_grid(uint32_t n) { return row_grid(n); }
 uint64_t& launch_counter();       // kernels launched by this library
 
 // Optional per-kernel timing with CUDA events recorded on the launching

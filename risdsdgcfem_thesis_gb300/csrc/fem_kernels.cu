@@ -1,24 +1,23 @@
 // fem_kernels.cu -- FP64 element products, node gathers and CG vector
 // kernels of the corotational linear-tet implicit-Euler step.
 //
-// Element products use the strain form of K0 = V B^T E B
-// (TetrahedronElement3::Compute_K, TetrahedronElement3.h:157-173): with
-// Dm^-1 rows = gradients of the shape functions of nodes 1..3 and node 0's
-// the negative sum, K0 u = V B^T sigma(eps(u)), eps = sym(H),
-// H = [u1-u0, u2-u0, u3-u0] Dm^-1. Mathematically identical to the
-// reference's 16 stored 3x3 blocks; 9+3 scalars per element instead of 144
-// and about 140 FMA per product instead of 216.
+// Element products use K0 = V B^T E B (TetrahedronElement3::Compute_K,
+// TetrahedronElement3.h:157-173) through the shape-function gradients (rows of
+// Dm^-1; node 0's the negative sum) instead of the reference's 16 stored 3x3
+// blocks: the C_WRP differential as one 9 x 9 matrix per element in fixed
+// point (fx.cuh), the forces and energies in the strain form
+// (elem_math.cuh).
 //
 // Scatter is atomics-free: each element writes its four nodal vectors to
-// eout, and one thread per node sums its entries in element order (the order
-// the reference's serial scatter adds them). Reductions are deterministic:
-// warp shuffles, a fixed block tree, then one block summing the block
-// partials in index order.
+// eout, and four lanes per node sum its entries in a fixed order. Reductions are
+// deterministic: integer warp sums (fx_warp_sum), a fixed block tree, then
+// the last block to finish summing the block partials.
 #include "bounds.cuh"
 #include "lcm.cuh"
 #include "fem_device.cuh"
 #include "msvd.cuh"
 #include "elem_math.cuh"
+#include "fx.cuh"
 
 #include <cooperative_groups.h>
 
@@ -123,14 +122,6 @@ uint64_t& launch_counter()
     return n;
 }
 
-uint32_t grid_for(uint32_t n)
-{
-    uint32_t g = (n + kBlock - 1) / kBlock;
-    if (g < 1) g = 1;
-    if (g > 4096) g = 4096;
-    return g;
-}
-
 __device__ __forceinline__ double warp_sum(double v)
 {
 #pragma unroll
@@ -138,19 +129,26 @@ __device__ __forceinline__ double warp_sum(double v)
     return v;
 }
 
-// Block sum with a fixed tree; result valid in thread 0.
+// Block sum, valid in every thread (two rounds of fx_warp_sum).
 __device__ __forceinline__ double block_sum(double v)
 {
     __shared__ double sh[32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    v = warp_sum(v);
+    v = fx_warp_sum(v);
+    if (blockDim.x == 32) return v;
     __syncthreads();
     if (lane == 0) sh[wid] = v;
     __syncthreads();
-    const int nw = (blockDim.x + 31) >> 5;
-    v = (threadIdx.x < nw) ? sh[threadIdx.x] : 0.0;
-    if (wid == 0) v = warp_sum(v);
-    return v;
+    return fx_warp_sum(lane < (int)((blockDim.x + 31) >> 5) ? sh[lane] : 0.0);
+}
+
+// The total of the previous kernel's block partials, valid in every thread
+// and the same in every block.
+__device__ __forceinline__ double grid_total(const double* __restrict__ partials, uint32_t count)
+{
+    double acc = 0.0;
+    for (uint32_t i = threadIdx.x; i < count; i += blockDim.x) acc += partials[i];
+    return block_sum(acc);
 }
 
 template <typename S>
@@ -208,7 +206,7 @@ __global__ void k_elem_lcm_force_fp64(MeshView<double> m, const double* __restri
 __global__ void k_elem_lcm_spmv_fp64(MeshView<double> m, const double* __restrict__ d, const double* __restrict__ F,
                                      PkMaterial mat, const StepScalars* st, int check_done)
 {
-    if (check_done && st->done) return;
+    if (check_done && st->done_pend) return;
     for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < m.T; e += gridDim.x * blockDim.x) {
         const int4 t = m.tets[e];
         const int ids[4] = {(int)bounds_idx((uint32_t)t.x, m.N, kSiteElemNode),
@@ -238,30 +236,78 @@ __global__ void k_elem_lcm_spmv_fp64(MeshView<double> m, const double* __restric
 
 // ---- element kernels ----
 
-__global__ void k_elem_spmv_fp64(MeshView<double> m, const double* __restrict__ d, const StepScalars* st,
-                                 int check_done)
+__device__ __forceinline__ void load_nodal(const MeshView<double>& m, uint32_t e, const double* __restrict__ d, double* dl)
 {
-    if (check_done && st->done) return;
+    const int4 t = m.tets[e];
+    const int ids[4] = {(int)bounds_idx((uint32_t)t.x, m.N, kSiteElemNode),
+                        (int)bounds_idx((uint32_t)t.y, m.N, kSiteElemNode),
+                        (int)bounds_idx((uint32_t)t.z, m.N, kSiteElemNode),
+                        (int)bounds_idx((uint32_t)t.w, m.N, kSiteElemNode)};
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        dl[3 * i] = d[3 * (size_t)ids[i]];
+        dl[3 * i + 1] = d[3 * (size_t)ids[i] + 1];
+        dl[3 * i + 2] = d[3 * (size_t)ids[i] + 2];
+    }
+}
+
+// Element e's fixed-point product matrix (fx.cuh) from R, Dm^-1 and the
+// material scalars: 45 entries and the scale, 368 bytes, written once per
+// evaluation. Integer-bound: about 250 products of three multiplies (284 us
+// for 1,080,000 tets, a fifth of their rotations).
+__global__ void __launch_bounds__(128, 3) k_elem_bake_fp64(MeshView<double> m)
+{
     for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < m.T; e += gridDim.x * blockDim.x) {
-        const int4 t = m.tets[e];
         double R[9], Di[9], k1, knu, k2;
         load_elem(m, e, R, Di, k1, knu, k2);
+        FxL even{0, 0};
+        auto put = [&](int k, FxL v) {  // two entries per 16-byte group
+            if ((k & 1) == 0) even = v;
+            else m.Kfx[(size_t)(k >> 1) * m.T + e] = make_int4(even.l, even.h, v.l, v.h);
+        };
+        const int32_t scale = fx_grade_ok(m.grade[e], knu, k2) ? fx_bake(R, Di, knu, k2, put) : kFxFp64;
+        m.Kfx[(size_t)(kFxGroups - 1) * m.T + e] = make_int4(even.l, even.h, scale, 0);
+    }
+}
+
+// The FP64 product of an element fx.cuh leaves out, as a record.
+__device__ __noinline__ void elem_record_fp64(const MeshView<double>& m, uint32_t e, const double* dl, int64_t* out)
+{
+    double R[9], Di[9], k1, knu, k2, o[12];
+    load_elem(m, e, R, Di, k1, knu, k2);
+    elem_RKRt(R, Di, k1, knu, k2, dl, o);
+    fx_stamp_doubles(o, out);
+}
+
+// R K0 R^T d per element as fixed-point records in eout. 368 bytes of matrix
+// per element: bound by the integer pipe while the matrices stay in L2 (up to
+// about 300k tets) and by HBM beyond. The FP64 strain form held the FP64 pipe
+// at 90 %: 7,215 tets 11.4 -> 4.0 us, 20,480 tets 11.7 -> 5.3 us, 1,080,000
+// tets 273 -> 119 us (540 MB, 4.5 TB/s).
+__global__ void __launch_bounds__(128, 3) k_elem_spmv_fp64(MeshView<double> m, const double* __restrict__ d,
+                                                           const StepScalars* st, int check_done)
+{
+    if (check_done && st->done_pend) return;
+    for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < m.T; e += gridDim.x * blockDim.x) {
         double dl[12];
-        const int ids[4] = {(int)bounds_idx((uint32_t)t.x, m.N, kSiteElemNode),
-                            (int)bounds_idx((uint32_t)t.y, m.N, kSiteElemNode),
-                            (int)bounds_idx((uint32_t)t.z, m.N, kSiteElemNode),
-                            (int)bounds_idx((uint32_t)t.w, m.N, kSiteElemNode)};
+        load_nodal(m, e, d, dl);
+        const int4* Kp = m.Kfx + e;
+        const int4 last = Kp[(size_t)(kFxGroups - 1) * m.T];
+        FxL D[9];
+        int64_t out[12];
+        int32_t x;
+        bool ok = fx_differences(dl, D, x) && last.z != kFxFp64;
+        int4 cur;
+        x += last.z + fx_product([&](int k) {
+            if (k == kFxK - 1) cur = last;
+            else if ((k & 1) == 0) cur = Kp[(size_t)(k >> 1) * m.T];
+            return (k & 1) ? FxL{cur.z, cur.w} : FxL{cur.x, cur.y};
+        }, D, out);
+        ok = ok && fx_stamp(out, x);
+        if (!ok) elem_record_fp64(m, e, dl, out);
+        longlong2* o = reinterpret_cast<longlong2*>(m.eout + 12 * (size_t)e);
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            dl[3 * i] = d[3 * (size_t)ids[i]];
-            dl[3 * i + 1] = d[3 * (size_t)ids[i] + 1];
-            dl[3 * i + 2] = d[3 * (size_t)ids[i] + 2];
-        }
-        double out[12];
-        elem_RKRt(R, Di, k1, knu, k2, dl, out);
-        double* o = m.eout + 12 * (size_t)e;
-#pragma unroll
-        for (int c = 0; c < 12; c++) o[c] = out[c];
+        for (int c = 0; c < 6; c++) o[c] = make_longlong2(out[2 * c], out[2 * c + 1]);
     }
 }
 
@@ -346,42 +392,81 @@ __global__ void k_potential_fp64(MeshView<double> m, StepConsts c, const double*
 
 // ---- node kernels ----
 
-__device__ __forceinline__ void gather3(const MeshView<double>& m, uint32_t n, double& a0, double& a1, double& a2)
+// The sums at a node are taken by four lanes of a warp (eight nodes per
+// warp): lanes 0 to 2 return the components, lane 3 zero. Every lane of a
+// warp calls them (on: the node exists). One thread per node left most of the
+// chip idle at 20,480 tets (node_q: 20 blocks, 15.9 us; now 5.6) and took
+// three FP64 adds per corner (1,080,000 tets: 74 us; now 40).
+
+// Element outputs in FP64 (forces, and the products of the P-K materials):
+// lane a adds component a of the node's corners in element order.
+__device__ __forceinline__ double gather_fp64(const MeshView<double>& m, uint32_t n, uint32_t a, bool on)
 {
+    double s = 0.0;
+    if (!on || a == 3) return s;
     const uint32_t beg = m.csr_ptr[n], end = m.csr_ptr[n + 1];
-    for (uint32_t j = beg; j < end; j++) {
-        const double* o = m.eout + 3 * (size_t)bounds_idx(m.csr_idx[j], 4ull * m.T, kSiteCsrEntry);
-        a0 += o[0];
-        a1 += o[1];
-        a2 += o[2];
+#pragma unroll 4
+    for (uint32_t j = beg; j < end; j++)
+        s += m.eout[3 * (size_t)bounds_idx(m.csr_idx[j], 4ull * m.T, kSiteCsrEntry) + a];
+    return s;
+}
+
+// Fixed-point records: lane l adds the corners beg + l, beg + l + 4, ... in
+// all three components (integer sums in block exponents, fx.cuh), then the
+// lanes' sums are brought to the largest exponent and added.
+__device__ __forceinline__ double gather_fx(const MeshView<double>& m, uint32_t n, uint32_t a, bool on)
+{
+    const int32_t guard = (int32_t)m.fx_guard;
+    FxSum s[3] = {{0, 0}, {0, 0}, {0, 0}};
+    if (on) {
+        const uint32_t beg = m.csr_ptr[n], end = m.csr_ptr[n + 1];
+        const long long* rec = reinterpret_cast<const long long*>(m.eout);
+#pragma unroll 2
+        for (uint32_t j = beg + a; j < end; j += 4) {
+            const long long* r = rec + 3 * (size_t)bounds_idx(m.csr_idx[j], 4ull * m.T, kSiteCsrEntry);
+            const int64_t v0 = r[0], v1 = r[1], v2 = r[2];
+            const int32_t x = fx_record_exp(v0, v1, v2);
+            fx_add(s[0], v0, x, guard);
+            fx_add(s[1], v1, x, guard);
+            fx_add(s[2], v2, x, guard);
+        }
     }
+    int32_t E = s[0].E;
+    E = max(E, __shfl_xor_sync(0xffffffffu, E, 1));
+    E = max(E, __shfl_xor_sync(0xffffffffu, E, 2));
+    const int32_t sh = fx_min63(E - s[0].E);
+    FxSum t{0, E};
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        long long v = s[c].acc >> sh;
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        if ((int)a == c) t.acc = v;
+    }
+    return fx_sum_value(t, guard);
 }
 
 // K u at node n for the solvers' node kernels: the assembled row when the
-// solid has one (9 FMAs per block), else the gather of the element outputs
-// of the product the solver launched before.
-__device__ __forceinline__ void node_Ku(const MeshView<double>& m, const double* __restrict__ u, uint32_t n,
-                                        double& a0, double& a1, double& a2)
+// solid has one (3 FMAs per block and lane), else the sum of the element
+// outputs of the product launched before.
+__device__ __forceinline__ double node_Ku(const MeshView<double>& m, const double* __restrict__ u, uint32_t n,
+                                          uint32_t a, bool on)
 {
     if (m.bsr_val) {
+        double s = 0.0;
+        if (!on || a == 3) return s;
         const uint32_t beg = m.bsr_row[n], end = m.bsr_row[n + 1];
+#pragma unroll 2
         for (uint32_t k = beg; k < end; k++) {
             const size_t j = 3 * (size_t)bounds_idx(m.bsr_col[k], m.N, kSiteBsrEntry);
-            const double* A = m.bsr_val + 9 * (size_t)k;
-            const double u0 = u[j], u1 = u[j + 1], u2 = u[j + 2];
-            a0 = fma(A[0], u0, a0);
-            a0 = fma(A[1], u1, a0);
-            a0 = fma(A[2], u2, a0);
-            a1 = fma(A[3], u0, a1);
-            a1 = fma(A[4], u1, a1);
-            a1 = fma(A[5], u2, a1);
-            a2 = fma(A[6], u0, a2);
-            a2 = fma(A[7], u1, a2);
-            a2 = fma(A[8], u2, a2);
+            const double* A = m.bsr_val + 9 * (size_t)k + 3 * a;
+            s = fma(A[0], u[j], s);
+            s = fma(A[1], u[j + 1], s);
+            s = fma(A[2], u[j + 2], s);
         }
-    } else {
-        gather3(m, n, a0, a1, a2);
+        return s;
     }
+    return m.Kfx ? gather_fx(m, n, a, on) : gather_fp64(m, n, a, on);
 }
 
 // One block of the assembled stiffness per thread (see
@@ -439,16 +524,16 @@ __global__ void k_bsr_assemble_fp64(MeshView<double> m, uint32_t nnzb, const uin
 // b = dt (m g + f_e) + m v ; y = v   (Step_QuasiImplicitEuler_v, :1211-1231)
 __global__ void k_node_b_fp64(MeshView<double> m, StepConsts c, const double* __restrict__ v, double* b, double* y)
 {
-    for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < m.N; n += gridDim.x * blockDim.x) {
-        double f0 = 0, f1 = 0, f2 = 0;
-        gather3(m, n, f0, f1, f2);
-        const size_t i = 3 * (size_t)n;
-        b[i] = (c.mass * c.gravity[0] - f0) * c.dt + c.mass * v[i];
-        b[i + 1] = (c.mass * c.gravity[1] - f1) * c.dt + c.mass * v[i + 1];
-        b[i + 2] = (c.mass * c.gravity[2] - f2) * c.dt + c.mass * v[i + 2];
-        y[i] = v[i];
-        y[i + 1] = v[i + 1];
-        y[i + 2] = v[i + 2];
+    const uint32_t a = threadIdx.x & 3u, step = (gridDim.x * blockDim.x) >> 2;
+    for (uint32_t n = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; (n & ~7u) < m.N; n += step) {
+        const bool on = n < m.N;
+        const double f = gather_fp64(m, n, a, on);
+        if (!on || a == 3) continue;
+        const size_t i = 3 * (size_t)n + a;
+        const double vi = v[i];
+        const double g = a == 0 ? c.gravity[0] : (a == 1 ? c.gravity[1] : c.gravity[2]);
+        b[i] = (c.mass * g - f) * c.dt + c.mass * vi;
+        y[i] = vi;
     }
 }
 
@@ -474,89 +559,73 @@ __global__ void k_knc_fp64(uint32_t N, uint32_t count, const uint32_t* __restric
 }
 
 // r = S (b - A y) ; d = r ; partial |r|^2   (ILSS_CG.h:53-64)
-__device__ __forceinline__ void fin_alpha(StepScalars* st, double total);
-__device__ __forceinline__ void fin_beta(StepScalars* st, double total);
-
-// The grid's total of the blocks' values (v in thread 0 of each), added in
-// the block that finishes last: each block leaves its value in its slot and
-// takes a ticket; the last one (true) adds the slots in order (a strided
-// sum per thread, then the block tree) into thread 0's total and resets
-// the ticket for the next kernel.
-__device__ __forceinline__ bool grid_total_last(double v, double* partials, uint32_t* ticket, double& total)
-{
-    __shared__ bool last;
-    if (threadIdx.x == 0) {
-        partials[blockIdx.x] = v;
-        __threadfence();
-        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last) return false;
-    __threadfence();
-    double acc = 0.0;
-    for (uint32_t i = threadIdx.x; i < gridDim.x; i += blockDim.x) acc += __ldcg(partials + i);
-    total = block_sum(acc);
-    if (threadIdx.x == 0) *ticket = 0;
-    return true;
-}
-
 __global__ void k_node_residual_fp64(MeshView<double> m, StepConsts c, const double* __restrict__ b,
                                      const double* __restrict__ y, double* r, double* d, double* partials)
 {
     double acc = 0.0;
     const double mfm = c.mass * c.factor_M;
-    for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < m.N; n += gridDim.x * blockDim.x) {
-        double s0 = 0, s1 = 0, s2 = 0;
-        node_Ku(m, y, n, s0, s1, s2);
-        const size_t i = 3 * (size_t)n;
-        double r0 = 0, r1 = 0, r2 = 0;
-        if (!m.fixed[n]) {
-            r0 = b[i] - (c.factor_K * s0 + mfm * y[i]);
-            r1 = b[i + 1] - (c.factor_K * s1 + mfm * y[i + 1]);
-            r2 = b[i + 2] - (c.factor_K * s2 + mfm * y[i + 2]);
-        }
-        r[i] = r0; r[i + 1] = r1; r[i + 2] = r2;
-        d[i] = r0; d[i + 1] = r1; d[i + 2] = r2;
-        acc += r0 * r0 + r1 * r1 + r2 * r2;
+    const uint32_t a = threadIdx.x & 3u, step = (gridDim.x * blockDim.x) >> 2;
+    for (uint32_t n = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; (n & ~7u) < m.N; n += step) {
+        const bool on = n < m.N;
+        const double s = node_Ku(m, y, n, a, on);
+        if (!on || a == 3) continue;
+        const size_t i = 3 * (size_t)n + a;
+        const double ri = m.fixed[n] ? 0.0 : b[i] - (c.factor_K * s + mfm * y[i]);
+        r[i] = ri;
+        d[i] = ri;
+        acc += ri * ri;
     }
     double s = block_sum(acc);
     if (threadIdx.x == 0) partials[blockIdx.x] = s;
 }
 
 // q = S A d ; partial d.q   (ILSS_CG.h:90-96)
-__global__ void k_node_q_fp64(MeshView<double> m, StepConsts c, const double* __restrict__ d, double* q,
-                              double* partials, StepScalars* st, cudaGraphConditionalHandle cond, int set_cond)
+__global__ void k_node_q_fp64(MeshView<double> m, StepConsts c, const double* __restrict__ d, double* q, double* pq,
+                              const StepScalars* st)
 {
-    if (st->done) return;
+    if (st->done_pend) return;
     double acc = 0.0;
     const double mfm = c.mass * c.factor_M;
-    for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < m.N; n += gridDim.x * blockDim.x) {
-        double s0 = 0, s1 = 0, s2 = 0;
-        node_Ku(m, d, n, s0, s1, s2);
-        const size_t i = 3 * (size_t)n;
-        double q0 = 0, q1 = 0, q2 = 0;
-        if (!m.fixed[n]) {
-            q0 = c.factor_K * s0 + mfm * d[i];
-            q1 = c.factor_K * s1 + mfm * d[i + 1];
-            q2 = c.factor_K * s2 + mfm * d[i + 2];
-        }
-        q[i] = q0; q[i + 1] = q1; q[i + 2] = q2;
-        acc += d[i] * q0 + d[i + 1] * q1 + d[i + 2] * q2;
+    const uint32_t a = threadIdx.x & 3u, step = (gridDim.x * blockDim.x) >> 2;
+    for (uint32_t n = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; (n & ~7u) < m.N; n += step) {
+        const bool on = n < m.N;
+        const double s = node_Ku(m, d, n, a, on);
+        if (!on || a == 3) continue;
+        const size_t i = 3 * (size_t)n + a;
+        const double di = d[i], qi = m.fixed[n] ? 0.0 : c.factor_K * s + mfm * di;
+        q[i] = qi;
+        acc += di * qi;
     }
-    double total = 0.0;
-    if (grid_total_last(block_sum(acc), partials, &st->fin_ticket, total) && threadIdx.x == 0) {
-        fin_alpha(st, total);
-        if (set_cond) cudaGraphSetConditional(cond, st->done ? 0u : 1u);
-    }
+    const double total = block_sum(acc);
+    if (threadIdx.x == 0) pq[blockIdx.x] = total;
 }
 
-// y += alpha d ; r -= alpha q ; partial |r|^2   (ILSS_CG.h:100-117)
+// alpha = |r|^2 / d.q ; y += alpha d ; r -= alpha q ; partial |r|^2
+// (ILSS_CG.h:96-117). One thread per block takes the division (a dozen FP64
+// instructions, each 64 clocks of its sub-partition per warp that runs it).
 __global__ void k_node_xr_fp64(uint32_t N, double* y, double* r, const double* __restrict__ d,
-                               const double* __restrict__ q, double* partials, StepScalars* st,
-                               cudaGraphConditionalHandle cond, int set_cond)
+                               const double* __restrict__ q, const double* __restrict__ pq, uint32_t npq, double* pr,
+                               StepScalars* st)
 {
-    if (st->done) return;
-    const double alpha = st->alpha, na = -alpha;
+    if (st->done_pend) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) st->done = 1;
+        return;
+    }
+    __shared__ double sh_alpha;
+    const double dq = grid_total(pq, npq), delta = st->delta_pend;
+    const bool brk = ::fabs(dq) < st->abs_eps_sq;  // breakdown: leave before the update (ILSS_CG.h:97)
+    if (threadIdx.x == 0) {
+        sh_alpha = delta / dq;
+        if (blockIdx.x == 0) {
+            st->dot_dq = dq;
+            st->delta_new = delta;
+            st->done = brk ? 1u : 0u;
+            if (!brk) st->alpha = sh_alpha;
+        }
+    }
+    if (brk) return;
+    __syncthreads();
+    const double alpha = sh_alpha, na = -alpha;
     double acc = 0.0;
     const uint32_t n3 = 3 * N;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n3; i += gridDim.x * blockDim.x) {
@@ -565,21 +634,42 @@ __global__ void k_node_xr_fp64(uint32_t N, double* y, double* r, const double* _
         r[i] = ri;
         acc += ri * ri;
     }
-    double total = 0.0;
-    if (grid_total_last(block_sum(acc), partials, &st->fin_ticket, total) && threadIdx.x == 0) {
-        fin_beta(st, total);
-        if (set_cond) cudaGraphSetConditional(cond, st->done ? 0u : 1u);
-    }
+    const double total = block_sum(acc);
+    if (threadIdx.x == 0) pr[blockIdx.x] = total;
 }
 
-// d = S (beta d + r)   (ILSS_CG.h:133-137)
+// beta = |r_new|^2 / |r|^2 and the loop test ; d = S (beta d + r)
+// (ILSS_CG.h:117-137)
 __global__ void k_node_d_fp64(uint32_t N, const uint8_t* __restrict__ fixed, double* d, const double* __restrict__ r,
-                              const StepScalars* st)
+                              const double* __restrict__ pr, uint32_t npr, StepScalars* st,
+                              cudaGraphConditionalHandle cond, int set_cond)
 {
-    // Once the loop has ended (including an iteration that just ended it in
-    // FIN_BETA) d is no longer read, so the update is skipped.
-    if (st->done) return;
-    const double beta = st->beta;
+    const bool first = blockIdx.x == 0 && threadIdx.x == 0;
+    if (st->done) {
+        if (first) {
+            st->done_pend = 1;
+            if (set_cond) cudaGraphSetConditional(cond, 0u);
+        }
+        return;
+    }
+    __shared__ double sh_beta;
+    const double total = grid_total(pr, npr);
+    if (threadIdx.x == 0) {
+        sh_beta = total / st->delta_new;
+        if (blockIdx.x == 0) {
+            st->delta_old = st->delta_new;
+            st->beta = sh_beta;
+            st->delta_pend = total;
+            st->k += 1;
+            st->total_iters += 1;
+            const bool go = total > st->abs_eps_sq && total > st->delta_target && st->k < st->max_iter;
+            st->done_pend = go ? 0u : 1u;
+            if (!isfinite(total)) st->status = 3;
+            if (set_cond) cudaGraphSetConditional(cond, go ? 1u : 0u);
+        }
+    }
+    __syncthreads();
+    const double beta = sh_beta;
     const uint32_t n3 = 3 * N;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n3; i += gridDim.x * blockDim.x) {
         const uint32_t n = i / 3;
@@ -610,16 +700,16 @@ __global__ void k_node_b_fie_fp64(MeshView<double> m, StepConsts c, const double
                                   double* b, double* y)
 {
     const double im = c.inv_dt * c.mass;
-    for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < m.N; n += gridDim.x * blockDim.x) {
-        double f[3] = {0, 0, 0};
-        gather3(m, n, f[0], f[1], f[2]);
-        const size_t i = 3 * (size_t)n;
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-            const double bf = c.mass * c.gravity[a] - f[a];
-            b[i + a] = bf + im * (vn[i + a] - c.inv_dt * (x[i + a] - xn[i + a]));
-            y[i + a] = warm ? c.dt * vn[i + a] : 0.0;
-        }
+    const uint32_t a = threadIdx.x & 3u, step = (gridDim.x * blockDim.x) >> 2;
+    for (uint32_t n = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; (n & ~7u) < m.N; n += step) {
+        const bool on = n < m.N;
+        const double f = gather_fp64(m, n, a, on);
+        if (!on || a == 3) continue;
+        const size_t i = 3 * (size_t)n + a;
+        const double g = a == 0 ? c.gravity[0] : (a == 1 ? c.gravity[1] : c.gravity[2]);
+        const double bf = c.mass * g - f;
+        b[i] = bf + im * (vn[i] - c.inv_dt * (x[i] - xn[i]));
+        y[i] = warm ? c.dt * vn[i] : 0.0;
     }
 }
 
@@ -675,16 +765,15 @@ __global__ void k_mr_init_fp64(MeshView<double> m, StepConsts c, const double* _
 {
     double acc = 0.0;
     const double mfm = c.mass * c.factor_M;
-    for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < m.N; n += gridDim.x * blockDim.x) {
-        double f[3] = {0, 0, 0};
-        node_Ku(m, y, n, f[0], f[1], f[2]);
-        const size_t i = 3 * (size_t)n;
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-            const double r = m.fixed[n] ? 0.0 : b[i + a] - (c.factor_K * f[a] + mfm * y[i + a]);
-            v1[i + a] = r;
-            acc += r * r;
-        }
+    const uint32_t a = threadIdx.x & 3u, step = (gridDim.x * blockDim.x) >> 2;
+    for (uint32_t n = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; (n & ~7u) < m.N; n += step) {
+        const bool on = n < m.N;
+        const double f = node_Ku(m, y, n, a, on);
+        if (!on || a == 3) continue;
+        const size_t i = 3 * (size_t)n + a;
+        const double r = m.fixed[n] ? 0.0 : b[i] - (c.factor_K * f + mfm * y[i]);
+        v1[i] = r;
+        acc += r * r;
     }
     double s = block_sum(acc);
     if (threadIdx.x == 0) partials[blockIdx.x] = s;
@@ -693,7 +782,7 @@ __global__ void k_mr_init_fp64(MeshView<double> m, StepConsts c, const double* _
 // v1 *= 1/beta_new ; v = p = p0 = 0   (:82-95)
 __global__ void k_mr_start_fp64(uint32_t N, double* v1, double* v, double* p, double* p0, const StepScalars* st)
 {
-    const double inv = 1.0 / st->mr.beta_new;
+    const double inv = 1.0 / st->mr_pend.beta_new;
     const uint32_t n3 = 3 * N;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n3; i += gridDim.x * blockDim.x) {
         v1[i] *= inv;
@@ -705,34 +794,43 @@ __global__ void k_mr_start_fp64(uint32_t N, double* v1, double* v, double* p, do
 
 // v1 = S A v - beta v0 ; partial v1.v   (:117-123)
 __global__ void k_mr_q_fp64(MeshView<double> m, StepConsts c, const double* __restrict__ v,
-                            const double* __restrict__ v0, double* v1, double* partials, const StepScalars* st)
+                            const double* __restrict__ v0, double* v1, double* pq, StepScalars* st)
 {
-    if (st->done) return;
-    const double mfm = c.mass * c.factor_M;
-    const double nb = -st->mr.beta_new;
-    double acc = 0.0;
-    for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < m.N; n += gridDim.x * blockDim.x) {
-        double f[3] = {0, 0, 0};
-        node_Ku(m, v, n, f[0], f[1], f[2]);
-        const size_t i = 3 * (size_t)n;
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-            const double q = m.fixed[n] ? 0.0 : c.factor_K * f[a] + mfm * v[i + a];
-            const double w1 = q + nb * v0[i + a];
-            v1[i + a] = w1;
-            acc += w1 * v[i + a];
-        }
+    const bool first = blockIdx.x == 0 && threadIdx.x == 0;
+    if (st->done_pend) {
+        if (first) st->done = 1;
+        return;
     }
-    double s = block_sum(acc);
-    if (threadIdx.x == 0) partials[blockIdx.x] = s;
+    const double mfm = c.mass * c.factor_M;
+    const double nb = -st->mr_pend.beta_new;
+    if (first) {
+        st->done = 0;
+        st->mr = st->mr_pend;
+        st->mr.beta = st->mr_pend.beta_new;
+    }
+    double acc = 0.0;
+    const uint32_t a = threadIdx.x & 3u, step = (gridDim.x * blockDim.x) >> 2;
+    for (uint32_t n = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; (n & ~7u) < m.N; n += step) {
+        const bool on = n < m.N;
+        const double f = node_Ku(m, v, n, a, on);
+        if (!on || a == 3) continue;
+        const size_t i = 3 * (size_t)n + a;
+        const double vi = v[i], qi = m.fixed[n] ? 0.0 : c.factor_K * f + mfm * vi;
+        const double w1 = qi + nb * v0[i];
+        v1[i] = w1;
+        acc += w1 * vi;
+    }
+    const double total = block_sum(acc);
+    if (threadIdx.x == 0) pq[blockIdx.x] = total;
 }
 
-// v1 -= alpha v ; partial |v1|^2   (:125-129)
-__global__ void k_mr_v1_fp64(uint32_t N, double* v1, const double* __restrict__ v, double* partials,
-                             const StepScalars* st)
+// alpha = v1.v ; v1 -= alpha v ; partial |v1|^2   (:123-129)
+__global__ void k_mr_v1_fp64(uint32_t N, double* v1, const double* __restrict__ v, const double* __restrict__ pq,
+                             uint32_t npq, double* pr, StepScalars* st)
 {
-    if (st->done) return;
-    const double na = -st->mr.alpha;
+    if (st->done_pend) return;
+    const double alpha = grid_total(pq, npq), na = -alpha;
+    if (blockIdx.x == 0 && threadIdx.x == 0) st->mr.alpha = alpha;
     double acc = 0.0;
     const uint32_t n3 = 3 * N;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n3; i += gridDim.x * blockDim.x) {
@@ -740,25 +838,49 @@ __global__ void k_mr_v1_fp64(uint32_t N, double* v1, const double* __restrict__ 
         v1[i] = r;
         acc += r * r;
     }
-    double s = block_sum(acc);
-    if (threadIdx.x == 0) partials[blockIdx.x] = s;
+    const double total = block_sum(acc);
+    if (threadIdx.x == 0) pr[blockIdx.x] = total;
 }
 
-// v1 *= 1/beta_new ; p_new = ((-r2) p + w + (-r3) p0) / r1 into p0's buffer ;
-// y += beta_one c eta p_new   (:131-156)
+// The Givens rotation and the loop test (:131-144) ; v1 *= 1/beta_new ;
+// p_new = ((-r2) p + w + (-r3) p0) / r1 into p0's buffer ;
+// y += beta_one c eta p_new   (:146-156)
 __global__ void k_mr_update_fp64(uint32_t N, double* v1, const double* __restrict__ v,
-                                 const double* __restrict__ p, double* p0, double* y, const StepScalars* st)
+                                 const double* __restrict__ p, double* p0, double* y, const double* __restrict__ pr,
+                                 uint32_t npr, StepScalars* st, cudaGraphConditionalHandle cond, int set_cond)
 {
-    if (st->done_prev) return;
-    const MinresScalars mr = st->mr;
+    if (st->done) {
+        if (set_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(cond, 0u);
+        return;
+    }
+    __shared__ MinresScalars sh;
+    const double total = grid_total(pr, npr);
+    if (threadIdx.x == 0) {
+        MinresScalars mr = st->mr;
+        minres_givens(mr, total);
+        sh = mr;
+        if (blockIdx.x == 0) {
+            st->mr_pend = mr;
+            st->delta_new = mr.norm_r_sq;
+            st->k += 1;
+            st->total_iters += 1;
+            const bool go =
+                mr.norm_r_sq > st->abs_eps_sq && mr.norm_r_sq > st->delta_target && st->k < st->max_iter;
+            st->done_pend = go ? 0u : 1u;
+            if (!isfinite(total) || !isfinite(mr.norm_r_sq)) st->status = 3;
+            if (set_cond) cudaGraphSetConditional(cond, go ? 1u : 0u);
+        }
+    }
+    __syncthreads();
+    const double inv_beta = sh.inv_beta, neg_r2 = sh.neg_r2, neg_r3 = sh.neg_r3, inv_r1 = sh.inv_r1, x_coef = sh.x_coef;
     const uint32_t n3 = 3 * N;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n3; i += gridDim.x * blockDim.x) {
-        v1[i] *= mr.inv_beta;
-        double pn = mr.neg_r2 * p[i] + v[i];
-        pn += mr.neg_r3 * p0[i];
-        pn *= mr.inv_r1;
+        v1[i] *= inv_beta;
+        double pn = neg_r2 * p[i] + v[i];
+        pn += neg_r3 * p0[i];
+        pn *= inv_r1;
         p0[i] = pn;
-        y[i] += mr.x_coef * pn;
+        y[i] += x_coef * pn;
     }
 }
 
@@ -767,18 +889,16 @@ __global__ void k_apply_A_fp64(MeshView<double> m, double factor_M, double facto
                                const double* __restrict__ d, double* q)
 {
     const double mfm = mass * factor_M;
-    for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < m.N; n += gridDim.x * blockDim.x) {
-        double s0 = 0, s1 = 0, s2 = 0;
-        gather3(m, n, s0, s1, s2);
-        const size_t i = 3 * (size_t)n;
-        if (m.fixed[n]) { q[i] = 0; q[i + 1] = 0; q[i + 2] = 0; continue; }
-        q[i] = factor_K * s0 + mfm * d[i];
-        q[i + 1] = factor_K * s1 + mfm * d[i + 1];
-        q[i + 2] = factor_K * s2 + mfm * d[i + 2];
+    const uint32_t a = threadIdx.x & 3u, step = (gridDim.x * blockDim.x) >> 2;
+    for (uint32_t n = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; (n & ~7u) < m.N; n += step) {
+        const bool on = n < m.N;
+        const double s = m.Kfx ? gather_fx(m, n, a, on) : gather_fp64(m, n, a, on);
+        if (!on || a == 3) continue;
+        const size_t i = 3 * (size_t)n + a;
+        q[i] = m.fixed[n] ? 0.0 : factor_K * s + mfm * d[i];
     }
 }
 
-// f += sign * sum(eout) per node
 // Material triple of every element from one E, nu (k_c = a (1 - nu), a nu,
 // a (0.5 - nu), formed on the host): mat[c][e] = V_e k_c, the product
 // EditableTetrahedronElementSet3::SetParams re-bakes for every element
@@ -797,18 +917,18 @@ __global__ void k_rebake_material_fp64(uint32_t T, const double* __restrict__ vo
 void launch_rebake_material_fp64(uint32_t T, const double* vol, double k0, double k1, double k2, double* mat,
                                  cudaStream_t s)
 {
-    k_rebake_material_fp64<<<grid_for(T), kBlock, 0, s>>>(T, vol, k0, k1, k2, mat);
+    k_rebake_material_fp64<<<vec_grid(T), row_block(T), 0, s>>>(T, vol, k0, k1, k2, mat);
     launch_counter()++;
 }
 
-__global__ void k_gather_sum_fp64(MeshView<double> m, double sign, double* f)
+// f += sign * sum(eout) per node; records: eout holds those of a product
+__global__ void k_gather_sum_fp64(MeshView<double> m, double sign, double* f, int records)
 {
-    for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < m.N; n += gridDim.x * blockDim.x) {
-        double s0 = 0, s1 = 0, s2 = 0;
-        gather3(m, n, s0, s1, s2);
-        f[3 * (size_t)n] += sign * s0;
-        f[3 * (size_t)n + 1] += sign * s1;
-        f[3 * (size_t)n + 2] += sign * s2;
+    const uint32_t a = threadIdx.x & 3u, step = (gridDim.x * blockDim.x) >> 2;
+    for (uint32_t n = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; (n & ~7u) < m.N; n += step) {
+        const bool on = n < m.N;
+        const double s = records ? gather_fx(m, n, a, on) : gather_fp64(m, n, a, on);
+        if (on && a < 3) f[3 * (size_t)n + a] += sign * s;
     }
 }
 
@@ -836,6 +956,8 @@ __device__ __forceinline__ void fin_init(StepScalars* st, const StepConsts& c, d
     st->alpha = 0.0;
     st->beta = 0.0;
     st->done = cg_continue(st) ? 0u : 1u;
+    st->delta_pend = total;
+    st->done_pend = st->done;
     if (!isfinite(total)) st->status = 3;  // FEM_E_NAN
 }
 __device__ __forceinline__ void fin_alpha(StepScalars* st, double total)
@@ -876,12 +998,6 @@ __global__ void k_finalize(int kind, const double* __restrict__ partials, uint32
     case FIN_INIT:
         fin_init(st, c, total);
         break;
-    case FIN_ALPHA:
-        fin_alpha(st, total);
-        break;
-    case FIN_BETA:
-        fin_beta(st, total);
-        break;
     case FIN_ENERGY_E:
         st->elastic_energy = total;
         break;
@@ -904,37 +1020,21 @@ __global__ void k_finalize(int kind, const double* __restrict__ partials, uint32
         st->k = 0;
         st->status = 0;
         st->done = (mr.norm_r_sq > st->abs_eps_sq && mr.norm_r_sq > st->delta_target && st->k < st->max_iter) ? 0u : 1u;
-        st->done_prev = st->done;
+        st->mr_pend = mr;
+        st->done_pend = st->done;
         if (!isfinite(total)) st->status = 3;
         break;
     }
-    case FIN_MR_ALPHA:
-        st->done_prev = st->done;
-        if (st->done) break;
-        st->mr.beta = st->mr.beta_new;
-        st->mr.alpha = total;
-        break;
-    case FIN_MR_BETA: {
-        if (st->done) break;
-        MinresScalars& mr = st->mr;
-        minres_givens(mr, total);  // Givens rotation (:135-144)
-        st->delta_new = mr.norm_r_sq;
-        st->k += 1;
-        st->total_iters += 1;
-        st->done = (mr.norm_r_sq > st->abs_eps_sq && mr.norm_r_sq > st->delta_target && st->k < st->max_iter) ? 0u : 1u;
-        if (!isfinite(total) || !isfinite(mr.norm_r_sq)) st->status = 3;
-        break;
-    }
     case FIN_MR_STATS:
-        st->rel_residual = ::sqrt(st->mr.norm_r_sq / st->mr.norm_b_sq);
-        st->abs_residual = ::sqrt(st->mr.norm_r_sq);
+        st->rel_residual = ::sqrt(st->mr_pend.norm_r_sq / st->mr_pend.norm_b_sq);
+        st->abs_residual = ::sqrt(st->mr_pend.norm_r_sq);
         break;
     case FIN_STATS:
+        st->delta_new = st->delta_pend;
         fin_stats(st);
         break;
     }
-    if (set_cond && (kind == FIN_INIT || kind == FIN_ALPHA || kind == FIN_BETA || kind == FIN_MR_INIT ||
-                     kind == FIN_MR_ALPHA || kind == FIN_MR_BETA))
+    if (set_cond && (kind == FIN_INIT || kind == FIN_MR_INIT))
         cudaGraphSetConditional(cond, st->done ? 0u : 1u);
 }
 
@@ -1269,137 +1369,143 @@ cudaError_t launch_cg_cluster_fp64(const MeshView<double>& m, const StepConsts& 
 
 // ---- launchers ----
 
-#define FEMGB_LAUNCH(kernel, grid, ...)                                   \
+#define FEMGB_LAUNCH(kernel, grid, block, ...)                            \
     do {                                                                  \
-        kernel<<<(grid), kBlock, 0, s>>>(__VA_ARGS__);                    \
+        kernel<<<(grid), (block), 0, s>>>(__VA_ARGS__);                   \
         launch_counter()++;                                               \
     } while (0)
 
+void launch_elem_bake_fp64(const MeshView<double>& m, cudaStream_t s)
+{
+    FEMGB_LAUNCH(k_elem_bake_fp64, elem_grid(m.T), elem_block(m.T), m);
+}
 void launch_elem_spmv_fp64(const MeshView<double>& m, const double* d, const StepScalars* st, int check_done,
                            cudaStream_t s)
 {
     prof_begin("elem_spmv_fp64", s);
-    FEMGB_LAUNCH(k_elem_spmv_fp64, grid_for(m.T), m, d, st, check_done);
+    FEMGB_LAUNCH(k_elem_spmv_fp64, elem_grid(m.T), elem_block(m.T), m, d, st, check_done);
     prof_end("elem_spmv_fp64", s);
 }
 void launch_elem_force_fp64(const MeshView<double>& m, const double* x, int write_out, double* energy_partials,
                             cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_elem_force_fp64, grid_for(m.T), m, x, write_out, energy_partials);
+    FEMGB_LAUNCH(k_elem_force_fp64, elem_grid(m.T), elem_block(m.T), m, x, write_out, energy_partials);
 }
 void launch_node_b_fp64(const MeshView<double>& m, const StepConsts& c, const double* v, double* b, double* y,
                         cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_node_b_fp64, grid_for(m.N), m, c, v, b, y);
+    FEMGB_LAUNCH(k_node_b_fp64, node_grid(m.N), row_block(node_rows(m.N)), m, c, v, b, y);
 }
 void launch_knc_fp64(uint32_t N, uint32_t count, const uint32_t* nodes, const double* targets, const double* x,
                      const StepConsts& c, double* b, double* y, cudaStream_t s)
 {
     if (count == 0) return;
-    FEMGB_LAUNCH(k_knc_fp64, grid_for(count), N, count, nodes, targets, x, c, b, y);
+    FEMGB_LAUNCH(k_knc_fp64, vec_grid(count), row_block(count), N, count, nodes, targets, x, c, b, y);
 }
 void launch_node_residual_fp64(const MeshView<double>& m, const StepConsts& c, const double* b, const double* y,
                                double* r, double* d, double* partials, cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_node_residual_fp64, grid_for(m.N), m, c, b, y, r, d, partials);
+    FEMGB_LAUNCH(k_node_residual_fp64, node_grid(m.N), row_block(node_rows(m.N)), m, c, b, y, r, d, partials);
 }
-void launch_node_q_fp64(const MeshView<double>& m, const StepConsts& c, const double* d, double* q,
-                        double* partials, StepScalars* st, cudaStream_t s, cudaGraphConditionalHandle cond,
-                        int set_cond)
+void launch_node_q_fp64(const MeshView<double>& m, const StepConsts& c, const double* d, double* q, double* pq,
+                        const StepScalars* st, cudaStream_t s)
 {
     prof_begin("node_q_fp64", s);
-    FEMGB_LAUNCH(k_node_q_fp64, grid_for(m.N), m, c, d, q, partials, st, cond, set_cond);
+    FEMGB_LAUNCH(k_node_q_fp64, node_grid(m.N), row_block(node_rows(m.N)), m, c, d, q, pq, st);
     prof_end("node_q_fp64", s);
 }
-void launch_node_xr_fp64(uint32_t N, double* y, double* r, const double* d, const double* q, double* partials,
-                         StepScalars* st, cudaStream_t s, cudaGraphConditionalHandle cond, int set_cond)
+void launch_node_xr_fp64(uint32_t N, double* y, double* r, const double* d, const double* q, const double* pq,
+                         double* pr, StepScalars* st, cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_node_xr_fp64, grid_for(3 * N), N, y, r, d, q, partials, st, cond, set_cond);
+    FEMGB_LAUNCH(k_node_xr_fp64, vec_grid(3 * N), row_block(3 * N), N, y, r, d, q, pq, node_grid(N), pr, st);
 }
-void launch_node_d_fp64(uint32_t N, const uint8_t* fixed, double* d, const double* r, const StepScalars* st,
-                        cudaStream_t s)
+void launch_node_d_fp64(uint32_t N, const uint8_t* fixed, double* d, const double* r, const double* pr,
+                        StepScalars* st, cudaStream_t s, cudaGraphConditionalHandle cond, int set_cond)
 {
-    FEMGB_LAUNCH(k_node_d_fp64, grid_for(3 * N), N, fixed, d, r, st);
+    FEMGB_LAUNCH(k_node_d_fp64, vec_grid(3 * N), row_block(3 * N), N, fixed, d, r, pr, vec_grid(3 * N), st, cond,
+                 set_cond);
 }
 void launch_integrate_fp64(uint32_t N, double dt, double* x, double* v, const double* y, cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_integrate_fp64, grid_for(3 * N), N, dt, x, v, y);
+    FEMGB_LAUNCH(k_integrate_fp64, vec_grid(3 * N), row_block(3 * N), N, dt, x, v, y);
 }
 void launch_node_b_fie_fp64(const MeshView<double>& m, const StepConsts& c, const double* x, const double* xn,
                             const double* vn, int warm, double* b, double* y, cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_node_b_fie_fp64, grid_for(m.N), m, c, x, xn, vn, warm, b, y);
+    FEMGB_LAUNCH(k_node_b_fie_fp64, node_grid(m.N), row_block(node_rows(m.N)), m, c, x, xn, vn, warm, b, y);
 }
 void launch_knc_fie_fp64(uint32_t N, uint32_t count, const uint32_t* nodes, const double* targets, const double* x,
                          double* b, double* y, cudaStream_t s)
 {
     if (count == 0) return;
-    FEMGB_LAUNCH(k_knc_fie_fp64, grid_for(count), N, count, nodes, targets, x, b, y);
+    FEMGB_LAUNCH(k_knc_fie_fp64, vec_grid(count), row_block(count), N, count, nodes, targets, x, b, y);
 }
 void launch_sq_norm_fp64(uint32_t n, const double* v, double* partials, cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_sq_norm_fp64, grid_for(n), n, v, partials);
+    FEMGB_LAUNCH(k_sq_norm_fp64, vec_grid(n), row_block(n), n, v, partials);
 }
 void launch_fie_update_fp64(uint32_t N, double inv_dt, double* x, double* v, const double* xn, const double* y,
                             double* partials, cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_fie_update_fp64, grid_for(3 * N), N, inv_dt, x, v, xn, y, partials);
+    FEMGB_LAUNCH(k_fie_update_fp64, vec_grid(3 * N), row_block(3 * N), N, inv_dt, x, v, xn, y, partials);
 }
 void launch_bsr_assemble_fp64(const MeshView<double>& m, uint32_t nnzb, const uint32_t* cptr,
                               const uint32_t* contrib, double* val, cudaStream_t s)
 {
     prof_begin("bsr_assemble_fp64", s);
-    FEMGB_LAUNCH(k_bsr_assemble_fp64, grid_for(nnzb), m, nnzb, cptr, contrib, val);
+    FEMGB_LAUNCH(k_bsr_assemble_fp64, capped((nnzb + 127) / 128, 16 * 1216u), 128u, m, nnzb, cptr, contrib, val);
     prof_end("bsr_assemble_fp64", s);
 }
 void launch_mr_init_fp64(const MeshView<double>& m, const StepConsts& c, const double* b, const double* y,
                          double* v1, double* partials, cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_mr_init_fp64, grid_for(m.N), m, c, b, y, v1, partials);
+    FEMGB_LAUNCH(k_mr_init_fp64, node_grid(m.N), row_block(node_rows(m.N)), m, c, b, y, v1, partials);
 }
 void launch_mr_start_fp64(uint32_t N, double* v1, double* v, double* p, double* p0, const StepScalars* st,
                           cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_mr_start_fp64, grid_for(3 * N), N, v1, v, p, p0, st);
+    FEMGB_LAUNCH(k_mr_start_fp64, vec_grid(3 * N), row_block(3 * N), N, v1, v, p, p0, st);
 }
 void launch_mr_q_fp64(const MeshView<double>& m, const StepConsts& c, const double* v, const double* v0,
-                      double* v1, double* partials, const StepScalars* st, cudaStream_t s)
+                      double* v1, double* pq, StepScalars* st, cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_mr_q_fp64, grid_for(m.N), m, c, v, v0, v1, partials, st);
+    FEMGB_LAUNCH(k_mr_q_fp64, node_grid(m.N), row_block(node_rows(m.N)), m, c, v, v0, v1, pq, st);
 }
-void launch_mr_v1_fp64(uint32_t N, double* v1, const double* v, double* partials, const StepScalars* st,
+void launch_mr_v1_fp64(uint32_t N, double* v1, const double* v, const double* pq, double* pr, StepScalars* st,
                        cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_mr_v1_fp64, grid_for(3 * N), N, v1, v, partials, st);
+    FEMGB_LAUNCH(k_mr_v1_fp64, vec_grid(3 * N), row_block(3 * N), N, v1, v, pq, node_grid(N), pr, st);
 }
 void launch_mr_update_fp64(uint32_t N, double* v1, const double* v, const double* p, double* p0, double* y,
-                           const StepScalars* st, cudaStream_t s)
+                           const double* pr, StepScalars* st, cudaStream_t s, cudaGraphConditionalHandle cond,
+                           int set_cond)
 {
-    FEMGB_LAUNCH(k_mr_update_fp64, grid_for(3 * N), N, v1, v, p, p0, y, st);
+    FEMGB_LAUNCH(k_mr_update_fp64, vec_grid(3 * N), row_block(3 * N), N, v1, v, p, p0, y, pr, vec_grid(3 * N), st,
+                 cond, set_cond);
 }
 void launch_elem_lcm_force_fp64(const MeshView<double>& m, const double* F, const PkMaterial& mat, int write_out,
                                 double* energy_partials, cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_elem_lcm_force_fp64, grid_for(m.T), m, F, mat, write_out, energy_partials);
+    FEMGB_LAUNCH(k_elem_lcm_force_fp64, elem_grid(m.T), elem_block(m.T), m, F, mat, write_out, energy_partials);
 }
 void launch_elem_lcm_spmv_fp64(const MeshView<double>& m, const double* d, const double* F, const PkMaterial& mat,
                                const StepScalars* st, int check_done, cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_elem_lcm_spmv_fp64, grid_for(m.T), m, d, F, mat, st, check_done);
+    FEMGB_LAUNCH(k_elem_lcm_spmv_fp64, elem_grid(m.T), elem_block(m.T), m, d, F, mat, st, check_done);
 }
 void launch_potential_fp64(const MeshView<double>& m, const StepConsts& c, const double* x, double* partials,
                            cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_potential_fp64, grid_for(m.T), m, c, x, partials);
+    FEMGB_LAUNCH(k_potential_fp64, elem_grid(m.T), elem_block(m.T), m, c, x, partials);
 }
 void launch_apply_A_fp64(const MeshView<double>& m, double factor_M, double factor_K, double mass,
                          const double* d, double* q, cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_apply_A_fp64, grid_for(m.N), m, factor_M, factor_K, mass, d, q);
+    FEMGB_LAUNCH(k_apply_A_fp64, node_grid(m.N), row_block(node_rows(m.N)), m, factor_M, factor_K, mass, d, q);
 }
-void launch_gather_sum_fp64(const MeshView<double>& m, double sign, double* f, cudaStream_t s)
+void launch_gather_sum_fp64(const MeshView<double>& m, double sign, double* f, bool records, cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_gather_sum_fp64, grid_for(m.N), m, sign, f);
+    FEMGB_LAUNCH(k_gather_sum_fp64, node_grid(m.N), row_block(node_rows(m.N)), m, sign, f, records ? 1 : 0);
 }
 void launch_finalize(int kind, const double* partials, uint32_t count, const StepConsts& c, StepScalars* st,
                      cudaStream_t s, cudaGraphConditionalHandle cond, int set_cond)

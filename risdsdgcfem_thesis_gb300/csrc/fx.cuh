@@ -1,0 +1,405 @@
+// fx.cuh -- the FP64 path's element products in fixed point, on the integer
+// pipe.
+//
+// GB300 issues one FP64 instruction per 64 clocks on each of an SM's four
+// sub-partitions (measured: DFMA 64.1 clocks, DADD 64 to 76, for dependent
+// and independent ones alike), and one 32 x 32 + 64 bit integer multiply-add
+// (IMAD.WIDE) per 2.07. A product of two 60-bit integers held as two signed
+// 32-bit limbs takes three of those (the low x low term is below the last
+// bit kept). The element product is therefore one symmetric 9 x 9 matrix per
+// element, K9 = the blocks (i, j), i, j = 1..3, of R K0 R^T, baked after each
+// evaluation, times the three node differences d_j - d_0 (node 0's output is
+// minus the sum of the others'): 81 products, about 500 clocks of
+// multiplies against 8,800 for the 138 FP64 operations of the strain form.
+//
+// Numbers are block fixed point: the nine differences share one exponent,
+// normalised to the largest, K9 one exponent, the twelve outputs one
+// exponent. Bounds are stated beside each stage. K9's entries are good to
+// about 2^-56 of the largest, the differences to 2^-60 and the sums to 2^-56,
+// where FP64 rounds every operation at 2^-53. Elements for which that does
+// not hold -- a non-finite or out-of-range operand, a rotation entry above
+// 1.125, a rest shape so graded that one exponent for Dm^-1 would cost more
+// than the spare bits -- take the FP64 product (elem_math.cuh).
+//
+// All functions are host callable: the arithmetic is checked on the CPU.
+#pragma once
+#include <stdint.h>
+#include <string.h>
+
+#ifdef __CUDACC__
+#define FX_HD __host__ __device__ __forceinline__
+#else
+#define FX_HD inline
+#endif
+
+namespace femgb {
+
+// v = h 2^32 + l, l signed.
+struct FxL {
+    int32_t l, h;
+};
+
+FX_HD FxL fx_split(int64_t v)
+{
+    FxL s;
+    s.l = (int32_t)v;
+    s.h = (int32_t)(v >> 32) + (int32_t)((uint32_t)s.l >> 31);
+    return s;
+}
+
+// hi += a.h b.h, mid += a.h b.l + a.l b.h: the product in units of 2^64 and 2^32.
+FX_HD void fx_mac(int64_t& hi, int64_t& mid, const FxL& a, const FxL& b)
+{
+    hi += (int64_t)a.h * b.h;
+    mid += (int64_t)a.h * b.l;
+    mid += (int64_t)a.l * b.h;
+}
+
+// The accumulated product in units of 2^(64 - K); mid in units of 2^(32 + half).
+template <int K>
+FX_HD int64_t fx_fin(int64_t hi, int64_t mid, int half = 0)
+{
+    return (int64_t)((uint64_t)hi << K) + (mid >> (32 - K - half));
+}
+
+FX_HD uint64_t fx_bits(double v)
+{
+#ifdef __CUDA_ARCH__
+    return (uint64_t)__double_as_longlong(v);
+#else
+    uint64_t u;
+    memcpy(&u, &v, 8);
+    return u;
+#endif
+}
+
+FX_HD double fx_from_bits(uint64_t u)
+{
+#ifdef __CUDA_ARCH__
+    return __longlong_as_double((long long)u);
+#else
+    double v;
+    memcpy(&v, &u, 8);
+    return v;
+#endif
+}
+
+// Biased exponent of a double (0: zero or denormal, 2047: Inf or NaN).
+FX_HD int32_t fx_exp(double v) { return (int32_t)(fx_bits(v) >> 52) & 0x7ff; }
+
+// v as an integer in units of 2^(E - 1022 - B), for E >= fx_exp(v), E <=
+// 2046: magnitude below 2^B, truncated. Denormals count as zero.
+template <int B>
+FX_HD int64_t fx_align(double v, int32_t E)
+{
+    const uint64_t u = fx_bits(v);
+    const int32_t e = (int32_t)(u >> 52) & 0x7ff;
+    const uint64_t m = ((u & 0xfffffffffffffull) | 0x10000000000000ull) << (B - 53);
+    const int32_t sh = E - e;
+    const int64_t a = (sh < 63 && e != 0) ? (int64_t)(m >> (sh & 63)) : 0;
+    const int64_t s = (int64_t)u >> 63;
+    return (a ^ s) - s;
+}
+
+// The scale of an element whose product runs in FP64 instead.
+constexpr int32_t kFxFp64 = 0x40000000;
+
+// A common exponent x of n values: every |v| < 2^x. False when all are zero
+// or one is not finite.
+FX_HD bool fx_common(const double* v, int n, int32_t& x)
+{
+    int32_t e = 0;
+    for (int i = 0; i < n; i++) {
+        const int32_t ei = fx_exp(v[i]);
+        e = ei > e ? ei : e;
+    }
+    x = e - 1022;
+    return e > 0 && e < 2047;
+}
+
+FX_HD uint64_t fx_mag(int64_t v) { return (uint64_t)(v ^ (v >> 63)); }  // |v| or |v| - 1
+
+FX_HD int fx_clz(uint64_t v)  // leading zeros, v > 0
+{
+#ifdef __CUDA_ARCH__
+    return __clzll((long long)v);
+#else
+    return __builtin_clzll(v);
+#endif
+}
+
+// m 2^x as a double, rounded to nearest (ties away); results below the
+// normal range become zero, above it infinity.
+FX_HD double fx_to_double(int64_t m, int32_t x)
+{
+    if (m == 0) return 0.0;
+    const uint64_t sign = (uint64_t)m & 0x8000000000000000ull;
+    uint64_t a = m < 0 ? 0ull - (uint64_t)m : (uint64_t)m;
+    const int lz = fx_clz(a);
+    a <<= lz;
+    const int32_t e = x + 63 - lz + 1023;  // biased exponent of the leading bit
+    if (e <= 0) return fx_from_bits(sign);
+    if (e >= 2047) return fx_from_bits(sign | 0x7ff0000000000000ull);
+    // the rounding carry moves on into the exponent
+    return fx_from_bits(sign | (((uint64_t)(e - 1) << 52) + ((a >> 11) + ((a >> 10) & 1ull))));
+}
+
+// A nodal output record: three integers of one element corner, their low four
+// bits holding the units' exponent: x + 2048 in 12 bits, low nibble first.
+// kFxNan marks a non-finite corner.
+constexpr int32_t kFxNan = 4095;
+FX_HD int32_t fx_record_exp(int64_t a, int64_t b, int64_t c)
+{
+    return (int32_t)(a & 15) | ((int32_t)(b & 15) << 4) | ((int32_t)(c & 15) << 8);
+}
+
+// Stamps the exponent x of 12 outputs' units into their low bits; false when
+// x has no place in a record above (the element takes FP64); far below, the
+// outputs become zero.
+FX_HD bool fx_stamp(int64_t* out, int32_t x)
+{
+    const int32_t b = x + 2048;
+    if (b >= kFxNan) return false;
+    const int32_t c = b < 0 ? 0 : b;
+#pragma unroll
+    for (int k = 0; k < 12; k++)
+        out[k] = b < 0 ? 0 : ((out[k] & ~15ll) | ((c >> (4 * (k % 3))) & 15));
+    return true;
+}
+
+// The record of 12 FP64 outputs.
+FX_HD void fx_stamp_doubles(const double* v, int64_t* out)
+{
+    int32_t E = 0;
+#pragma unroll
+    for (int k = 0; k < 12; k++) {
+        const int32_t e = fx_exp(v[k]);
+        E = e > E ? e : E;
+    }
+    if (E == 2047) {
+#pragma unroll
+        for (int k = 0; k < 12; k++) out[k] = 15;
+        return;
+    }
+#pragma unroll
+    for (int k = 0; k < 12; k++) out[k] = fx_align<61>(v[k], E);
+    fx_stamp(out, E - 1022 - 61);
+}
+
+// The running sum of one component's records: acc in units of 2^(E - 2048 +
+// guard), the guard bits sized so that a node's entries cannot overflow.
+struct FxSum {
+    int64_t acc;
+    int32_t E;
+};
+FX_HD int32_t fx_min63(int32_t s) { return s > 63 ? 63 : s; }
+FX_HD void fx_add(FxSum& s, int64_t m, int32_t e, int32_t guard)
+{
+    const int32_t up = e > s.E ? e - s.E : 0, down = (e < s.E ? s.E - e : 0) + guard;
+    s.acc = (s.acc >> fx_min63(up)) + (m >> fx_min63(down));
+    s.E = e > s.E ? e : s.E;
+}
+FX_HD double fx_sum_value(const FxSum& s, int32_t guard)
+{
+    return s.E == kFxNan ? fx_from_bits(0x7ff8000000000000ull) : fx_to_double(s.acc, s.E - 2048 + guard);
+}
+
+// K9's packed upper triangle: entry (r, c), r <= c, of the 9 x 9 matrix whose
+// index 3 (i - 1) + a is component a of node i.
+constexpr int kFxK = 45;
+FX_HD constexpr int fx_at(int r, int c)  // r <= c
+{
+    return 9 * r - r * (r - 1) / 2 + (c - r);
+}
+
+// An element's grade max|Dm| max|Dm^-1| (1 for a cube corner): one exponent
+// for all of Dm^-1 costs bits of K9 with it. Measured against 128-bit products
+// (random shapes, rotations and fields): below grade 3 the error is 0.2 to
+// 0.9 of the FP64 strain form's for nu up to 0.45, between 3 and 4 it passes
+// it; near incompressibility both lose bits and the line lies at 1.2.
+constexpr float kFxMaxGrade = 3.0f, kFxMaxGradeStiff = 1.2f;
+constexpr double kFxStiff = 9.5;  // lambda / mu
+
+// Whether an element of this rest shape and material may take fx_bake:
+// grade = max|Dm| max|Dm^-1|.
+FX_HD bool fx_grade_ok(float grade, double kl, double km)
+{
+    return grade <= (kl <= kFxStiff * km ? kFxMaxGrade : kFxMaxGradeStiff);  // false for NaN
+}
+
+// Bakes K9 = V (lambda m_i m_j^T + mu m_j m_i^T + mu (g_i . g_j) R R^T) with g_i
+// the rows of Dm^-1 and m_i = R g_i (the strain form's product for any R,
+// orthonormal or not). kl = V lambda, km = V mu; the caller has checked
+// fx_grade_ok. K9 in units of 2^scale (returned), |K9| < 2^60 and its largest
+// entry at least 2^59; kFxFp64 when the element takes FP64 (a row of R longer
+// than 1.015, a non-finite or extreme operand); put(k, entry) takes the packed
+// triangle in order. No FP64 operation.
+template <typename FP>
+FX_HD int32_t fx_bake(const double* R, const double* Di, double kl, double km, FP&& put)
+{
+    const double mat[2] = {kl, km};
+    int32_t xd = 0, xm = 0;
+    bool ok = fx_common(Di, 9, xd) && fx_common(mat, 2, xm) && xd > -400 && xd < 400 && xm > -400 && xm < 400;
+#pragma unroll
+    for (int i = 0; i < 9; i++)  // |R| < 1.0157 by its high word; false for NaN
+        ok = ok && ((uint32_t)(fx_bits(R[i]) >> 32) & 0x7fffffffu) < 0x3ff04000u;
+    if (!ok) return kFxFp64;
+    FxL r[9], g[9];
+#pragma unroll
+    for (int i = 0; i < 9; i++) {
+        r[i] = fx_split(fx_align<62>(R[i], 1023));        // R 2^61, below 2^61.03
+        g[i] = fx_split(fx_align<61>(Di[i], xd + 1022));  // g 2^(61 - xd), below 2^61
+    }
+    FxL m[9], C[6], W[6];
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            int64_t hi = 0, mid = 0;
+#pragma unroll
+            for (int b = 0; b < 3; b++) fx_mac(hi, mid, r[3 * a + b], g[3 * i + b]);
+            m[3 * i + a] = fx_split(fx_fin<2>(hi, mid));  // m 2^(60 - xd), below 2^60.82
+        }
+    const int pa[6] = {0, 0, 0, 1, 1, 2}, pb[6] = {0, 1, 2, 1, 2, 2};  // (0,0) (0,1) (0,2) (1,1) (1,2) (2,2)
+    const FxL lam = fx_split(fx_align<61>(kl, xm + 1022)), mu = fx_split(fx_align<61>(km, xm + 1022));  // 2^(61 - xm)
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+        int64_t hi = 0, mid = 0;
+#pragma unroll
+        for (int b = 0; b < 3; b++) fx_mac(hi, mid, r[3 * pa[k] + b], r[3 * pb[k] + b]);
+        const int64_t ck = fx_fin<2>(hi, mid);  // C 2^60, below 2^61.7
+        if (pa[k] == pb[k]) ok = ok && ck < (int64_t)(1.03 * 1152921504606846976.0);
+        C[k] = fx_split(ck);
+        hi = mid = 0;
+#pragma unroll
+        for (int b = 0; b < 3; b++) fx_mac(hi, mid, g[3 * pa[k] + b], g[3 * pb[k] + b]);
+        const FxL G = fx_split(fx_fin<2>(hi, mid));  // G 2^(60 - 2 xd), below 2^61.6
+        hi = mid = 0;
+        fx_mac(hi, mid, mu, G);
+        W[k] = fx_split(fx_fin<2>(hi, mid));  // mu G 2^(59 - xm - 2 xd), below 2^60.6
+    }
+    FxL L[9], U[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+        int64_t hi = 0, mid = 0;
+        fx_mac(hi, mid, lam, m[k]);
+        L[k] = fx_split(fx_fin<2>(hi, mid));  // lambda m 2^(59 - xm - xd), below 2^59.82
+        hi = mid = 0;
+        fx_mac(hi, mid, mu, m[k]);
+        U[k] = fx_split(fx_fin<2>(hi, mid));
+    }
+    // (mid stays below (2 (2^27.82 + 2^28.82) + 2^28.6 + 2^28.05) 2^31 < 2^63).
+    // K9 is positive semidefinite, so its largest entry is on the diagonal:
+    // that gives the shift that moves it to [2^59, 2^60).
+    const int sym[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
+    auto entry = [&](int r, int c) {
+        const int i = r / 3, a = r % 3, j = c / 3, b = c % 3;
+        int64_t hi = 0, mid = 0;
+        fx_mac(hi, mid, L[3 * i + a], m[3 * j + b]);
+        fx_mac(hi, mid, U[3 * j + a], m[3 * i + b]);
+        fx_mac(hi, mid, W[sym[3 * i + j]], C[sym[3 * a + b]]);
+        return fx_fin<4>(hi, mid);  // K9 2^(59 - xm - 2 xd), below 9.4 2^59
+    };
+    uint64_t any = 0;
+#pragma unroll
+    for (int r = 0; r < 9; r++) any |= fx_mag(entry(r, r));
+    if (any == 0 || !ok) return kFxFp64;
+    const int lz = fx_clz(any);  // 1 at least
+#pragma unroll
+    for (int r = 0; r < 9; r++)
+#pragma unroll
+        for (int c = r; c < 9; c++) put(fx_at(r, c), fx_split((int64_t)((uint64_t)entry(r, c) << (lz - 1)) >> 3));
+    return xm + 2 * xd - 59 - (lz - 1) + 3;
+}
+
+// The node differences d_j - d_0 (D[3 (j - 1) + a]) in limbs, |D| < 2^60, from
+// the four nodes' vectors; returns the exponent x of their units (2^x). False
+// when a component is not finite (the element takes FP64); all-zero
+// differences give zeros.
+FX_HD bool fx_differences(const double* d, FxL* D, int32_t& x)
+{
+    int32_t E = 0;
+#pragma unroll
+    for (int i = 0; i < 12; i++) {
+        const int32_t e = fx_exp(d[i]);
+        E = e > E ? e : E;
+    }
+    int64_t v[9];
+    uint64_t any = 1;
+    int64_t d0[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) d0[a] = fx_align<62>(d[a], E);
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            v[3 * j + a] = fx_align<62>(d[3 * (j + 1) + a], E) - d0[a];
+            any |= fx_mag(v[3 * j + a]);
+        }
+    const int lz = fx_clz(any);  // 1 at least
+#pragma unroll
+    for (int k = 0; k < 9; k++) D[k] = fx_split((int64_t)((uint64_t)v[k] << (lz - 1)) >> 3);
+    x = E - 1022 - 62 - (lz - 1) + 3;
+    return E < 2047;
+}
+
+// K9 D: out[3 i + a] for the nodes i = 0..3, normalised (|out| < 2^61, node 0's
+// below 3 2^61) in units of 2^(scale + x + the returned shift). K(k) gives
+// entry k of the packed triangle. Each of the two mid sums stays below
+// 9 2^28 2^31 = 2^62.2, the outputs before their normalisation below 2^62.2.
+template <typename FK>
+FX_HD int32_t fx_product(FK&& K, const FxL* D, int64_t* out)
+{
+    int64_t hi[9], m1[9], m2[9];
+#pragma unroll
+    for (int r = 0; r < 9; r++) hi[r] = m1[r] = m2[r] = 0;
+#pragma unroll
+    for (int r = 0; r < 9; r++)
+#pragma unroll
+        for (int c = r; c < 9; c++) {  // entry (r, c) goes to rows r and c as it arrives
+            const FxL k = K(fx_at(r, c));
+            hi[r] += (int64_t)k.h * D[c].h;
+            m1[r] += (int64_t)k.h * D[c].l;
+            m2[r] += (int64_t)k.l * D[c].h;
+            if (c > r) {
+                hi[c] += (int64_t)k.h * D[r].h;
+                m1[c] += (int64_t)k.h * D[r].l;
+                m2[c] += (int64_t)k.l * D[r].h;
+            }
+        }
+    int64_t sum[3] = {0, 0, 0};
+    uint64_t any = 1;
+#pragma unroll
+    for (int r = 0; r < 9; r++) {
+        out[3 + r] = fx_fin<3>(hi[r], (m1[r] >> 1) + (m2[r] >> 1), 1);
+        any |= fx_mag(out[3 + r]);
+    }
+    const int lz = fx_clz(any);  // 2 at least
+#pragma unroll
+    for (int r = 0; r < 9; r++) {
+        out[3 + r] = (int64_t)((uint64_t)out[3 + r] << (lz - 2)) >> 1;
+        sum[r % 3] += out[3 + r];
+    }
+#pragma unroll
+    for (int a = 0; a < 3; a++) out[a] = -sum[a];
+    return 61 - (lz - 2) + 1;
+}
+
+#ifdef __CUDACC__
+// The sum of a warp's doubles, the same in every lane: aligned to the largest
+// exponent and added exactly in three limbs by integer reductions. About 150
+// clocks; five FP64 adds and ten shuffles take about 600. The result is
+// within 2^-52 of the largest term.
+__device__ __forceinline__ double fx_warp_sum(double v)
+{
+    const int32_t E = __reduce_max_sync(0xffffffffu, fx_exp(v));
+    if (E == 2047) return __longlong_as_double(0x7ff8000000000000ll);
+    const int64_t m = fx_align<57>(v, E);
+    const uint32_t l0 = __reduce_add_sync(0xffffffffu, (uint32_t)m & 0xffffffu);
+    const uint32_t l1 = __reduce_add_sync(0xffffffffu, (uint32_t)(m >> 24) & 0xffffffu);
+    const int32_t l2 = __reduce_add_sync(0xffffffffu, (int32_t)(m >> 48));
+    return fx_to_double((int64_t)l0 + ((int64_t)l1 << 24) + ((int64_t)((uint64_t)(int64_t)l2 << 48)), E - 1022 - 57);
+}
+#endif
+
+}  // namespace femgb

@@ -54,7 +54,7 @@ void launch_begin_eval_fp64(const MeshView<double>& m, const double* x, double* 
                             cudaStream_t s)
 {
     prof_begin("begin_eval_msvd_fp64", s);
-    k_begin_eval_fp64<<<grid_for(m.T), kBlock, 0, s>>>(m, x, F_out, st);
+    k_begin_eval_fp64<<<elem_grid(m.T), elem_block(m.T), 0, s>>>(m, x, F_out, st);
     prof_end("begin_eval_msvd_fp64", s);
     launch_counter()++;
 }
@@ -111,7 +111,7 @@ void launch_begin_eval_dapd_fp64(const MeshView<double>& m, const double* xprev,
                                  const DapdParams& p, double* F_out, StepScalars* st, cudaStream_t s)
 {
     prof_begin("begin_eval_dapd_fp64", s);
-    k_begin_eval_dapd_fp64<<<grid_for(m.T), kBlock, 0, s>>>(m, xprev, x, doc, p, F_out, st);
+    k_begin_eval_dapd_fp64<<<elem_grid(m.T), elem_block(m.T), 0, s>>>(m, xprev, x, doc, p, F_out, st);
     prof_end("begin_eval_dapd_fp64", s);
     launch_counter()++;
 }

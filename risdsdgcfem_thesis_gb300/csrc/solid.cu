@@ -105,6 +105,13 @@ struct fem_solid_s {
     // element data
     DevBuf<int4> tets;
     DevBuf<double> Dinv, mat, vol, R, detF, eout;
+    // the fixed-point product matrices (MeshView::Kfx), baked from the
+    // rotations and the material; kfx_fresh: they are those of the last
+    // evaluation
+    DevBuf<int4> Kfx;
+    DevBuf<float> grade;
+    uint32_t fx_guard = 0;
+    bool kfx_fresh = false;
     DevBuf<uint32_t> csr_ptr, csr_idx;
     DevBuf<uint8_t> fixed;
     // the one-cluster CG of a small solid (ctas 0: none); cl_ent as csr_idx,
@@ -184,6 +191,9 @@ struct fem_solid_s {
         m.csr_idx = csr_idx.p;
         m.fixed = fixed.p;
         m.eout = eout.p;
+        if (params.material == FEM_MATERIAL_C_WRP) m.Kfx = Kfx.p;
+        m.fx_guard = fx_guard;
+        m.grade = grade.p;
         if (bsr_use) {
             m.bsr_row = bsr_row.p;
             m.bsr_col = bsr_col.p;
@@ -199,6 +209,8 @@ struct fem_solid_s {
                                  &lk_x, &lk_v};
         for (auto* p : dbl) p->release();
         doc.release();
+        Kfx.release();
+        grade.release();
         tets.release();
         csr_ptr.release();
         csr_idx.release();
@@ -313,6 +325,14 @@ void set_consts(fem_solid s)
     s->dapd.eNL = (double)(float)params->dapd_nl_exponent;
 }
 
+// The fixed-point product matrices of a C_WRP solid on its last rotations.
+void bake_products(fem_solid s)
+{
+    if (uses_lcm(s) || s->kfx_fresh) return;
+    launch_elem_bake_fp64(s->view(), s->stream);
+    s->kfx_fresh = true;
+}
+
 // TetrahedronElementSet3::BeginEvaluation(x0 = xprev, x): F, det F and the
 // rotations at x; xprev feeds the DAPD collapse detection only. C_LCM keeps F.
 void begin_eval(fem_solid s, const double* xprev, const double* x)
@@ -323,8 +343,12 @@ void begin_eval(fem_solid s, const double* xprev, const double* x)
         launch_begin_eval_dapd_fp64(m, xprev, x, s->doc.p, s->dapd, F_out, s->st.p, s->stream);
     else
         launch_begin_eval_fp64(m, x, F_out, s->st.p, s->stream);
-    if (s->bsr_use)  // the solvers' operator on the new rotations
+    // the solvers' operator on the new rotations
+    s->kfx_fresh = false;
+    if (s->bsr_use)
         launch_bsr_assemble_fp64(m, s->bsr_nnzb, s->bsr_cptr.p, s->bsr_contrib.p, s->bsr_val.p, s->stream);
+    else
+        bake_products(s);
 }
 
 // The material's element force at x (C_f_e / C_LCM_f_e) into m.eout and/or
@@ -342,8 +366,10 @@ void elem_spmv(fem_solid s, const MeshView<double>& m, const double* d, int chec
 {
     if (uses_lcm(s))
         launch_elem_lcm_spmv_fp64(m, d, s->Fe.p, pk_material(s), s->st.p, check_done, s->stream);
-    else
+    else {
+        bake_products(s);
         launch_elem_spmv_fp64(m, d, s->st.p, check_done, s->stream);
+    }
 }
 
 // The solvers' product ahead of their node kernels: nothing when those take
@@ -501,7 +527,7 @@ int cg_solve(fem_solid s, const StepConsts& c, int chunk)
         CK(cudaGetLastError());
         return FEM_OK;
     }
-    const uint32_t gN = grid_for(s->N), gV = grid_for(3 * s->N);
+    const uint32_t gN = node_grid(s->N), gV = vec_grid(3 * s->N);
     solve_product(s, m, s->y.p, 0);
     launch_node_residual_fp64(m, c, s->b.p, s->y.p, s->r.p, s->d.p, s->partials.p, st);
     launch_finalize(FIN_INIT, s->partials.p, gN, c, s->st.p, st);
@@ -509,12 +535,12 @@ int cg_solve(fem_solid s, const StepConsts& c, int chunk)
         for (int i = 0; i < chunk; i++) {
             solve_product(s, m, s->d.p, 1);
             launch_node_q_fp64(m, c, s->d.p, s->q.p, s->partials.p, s->st.p, st);
-            launch_node_xr_fp64(s->N, s->y.p, s->r.p, s->d.p, s->q.p, s->partials.p, s->st.p, st);
-            launch_node_d_fp64(s->N, s->fixed.p, s->d.p, s->r.p, s->st.p, st);
+            launch_node_xr_fp64(s->N, s->y.p, s->r.p, s->d.p, s->q.p, s->partials.p, s->partials2.p, s->st.p, st);
+            launch_node_d_fp64(s->N, s->fixed.p, s->d.p, s->r.p, s->partials2.p, s->st.p, st);
         }
         CK(cudaMemcpyAsync(s->st_host, s->st.p, sizeof(StepScalars), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
-        if (s->st_host->done) break;
+        if (s->st_host->done_pend) break;
     }
     launch_finalize(FIN_STATS, s->partials.p, 0, c, s->st.p, st);
     CK(cudaGetLastError());
@@ -529,7 +555,7 @@ int minres_solve(fem_solid s, const StepConsts& c, int chunk)
 {
     cudaStream_t st = s->stream;
     MeshView<double> m = s->view();
-    const uint32_t gN = grid_for(s->N), gV = grid_for(3 * s->N);
+    const uint32_t gN = node_grid(s->N), gV = vec_grid(3 * s->N);
     double *v = s->r.p, *v0 = s->d.p, *v1 = s->q.p, *p = s->mr_p.p, *p0 = s->mr_p0.p;
     launch_sq_norm_fp64(3 * s->N, s->b.p, s->partials.p, st);
     launch_finalize(FIN_SUM, s->partials.p, gV, c, s->st.p, st);  // |b|^2
@@ -545,17 +571,15 @@ int minres_solve(fem_solid s, const StepConsts& c, int chunk)
             v1 = t;
             solve_product(s, m, v, 1);
             launch_mr_q_fp64(m, c, v, v0, v1, s->partials.p, s->st.p, st);
-            launch_finalize(FIN_MR_ALPHA, s->partials.p, gN, c, s->st.p, st);
-            launch_mr_v1_fp64(s->N, v1, v, s->partials.p, s->st.p, st);
-            launch_finalize(FIN_MR_BETA, s->partials.p, gV, c, s->st.p, st);
-            launch_mr_update_fp64(s->N, v1, v, p, p0, s->y.p, s->st.p, st);
+            launch_mr_v1_fp64(s->N, v1, v, s->partials.p, s->partials2.p, s->st.p, st);
+            launch_mr_update_fp64(s->N, v1, v, p, p0, s->y.p, s->partials2.p, s->st.p, st);
             t = p;  // the new p was written into p0's buffer
             p = p0;
             p0 = t;
         }
         CK(cudaMemcpyAsync(s->st_host, s->st.p, sizeof(StepScalars), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
-        if (s->st_host->done) break;
+        if (s->st_host->done_pend) break;
     }
     launch_finalize(FIN_MR_STATS, s->partials.p, 0, c, s->st.p, st);
     CK(cudaGetLastError());
@@ -577,7 +601,7 @@ cudaError_t ls_solve_capture(fem_solid s, const StepConsts& c, cudaGraph_t top)
 {
     cudaStream_t st = s->stream;
     MeshView<double> m = s->view();
-    const uint32_t gN = grid_for(s->N), gV = grid_for(3 * s->N);
+    const uint32_t gN = node_grid(s->N), gV = vec_grid(3 * s->N);
     if (s->params.ls_solver != FEM_LS_MINRES && cg_on_cluster(s))
         return launch_cg_cluster_fp64(m, c, s->cl_plan, s->cl_ent.p, s->b.p, s->y.p, s->st.p, st);
     cudaGraphConditionalHandle cond = 0;
@@ -590,9 +614,9 @@ cudaError_t ls_solve_capture(fem_solid s, const StepConsts& c, cudaGraph_t top)
         e = capture_conditional(st, cond, cudaGraphCondTypeWhile, [&](cudaStream_t bs, cudaGraph_t) {
             s->stream = bs;
             solve_product(s, m, s->d.p, 1);
-            launch_node_q_fp64(m, c, s->d.p, s->q.p, s->partials.p, s->st.p, bs, cond, 1);
-            launch_node_xr_fp64(s->N, s->y.p, s->r.p, s->d.p, s->q.p, s->partials.p, s->st.p, bs, cond, 1);
-            launch_node_d_fp64(s->N, s->fixed.p, s->d.p, s->r.p, s->st.p, bs);
+            launch_node_q_fp64(m, c, s->d.p, s->q.p, s->partials.p, s->st.p, bs);
+            launch_node_xr_fp64(s->N, s->y.p, s->r.p, s->d.p, s->q.p, s->partials.p, s->partials2.p, s->st.p, bs);
+            launch_node_d_fp64(s->N, s->fixed.p, s->d.p, s->r.p, s->partials2.p, s->st.p, bs, cond, 1);
             s->stream = st;
             return cudaGetLastError();
         });
@@ -619,10 +643,8 @@ cudaError_t ls_solve_capture(fem_solid s, const StepConsts& c, cudaGraph_t top)
             v1 = t;
             solve_product(s, m, v, 1);
             launch_mr_q_fp64(m, c, v, v0, v1, s->partials.p, s->st.p, bs);
-            launch_finalize(FIN_MR_ALPHA, s->partials.p, gN, c, s->st.p, bs, cond, 1);
-            launch_mr_v1_fp64(s->N, v1, v, s->partials.p, s->st.p, bs);
-            launch_finalize(FIN_MR_BETA, s->partials.p, gV, c, s->st.p, bs, cond, 1);
-            launch_mr_update_fp64(s->N, v1, v, p, p0, s->y.p, s->st.p, bs);
+            launch_mr_v1_fp64(s->N, v1, v, s->partials.p, s->partials2.p, s->st.p, bs);
+            launch_mr_update_fp64(s->N, v1, v, p, p0, s->y.p, s->partials2.p, s->st.p, bs, cond, 1);
             t = p;  // the new p was written into p0's buffer
             p = p0;
             p0 = t;
@@ -653,7 +675,7 @@ void energy(fem_solid s)
     cudaStream_t st = s->stream;
     MeshView<double> m = s->view();
     const StepConsts& c = s->consts;
-    const uint32_t gE = grid_for(s->T);
+    const uint32_t gE = elem_grid(s->T);
     elem_force(s, m, s->x.p, 0, s->partials2.p);
     launch_finalize(FIN_ENERGY_E, s->partials2.p, gE, c, s->st.p, st);
     launch_potential_fp64(m, c, s->x.p, s->partials2.p, st);
@@ -678,7 +700,7 @@ int step_fie(fem_solid s, int chunk)
     c.factor_M = c.inv_dt * c.inv_dt + c.inv_dt * s->rayleigh[0];
     c.factor_K = 1.0 + c.inv_dt * s->rayleigh[1];
     const size_t bytes = sizeof(double) * 3 * (size_t)s->N;
-    const uint32_t gV = grid_for(3 * s->N);
+    const uint32_t gV = vec_grid(3 * s->N);
     if (int e = open_step(s)) return e;
     CK(cudaMemcpyAsync(s->xn.p, s->x.p, bytes, cudaMemcpyDeviceToDevice, st));
     CK(cudaMemcpyAsync(s->vn.p, s->v.p, bytes, cudaMemcpyDeviceToDevice, st));
@@ -774,6 +796,7 @@ int step_once(fem_solid s, int chunk)
     if (!s->exec)
         if (int e = capture_step(s)) return e;
     CK(cudaGraphLaunch(s->exec, s->stream));
+    s->kfx_fresh = !uses_lcm(s) && !s->bsr_use;  // baked by the graph's evaluation
     return FEM_OK;
 }
 void fill_stats(fem_solid s, const StepScalars& h, fem_step_stats* out)
@@ -913,6 +936,7 @@ int fem_solid_create(const double* rest_xyz, uint32_t N, const uint32_t* tets, u
 
     // ---- host set-up (EndEdition + RebuildMass + Rayleigh) ----
     std::vector<double> Dinv(9 * (size_t)T), mat(3 * (size_t)T), vol(T);
+    std::vector<float> grade(T);
     double acc_total_volume = 0.0;
     for (uint32_t e = 0; e < T; e++) {
         const double* r0 = rest_xyz + 3 * (size_t)tets[4 * (size_t)e];
@@ -931,7 +955,13 @@ int fem_solid_create(const double* rest_xyz, uint32_t N, const uint32_t* tets, u
         acc_total_volume += V;
         double Di[9];
         inverse3(D, Di);
-        for (int c = 0; c < 9; c++) Dinv[(size_t)c * T + e] = Di[c];
+        double edge = 0.0, slope = 0.0;
+        for (int c = 0; c < 9; c++) {
+            Dinv[(size_t)c * T + e] = Di[c];
+            edge = std::max(edge, std::fabs(D[c]));
+            slope = std::max(slope, std::fabs(Di[c]));
+        }
+        grade[e] = (float)(edge * slope);
         const double E = young_per_elem ? young_per_elem[e] : params->young_modulus;
         const double nu = poisson_per_elem ? poisson_per_elem[e] : params->poisson_ratio;
         // Compute_E (TetrahedronElement3.h:141-156)
@@ -956,6 +986,8 @@ int fem_solid_create(const double* rest_xyz, uint32_t N, const uint32_t* tets, u
         std::vector<uint32_t> fill(ptr.begin(), ptr.end() - 1);
         for (size_t i = 0; i < 4 * (size_t)T; i++) idx[fill[tets[i]]++] = (uint32_t)i;
     }
+    for (uint32_t n = 0; n < N; n++)
+        while ((1u << s->fx_guard) < ptr[n + 1] - ptr[n]) s->fx_guard++;
     std::vector<int4> t4(T);
     for (uint32_t e = 0; e < T; e++)
         t4[e] = make_int4((int)tets[4 * (size_t)e], (int)tets[4 * (size_t)e + 1], (int)tets[4 * (size_t)e + 2],
@@ -983,6 +1015,8 @@ int fem_solid_create(const double* rest_xyz, uint32_t N, const uint32_t* tets, u
     CKC(s->R.alloc(9 * (size_t)T));
     CKC(s->detF.alloc(T));
     CKC(s->eout.alloc(12 * (size_t)T));
+    CKC(s->Kfx.alloc(kFxGroups * (size_t)T));
+    CKC(s->grade.alloc(T));
     CKC(s->csr_ptr.alloc(N + 1));
     CKC(s->csr_idx.alloc(4 * (size_t)T));
     CKC(s->fixed.alloc(N));
@@ -1013,6 +1047,7 @@ int fem_solid_create(const double* rest_xyz, uint32_t N, const uint32_t* tets, u
     CKC(cudaMemcpyAsync(s->Dinv.p, Dinv.data(), sizeof(double) * Dinv.size(), cudaMemcpyHostToDevice, st));
     CKC(cudaMemcpyAsync(s->mat.p, mat.data(), sizeof(double) * mat.size(), cudaMemcpyHostToDevice, st));
     CKC(cudaMemcpyAsync(s->vol.p, vol.data(), sizeof(double) * T, cudaMemcpyHostToDevice, st));
+    CKC(cudaMemcpyAsync(s->grade.p, grade.data(), sizeof(float) * T, cudaMemcpyHostToDevice, st));
     CKC(cudaMemcpyAsync(s->csr_ptr.p, ptr.data(), sizeof(uint32_t) * (N + 1), cudaMemcpyHostToDevice, st));
     CKC(cudaMemcpyAsync(s->csr_idx.p, idx.data(), sizeof(uint32_t) * idx.size(), cudaMemcpyHostToDevice, st));
     s->cl_plan = plan_cg_cluster(N, T, ptr);
@@ -1207,6 +1242,7 @@ int fem_solid_set_params(fem_solid s, const fem_params* params)
         const double E = params->young_modulus, nu = params->poisson_ratio;
         const double a = E / ((1.0 + nu) * (1.0 - 2.0 * nu));  // Compute_E (TetrahedronElement3.h:141-156)
         launch_rebake_material_fp64(s->T, s->vol.p, a * (1.0 - nu), a * nu, a * (0.5 - nu), s->mat.p, s->stream);
+        s->kfx_fresh = false;
         CK(cudaGetLastError());
     }
     CK(cudaStreamSynchronize(s->stream));
@@ -1319,7 +1355,7 @@ int fem_solid_nr_end(fem_solid s, double dt)
     if (s->params.compute_energy) {
         MeshView<double> m = s->view();
         launch_potential_fp64(m, s->consts, s->x.p, s->partials2.p, s->stream);
-        launch_finalize(FIN_ENERGY_P, s->partials2.p, grid_for(s->T), s->consts, s->st.p, s->stream);
+        launch_finalize(FIN_ENERGY_P, s->partials2.p, elem_grid(s->T), s->consts, s->st.p, s->stream);
     }
     s->lock_stats = true;
     CK(cudaStreamSynchronize(s->stream));
@@ -1495,7 +1531,7 @@ int fem_solid_force_elastic(fem_solid s, double* f)
     // positions of the last evaluation are in tmp
     CK(cudaMemcpyAsync(s->q.p, f, bytes, cudaMemcpyHostToDevice, s->stream));
     elem_force(s, s->view(), s->tmp.p, 1, nullptr);
-    launch_gather_sum_fp64(s->view(), -1.0, s->q.p, s->stream);
+    launch_gather_sum_fp64(s->view(), -1.0, s->q.p, false, s->stream);
     CK(cudaMemcpyAsync(f, s->q.p, bytes, cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     return FEM_OK;
@@ -1509,7 +1545,7 @@ int fem_solid_df_x(fem_solid s, const double* dx, double* df)
     CK(cudaMemcpyAsync(s->d.p, dx, bytes, cudaMemcpyHostToDevice, s->stream));
     CK(cudaMemcpyAsync(s->q.p, df, bytes, cudaMemcpyHostToDevice, s->stream));
     elem_spmv(s, s->view(), s->d.p, 0);
-    launch_gather_sum_fp64(s->view(), -1.0, s->q.p, s->stream);
+    launch_gather_sum_fp64(s->view(), -1.0, s->q.p, !uses_lcm(s), s->stream);
     CK(cudaMemcpyAsync(df, s->q.p, bytes, cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     return FEM_OK;
@@ -1534,7 +1570,7 @@ int fem_solid_energy(fem_solid s, double* V)
     if (!V) return fail(FEM_E_ARG, "null output");
     if (!s->evaluated) return fail(FEM_E_ARG, "fem_solid_begin_eval must come first");
     elem_force(s, s->view(), s->tmp.p, 0, s->partials2.p);
-    launch_finalize(FIN_ENERGY_E, s->partials2.p, grid_for(s->T), s->consts, s->st.p, s->stream);
+    launch_finalize(FIN_ENERGY_E, s->partials2.p, elem_grid(s->T), s->consts, s->st.p, s->stream);
     CK(cudaMemcpyAsync(s->st_host, s->st.p, sizeof(StepScalars), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     *V = s->st_host->elastic_energy;
