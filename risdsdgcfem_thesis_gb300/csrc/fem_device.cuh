@@ -134,9 +134,10 @@ struct MeshView {
     const uint32_t* bsr_col = nullptr;
     const double* bsr_val = nullptr;
     // FP64 solid, C_WRP: each element's fixed-point product matrix (fx.cuh),
-    // kFxGroups 16-byte groups of two entries, [kFxGroups][T], the last
-    // group's second half the scale; when set, eout holds fixed-point records
-    // of the product instead of doubles. fx_guard: log2 of the largest
+    // kFxGroups 16-byte groups of two entries, the last group's second half
+    // the scale, [T / 32][kFxGroups][32] (a warp's groups at fixed offsets);
+    // when set, eout holds fixed-point records of the product instead of
+    // doubles. fx_guard: log2 of the largest
     // number of element corners at a node, rounded up.
     int4* Kfx = nullptr;
     uint32_t fx_guard = 0;
@@ -250,11 +251,11 @@ void launch_bsr_assemble_fp64(const MeshView<double>& m, uint32_t nnzb, const ui
 // (fem_kernels.cu): CTA r of `ctas` owns the elements [r ept, (r+1) ept) and
 // the nodes [r npt, (r+1) npt); ent_max bounds a CTA's CSR entries; smem is
 // its dynamic shared memory (cg_cluster_smem_bytes).
-constexpr uint32_t kCgClusterMaxCtas = 16, kCgClusterMaxThreads = 512;
+constexpr uint32_t kCgClusterMaxCtas = 16, kCgClusterMaxThreads = 512, kCgClusterRegThreads = 256;
 constexpr size_t kCgClusterMaxSmem = 200 * 1024;
-// split: three lanes per element (ten elements per warp), else one.
+// nodes: per four lanes (1, 2 or 4; npt <= nodes threads / 4).
 struct CgClusterPlan {
-    uint32_t ctas, threads, ept, npt, ent_max, split;
+    uint32_t ctas, threads, ept, npt, ent_max, nodes;
     size_t smem;
 };
 size_t cg_cluster_smem_bytes(uint32_t ept, uint32_t npt, uint32_t ent_max);

@@ -236,78 +236,107 @@ __global__ void k_elem_lcm_spmv_fp64(MeshView<double> m, const double* __restric
 
 // ---- element kernels ----
 
-__device__ __forceinline__ void load_nodal(const MeshView<double>& m, uint32_t e, const double* __restrict__ d, double* dl)
+// Element e's groups: 32 apart.
+template <typename P>
+__device__ __forceinline__ P* fx_matrix(P* K, uint32_t e)
 {
-    const int4 t = m.tets[e];
-    const int ids[4] = {(int)bounds_idx((uint32_t)t.x, m.N, kSiteElemNode),
-                        (int)bounds_idx((uint32_t)t.y, m.N, kSiteElemNode),
-                        (int)bounds_idx((uint32_t)t.z, m.N, kSiteElemNode),
-                        (int)bounds_idx((uint32_t)t.w, m.N, kSiteElemNode)};
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        dl[3 * i] = d[3 * (size_t)ids[i]];
-        dl[3 * i + 1] = d[3 * (size_t)ids[i] + 1];
-        dl[3 * i + 2] = d[3 * (size_t)ids[i] + 2];
-    }
+    return K + (size_t)kFxGroups * (e & ~31u) + (e & 31u);
 }
 
 // Element e's fixed-point product matrix (fx.cuh) from R, Dm^-1 and the
 // material scalars: 45 entries and the scale, 368 bytes, written once per
-// evaluation. Integer-bound: about 250 products of three multiplies (284 us
-// for 1,080,000 tets, a fifth of their rotations).
+// evaluation. Integer-bound: about 250 products of three multiplies (224 us
+// for 1,080,000 tets, a sixth of their rotations).
 __global__ void __launch_bounds__(128, 3) k_elem_bake_fp64(MeshView<double> m)
 {
     for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < m.T; e += gridDim.x * blockDim.x) {
         double R[9], Di[9], k1, knu, k2;
         load_elem(m, e, R, Di, k1, knu, k2);
         FxL even{0, 0};
+        int4* Kp = fx_matrix(m.Kfx, e);
         auto put = [&](int k, FxL v) {  // two entries per 16-byte group
             if ((k & 1) == 0) even = v;
-            else m.Kfx[(size_t)(k >> 1) * m.T + e] = make_int4(even.l, even.h, v.l, v.h);
+            else Kp[32 * (k >> 1)] = make_int4(even.l, even.h, v.l, v.h);
         };
         const int32_t scale = fx_grade_ok(m.grade[e], knu, k2) ? fx_bake(R, Di, knu, k2, put) : kFxFp64;
-        m.Kfx[(size_t)(kFxGroups - 1) * m.T + e] = make_int4(even.l, even.h, scale, 0);
+        Kp[32 * (kFxGroups - 1)] = make_int4(even.l, even.h, scale, 0);
     }
 }
 
-// The FP64 product of an element fx.cuh leaves out, as a record.
-__device__ __noinline__ void elem_record_fp64(const MeshView<double>& m, uint32_t e, const double* dl, int64_t* out)
+// The FP64 product of an element fx.cuh leaves out, from its nodes' vectors,
+// as records in o. Out of line and from pointers, so that the fixed-point
+// path keeps its values in registers.
+__device__ __noinline__ void elem_record_fp64(const double* Rp, const double* Dp, const double* mat, size_t T, const double* p0,
+                                              const double* p1, const double* p2, const double* p3, longlong2* o)
 {
-    double R[9], Di[9], k1, knu, k2, o[12];
-    load_elem(m, e, R, Di, k1, knu, k2);
-    elem_RKRt(R, Di, k1, knu, k2, dl, o);
-    fx_stamp_doubles(o, out);
+    double R[9], Di[9], d[12], f[12];
+    int64_t out[12];
+#pragma unroll
+    for (int c = 0; c < 9; c++) {
+        R[c] = Rp[c * T];
+        Di[c] = Dp[c * T];
+    }
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        d[a] = p0[a];
+        d[3 + a] = p1[a];
+        d[6 + a] = p2[a];
+        d[9 + a] = p3[a];
+    }
+    elem_RKRt(R, Di, mat[0], mat[T], mat[2 * T], d, f);
+    fx_stamp_doubles(f, out);
+#pragma unroll
+    for (int c = 0; c < 6; c++) o[c] = make_longlong2(out[2 * c], out[2 * c + 1]);
+}
+
+// Element e's product from its nodes' vectors into six 16-byte words of
+// records. K(k): the matrix entries, in order.
+template <typename FK>
+__device__ __forceinline__ void elem_records(const MeshView<double>& m, uint32_t e, int32_t scale, FK&& K,
+                                             const double* const* p, longlong2* o)
+{
+    double dl[12];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int a = 0; a < 3; a++) dl[3 * i + a] = p[i][a];
+    FxL D[9];
+    int64_t out[12];
+    int32_t x;
+    bool ok = fx_differences(dl, D, x) && scale != kFxFp64;
+    x += scale + fx_product(K, D, out);
+    ok = ok && fx_stamp(out, x);
+    if (ok) {
+#pragma unroll
+        for (int c = 0; c < 6; c++) o[c] = make_longlong2(out[2 * c], out[2 * c + 1]);
+    } else {
+        elem_record_fp64(m.R + e, m.Dinv + e, m.mat + e, m.T, p[0], p[1], p[2], p[3], o);
+    }
 }
 
 // R K0 R^T d per element as fixed-point records in eout. 368 bytes of matrix
 // per element: bound by the integer pipe while the matrices stay in L2 (up to
 // about 300k tets) and by HBM beyond. The FP64 strain form held the FP64 pipe
-// at 90 %: 7,215 tets 11.4 -> 4.0 us, 20,480 tets 11.7 -> 5.3 us, 1,080,000
-// tets 273 -> 119 us (540 MB, 4.5 TB/s).
+// at 90 %: 7,215 tets 11.4 -> 3.6 us, 20,480 tets 11.7 -> 4.8 us, 1,080,000
+// tets 273 -> 91 us (540 MB, 5.9 TB/s).
 __global__ void __launch_bounds__(128, 3) k_elem_spmv_fp64(MeshView<double> m, const double* __restrict__ d,
                                                            const StepScalars* st, int check_done)
 {
     if (check_done && st->done_pend) return;
     for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < m.T; e += gridDim.x * blockDim.x) {
-        double dl[12];
-        load_nodal(m, e, d, dl);
-        const int4* Kp = m.Kfx + e;
-        const int4 last = Kp[(size_t)(kFxGroups - 1) * m.T];
-        FxL D[9];
-        int64_t out[12];
-        int32_t x;
-        bool ok = fx_differences(dl, D, x) && last.z != kFxFp64;
+        const int4 t = m.tets[e];
+        const double* p[4] = {d + 3 * (size_t)bounds_idx((uint32_t)t.x, m.N, kSiteElemNode),
+                              d + 3 * (size_t)bounds_idx((uint32_t)t.y, m.N, kSiteElemNode),
+                              d + 3 * (size_t)bounds_idx((uint32_t)t.z, m.N, kSiteElemNode),
+                              d + 3 * (size_t)bounds_idx((uint32_t)t.w, m.N, kSiteElemNode)};
+        const int4* Kp = fx_matrix(m.Kfx, e);
+        const int4 last = Kp[32 * (kFxGroups - 1)];
         int4 cur;
-        x += last.z + fx_product([&](int k) {
+        elem_records(m, e, last.z, [&](int k) {
             if (k == kFxK - 1) cur = last;
-            else if ((k & 1) == 0) cur = Kp[(size_t)(k >> 1) * m.T];
+            else if ((k & 1) == 0) cur = Kp[32 * (k >> 1)];
             return (k & 1) ? FxL{cur.z, cur.w} : FxL{cur.x, cur.y};
-        }, D, out);
-        ok = ok && fx_stamp(out, x);
-        if (!ok) elem_record_fp64(m, e, dl, out);
-        longlong2* o = reinterpret_cast<longlong2*>(m.eout + 12 * (size_t)e);
-#pragma unroll
-        for (int c = 0; c < 6; c++) o[c] = make_longlong2(out[2 * c], out[2 * c + 1]);
+        }, p, reinterpret_cast<longlong2*>(m.eout + 12 * (size_t)e));
     }
 }
 
@@ -411,9 +440,27 @@ __device__ __forceinline__ double gather_fp64(const MeshView<double>& m, uint32_
     return s;
 }
 
+// The four lanes' record sums of a node (three components with one exponent
+// each) brought to the largest exponent and added: lane a's component.
+__device__ __forceinline__ double fx_quad_sum(const FxSum* s, uint32_t a, int32_t guard)
+{
+    int32_t E = s[0].E;
+    E = max(E, __shfl_xor_sync(0xffffffffu, E, 1));
+    E = max(E, __shfl_xor_sync(0xffffffffu, E, 2));
+    const int32_t sh = fx_min63(E - s[0].E);
+    FxSum t{0, E};
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        long long v = s[c].acc >> sh;
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        if ((int)a == c) t.acc = v;
+    }
+    return fx_sum_value(t, guard);
+}
+
 // Fixed-point records: lane l adds the corners beg + l, beg + l + 4, ... in
-// all three components (integer sums in block exponents, fx.cuh), then the
-// lanes' sums are brought to the largest exponent and added.
+// all three components (integer sums in block exponents, fx.cuh).
 __device__ __forceinline__ double gather_fx(const MeshView<double>& m, uint32_t n, uint32_t a, bool on)
 {
     const int32_t guard = (int32_t)m.fx_guard;
@@ -431,19 +478,7 @@ __device__ __forceinline__ double gather_fx(const MeshView<double>& m, uint32_t 
             fx_add(s[2], v2, x, guard);
         }
     }
-    int32_t E = s[0].E;
-    E = max(E, __shfl_xor_sync(0xffffffffu, E, 1));
-    E = max(E, __shfl_xor_sync(0xffffffffu, E, 2));
-    const int32_t sh = fx_min63(E - s[0].E);
-    FxSum t{0, E};
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-        long long v = s[c].acc >> sh;
-        v += __shfl_xor_sync(0xffffffffu, v, 1);
-        v += __shfl_xor_sync(0xffffffffu, v, 2);
-        if ((int)a == c) t.acc = v;
-    }
-    return fx_sum_value(t, guard);
+    return fx_quad_sum(s, a, guard);
 }
 
 // K u at node n for the solvers' node kernels: the assembled row when the
@@ -1038,248 +1073,162 @@ __global__ void k_finalize(int kind, const double* __restrict__ partials, uint32
         cudaGraphSetConditional(cond, st->done ? 0u : 1u);
 }
 
-// elem_RKRt over three lanes of a warp (lane a of lanes 3g..3g+2 computes
-// component a): u_i = R^T d_i, the element-frame gradient row a, the stress
-// row a after exchanging the gradient's diagonal and column a, the force
-// row a, and after exchanging the force rows component a of R P (node 0:
-// minus the sum). About 50 FP64 instructions per lane against 140 for one
-// lane; GB300 gives a warp's FP64 instruction about 64 clocks whatever the
-// lanes, so a few warps of elements take a third of the time. Every lane of
-// the warp must call it (invalid lanes with zeros); out4 = component a of
-// nodes 0..3.
-// Rc: column a of R; Rr: row a of R as (R[a][a], R[a][a+1], R[a][a+2])
-// (indexes mod 3).
-__device__ __forceinline__ void elem_RKRt_lanes(const double* Rc, const double* Rr, const double* Di, double k1,
-                                                double knu, double k2, const double* d, uint32_t a, uint32_t base,
-                                                double* out4)
-{
-    const uint32_t l1 = base + (a == 2 ? 0u : a + 1), l2 = base + (a == 0 ? 2u : a - 1);  // lanes of a+1, a+2 (mod 3)
-    double u[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) u[i] = Rc[0] * d[3 * i] + Rc[1] * d[3 * i + 1] + Rc[2] * d[3 * i + 2];
-    const double D0 = u[1] - u[0], D1 = u[2] - u[0], D2 = u[3] - u[0];
-    double H[3];  // row a of the element-frame gradient
-#pragma unroll
-    for (int b = 0; b < 3; b++) H[b] = D0 * Di[b] + D1 * Di[3 + b] + D2 * Di[6 + b];
-    // the lane of component b sends H[b][a'] for the receiver a' = b - 1 or b - 2
-    const double Ha = a == 0 ? H[0] : (a == 1 ? H[1] : H[2]);
-    const double send1 = a == 0 ? H[2] : (a == 1 ? H[0] : H[1]);  // to a - 1
-    const double send2 = a == 0 ? H[1] : (a == 1 ? H[2] : H[0]);  // to a - 2
-    const double e1 = __shfl_sync(0xffffffffu, Ha, l1), e2 = __shfl_sync(0xffffffffu, Ha, l2);
-    const double c1 = __shfl_sync(0xffffffffu, send1, l1), c2 = __shfl_sync(0xffffffffu, send2, l2);
-    const double h1 = a == 0 ? H[1] : (a == 1 ? H[2] : H[0]), h2 = a == 0 ? H[2] : (a == 1 ? H[0] : H[1]);
-    const double saa = k1 * Ha + knu * (e1 + e2);
-    const double s1 = k2 * (h1 + c1), s2 = k2 * (h2 + c2);
-    double Sg[3];  // row a of the stress
-    Sg[0] = a == 0 ? saa : (a == 1 ? s2 : s1);
-    Sg[1] = a == 1 ? saa : (a == 2 ? s2 : s1);
-    Sg[2] = a == 2 ? saa : (a == 0 ? s2 : s1);
-    double P[3];
-#pragma unroll
-    for (int i = 0; i < 3; i++) P[i] = Sg[0] * Di[3 * i] + Sg[1] * Di[3 * i + 1] + Sg[2] * Di[3 * i + 2];
-    double Q1[3], Q2[3];
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-        Q1[i] = __shfl_sync(0xffffffffu, P[i], l1);
-        Q2[i] = __shfl_sync(0xffffffffu, P[i], l2);
-    }
-    double w[3];
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-        w[i] = Rr[0] * P[i] + Rr[1] * Q1[i] + Rr[2] * Q2[i];
-        out4[i + 1] = w[i];
-    }
-    out4[0] = -(w[0] + w[1] + w[2]);
-}
-
 // The whole of ILSS_CG::Solve (ILSS_CG.h:38-151) for a C_WRP solid of up to
 // kCgClusterMaxCtas x kCgClusterMaxThreads tets on one thread-block cluster,
-// on chip. CTA r owns the elements [r ept, (r+1) ept) and the nodes
-// [r npt, (r+1) npt): a thread (kSplit: three lanes, elem_RKRt_lanes)
-// keeps one element's R, Dm^-1 and material scalars in registers and its
-// element output in its CTA's shared memory; the CTA keeps its nodes' y,
-// r, d, q, b, CSR rows and fixed flags. An element product reads its four
-// nodes' d from the owning CTAs' shared memory (distributed shared memory);
-// a node component's gather (one thread per component) reads its element
-// corners' outputs the same way (ent: per CSR entry, the owning CTA << 24 |
-// its local corner). A reduction sums each CTA's block total into a slot of
-// every CTA, then every CTA adds the slots in rank order, so all CTAs take
-// the same scalar steps and leave the loop together. Four cluster barriers
-// per iteration: element outputs complete, d.q, |r|^2, the new d. y and the
-// statistics are written back at the end; the loop ends on the solver's own
-// tests (at most max_iter iterations).
-template <int kSplit>
-__global__ void __launch_bounds__(kCgClusterMaxThreads, 1)
+// on chip. CTA r owns the elements [r ept, (r+1) ept), one per thread, and the
+// nodes [r npt, (r+1) npt), kNodes per four lanes, whose y, r, d, q and b
+// components stay in the lanes' registers. An element product (fx.cuh; kReg:
+// the matrix in registers, else read from L2 each time) reads its four nodes'
+// d from the owning CTAs' shared memory (distributed shared memory) and
+// leaves its records in its own; a node's lanes add its corners' records the
+// same way (ent: per CSR entry, the owning CTA << 24 | its local corner). A
+// reduction leaves each CTA's block total in a slot of every CTA, and every
+// warp adds the slots, so all CTAs take the same scalar steps and leave the
+// loop together. Four cluster barriers per iteration: element records
+// complete, d.q, |r|^2, the new d. y and the statistics are written back at
+// the end; the loop ends on the solver's own tests (at most max_iter
+// iterations).
+template <bool kReg, int kNodes>
+__global__ void __launch_bounds__(kReg ? kCgClusterRegThreads : kCgClusterMaxThreads, 1)
     k_cg_cluster_fp64(MeshView<double> m, StepConsts c, CgClusterPlan p, const uint32_t* __restrict__ ent,
                       const double* __restrict__ b, double* y, StepScalars* st)
 {
     namespace cgr = cooperative_groups;
     cgr::cluster_group cl = cgr::this_cluster();
     extern __shared__ __align__(16) unsigned char cl_smem[];
-    const uint32_t tid = threadIdx.x, nt = blockDim.x, rank = cl.block_rank(), C = p.ctas;
+    const uint32_t tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, rank = cl.block_rank(), C = p.ctas;
     const uint32_t N = m.N, T = m.T;
     const uint32_t e0 = rank * p.ept, n0 = rank * p.npt;
-    const uint32_t ne = e0 < T ? min(p.ept, T - e0) : 0u, nn = n0 < N ? min(p.npt, N - n0) : 0u, n3 = 3 * nn;
-    const size_t v3 = 3 * (size_t)p.npt;
-    double* eo = reinterpret_cast<double*>(cl_smem);  // [12 ept]
-    double* vy = eo + 12 * (size_t)p.ept;               // [3 npt] each
-    double* vr = vy + v3;
-    double* vd = vr + v3;
-    double* vq = vd + v3;
-    double* vb = vq + v3;
-    double* part = vb + v3;                                   // [3][kCgClusterMaxCtas]
-    uint32_t* cptr = reinterpret_cast<uint32_t*>(part + 3 * kCgClusterMaxCtas);  // [npt + 1]
-    uint32_t* cent = cptr + p.npt + 1;                                          // [ent_max]
-    uint8_t* fx = reinterpret_cast<uint8_t*>(cent + p.ent_max);                 // [npt]
+    const uint32_t ne = e0 < T ? min(p.ept, T - e0) : 0u, nn = n0 < N ? min(p.npt, N - n0) : 0u;
+    longlong2* eo = reinterpret_cast<longlong2*>(cl_smem);                 // [6 ept]
+    double* vd = reinterpret_cast<double*>(eo + 6 * (size_t)p.ept);          // [3 npt]
+    double* part = vd + 3 * (size_t)p.npt;                                  // [3][kCgClusterMaxCtas]
+    uint32_t* cent = reinterpret_cast<uint32_t*>(part + 3 * kCgClusterMaxCtas);  // [ent_max]
     __shared__ StepScalars sst;
+    __shared__ double wsum[kCgClusterMaxThreads / 32];
     const double mfm = c.mass * c.factor_M;
+    const int32_t guard = (int32_t)m.fx_guard;
     const uint32_t base = nn ? m.csr_ptr[n0] : 0u;
-    for (uint32_t i = tid; i < n3; i += nt) {
-        vy[i] = y[3 * (size_t)n0 + i];
-        vb[i] = b[3 * (size_t)n0 + i];
-    }
-    for (uint32_t i = tid; i <= nn; i += nt) cptr[i] = nn ? m.csr_ptr[n0 + i] - base : 0u;
     const uint32_t ne_ent = nn ? min(m.csr_ptr[n0 + nn] - base, p.ent_max) : 0u;
     for (uint32_t i = tid; i < ne_ent; i += nt) cent[i] = ent[base + i];
-    for (uint32_t i = tid; i < nn; i += nt) fx[i] = m.fixed[n0 + i];
     if (tid == 0) sst = *st;
-    // this thread's element and where its nodes live: element tid, or with
-    // kSplit lane 3g + a (a < 3, g < 10) of warp w takes component a of
-    // element 10 w + g
-    const uint32_t lane = tid & 31, ca = kSplit ? lane % 3 : 0u, cbase = lane - ca;
-    const uint32_t le = kSplit ? (lane < 30 ? 10 * (tid >> 5) + lane / 3 : 0xffffffffu) : tid;
-    const bool has_elem = le < ne;
-    double R[9], Di[9], k1 = 0, knu = 0, k2 = 0;
+    auto sync = [&] {
+        if (C == 1) __syncthreads();
+        else cl.sync();
+    };
+    // this lane's components: node tid / 4 + k nt / 4, component a
+    const uint32_t a = tid & 3u;
+    double ny[kNodes], nr[kNodes], nd[kNodes], nq[kNodes];
+    uint32_t cb[kNodes], ce[kNodes];
+    bool live[kNodes];  // the component exists and is not constrained
 #pragma unroll
-    for (int k = 0; k < 9; k++) R[k] = Di[k] = 0.0;
-    double Rc[3] = {0, 0, 0}, Rr[3] = {0, 0, 0};  // kSplit: column a of R, row a from (a, a)
-    uint32_t nr[4] = {0, 0, 0, 0}, nl[4] = {0, 0, 0, 0};
-    if (has_elem) {
-        load_elem(m, e0 + le, R, Di, k1, knu, k2);
-        if constexpr (kSplit != 0) {
-            double row[3];
+    for (int k = 0; k < kNodes; k++) {
+        const uint32_t ln = (tid >> 2) + k * (nt >> 2);
+        const bool on = ln < nn;
+        cb[k] = on ? m.csr_ptr[n0 + ln] - base + a : 0u;
+        ce[k] = on ? min(m.csr_ptr[n0 + ln + 1] - base, ne_ent) : 0u;
+        live[k] = on && a < 3 && !m.fixed[n0 + ln];
+        ny[k] = on && a < 3 ? y[3 * (size_t)(n0 + ln) + a] : 0.0;
+        nr[k] = nd[k] = nq[k] = 0.0;
+        if (on && a < 3) vd[3 * ln + a] = ny[k];
+    }
+    // this thread's element
+    const bool has_elem = tid < ne;
+    const uint32_t e = has_elem ? e0 + tid : 0u;
+    const int4* Kp = fx_matrix(m.Kfx, e);
+    const int32_t scale = has_elem ? Kp[32 * (kFxGroups - 1)].z : kFxFp64;
+    FxL K[kReg ? kFxK : 1];
+    if constexpr (kReg) {
 #pragma unroll
-            for (int k = 0; k < 3; k++) {
-                Rc[k] = ca == 0 ? R[3 * k] : (ca == 1 ? R[3 * k + 1] : R[3 * k + 2]);
-                row[k] = ca == 0 ? R[k] : (ca == 1 ? R[3 + k] : R[6 + k]);
-            }
-            Rr[0] = ca == 0 ? row[0] : (ca == 1 ? row[1] : row[2]);
-            Rr[1] = ca == 0 ? row[1] : (ca == 1 ? row[2] : row[0]);
-            Rr[2] = ca == 0 ? row[2] : (ca == 1 ? row[0] : row[1]);
+        for (int g = 0; g < (int)kFxGroups; g++) {
+            const int4 v = has_elem ? Kp[32 * g] : make_int4(0, 0, 0, 0);
+            K[2 * g] = FxL{v.x, v.y};
+            if (2 * g + 1 < kFxK) K[2 * g + 1] = FxL{v.z, v.w};
         }
-        const int4 t = m.tets[e0 + le];
+    }
+    const double* pd[4] = {vd, vd, vd, vd};
+    if (has_elem) {
+        const int4 t = m.tets[e];
         const uint32_t ids[4] = {bounds_idx((uint32_t)t.x, N, kSiteElemNode), bounds_idx((uint32_t)t.y, N, kSiteElemNode),
                                  bounds_idx((uint32_t)t.z, N, kSiteElemNode), bounds_idx((uint32_t)t.w, N, kSiteElemNode)};
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-            nr[k] = ids[k] / p.npt;
-            nl[k] = 3 * (ids[k] - nr[k] * p.npt);
+            const uint32_t nrk = ids[k] / p.npt;
+            pd[k] = cl.map_shared_rank(vd, nrk) + 3 * (ids[k] - nrk * p.npt);
         }
     }
-    const double* pd[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) pd[k] = cl.map_shared_rank(vd, nr[k]) + nl[k];
-    cl.sync();  // every CTA's y, d and CSR rows are in place
-    auto elem_products = [&](const double* const* u) {
-        double dl[12];
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            dl[3 * k] = has_elem ? u[k][0] : 0.0;
-            dl[3 * k + 1] = has_elem ? u[k][1] : 0.0;
-            dl[3 * k + 2] = has_elem ? u[k][2] : 0.0;
+    auto product = [&] {
+        if (has_elem) {
+            int4 cur;
+            elem_records(m, e, scale, [&](int k) {
+                if constexpr (kReg) return K[k];
+                if ((k & 1) == 0) cur = __ldg(Kp + 32 * (k >> 1));
+                return (k & 1) ? FxL{cur.z, cur.w} : FxL{cur.x, cur.y};
+            }, pd, eo + 6 * tid);
         }
-        if constexpr (kSplit != 0) {
-            double o4[4];
-            elem_RKRt_lanes(Rc, Rr, Di, k1, knu, k2, dl, ca, cbase, o4);
-            if (has_elem)
-#pragma unroll
-                for (int k = 0; k < 4; k++) eo[12 * le + 3 * k + ca] = o4[k];
-        } else if (has_elem) {
-            double out[12];
-            elem_RKRt(R, Di, k1, knu, k2, dl, out);
-#pragma unroll
-            for (int k = 0; k < 12; k++) eo[12 * le + k] = out[k];
-        }
-        cl.sync();  // all element outputs complete
+        sync();  // all element records complete
     };
-    // component a of node ln's element sum
-    auto gather = [&](uint32_t ln, uint32_t a) {
-        const uint32_t jend = min(cptr[ln + 1], ne_ent);
-        double acc = 0.0;
-#pragma unroll 4
-        for (uint32_t j = cptr[ln]; j < jend; j++) {
-            const uint32_t e = cent[j];
-            acc += cl.map_shared_rank(eo, e >> 24)[3 * (e & 0xffffffu) + a];
+    // the lane's component of node k's sum (gather_fx over the CTAs)
+    auto gather = [&](int k) {
+        FxSum s[3] = {{0, 0}, {0, 0}, {0, 0}};
+#pragma unroll 2
+        for (uint32_t j = cb[k]; j < ce[k]; j += 4) {
+            const uint32_t w = cent[j];
+            const long long* r = reinterpret_cast<const long long*>(cl.map_shared_rank(eo, w >> 24)) + 3 * (w & 0xffffffu);
+            const int64_t v0 = r[0], v1 = r[1], v2 = r[2];
+            const int32_t x = fx_record_exp(v0, v1, v2);
+            fx_add(s[0], v0, x, guard);
+            fx_add(s[1], v1, x, guard);
+            fx_add(s[2], v2, x, guard);
         }
-        return acc;
+        return fx_quad_sum(s, a, guard);
     };
-    // the cluster's total of every thread's acc (valid in thread 0)
-    // (each FP64 add costs a warp about 64 clocks: the CTA's warp totals and
-    // the CTAs' totals are added in shuffle trees of log2 depth, the same
-    // fixed trees in every CTA)
-    __shared__ double wsum[kCgClusterMaxThreads / 32];
-    const uint32_t nw = nt >> 5;
-    const uint32_t wtop = nw > 1 ? 1u << (31 - __clz(nw - 1)) : 0u, ctop = C > 1 ? 1u << (31 - __clz(C - 1)) : 0u;
+    // the cluster's total of every thread's acc, in every thread
     auto cluster_total = [&](double acc, int slot) -> double {
-        double v = warp_sum(acc);
-        if (lane == 0) wsum[tid >> 5] = v;
-        __syncthreads();
-        if (tid < 32) {
-            v = lane < nw ? wsum[lane] : 0.0;
-            for (uint32_t o = wtop; o >= 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            v = __shfl_sync(0xffffffffu, v, 0);
-            if (lane < C) cl.map_shared_rank(part, lane)[slot * kCgClusterMaxCtas + rank] = v;
+        double v = fx_warp_sum(acc);
+        if (nt > 32) {
+            if (lane == 0) wsum[tid >> 5] = v;
+            __syncthreads();
+            if (tid < 32) v = fx_warp_sum(lane < (nt >> 5) ? wsum[lane] : 0.0);
         }
-        cl.sync();
-        double total = 0.0;
-        if (tid < 32) {
-            total = lane < C ? part[slot * kCgClusterMaxCtas + lane] : 0.0;
-            for (uint32_t o = ctop; o >= 1; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-        }
-        return total;
+        if (tid < C) cl.map_shared_rank(part, tid)[slot * kCgClusterMaxCtas + rank] = v;
+        sync();
+        return fx_warp_sum(lane < C ? part[slot * kCgClusterMaxCtas + lane] : 0.0);
     };
-    // r = S(b - A y), d = r, |r|^2
-    {
-        const double* py[4];
+    sync();  // every CTA's y is in place
+    for (bool start = true;; start = false) {
+        // the start: r = S(b - A y), d = r, |r|^2; then q = S A d, d.q, alpha
+        product();
+        double acc = 0.0;
 #pragma unroll
-        for (int k = 0; k < 4; k++) py[k] = cl.map_shared_rank(vy, nr[k]) + nl[k];
-        elem_products(py);
-    }
-    double acc = 0.0;
-    for (uint32_t i = tid; i < n3; i += nt) {
-        const uint32_t ln = i / 3;
-        const double s = gather(ln, i - 3 * ln);
-        const double ri = fx[ln] ? 0.0 : vb[i] - (c.factor_K * s + mfm * vy[i]);
-        vr[i] = ri;
-        vd[i] = ri;
-        acc += ri * ri;
-    }
-    double total = cluster_total(acc, 0);
-    if (tid == 0) fin_init(&sst, c, total);
-    __syncthreads();
-    while (!sst.done) {
-        // q = S A d, d.q, alpha
-        elem_products(pd);
-        acc = 0.0;
-        for (uint32_t i = tid; i < n3; i += nt) {
-            const uint32_t ln = i / 3;
-            const double s = gather(ln, i - 3 * ln);
-            const double qi = fx[ln] ? 0.0 : c.factor_K * s + mfm * vd[i];
-            vq[i] = qi;
-            acc += vd[i] * qi;
+        for (int k = 0; k < kNodes; k++) {
+            const double s = gather(k);
+            const uint32_t ln = (tid >> 2) + k * (nt >> 2);
+            if (start) {
+                if (live[k]) nr[k] = nd[k] = b[3 * (size_t)(n0 + ln) + a] - (c.factor_K * s + mfm * ny[k]);
+                if (ln < nn && a < 3) vd[3 * ln + a] = nd[k];
+                acc += nr[k] * nr[k];
+            } else {
+                if (live[k]) nq[k] = c.factor_K * s + mfm * nd[k];
+                acc += nd[k] * nq[k];
+            }
         }
-        total = cluster_total(acc, 1);
-        if (tid == 0) fin_alpha(&sst, total);
+        double total = cluster_total(acc, start ? 0 : 1);  // at the start its barrier completes d too
+        if (tid == 0) {
+            if (start) fin_init(&sst, c, total);
+            else fin_alpha(&sst, total);
+        }
         __syncthreads();
         if (sst.done) break;
+        if (start) continue;
         // y += alpha d, r -= alpha q, |r|^2, beta and the loop test
         const double alpha = sst.alpha, na = -alpha;
         acc = 0.0;
-        for (uint32_t i = tid; i < n3; i += nt) {
-            vy[i] += alpha * vd[i];
-            const double ri = vr[i] + na * vq[i];
-            vr[i] = ri;
-            acc += ri * ri;
+#pragma unroll
+        for (int k = 0; k < kNodes; k++) {
+            ny[k] += alpha * nd[k];
+            nr[k] += na * nq[k];
+            acc += nr[k] * nr[k];
         }
         total = cluster_total(acc, 2);
         if (tid == 0) fin_beta(&sst, total);
@@ -1287,33 +1236,51 @@ __global__ void __launch_bounds__(kCgClusterMaxThreads, 1)
         if (sst.done) break;
         // d = S (beta d + r)
         const double beta = sst.beta;
-        for (uint32_t i = tid; i < n3; i += nt) vd[i] = fx[i / 3] ? 0.0 : beta * vd[i] + vr[i];
-        cl.sync();  // the new d is complete
+#pragma unroll
+        for (int k = 0; k < kNodes; k++) {
+            const uint32_t ln = (tid >> 2) + k * (nt >> 2);
+            nd[k] = beta * nd[k] + nr[k];
+            if (ln < nn && a < 3) vd[3 * ln + a] = nd[k];
+        }
+        sync();  // the new d is complete
     }
-    for (uint32_t i = tid; i < n3; i += nt) y[3 * (size_t)n0 + i] = vy[i];
+#pragma unroll
+    for (int k = 0; k < kNodes; k++) {
+        const uint32_t ln = (tid >> 2) + k * (nt >> 2);
+        if (ln < nn && a < 3) y[3 * (size_t)(n0 + ln) + a] = ny[k];
+    }
     if (rank == 0 && tid == 0) {
         fin_stats(&sst);
         *st = sst;
     }
-    cl.sync();  // no CTA leaves while another may still read its shared memory
+    sync();  // no CTA leaves while another may still read its shared memory
 }
 
 size_t cg_cluster_smem_bytes(uint32_t ept, uint32_t npt, uint32_t ent_max)
 {
-    return sizeof(double) * (12 * (size_t)ept + 15 * (size_t)npt + 3 * kCgClusterMaxCtas) +
-           sizeof(uint32_t) * ((size_t)npt + 1 + ent_max) + npt;
+    return sizeof(double) * (12 * (size_t)ept + 3 * (size_t)npt + 3 * kCgClusterMaxCtas) + sizeof(uint32_t) * (size_t)ent_max;
 }
 
 namespace {
-template <int kSplit>
+using CgClusterKernel = void (*)(MeshView<double>, StepConsts, CgClusterPlan, const uint32_t*, const double*, double*,
+                                 StepScalars*);
+// The instance for a plan: matrices in registers while the threads leave room
+// for them, else one, two or four nodes per four lanes.
+CgClusterKernel cg_cluster_kernel(const CgClusterPlan& p)
+{
+    if (p.nodes == 1) return p.threads <= kCgClusterRegThreads ? k_cg_cluster_fp64<true, 1> : k_cg_cluster_fp64<false, 1>;
+    return p.nodes == 2 ? k_cg_cluster_fp64<false, 2> : k_cg_cluster_fp64<false, 4>;
+}
 cudaError_t cg_cluster_attrs()
 {
     static const cudaError_t e = [] {
-        cudaError_t r = cudaFuncSetAttribute(k_cg_cluster_fp64<kSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)kCgClusterMaxSmem);
-        if (r == cudaSuccess)
-            r = cudaFuncSetAttribute(k_cg_cluster_fp64<kSplit>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        return r;
+        for (auto* k : {k_cg_cluster_fp64<true, 1>, k_cg_cluster_fp64<false, 1>, k_cg_cluster_fp64<false, 2>,
+                        k_cg_cluster_fp64<false, 4>}) {
+            cudaError_t r = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCgClusterMaxSmem);
+            if (r == cudaSuccess) r = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+            if (r != cudaSuccess) return r;
+        }
+        return cudaSuccess;
     }();
     return e;
 }
@@ -1336,17 +1303,15 @@ void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& at, const CgCl
 bool cg_cluster_fits(const CgClusterPlan& p)
 {
     if (p.ctas < 1 || p.ctas > kCgClusterMaxCtas || p.threads < 32 || p.threads > kCgClusterMaxThreads ||
-        p.threads % 32 || p.smem > kCgClusterMaxSmem ||
-        p.ept > (p.split ? 10 * (p.threads / 32) : p.threads) ||
-        (p.split ? cg_cluster_attrs<1>() : cg_cluster_attrs<0>()) != cudaSuccess)
+        p.threads % 32 || p.smem > kCgClusterMaxSmem || p.ept > p.threads ||
+        (p.nodes != 1 && p.nodes != 2 && p.nodes != 4) || 4 * (size_t)p.npt > (size_t)p.nodes * p.threads ||
+        cg_cluster_attrs() != cudaSuccess)
         return false;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at;
     cluster_config(cfg, at, p, nullptr);
     int n = 0;
-    const cudaError_t e = p.split ? cudaOccupancyMaxActiveClusters(&n, k_cg_cluster_fp64<1>, &cfg)
-                                  : cudaOccupancyMaxActiveClusters(&n, k_cg_cluster_fp64<0>, &cfg);
-    if (e != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&n, cg_cluster_kernel(p), &cfg) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
@@ -1356,15 +1321,12 @@ bool cg_cluster_fits(const CgClusterPlan& p)
 cudaError_t launch_cg_cluster_fp64(const MeshView<double>& m, const StepConsts& c, const CgClusterPlan& p,
                                    const uint32_t* ent, const double* b, double* y, StepScalars* st, cudaStream_t s)
 {
-    cudaError_t e = p.split ? cg_cluster_attrs<1>() : cg_cluster_attrs<0>();
-    if (e != cudaSuccess) return e;
+    if (const cudaError_t e = cg_cluster_attrs(); e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at;
     cluster_config(cfg, at, p, s);
-    e = p.split ? cudaLaunchKernelEx(&cfg, k_cg_cluster_fp64<1>, m, c, p, ent, b, y, st)
-                : cudaLaunchKernelEx(&cfg, k_cg_cluster_fp64<0>, m, c, p, ent, b, y, st);
     launch_counter()++;
-    return e;
+    return cudaLaunchKernelEx(&cfg, cg_cluster_kernel(p), m, c, p, ent, b, y, st);
 }
 
 // ---- launchers ----

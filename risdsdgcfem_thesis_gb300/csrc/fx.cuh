@@ -4,18 +4,19 @@
 // GB300 issues one FP64 instruction per 64 clocks on each of an SM's four
 // sub-partitions (measured: DFMA 64.1 clocks, DADD 64 to 76, for dependent
 // and independent ones alike), and one 32 x 32 + 64 bit integer multiply-add
-// (IMAD.WIDE) per 2.07. A product of two 60-bit integers held as two signed
+// (IMAD.WIDE) per 4.3. A product of two 60-bit integers held as two signed
 // 32-bit limbs takes three of those (the low x low term is below the last
 // bit kept). The element product is therefore one symmetric 9 x 9 matrix per
 // element, K9 = the blocks (i, j), i, j = 1..3, of R K0 R^T, baked after each
 // evaluation, times the three node differences d_j - d_0 (node 0's output is
-// minus the sum of the others'): 81 products, about 500 clocks of
-// multiplies against 8,800 for the 138 FP64 operations of the strain form.
+// minus the sum of the others'): 81 products, about 1,050 clocks of
+// multiplies (1,200 with the rest of the product, 800 for the differences)
+// against 8,800 for the 138 FP64 operations of the strain form.
 //
 // Numbers are block fixed point: the nine differences share one exponent,
 // normalised to the largest, K9 one exponent, the twelve outputs one
 // exponent. Bounds are stated beside each stage. K9's entries are good to
-// about 2^-56 of the largest, the differences to 2^-60 and the sums to 2^-56,
+// about 2^-56 of the largest, the differences to 2^-59 and the sums to 2^-56,
 // where FP64 rounds every operation at 2^-53. Elements for which that does
 // not hold -- a non-finite or out-of-range operand, a rotation entry above
 // 1.125, a rest shape so graded that one exponent for Dm^-1 would cost more
@@ -44,6 +45,11 @@ FX_HD FxL fx_split(int64_t v)
     FxL s;
     s.l = (int32_t)v;
     s.h = (int32_t)(v >> 32) + (int32_t)((uint32_t)s.l >> 31);
+#ifdef __CUDA_ARCH__
+    // two plain 32-bit values from here on: otherwise the compiler carries the
+    // limb as a 64-bit one and multiplies 64 x 64 (four instructions)
+    asm("" : "+r"(s.l), "+r"(s.h));
+#endif
     return s;
 }
 
@@ -55,11 +61,11 @@ FX_HD void fx_mac(int64_t& hi, int64_t& mid, const FxL& a, const FxL& b)
     mid += (int64_t)a.l * b.h;
 }
 
-// The accumulated product in units of 2^(64 - K); mid in units of 2^(32 + half).
+// The accumulated product in units of 2^(64 - K).
 template <int K>
-FX_HD int64_t fx_fin(int64_t hi, int64_t mid, int half = 0)
+FX_HD int64_t fx_fin(int64_t hi, int64_t mid)
 {
-    return (int64_t)((uint64_t)hi << K) + (mid >> (32 - K - half));
+    return (int64_t)((uint64_t)hi << K) + (mid >> (32 - K));
 }
 
 FX_HD uint64_t fx_bits(double v)
@@ -95,10 +101,9 @@ FX_HD int64_t fx_align(double v, int32_t E)
     const uint64_t u = fx_bits(v);
     const int32_t e = (int32_t)(u >> 52) & 0x7ff;
     const uint64_t m = ((u & 0xfffffffffffffull) | 0x10000000000000ull) << (B - 53);
-    const int32_t sh = E - e;
-    const int64_t a = (sh < 63 && e != 0) ? (int64_t)(m >> (sh & 63)) : 0;
+    const int32_t sh = e == 0 || E - e > 63 ? 63 : E - e;
     const int64_t s = (int64_t)u >> 63;
-    return (a ^ s) - s;
+    return ((int64_t)(m >> sh) ^ s) - s;
 }
 
 // The scale of an element whose product runs in FP64 instead.
@@ -213,18 +218,19 @@ FX_HD constexpr int fx_at(int r, int c)  // r <= c
 }
 
 // An element's grade max|Dm| max|Dm^-1| (1 for a cube corner): one exponent
-// for all of Dm^-1 costs bits of K9 with it. Measured against 128-bit products
-// (random shapes, rotations and fields): below grade 3 the error is 0.2 to
-// 0.9 of the FP64 strain form's for nu up to 0.45, between 3 and 4 it passes
-// it; near incompressibility both lose bits and the line lies at 1.2.
-constexpr float kFxMaxGrade = 3.0f, kFxMaxGradeStiff = 1.2f;
-constexpr double kFxStiff = 9.5;  // lambda / mu
+// for all of Dm^-1 costs bits of K9 with it, and stiff materials cost bits of
+// the shear terms. Measured against 128-bit products (random shapes,
+// rotations and fields), the error below these grades is 0.4 to 0.95 of the
+// FP64 strain form's; above them it passes it (grade 2 to 3 at nu 0.45: up to
+// 1.2 times).
+constexpr float kFxMaxGrade = 3.0f, kFxMaxGradeStiff = 2.0f, kFxMaxGradeRigid = 1.2f;
+constexpr double kFxStiff = 2.0, kFxRigid = 9.5;  // lambda / mu
 
 // Whether an element of this rest shape and material may take fx_bake:
 // grade = max|Dm| max|Dm^-1|.
 FX_HD bool fx_grade_ok(float grade, double kl, double km)
 {
-    return grade <= (kl <= kFxStiff * km ? kFxMaxGrade : kFxMaxGradeStiff);  // false for NaN
+    return grade <= (kl <= kFxStiff * km ? kFxMaxGrade : (kl <= kFxRigid * km ? kFxMaxGradeStiff : kFxMaxGradeRigid));
 }
 
 // Bakes K9 = V (lambda m_i m_j^T + mu m_j m_i^T + mu (g_i . g_j) R R^T) with g_i
@@ -312,77 +318,80 @@ FX_HD int32_t fx_bake(const double* R, const double* Di, double kl, double km, F
     return xm + 2 * xd - 59 - (lz - 1) + 3;
 }
 
-// The node differences d_j - d_0 (D[3 (j - 1) + a]) in limbs, |D| < 2^60, from
+// The leading zeros of the largest magnitude of several values, from the
+// words fx_top accumulates (31 when all their high words are zero: the values
+// are then below 2^32 and moving them up by less is exact).
+FX_HD uint32_t fx_top(int64_t v)
+{
+    const int32_t h = (int32_t)(v >> 32);
+    return (uint32_t)(h ^ (h >> 31));
+}
+FX_HD int fx_clz_top(uint32_t any)
+{
+#ifdef __CUDA_ARCH__
+    return __clz((int)(any | 1u));
+#else
+    return __builtin_clz(any | 1u);
+#endif
+}
+
+// The node differences d_j - d_0 (D[3 (j - 1) + a]) in limbs, |D| < 2^59, from
 // the four nodes' vectors; returns the exponent x of their units (2^x). False
-// when a component is not finite (the element takes FP64); all-zero
-// differences give zeros.
+// when one is not finite (the element takes FP64); all-zero differences give
+// zeros. The nine subtractions are FP64's own (the pipe is idle otherwise).
 FX_HD bool fx_differences(const double* d, FxL* D, int32_t& x)
 {
+    double v[9];
     int32_t E = 0;
-#pragma unroll
-    for (int i = 0; i < 12; i++) {
-        const int32_t e = fx_exp(d[i]);
-        E = e > E ? e : E;
-    }
-    int64_t v[9];
-    uint64_t any = 1;
-    int64_t d0[3];
-#pragma unroll
-    for (int a = 0; a < 3; a++) d0[a] = fx_align<62>(d[a], E);
 #pragma unroll
     for (int j = 0; j < 3; j++)
 #pragma unroll
         for (int a = 0; a < 3; a++) {
-            v[3 * j + a] = fx_align<62>(d[3 * (j + 1) + a], E) - d0[a];
-            any |= fx_mag(v[3 * j + a]);
+            v[3 * j + a] = d[3 * (j + 1) + a] - d[a];
+            const int32_t e = fx_exp(v[3 * j + a]);
+            E = e > E ? e : E;
         }
-    const int lz = fx_clz(any);  // 1 at least
 #pragma unroll
-    for (int k = 0; k < 9; k++) D[k] = fx_split((int64_t)((uint64_t)v[k] << (lz - 1)) >> 3);
-    x = E - 1022 - 62 - (lz - 1) + 3;
+    for (int k = 0; k < 9; k++) D[k] = fx_split(fx_align<59>(v[k], E));
+    x = E - 1022 - 59;
     return E < 2047;
 }
 
 // K9 D: out[3 i + a] for the nodes i = 0..3, normalised (|out| < 2^61, node 0's
 // below 3 2^61) in units of 2^(scale + x + the returned shift). K(k) gives
-// entry k of the packed triangle. Each of the two mid sums stays below
-// 9 2^28 2^31 = 2^62.2, the outputs before their normalisation below 2^62.2.
+// entry k of the packed triangle, in order. The mid sums stay below
+// 9 (2^28 + 2^27) 2^31 < 2^63, the outputs before their normalisation below
+// 2^60.2.
 template <typename FK>
 FX_HD int32_t fx_product(FK&& K, const FxL* D, int64_t* out)
 {
-    int64_t hi[9], m1[9], m2[9];
+    int64_t hi[9], mid[9];
 #pragma unroll
-    for (int r = 0; r < 9; r++) hi[r] = m1[r] = m2[r] = 0;
+    for (int r = 0; r < 9; r++) hi[r] = mid[r] = 0;
 #pragma unroll
     for (int r = 0; r < 9; r++)
 #pragma unroll
         for (int c = r; c < 9; c++) {  // entry (r, c) goes to rows r and c as it arrives
             const FxL k = K(fx_at(r, c));
-            hi[r] += (int64_t)k.h * D[c].h;
-            m1[r] += (int64_t)k.h * D[c].l;
-            m2[r] += (int64_t)k.l * D[c].h;
-            if (c > r) {
-                hi[c] += (int64_t)k.h * D[r].h;
-                m1[c] += (int64_t)k.h * D[r].l;
-                m2[c] += (int64_t)k.l * D[r].h;
-            }
+            fx_mac(hi[r], mid[r], k, D[c]);
+            if (c > r) fx_mac(hi[c], mid[c], k, D[r]);
         }
-    int64_t sum[3] = {0, 0, 0};
-    uint64_t any = 1;
+    uint32_t any = 0;
 #pragma unroll
     for (int r = 0; r < 9; r++) {
-        out[3 + r] = fx_fin<3>(hi[r], (m1[r] >> 1) + (m2[r] >> 1), 1);
-        any |= fx_mag(out[3 + r]);
+        out[3 + r] = fx_fin<2>(hi[r], mid[r]);
+        any |= fx_top(out[3 + r]);
     }
-    const int lz = fx_clz(any);  // 2 at least
+    const int up = fx_clz_top(any) - 3;
+    int64_t sum[3] = {0, 0, 0};
 #pragma unroll
     for (int r = 0; r < 9; r++) {
-        out[3 + r] = (int64_t)((uint64_t)out[3 + r] << (lz - 2)) >> 1;
+        out[3 + r] = (int64_t)((uint64_t)out[3 + r] << up);
         sum[r % 3] += out[3 + r];
     }
 #pragma unroll
     for (int a = 0; a < 3; a++) out[a] = -sum[a];
-    return 61 - (lz - 2) + 1;
+    return 62 - up;
 }
 
 #ifdef __CUDACC__

@@ -391,12 +391,8 @@ int open_step(fem_solid s)
     return FEM_OK;
 }
 
-// A C_WRP solid with a one-cluster CG plan. GB300 gives a warp's FP64
-// instruction about 64 clocks whatever its active lanes, and an SM about
-// one every 19 clocks over all its warps: a 140-instruction element product
-// takes about 9k clocks, so the plan spreads the elements thin (at most a
-// few warps of them per SM) over up to 16 CTAs, and its iteration is four
-// cluster barriers instead of six launches.
+// A C_WRP solid with a one-cluster CG plan: its iteration is four cluster
+// barriers instead of four launches.
 bool cg_on_cluster(const fem_solid s)
 {
     return s->params.material == FEM_MATERIAL_C_WRP && s->cl_plan.ctas > 0;
@@ -472,19 +468,18 @@ int build_bsr(fem_solid s, const uint32_t* tets, const std::vector<uint32_t>& pt
     return FEM_OK;
 }
 
-// The one-cluster CG plan of a solid (see cg_on_cluster). Up to 1,440 tets,
-// three lanes per element (about 50 FP64 instructions each) and 30
-// elements per CTA on ceil(T / 30) CTAs; beyond, one lane per element and
-// 128 per CTA on ceil(T / 128). When a cluster of that size does not fit,
-// the fewest CTAs below it that do, with at most kCgClusterMaxThreads
-// threads; none when the solid is too large. ptr: the node CSR's row starts.
+// The one-cluster CG plan of a solid (see cg_on_cluster): one element per
+// thread and one node per four lanes, one CTA up to 192 tets (160 tets: 545 us
+// per step against 617 on two to sixteen, whose barriers cost more than the
+// spread saves), then 96 tets per CTA (1,080: 691 us; 256 per CTA: 750). When
+// a cluster of that size does not fit, the fewest CTAs below it that do; none
+// when the solid is too large. ptr: the node CSR's row starts.
 CgClusterPlan plan_cg_cluster(uint32_t N, uint32_t T, const std::vector<uint32_t>& ptr)
 {
     if (T == 0 || N == 0) return CgClusterPlan{};
-    auto try_plan = [&](uint32_t C, uint32_t split, CgClusterPlan& p) {
+    auto try_plan = [&](uint32_t C, CgClusterPlan& p) {
         p = CgClusterPlan{};
         p.ctas = C;
-        p.split = split;
         p.ept = (T + C - 1) / C;
         p.npt = (N + C - 1) / C;
         uint32_t emax = 0;
@@ -493,21 +488,17 @@ CgClusterPlan plan_cg_cluster(uint32_t N, uint32_t T, const std::vector<uint32_t
             emax = std::max(emax, ptr[b] - ptr[a]);
         }
         p.ent_max = emax;
-        const uint32_t need = split ? 32 * ((p.ept + 9) / 10) : (p.ept + 31) / 32 * 32;
-        p.threads = std::max<uint32_t>(128u, need);
+        const uint32_t lanes = 4 * p.npt;
+        p.nodes = lanes <= kCgClusterMaxThreads ? 1 : (lanes <= 2 * kCgClusterMaxThreads ? 2 : 4);
+        p.threads = (std::max(p.ept, (lanes + p.nodes - 1) / p.nodes) + 31) / 32 * 32;
         p.smem = cg_cluster_smem_bytes(p.ept, p.npt, p.ent_max);
         return p.threads <= kCgClusterMaxThreads && cg_cluster_fits(p);
     };
     CgClusterPlan p{};
-    if (T <= 1440) {
-        const uint32_t want = std::min<uint32_t>(kCgClusterMaxCtas, std::max<uint32_t>(1u, (T + 29) / 30));
-        for (uint32_t C = want; C >= 1; C--)
-            if (try_plan(C, 1, p)) return p;
-    }
-    const uint32_t want = std::min<uint32_t>(kCgClusterMaxCtas, std::max<uint32_t>(1u, (T + 127) / 128));
+    const uint32_t want = T <= 192 ? 1u : std::min<uint32_t>(kCgClusterMaxCtas, (T + 95) / 96);
     for (uint32_t C = want; C >= 1; C--) {
         if ((T + C - 1) / C > kCgClusterMaxThreads) break;  // fewer CTAs only take more
-        if (try_plan(C, 0, p)) return p;
+        if (try_plan(C, p)) return p;
     }
     return CgClusterPlan{};
 }
@@ -1015,7 +1006,7 @@ int fem_solid_create(const double* rest_xyz, uint32_t N, const uint32_t* tets, u
     CKC(s->R.alloc(9 * (size_t)T));
     CKC(s->detF.alloc(T));
     CKC(s->eout.alloc(12 * (size_t)T));
-    CKC(s->Kfx.alloc(kFxGroups * (size_t)T));
+    CKC(s->Kfx.alloc(kFxGroups * (((size_t)T + 31) / 32 * 32)));
     CKC(s->grade.alloc(T));
     CKC(s->csr_ptr.alloc(N + 1));
     CKC(s->csr_idx.alloc(4 * (size_t)T));
