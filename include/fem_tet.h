@@ -268,11 +268,12 @@ int fem_solid_get_params(fem_solid s, fem_params* params);
  * (ILSS_CG.h:38-151 over TetrahedronElementSet3's R K0 R^T products), and
  * so does this solid by default (on = 0). With on = 1 a C_WRP solid keeps
  * K = sum_e R K0 R^T as 3x3 blocks over the node graph, rebuilt at every
- * evaluation, and CG and MINRES take K u from its rows: about 24 FP64 FMAs
- * per tet and iteration against about 140, at the price of 76 B per block
- * (12.6 blocks per node on grid meshes) and one assembly per evaluation;
- * the sums run in another order, so other bits, within the same parity
- * tolerances. Other materials keep the element product, and so does the
+ * evaluation, and CG and MINRES take K u from its rows: about 230 bytes per
+ * tet and iteration against about 580, at the price of 76 B per block (14.1
+ * blocks per node on grid meshes, rows padded to a multiple of four), 628 B
+ * per tet for the assembly and one assembly per evaluation (about five
+ * iterations' time); the sums run in another order, so other bits, within
+ * the same parity tolerances. Other materials keep the element product, and so does the
  * one-cluster CG of solids of at most 8,192 tets. FEM_E_OOM when the blocks
  * do not fit. */
 int fem_solid_set_assembled(fem_solid s, int on);

@@ -126,13 +126,18 @@ struct MeshView {
     const uint32_t* csr_idx;     // [4T]
     const uint8_t* fixed;        // [N]
     S* eout;                     // [12T]
-    // FP64 solid: the assembled stiffness K = sum_e R K0 R^T as 3x3 blocks
-    // (row starts [N+1], columns [nnzb], blocks [nnzb][9] row-major); when
-    // set, the solvers' node kernels take K u from it instead of gathering
-    // the element outputs
+    // FP64 solid: the assembled stiffness K = sum_e R K0 R^T as 3x3 blocks of
+    // fixed-point entries (fx.cuh), rows padded to groups of four blocks: the
+    // groups' row starts [N+1], columns [4 groups] (a pad: the row itself with
+    // a zero block), entries [group][9][4], each row's exponent [N] (units
+    // 2^x); and the vector a product reads, a 32-byte record per node (three
+    // integers in units of 2^(e - 1081), e). When set, the solvers' node
+    // kernels take K u from it instead of gathering the element outputs.
     const uint32_t* bsr_row = nullptr;
     const uint32_t* bsr_col = nullptr;
-    const double* bsr_val = nullptr;
+    const int2* bsr_val = nullptr;
+    const int32_t* bsr_x = nullptr;
+    longlong2* bsr_u = nullptr;  // [2 N]
     // FP64 solid, C_WRP: each element's fixed-point product matrix (fx.cuh),
     // kFxGroups 16-byte groups of two entries, the last group's second half
     // the scale, [T / 32][kFxGroups][32] (a warp's groups at fixed offsets);
@@ -185,10 +190,11 @@ void launch_node_residual_fp64(const MeshView<double>& m, const StepConsts& c, c
 // condition.
 void launch_node_q_fp64(const MeshView<double>& m, const StepConsts& c, const double* d, double* q, double* pq,
                         const StepScalars* st, cudaStream_t s);
-void launch_node_xr_fp64(uint32_t N, double* y, double* r, const double* d, const double* q, const double* pq,
-                         double* pr, StepScalars* st, cudaStream_t s);
-void launch_node_d_fp64(uint32_t N, const uint8_t* fixed, double* d, const double* r, const double* pr,
-                        StepScalars* st, cudaStream_t s, cudaGraphConditionalHandle cond = 0, int set_cond = 0);
+void launch_node_xr_fp64(const MeshView<double>& m, double* y, double* r, const double* d, const double* q,
+                         const double* pq, double* pr, StepScalars* st, cudaStream_t s);
+// (with the assembled stiffness also the records of d)
+void launch_node_d_fp64(const MeshView<double>& m, double* d, const double* r, const double* pr, StepScalars* st,
+                        cudaStream_t s, cudaGraphConditionalHandle cond = 0, int set_cond = 0);
 void launch_integrate_fp64(uint32_t N, double dt, double* x, double* v, const double* y, cudaStream_t s);
 // Fully-implicit Euler (Newton on Delta x) pieces, FP64 solid path.
 void launch_node_b_fie_fp64(const MeshView<double>& m, const StepConsts& c, const double* x, const double* xn,
@@ -214,8 +220,8 @@ void launch_mr_start_fp64(uint32_t N, double* v1, double* v, double* p, double* 
 void launch_mr_q_fp64(const MeshView<double>& m, const StepConsts& c, const double* v, const double* v0,
                       double* v1, double* pq, StepScalars* st, cudaStream_t s);
 // alpha = v1.v ; v1 -= alpha v ; partial |v1|^2
-void launch_mr_v1_fp64(uint32_t N, double* v1, const double* v, const double* pq, double* pr, StepScalars* st,
-                       cudaStream_t s);
+void launch_mr_v1_fp64(const MeshView<double>& m, double* v1, const double* v, const double* pq, double* pr,
+                       StepScalars* st, cudaStream_t s);
 // |v1|^2, the Givens rotation and the loop test, then
 // v1 /= beta_new ; p0 <- (w - r2 p - r3 p0) / r1 (the new p, in p0's buffer) ; y += coef p_new
 void launch_mr_update_fp64(uint32_t N, double* v1, const double* v, const double* p, double* p0, double* y,
@@ -226,6 +232,7 @@ void launch_potential_fp64(const MeshView<double>& m, const StepConsts& c, const
 void launch_apply_A_fp64(const MeshView<double>& m, double factor_M, double factor_K, double mass,
                          const double* d, double* q, cudaStream_t s);
 void launch_gather_sum_fp64(const MeshView<double>& m, double sign, double* f, bool records, cudaStream_t s);
+void launch_rest_rotations_fp64(uint32_t T, double* R, double* detF, cudaStream_t s);
 void launch_rebake_material_fp64(uint32_t T, const double* vol, double k0, double k1, double k2, double* mat,
                                  cudaStream_t s);
 
@@ -241,11 +248,24 @@ enum FinalizeKind {
 void launch_finalize(int kind, const double* partials, uint32_t count, const StepConsts& c, StepScalars* st,
                      cudaStream_t s, cudaGraphConditionalHandle cond = 0, int set_cond = 0);
 
-// The assembled stiffness's blocks (MeshView::bsr_*): block slot s sums, in
-// element order, R K0[li][lj] R^T over its contributions contrib[cptr[s]..
-// cptr[s+1]) = element << 4 | li << 2 | lj.
-void launch_bsr_assemble_fp64(const MeshView<double>& m, uint32_t nnzb, const uint32_t* cptr,
-                              const uint32_t* contrib, double* val, cudaStream_t s);
+// The assembled stiffness (MeshView::bsr_*) of the current rotations. The
+// elements' corner blocks go to eblk ([T][kBsrElemWords], their exponents to
+// ex); block slot s then sums, in element order, its contributions
+// contrib[cptr[s] .. cptr[s+1]) = element << 4 | li << 2 | lj; last the rows
+// are brought to one exponent each and get their diagonal blocks.
+constexpr uint32_t kBsrElemWords = 78;
+struct BsrBuild {
+    uint32_t groups;
+    const uint32_t *cptr, *contrib;
+    long long* eblk;
+    int32_t* ex;
+    int2* val;
+    int32_t* x;
+};
+void launch_bsr_assemble_fp64(const MeshView<double>& m, const BsrBuild& a, cudaStream_t s);
+// The records (bsr_u) of the vector the next product multiplies.
+void launch_bsr_vector_fp64(const MeshView<double>& m, const double* u, const StepScalars* st, int check_done,
+                            cudaStream_t s);
 
 // The whole CG solve of a small C_WRP solid on one thread-block cluster
 // (fem_kernels.cu): CTA r of `ctas` owns the elements [r ept, (r+1) ept) and
@@ -275,14 +295,19 @@ inline uint32_t elem_block(uint32_t T) { return T <= 32 * kSubPartitions ? 32u :
 inline uint32_t capped(uint32_t g, uint32_t cap) { return g < 1 ? 1 : (g > cap ? cap : g); }
 inline uint32_t elem_grid(uint32_t T) { return capped((T + elem_block(T) - 1) / elem_block(T), 4096u); }
 // Node kernels (four lanes per node) and vector kernels (one per component):
-// 128 threads until every SM has two blocks, then 512; at most three blocks
-// per SM, so that the block that ends a reduction adds at most one partial
-// per thread.
+// 128 threads until every SM has two blocks, then 512 (the assembled rows'
+// kernels, which hold more registers, 256); at most three, two or four blocks
+// per SM, so that a block adds few of the previous kernel's partials per
+// thread.
 inline uint32_t row_block(uint32_t n) { return n <= 304u * 128u ? 128u : 512u; }
-inline uint32_t row_grid(uint32_t n) { return capped((n + row_block(n) - 1) / row_block(n), 456u); }
+inline uint32_t vec_grid(uint32_t n) { return capped((n + row_block(n) - 1) / row_block(n), 304u); }
 inline uint32_t node_rows(uint32_t N) { return 4u * (N < (1u << 29) ? N : (1u << 29)); }
-inline uint32_t node_grid(uint32_t N) { return row_grid(node_rows(N)); }
-inline uint32_t vec_grid(uint32_t n) { return row_grid(n); }
+inline uint32_t node_block(uint32_t N, bool bsr) { return bsr ? (row_block(node_rows(N)) == 128u ? 128u : 256u) : row_block(node_rows(N)); }
+inline uint32_t node_grid(uint32_t N, bool bsr)
+{
+    const uint32_t b = node_block(N, bsr);
+    return capped((node_rows(N) + b - 1) / b, bsr ? 608u : 456u);
+}
 uint64_t& launch_counter();       // kernels launched by this library
 
 // Optional per-kernel timing with CUDA events recorded on the launching

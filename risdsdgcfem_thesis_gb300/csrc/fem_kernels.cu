@@ -254,7 +254,8 @@ __global__ void __launch_bounds__(128, 3) k_elem_bake_fp64(MeshView<double> m)
         load_elem(m, e, R, Di, k1, knu, k2);
         FxL even{0, 0};
         int4* Kp = fx_matrix(m.Kfx, e);
-        auto put = [&](int k, FxL v) {  // two entries per 16-byte group
+        auto put = [&](int k, int64_t w) {  // two entries per 16-byte group
+            const FxL v = fx_split(w);
             if ((k & 1) == 0) even = v;
             else Kp[32 * (k >> 1)] = make_int4(even.l, even.h, v.l, v.h);
         };
@@ -463,96 +464,285 @@ __device__ __forceinline__ double fx_quad_sum(const FxSum* s, uint32_t a, int32_
 // all three components (integer sums in block exponents, fx.cuh).
 __device__ __forceinline__ double gather_fx(const MeshView<double>& m, uint32_t n, uint32_t a, bool on)
 {
+    constexpr int kBatch = 3;  // records in flight per lane
     const int32_t guard = (int32_t)m.fx_guard;
     FxSum s[3] = {{0, 0}, {0, 0}, {0, 0}};
     if (on) {
         const uint32_t beg = m.csr_ptr[n], end = m.csr_ptr[n + 1];
         const long long* rec = reinterpret_cast<const long long*>(m.eout);
-#pragma unroll 2
-        for (uint32_t j = beg + a; j < end; j += 4) {
-            const long long* r = rec + 3 * (size_t)bounds_idx(m.csr_idx[j], 4ull * m.T, kSiteCsrEntry);
-            const int64_t v0 = r[0], v1 = r[1], v2 = r[2];
-            const int32_t x = fx_record_exp(v0, v1, v2);
-            fx_add(s[0], v0, x, guard);
-            fx_add(s[1], v1, x, guard);
-            fx_add(s[2], v2, x, guard);
+        for (uint32_t j = beg + a; j < end; j += 4 * kBatch) {
+            int64_t v[kBatch][3];
+#pragma unroll
+            for (int k = 0; k < kBatch; k++) {
+                v[k][0] = v[k][1] = v[k][2] = 0;  // an empty record: the lowest exponent
+                if (j + 4 * k < end) {
+                    const long long* r = rec + 3 * (size_t)bounds_idx(m.csr_idx[j + 4 * k], 4ull * m.T, kSiteCsrEntry);
+                    v[k][0] = r[0];
+                    v[k][1] = r[1];
+                    v[k][2] = r[2];
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < kBatch; k++) {
+                const int32_t x = fx_record_exp(v[k][0], v[k][1], v[k][2]);
+                fx_add(s[0], v[k][0], x, guard);
+                fx_add(s[1], v[k][1], x, guard);
+                fx_add(s[2], v[k][2], x, guard);
+            }
         }
     }
     return fx_quad_sum(s, a, guard);
 }
 
-// K u at node n for the solvers' node kernels: the assembled row when the
-// solid has one (3 FMAs per block and lane), else the sum of the element
-// outputs of the product launched before.
-__device__ __forceinline__ double node_Ku(const MeshView<double>& m, const double* __restrict__ u, uint32_t n,
-                                          uint32_t a, bool on)
+// The assembled row times the vector's records: lane l takes the blocks l,
+// l + 4, ...; the vector's entries are brought to the largest exponent among
+// the row's columns. The first four groups' records (rows of up to 16 blocks
+// whole) are loaded once, ahead of everything that waits for them. A block's
+// nine products keep mid below 3 (2^28 + 2^27) 2^31 + 2^32; the row's exponent
+// holds bits free for its length.
+__device__ __forceinline__ double bsr_row_fx(const MeshView<double>& m, uint32_t n, uint32_t a, bool on)
 {
-    if (m.bsr_val) {
-        double s = 0.0;
-        if (!on || a == 3) return s;
-        const uint32_t beg = m.bsr_row[n], end = m.bsr_row[n + 1];
-#pragma unroll 2
-        for (uint32_t k = beg; k < end; k++) {
-            const size_t j = 3 * (size_t)bounds_idx(m.bsr_col[k], m.N, kSiteBsrEntry);
-            const double* A = m.bsr_val + 9 * (size_t)k + 3 * a;
-            s = fma(A[0], u[j], s);
-            s = fma(A[1], u[j + 1], s);
-            s = fma(A[2], u[j + 2], s);
-        }
-        return s;
-    }
-    return m.Kfx ? gather_fx(m, n, a, on) : gather_fp64(m, n, a, on);
-}
-
-// One block of the assembled stiffness per thread (see
-// launch_bsr_assemble_fp64). The element block in the element frame, from
-// the strain form of elem_RKRt (g_i the shape gradients: rows of Dm^-1,
-// node 0 minus their sum; k1 = V(lambda + 2 mu), knu = V lambda, k2 = V mu):
-// K0[a][a] = k1 gi_a gj_a + k2 (gi.gj - gi_a gj_a),
-// K0[a][b] = knu gi_a gj_b + k2 gj_a gi_b (a != b); the world block R K0 R^T.
-__global__ void k_bsr_assemble_fp64(MeshView<double> m, uint32_t nnzb, const uint32_t* __restrict__ cptr,
-                                    const uint32_t* __restrict__ contrib, double* __restrict__ val)
-{
-    for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < nnzb; s += gridDim.x * blockDim.x) {
-        double acc[9];
+    constexpr int kHeld = 4;
+    const uint32_t beg = on ? m.bsr_row[n] : 0u, end = on ? m.bsr_row[n + 1] : 0u;
+    const int32_t xr = on ? m.bsr_x[n] : 0;
+    auto column = [&](uint32_t g) { return (size_t)bounds_idx(m.bsr_col[4 * (size_t)g + a], m.N, kSiteBsrEntry); };
+    longlong2 u01[kHeld], u2e[kHeld];
+    int32_t E = 0;
 #pragma unroll
-        for (int k = 0; k < 9; k++) acc[k] = 0.0;
-        for (uint32_t k = cptr[s]; k < cptr[s + 1]; k++) {
-            const uint32_t cb = contrib[k], e = bounds_idx(cb >> 4, m.T, kSiteBsrEntry);
-            const uint32_t li = (cb >> 2) & 3u, lj = cb & 3u;
-            double R[9], Di[9], k1, knu, k2;
-            load_elem(m, e, R, Di, k1, knu, k2);
-            double gi[3], gj[3];
+    for (int h = 0; h < kHeld; h++) {
+        u01[h] = u2e[h] = make_longlong2(0, 0);
+        if (beg + h < end) {
+            const size_t j = column(beg + h);
+            u01[h] = m.bsr_u[2 * j];
+            u2e[h] = m.bsr_u[2 * j + 1];
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < kHeld; h++) E = max(E, (int32_t)u2e[h].y);
+    for (uint32_t g = beg + kHeld; g < end; g++) E = max(E, (int32_t)m.bsr_u[2 * column(g) + 1].y);
+    E = max(E, __shfl_xor_sync(0xffffffffu, E, 1));
+    E = max(E, __shfl_xor_sync(0xffffffffu, E, 2));
+    int64_t hi[3] = {0, 0, 0}, mid[3] = {0, 0, 0};
+    auto block = [&](uint32_t g, const longlong2& v01, const longlong2& v2e) {
+        const int32_t sh = fx_min63(E - (int32_t)v2e.y);
+        const FxL u[3] = {fx_split(v01.x >> sh), fx_split(v01.y >> sh), fx_split(v2e.x >> sh)};
+        const int2* A = m.bsr_val + 36 * (size_t)g + a;
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
 #pragma unroll
             for (int c = 0; c < 3; c++) {
-                const double g0 = -(Di[c] + Di[3 + c] + Di[6 + c]);
-                gi[c] = li == 0 ? g0 : (li == 1 ? Di[c] : (li == 2 ? Di[3 + c] : Di[6 + c]));
-                gj[c] = lj == 0 ? g0 : (lj == 1 ? Di[c] : (lj == 2 ? Di[3 + c] : Di[6 + c]));
+                const int2 k = A[4 * (3 * r + c)];
+                fx_mac(hi[r], mid[r], FxL{k.x, k.y}, u[c]);
             }
-            const double dot = gi[0] * gj[0] + gi[1] * gj[1] + gi[2] * gj[2];
-            double K0[9];
-#pragma unroll
-            for (int a = 0; a < 3; a++)
-#pragma unroll
-                for (int b = 0; b < 3; b++) {
-                    const double p = gi[a] * gj[b];
-                    K0[3 * a + b] = a == b ? k1 * p + k2 * (dot - p) : knu * p + k2 * gj[a] * gi[b];
-                }
-            double T1[9];  // R K0
-#pragma unroll
-            for (int a = 0; a < 3; a++)
-#pragma unroll
-                for (int b = 0; b < 3; b++)
-                    T1[3 * a + b] = R[3 * a] * K0[b] + R[3 * a + 1] * K0[3 + b] + R[3 * a + 2] * K0[6 + b];
-#pragma unroll
-            for (int a = 0; a < 3; a++)
-#pragma unroll
-                for (int b = 0; b < 3; b++)
-                    acc[3 * a + b] += T1[3 * a] * R[3 * b] + T1[3 * a + 1] * R[3 * b + 1] + T1[3 * a + 2] * R[3 * b + 2];
+            hi[r] += mid[r] >> 32;
+            mid[r] &= 0xffffffffll;
         }
-        double* o = val + 9 * (size_t)s;
+    };
 #pragma unroll
-        for (int k = 0; k < 9; k++) o[k] = acc[k];
+    for (int h = 0; h < kHeld; h++)
+        if (beg + h < end) block(beg + h, u01[h], u2e[h]);
+    for (uint32_t g = beg + kHeld; g < end; g++) {
+        const size_t j = column(g);
+        block(g, m.bsr_u[2 * j], m.bsr_u[2 * j + 1]);
+    }
+    int64_t t = 0;
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+        long long v = fx_fin<4>(hi[r], mid[r]) >> 2;
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        if ((int)a == r) t = v;
+    }
+    if (E == 2047 || xr == kFxFp64) return fx_from_bits(0x7ff8000000000000ull);
+    return a == 3 ? 0.0 : fx_to_double(t, xr + (E - 1081) + 62);
+}
+
+// A node's record: its components in units of its own largest.
+__device__ __forceinline__ void bsr_record(const MeshView<double>& m, uint32_t n, double v0, double v1, double v2)
+{
+    const int32_t E = max(fx_exp(v0), max(fx_exp(v1), fx_exp(v2)));
+    m.bsr_u[2 * (size_t)n] = make_longlong2(fx_align<59>(v0, E), fx_align<59>(v1, E));
+    m.bsr_u[2 * (size_t)n + 1] = make_longlong2(fx_align<59>(v2, E), E);
+}
+__global__ void k_bsr_vector_fp64(MeshView<double> m, const double* __restrict__ u, const StepScalars* st,
+                                  int check_done)
+{
+    if (check_done && st->done_pend) return;
+    for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < m.N; n += gridDim.x * blockDim.x)
+        bsr_record(m, n, u[3 * (size_t)n], u[3 * (size_t)n + 1], u[3 * (size_t)n + 2]);
+}
+
+// K u at node n for the solvers' node kernels: the assembled row when the
+// solid has one, else the sum of the element outputs of the product launched
+// before.
+enum NodeKu { kKuRecords = 0, kKuFp64 = 1, kKuBsr = 2 };
+template <int kKu>
+__device__ __forceinline__ double node_Ku(const MeshView<double>& m, uint32_t n, uint32_t a, bool on)
+{
+    if constexpr (kKu == kKuBsr) return bsr_row_fx(m, n, a, on);
+    else if constexpr (kKu == kKuRecords) return gather_fx(m, n, a, on);
+    else return gather_fp64(m, n, a, on);
+}
+
+// An element fx.cuh leaves out: K9 / 2 from FP64 (V (lambda m_i m_j^T +
+// mu m_j m_i^T + mu (g_i . g_j) R R^T), m = R g) in the block words; returns
+// the units' exponent, kFxFp64 when an entry is not finite.
+__device__ __noinline__ int32_t elem_blocks_fp64(const double* Rp, const double* Dp, double kl, double km, size_t T, int64_t* w)
+{
+    double R[9], g[9], mm[9], C[9], K[45];
+    for (int c = 0; c < 9; c++) {
+        R[c] = Rp[c * T];
+        g[c] = Dp[c * T];
+    }
+    for (int i = 0; i < 3; i++)
+        for (int a = 0; a < 3; a++) {
+            mm[3 * i + a] = R[3 * a] * g[3 * i] + R[3 * a + 1] * g[3 * i + 1] + R[3 * a + 2] * g[3 * i + 2];
+            C[3 * i + a] = R[3 * i] * R[3 * a] + R[3 * i + 1] * R[3 * a + 1] + R[3 * i + 2] * R[3 * a + 2];
+        }
+    int32_t E = 0;
+    for (int r = 0; r < 9; r++)
+        for (int c = r; c < 9; c++) {
+            const int i = r / 3, a = r % 3, j = c / 3, b = c % 3;
+            const double G = g[3 * i] * g[3 * j] + g[3 * i + 1] * g[3 * j + 1] + g[3 * i + 2] * g[3 * j + 2];
+            const double v = kl * mm[3 * i + a] * mm[3 * j + b] + km * mm[3 * j + a] * mm[3 * i + b] + km * G * C[3 * a + b];
+            K[fx_at(r, c)] = v;
+            E = max(E, fx_exp(v));
+        }
+    for (int r = 0; r < 9; r++)
+        for (int c = r; c < 9; c++) {
+            const int i = r / 3 + 1, j = c / 3 + 1;
+            if (E < 2047) w[fx_block_word(i, j, r % 3, c % 3)] = fx_align<59>(K[fx_at(r, c)], E);
+        }
+    return E < 2047 ? E - 1022 - 59 : kFxFp64;
+}
+
+// The elements' corner blocks: one element per thread, its words staged in
+// shared memory (rows of an odd number of words) and written out in whole
+// lines. Bound by the integer products of fx_bake and by the writes (632
+// bytes per element).
+constexpr int kBsrElemBlock = 64, kBsrElemRow = 79;
+__global__ void __launch_bounds__(kBsrElemBlock) k_bsr_elements_fp64(MeshView<double> m, BsrBuild a)
+{
+    extern __shared__ long long el_smem[];
+    int64_t* w = reinterpret_cast<int64_t*>(el_smem) + kBsrElemRow * threadIdx.x;
+    for (uint32_t e0 = blockIdx.x * kBsrElemBlock; e0 < m.T; e0 += gridDim.x * kBsrElemBlock) {
+        const uint32_t e = e0 + threadIdx.x;
+        if (e < m.T) {
+            double R[9], Di[9], k1, knu, k2;
+            load_elem(m, e, R, Di, k1, knu, k2);
+            int32_t scale = kFxFp64;
+            if (fx_grade_ok(m.grade[e], knu, k2)) {
+                int r = 0, c = 0;
+                scale = fx_bake(R, Di, knu, k2, [&](int, int64_t v) {
+                    w[fx_block_word(r / 3 + 1, c / 3 + 1, r % 3, c % 3)] = v >> 1;
+                    if (++c == 9) c = ++r;
+                });
+            }
+            scale = scale != kFxFp64 ? scale + 1 : elem_blocks_fp64(m.R + e, m.Dinv + e, knu, k2, m.T, w);
+            fx_node0_blocks(w);
+            a.ex[e] = scale;
+        }
+        __syncthreads();
+        const uint32_t words = kBsrElemWords * min((uint32_t)kBsrElemBlock, m.T - e0);
+        for (uint32_t i = threadIdx.x; i < words; i += kBsrElemBlock)
+            a.eblk[kBsrElemWords * (size_t)e0 + i] = el_smem[kBsrElemRow * (i / kBsrElemWords) + i % kBsrElemWords];
+        __syncthreads();
+    }
+}
+
+// One block slot per thread: the contributions at the largest exponent among
+// them, added exactly, as nine doubles in the slot's entries (the rows' kernel
+// converts them in place). Diagonal blocks have four times the contributions
+// of the others; they come from the row instead.
+__global__ void __launch_bounds__(128) k_bsr_slots_fp64(MeshView<double> m, BsrBuild b)
+{
+    const uint32_t count = 4 * b.groups;
+    double* val = reinterpret_cast<double*>(b.val);
+    for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < count; s += gridDim.x * blockDim.x) {
+        const uint32_t beg = b.cptr[s], end = b.cptr[s + 1];
+        int32_t X = INT32_MIN;
+        for (uint32_t k = beg; k < end; k++) X = max(X, b.ex[bounds_idx(b.contrib[k] >> 4, m.T, kSiteBsrEntry)]);
+        FxWide acc[9];
+#pragma unroll
+        for (int c = 0; c < 9; c++) acc[c] = FxWide{0, 0};
+        for (uint32_t k = beg; k < end; k++) {
+            const uint32_t cb = b.contrib[k], e = bounds_idx(cb >> 4, m.T, kSiteBsrEntry);
+            const uint32_t li = (cb >> 2) & 3u, lj = cb & 3u, p = min(li, lj), q = max(li, lj);
+            const int32_t sh = fx_min63(X - b.ex[e]);
+            const long long* w = b.eblk + kBsrElemWords * (size_t)e + fx_block(p, q);
+            int64_t v[9];
+#pragma unroll
+            for (int c = 0; c < 9; c++) v[c] = w[c] >> sh;
+#pragma unroll
+            for (int r = 0; r < 3; r++)
+#pragma unroll
+                for (int c = 0; c < 3; c++) fx_wide_add(acc[3 * r + c], li < lj ? v[3 * r + c] : v[3 * c + r]);
+        }
+        double* o = val + 36 * (size_t)(s >> 2) + (s & 3u);
+#pragma unroll
+        for (int c = 0; c < 9; c++)
+            o[4 * c] = beg == end ? 0.0
+                                  : (X == kFxFp64 ? fx_from_bits(0x7ff8000000000000ull) : fx_wide_value(acc[c], X));
+    }
+}
+
+// Each row to one exponent, in place, and its diagonal block as minus the sum
+// of the others (an element's blocks sum to zero along a row), exactly as the
+// row now holds them: rigid translations have no force. Entries below 2^60,
+// less a bit per doubling of the row beyond 16 blocks (the product's
+// headroom).
+__global__ void k_bsr_rows_fp64(MeshView<double> m, BsrBuild b)
+{
+    const uint32_t a = threadIdx.x & 3u, step = (gridDim.x * blockDim.x) >> 2;
+    const double* val = reinterpret_cast<const double*>(b.val);
+    for (uint32_t n = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; (n & ~7u) < m.N; n += step) {
+        const bool on = n < m.N;
+        const uint32_t beg = on ? m.bsr_row[n] : 0u, end = on ? m.bsr_row[n + 1] : 0u;
+        int32_t E = 0;
+        uint32_t diag = 0xffffffffu;  // the first slot of column n (pads follow it)
+        for (uint32_t g = beg; g < end; g++) {
+            if (m.bsr_col[4 * (size_t)g + a] == n) diag = min(diag, 4 * g + a);
+#pragma unroll
+            for (int k = 0; k < 9; k++) E = max(E, fx_exp(val[36 * (size_t)g + 4 * k + a]));
+        }
+        int32_t room = 0, guard = 0;  // bits for the diagonal's sum, and for the product
+        while ((2u << room) < end - beg) room++;
+        while ((4u << guard) < end - beg) guard++;
+#pragma unroll
+        for (int o = 1; o <= 2; o <<= 1) {
+            E = max(E, __shfl_xor_sync(0xffffffffu, E, o));
+            diag = min(diag, __shfl_xor_sync(0xffffffffu, diag, o));
+        }
+        long long sum[9];
+#pragma unroll
+        for (int k = 0; k < 9; k++) sum[k] = 0;
+        uint64_t top = 1;
+        for (uint32_t g = beg; g < end; g++)
+#pragma unroll
+            for (int k = 0; k < 9; k++) {
+                const int64_t v = fx_align<60>(val[36 * (size_t)g + 4 * k + a], E) >> room;
+                sum[k] += v;
+                top |= fx_mag(v);
+            }
+#pragma unroll
+        for (int k = 0; k < 9; k++) {
+            sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], 1);
+            sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], 2);
+            top |= fx_mag(sum[k]);
+        }
+        uint32_t bits = 64 - fx_clz(top);
+        bits = max(bits, __shfl_xor_sync(0xffffffffu, bits, 1));
+        bits = max(bits, __shfl_xor_sync(0xffffffffu, bits, 2));
+        const int32_t down = max(0, (int32_t)bits - (60 - guard));
+        for (uint32_t g = beg; g < end; g++)
+#pragma unroll
+            for (int k = 0; k < 9; k++) {
+                const size_t i = 36 * (size_t)g + 4 * k + a;
+                const int64_t v = 4 * g + a == diag ? -sum[k] : fx_align<60>(val[i], E) >> room;
+                const FxL l = fx_split(v >> down);
+                b.val[i] = make_int2(l.l, l.h);
+            }
+        if (on && a == 0) b.x[n] = E < 2047 ? E - 1082 + room + down : kFxFp64;
     }
 }
 
@@ -594,6 +784,7 @@ __global__ void k_knc_fp64(uint32_t N, uint32_t count, const uint32_t* __restric
 }
 
 // r = S (b - A y) ; d = r ; partial |r|^2   (ILSS_CG.h:53-64)
+template <int kKu>
 __global__ void k_node_residual_fp64(MeshView<double> m, StepConsts c, const double* __restrict__ b,
                                      const double* __restrict__ y, double* r, double* d, double* partials)
 {
@@ -602,7 +793,7 @@ __global__ void k_node_residual_fp64(MeshView<double> m, StepConsts c, const dou
     const uint32_t a = threadIdx.x & 3u, step = (gridDim.x * blockDim.x) >> 2;
     for (uint32_t n = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; (n & ~7u) < m.N; n += step) {
         const bool on = n < m.N;
-        const double s = node_Ku(m, y, n, a, on);
+        const double s = node_Ku<kKu>(m, n, a, on);
         if (!on || a == 3) continue;
         const size_t i = 3 * (size_t)n + a;
         const double ri = m.fixed[n] ? 0.0 : b[i] - (c.factor_K * s + mfm * y[i]);
@@ -615,6 +806,7 @@ __global__ void k_node_residual_fp64(MeshView<double> m, StepConsts c, const dou
 }
 
 // q = S A d ; partial d.q   (ILSS_CG.h:90-96)
+template <int kKu>
 __global__ void k_node_q_fp64(MeshView<double> m, StepConsts c, const double* __restrict__ d, double* q, double* pq,
                               const StepScalars* st)
 {
@@ -624,7 +816,7 @@ __global__ void k_node_q_fp64(MeshView<double> m, StepConsts c, const double* __
     const uint32_t a = threadIdx.x & 3u, step = (gridDim.x * blockDim.x) >> 2;
     for (uint32_t n = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; (n & ~7u) < m.N; n += step) {
         const bool on = n < m.N;
-        const double s = node_Ku(m, d, n, a, on);
+        const double s = node_Ku<kKu>(m, n, a, on);
         if (!on || a == 3) continue;
         const size_t i = 3 * (size_t)n + a;
         const double di = d[i], qi = m.fixed[n] ? 0.0 : c.factor_K * s + mfm * di;
@@ -646,6 +838,14 @@ __global__ void k_node_xr_fp64(uint32_t N, double* y, double* r, const double* _
         if (blockIdx.x == 0 && threadIdx.x == 0) st->done = 1;
         return;
     }
+    const uint32_t n3 = 3 * N, i0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    double y0 = 0.0, r0 = 0.0, d0 = 0.0, q0 = 0.0;  // the first component, loaded ahead of alpha
+    if (i0 < n3) {
+        y0 = y[i0];
+        r0 = r[i0];
+        d0 = d[i0];
+        q0 = q[i0];
+    }
     __shared__ double sh_alpha;
     const double dq = grid_total(pq, npq), delta = st->delta_pend;
     const bool brk = ::fabs(dq) < st->abs_eps_sq;  // breakdown: leave before the update (ILSS_CG.h:97)
@@ -662,12 +862,18 @@ __global__ void k_node_xr_fp64(uint32_t N, double* y, double* r, const double* _
     __syncthreads();
     const double alpha = sh_alpha, na = -alpha;
     double acc = 0.0;
-    const uint32_t n3 = 3 * N;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n3; i += gridDim.x * blockDim.x) {
-        y[i] += alpha * d[i];
-        double ri = r[i] + na * q[i];
+    for (uint32_t i = i0; i < n3;) {
+        y[i] = y0 + alpha * d0;
+        const double ri = r0 + na * q0;
         r[i] = ri;
         acc += ri * ri;
+        i += step;
+        if (i < n3) {
+            y0 = y[i];
+            r0 = r[i];
+            d0 = d[i];
+            q0 = q[i];
+        }
     }
     const double total = block_sum(acc);
     if (threadIdx.x == 0) pr[blockIdx.x] = total;
@@ -675,7 +881,8 @@ __global__ void k_node_xr_fp64(uint32_t N, double* y, double* r, const double* _
 
 // beta = |r_new|^2 / |r|^2 and the loop test ; d = S (beta d + r)
 // (ILSS_CG.h:117-137)
-__global__ void k_node_d_fp64(uint32_t N, const uint8_t* __restrict__ fixed, double* d, const double* __restrict__ r,
+template <bool kBsr>
+__global__ void k_node_d_fp64(MeshView<double> m, double* d, const double* __restrict__ r,
                               const double* __restrict__ pr, uint32_t npr, StepScalars* st,
                               cudaGraphConditionalHandle cond, int set_cond)
 {
@@ -687,6 +894,20 @@ __global__ void k_node_d_fp64(uint32_t N, const uint8_t* __restrict__ fixed, dou
         }
         return;
     }
+    // one component per thread, or (kBsr) one node; the first loaded ahead of beta
+    constexpr int kW = kBsr ? 3 : 1;
+    const uint32_t count = kBsr ? m.N : 3 * m.N, i0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    double d0[kW], r0[kW];
+    bool f0 = false;
+    auto load = [&](uint32_t i) {
+#pragma unroll
+        for (int k = 0; k < kW; k++) {
+            d0[k] = d[kW * (size_t)i + k];
+            r0[k] = r[kW * (size_t)i + k];
+        }
+        f0 = m.fixed[kBsr ? i : i / 3];
+    };
+    if (i0 < count) load(i0);
     __shared__ double sh_beta;
     const double total = grid_total(pr, npr);
     if (threadIdx.x == 0) {
@@ -705,10 +926,13 @@ __global__ void k_node_d_fp64(uint32_t N, const uint8_t* __restrict__ fixed, dou
     }
     __syncthreads();
     const double beta = sh_beta;
-    const uint32_t n3 = 3 * N;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n3; i += gridDim.x * blockDim.x) {
-        const uint32_t n = i / 3;
-        d[i] = fixed[n] ? 0.0 : beta * d[i] + r[i];
+    for (uint32_t i = i0; i < count;) {
+        double v[kW];
+#pragma unroll
+        for (int k = 0; k < kW; k++) d[kW * (size_t)i + k] = v[k] = f0 ? 0.0 : beta * d0[k] + r0[k];
+        if constexpr (kBsr) bsr_record(m, i, v[0], v[1], v[2]);
+        i += step;
+        if (i < count) load(i);
     }
 }
 
@@ -795,6 +1019,7 @@ __global__ void k_fie_update_fp64(uint32_t N, double inv_dt, double* x, double* 
 // iterations; every kernel is a no-op once the loop has ended.
 
 // v1 = S (b - A y) ; partial |v1|^2   (:66-74)
+template <int kKu>
 __global__ void k_mr_init_fp64(MeshView<double> m, StepConsts c, const double* __restrict__ b,
                                const double* __restrict__ y, double* v1, double* partials)
 {
@@ -803,7 +1028,7 @@ __global__ void k_mr_init_fp64(MeshView<double> m, StepConsts c, const double* _
     const uint32_t a = threadIdx.x & 3u, step = (gridDim.x * blockDim.x) >> 2;
     for (uint32_t n = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; (n & ~7u) < m.N; n += step) {
         const bool on = n < m.N;
-        const double f = node_Ku(m, y, n, a, on);
+        const double f = node_Ku<kKu>(m, n, a, on);
         if (!on || a == 3) continue;
         const size_t i = 3 * (size_t)n + a;
         const double r = m.fixed[n] ? 0.0 : b[i] - (c.factor_K * f + mfm * y[i]);
@@ -828,6 +1053,7 @@ __global__ void k_mr_start_fp64(uint32_t N, double* v1, double* v, double* p, do
 }
 
 // v1 = S A v - beta v0 ; partial v1.v   (:117-123)
+template <int kKu>
 __global__ void k_mr_q_fp64(MeshView<double> m, StepConsts c, const double* __restrict__ v,
                             const double* __restrict__ v0, double* v1, double* pq, StepScalars* st)
 {
@@ -847,7 +1073,7 @@ __global__ void k_mr_q_fp64(MeshView<double> m, StepConsts c, const double* __re
     const uint32_t a = threadIdx.x & 3u, step = (gridDim.x * blockDim.x) >> 2;
     for (uint32_t n = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; (n & ~7u) < m.N; n += step) {
         const bool on = n < m.N;
-        const double f = node_Ku(m, v, n, a, on);
+        const double f = node_Ku<kKu>(m, n, a, on);
         if (!on || a == 3) continue;
         const size_t i = 3 * (size_t)n + a;
         const double vi = v[i], qi = m.fixed[n] ? 0.0 : c.factor_K * f + mfm * vi;
@@ -947,6 +1173,23 @@ __global__ void k_rebake_material_fp64(uint32_t T, const double* __restrict__ vo
         mat[(size_t)T + e] = V * k1;
         mat[2 * (size_t)T + e] = V * k2;
     }
+}
+
+// R = I, det F = 1 until the first evaluation (CreateCache,
+// TetrahedronElementSet3.cpp:190-209).
+__global__ void k_rest_rotations_fp64(uint32_t T, double* R, double* detF)
+{
+    for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < T; e += gridDim.x * blockDim.x) {
+#pragma unroll
+        for (int c = 0; c < 9; c++) R[c * (size_t)T + e] = c % 4 == 0 ? 1.0 : 0.0;
+        detF[e] = 1.0;
+    }
+}
+
+void launch_rest_rotations_fp64(uint32_t T, double* R, double* detF, cudaStream_t s)
+{
+    k_rest_rotations_fp64<<<vec_grid(T), row_block(T), 0, s>>>(T, R, detF);
+    launch_counter()++;
 }
 
 void launch_rebake_material_fp64(uint32_t T, const double* vol, double k0, double k1, double k2, double* mat,
@@ -1331,6 +1574,16 @@ cudaError_t launch_cg_cluster_fp64(const MeshView<double>& m, const StepConsts& 
 
 // ---- launchers ----
 
+// A node kernel in the form of the solid's operator (MeshView).
+#define FEMGB_LAUNCH_KU(kernel, m, ...)                                                                              \
+    do {                                                                                                             \
+        const bool bsr_ = (m).bsr_val != nullptr;                                                                    \
+        const uint32_t g_ = node_grid((m).N, bsr_), b_ = node_block((m).N, bsr_);                                    \
+        if (bsr_) kernel<kKuBsr><<<g_, b_, 0, s>>>(m, __VA_ARGS__);                                                  \
+        else if ((m).Kfx) kernel<kKuRecords><<<g_, b_, 0, s>>>(m, __VA_ARGS__);                                      \
+        else kernel<kKuFp64><<<g_, b_, 0, s>>>(m, __VA_ARGS__);                                                      \
+        launch_counter()++;                                                                                          \
+    } while (0)
 #define FEMGB_LAUNCH(kernel, grid, block, ...)                            \
     do {                                                                  \
         kernel<<<(grid), (block), 0, s>>>(__VA_ARGS__);                   \
@@ -1356,7 +1609,7 @@ void launch_elem_force_fp64(const MeshView<double>& m, const double* x, int writ
 void launch_node_b_fp64(const MeshView<double>& m, const StepConsts& c, const double* v, double* b, double* y,
                         cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_node_b_fp64, node_grid(m.N), row_block(node_rows(m.N)), m, c, v, b, y);
+    FEMGB_LAUNCH(k_node_b_fp64, node_grid(m.N, false), node_block(m.N, false), m, c, v, b, y);
 }
 void launch_knc_fp64(uint32_t N, uint32_t count, const uint32_t* nodes, const double* targets, const double* x,
                      const StepConsts& c, double* b, double* y, cudaStream_t s)
@@ -1367,25 +1620,29 @@ void launch_knc_fp64(uint32_t N, uint32_t count, const uint32_t* nodes, const do
 void launch_node_residual_fp64(const MeshView<double>& m, const StepConsts& c, const double* b, const double* y,
                                double* r, double* d, double* partials, cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_node_residual_fp64, node_grid(m.N), row_block(node_rows(m.N)), m, c, b, y, r, d, partials);
+    FEMGB_LAUNCH_KU(k_node_residual_fp64, m, c, b, y, r, d, partials);
 }
 void launch_node_q_fp64(const MeshView<double>& m, const StepConsts& c, const double* d, double* q, double* pq,
                         const StepScalars* st, cudaStream_t s)
 {
     prof_begin("node_q_fp64", s);
-    FEMGB_LAUNCH(k_node_q_fp64, node_grid(m.N), row_block(node_rows(m.N)), m, c, d, q, pq, st);
+    FEMGB_LAUNCH_KU(k_node_q_fp64, m, c, d, q, pq, st);
     prof_end("node_q_fp64", s);
 }
-void launch_node_xr_fp64(uint32_t N, double* y, double* r, const double* d, const double* q, const double* pq,
-                         double* pr, StepScalars* st, cudaStream_t s)
+void launch_node_xr_fp64(const MeshView<double>& m, double* y, double* r, const double* d, const double* q,
+                         const double* pq, double* pr, StepScalars* st, cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_node_xr_fp64, vec_grid(3 * N), row_block(3 * N), N, y, r, d, q, pq, node_grid(N), pr, st);
+    FEMGB_LAUNCH(k_node_xr_fp64, vec_grid(3 * m.N), row_block(3 * m.N), m.N, y, r, d, q, pq,
+                 node_grid(m.N, m.bsr_val != nullptr), pr, st);
 }
-void launch_node_d_fp64(uint32_t N, const uint8_t* fixed, double* d, const double* r, const double* pr,
-                        StepScalars* st, cudaStream_t s, cudaGraphConditionalHandle cond, int set_cond)
+void launch_node_d_fp64(const MeshView<double>& m, double* d, const double* r, const double* pr, StepScalars* st,
+                        cudaStream_t s, cudaGraphConditionalHandle cond, int set_cond)
 {
-    FEMGB_LAUNCH(k_node_d_fp64, vec_grid(3 * N), row_block(3 * N), N, fixed, d, r, pr, vec_grid(3 * N), st, cond,
-                 set_cond);
+    const uint32_t npr = vec_grid(3 * m.N);
+    if (m.bsr_val)
+        FEMGB_LAUNCH(k_node_d_fp64<true>, vec_grid(m.N), row_block(m.N), m, d, r, pr, npr, st, cond, set_cond);
+    else
+        FEMGB_LAUNCH(k_node_d_fp64<false>, npr, row_block(3 * m.N), m, d, r, pr, npr, st, cond, set_cond);
 }
 void launch_integrate_fp64(uint32_t N, double dt, double* x, double* v, const double* y, cudaStream_t s)
 {
@@ -1394,7 +1651,7 @@ void launch_integrate_fp64(uint32_t N, double dt, double* x, double* v, const do
 void launch_node_b_fie_fp64(const MeshView<double>& m, const StepConsts& c, const double* x, const double* xn,
                             const double* vn, int warm, double* b, double* y, cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_node_b_fie_fp64, node_grid(m.N), row_block(node_rows(m.N)), m, c, x, xn, vn, warm, b, y);
+    FEMGB_LAUNCH(k_node_b_fie_fp64, node_grid(m.N, false), node_block(m.N, false), m, c, x, xn, vn, warm, b, y);
 }
 void launch_knc_fie_fp64(uint32_t N, uint32_t count, const uint32_t* nodes, const double* targets, const double* x,
                          double* b, double* y, cudaStream_t s)
@@ -1411,17 +1668,26 @@ void launch_fie_update_fp64(uint32_t N, double inv_dt, double* x, double* v, con
 {
     FEMGB_LAUNCH(k_fie_update_fp64, vec_grid(3 * N), row_block(3 * N), N, inv_dt, x, v, xn, y, partials);
 }
-void launch_bsr_assemble_fp64(const MeshView<double>& m, uint32_t nnzb, const uint32_t* cptr,
-                              const uint32_t* contrib, double* val, cudaStream_t s)
+void launch_bsr_assemble_fp64(const MeshView<double>& m, const BsrBuild& a, cudaStream_t s)
 {
+    static_assert(kBsrElemWords == kFxBlockWords, "an element's block words");
     prof_begin("bsr_assemble_fp64", s);
-    FEMGB_LAUNCH(k_bsr_assemble_fp64, capped((nnzb + 127) / 128, 16 * 1216u), 128u, m, nnzb, cptr, contrib, val);
+    const uint32_t blocks = capped((m.T + kBsrElemBlock - 1) / kBsrElemBlock, 65535u);
+    k_bsr_elements_fp64<<<blocks, kBsrElemBlock, sizeof(long long) * kBsrElemRow * kBsrElemBlock, s>>>(m, a);
+    launch_counter()++;
+    FEMGB_LAUNCH(k_bsr_slots_fp64, capped((4 * a.groups + 127) / 128, 65535u), 128u, m, a);
+    FEMGB_LAUNCH(k_bsr_rows_fp64, capped((node_rows(m.N) + 127) / 128, 65535u), 128u, m, a);
     prof_end("bsr_assemble_fp64", s);
+}
+void launch_bsr_vector_fp64(const MeshView<double>& m, const double* u, const StepScalars* st, int check_done,
+                            cudaStream_t s)
+{
+    FEMGB_LAUNCH(k_bsr_vector_fp64, vec_grid(m.N), row_block(m.N), m, u, st, check_done);
 }
 void launch_mr_init_fp64(const MeshView<double>& m, const StepConsts& c, const double* b, const double* y,
                          double* v1, double* partials, cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_mr_init_fp64, node_grid(m.N), row_block(node_rows(m.N)), m, c, b, y, v1, partials);
+    FEMGB_LAUNCH_KU(k_mr_init_fp64, m, c, b, y, v1, partials);
 }
 void launch_mr_start_fp64(uint32_t N, double* v1, double* v, double* p, double* p0, const StepScalars* st,
                           cudaStream_t s)
@@ -1431,12 +1697,13 @@ void launch_mr_start_fp64(uint32_t N, double* v1, double* v, double* p, double* 
 void launch_mr_q_fp64(const MeshView<double>& m, const StepConsts& c, const double* v, const double* v0,
                       double* v1, double* pq, StepScalars* st, cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_mr_q_fp64, node_grid(m.N), row_block(node_rows(m.N)), m, c, v, v0, v1, pq, st);
+    FEMGB_LAUNCH_KU(k_mr_q_fp64, m, c, v, v0, v1, pq, st);
 }
-void launch_mr_v1_fp64(uint32_t N, double* v1, const double* v, const double* pq, double* pr, StepScalars* st,
-                       cudaStream_t s)
+void launch_mr_v1_fp64(const MeshView<double>& m, double* v1, const double* v, const double* pq, double* pr,
+                       StepScalars* st, cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_mr_v1_fp64, vec_grid(3 * N), row_block(3 * N), N, v1, v, pq, node_grid(N), pr, st);
+    FEMGB_LAUNCH(k_mr_v1_fp64, vec_grid(3 * m.N), row_block(3 * m.N), m.N, v1, v, pq,
+                 node_grid(m.N, m.bsr_val != nullptr), pr, st);
 }
 void launch_mr_update_fp64(uint32_t N, double* v1, const double* v, const double* p, double* p0, double* y,
                            const double* pr, StepScalars* st, cudaStream_t s, cudaGraphConditionalHandle cond,
@@ -1463,11 +1730,11 @@ void launch_potential_fp64(const MeshView<double>& m, const StepConsts& c, const
 void launch_apply_A_fp64(const MeshView<double>& m, double factor_M, double factor_K, double mass,
                          const double* d, double* q, cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_apply_A_fp64, node_grid(m.N), row_block(node_rows(m.N)), m, factor_M, factor_K, mass, d, q);
+    FEMGB_LAUNCH(k_apply_A_fp64, node_grid(m.N, false), node_block(m.N, false), m, factor_M, factor_K, mass, d, q);
 }
 void launch_gather_sum_fp64(const MeshView<double>& m, double sign, double* f, bool records, cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_gather_sum_fp64, node_grid(m.N), row_block(node_rows(m.N)), m, sign, f, records ? 1 : 0);
+    FEMGB_LAUNCH(k_gather_sum_fp64, node_grid(m.N, false), node_block(m.N, false), m, sign, f, records ? 1 : 0);
 }
 void launch_finalize(int kind, const double* partials, uint32_t count, const StepConsts& c, StepScalars* st,
                      cudaStream_t s, cudaGraphConditionalHandle cond, int set_cond)

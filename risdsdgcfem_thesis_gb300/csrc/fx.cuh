@@ -314,7 +314,7 @@ FX_HD int32_t fx_bake(const double* R, const double* Di, double kl, double km, F
 #pragma unroll
     for (int r = 0; r < 9; r++)
 #pragma unroll
-        for (int c = r; c < 9; c++) put(fx_at(r, c), fx_split((int64_t)((uint64_t)entry(r, c) << (lz - 1)) >> 3));
+        for (int c = r; c < 9; c++) put(fx_at(r, c), (int64_t)((uint64_t)entry(r, c) << (lz - 1)) >> 3);
     return xm + 2 * xd - 59 - (lz - 1) + 3;
 }
 
@@ -392,6 +392,63 @@ FX_HD int32_t fx_product(FK&& K, const FxL* D, int64_t* out)
 #pragma unroll
     for (int a = 0; a < 3; a++) out[a] = -sum[a];
     return 62 - up;
+}
+
+// The 4 x 4 corner blocks of an element's stiffness from K9, as kFxBlockWords
+// integers: blocks (p, q), p <= q, in the order 00 01 02 03 11 12 13 22 23 33,
+// a diagonal block's upper triangle (6), another block's rows (9). K9 / 2 in
+// words 24 + 9 ... : node 0's blocks are minus the sums of the others'.
+constexpr int kFxBlockWords = 78;
+FX_HD constexpr int fx_block(int p, int q)  // first word of block (p, q), p <= q
+{
+    return p == 0 ? (q == 0 ? 0 : 6 + 9 * (q - 1))
+                  : (p == 1 ? (q == 1 ? 33 : 39 + 9 * (q - 2)) : (p == 2 ? (q == 2 ? 57 : 63) : 72));
+}
+FX_HD constexpr int fx_tri(int a, int b)  // a, b in a diagonal block's triangle
+{
+    return a <= b ? 3 * a - a * (a - 1) / 2 + (b - a) : fx_tri(b, a);
+}
+// Word of entry (a, b) of block (p, q) in either order.
+FX_HD int fx_block_word(int p, int q, int a, int b)
+{
+    if (p == q) return fx_block(p, p) + fx_tri(a, b);
+    return p < q ? fx_block(p, q) + 3 * a + b : fx_block(q, p) + 3 * b + a;
+}
+// w[] holds K9 / 2 (entries (r, c), r <= c, of nodes 1 to 3) in its block words;
+// fills in node 0's blocks (below 9 2^59).
+FX_HD void fx_node0_blocks(int64_t* w)
+{
+    int64_t s00[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll
+    for (int j = 1; j < 4; j++)
+#pragma unroll
+        for (int a = 0; a < 3; a++)
+#pragma unroll
+            for (int b = 0; b < 3; b++) {
+                int64_t v = 0;
+#pragma unroll
+                for (int i = 1; i < 4; i++) v += w[fx_block_word(i, j, a, b)];
+                w[fx_block(0, j) + 3 * a + b] = -v;
+                if (a <= b) s00[fx_tri(a, b)] += v;
+            }
+#pragma unroll
+    for (int k = 0; k < 6; k++) w[k] = s00[k];
+}
+
+// A sum of 64-bit integers of any number (up to 2^31), in two words.
+struct FxWide {
+    int64_t hi, lo;  // hi 2^32 + lo
+};
+FX_HD void fx_wide_add(FxWide& s, int64_t v)
+{
+    s.hi += v >> 32;
+    s.lo += (uint32_t)v;
+}
+FX_HD double fx_wide_value(const FxWide& s, int32_t x)
+{
+    const int64_t hi = s.hi + (s.lo >> 32);
+    const int32_t bits = 64 - fx_clz(fx_mag(hi) | 1u), r = bits > 30 ? bits - 30 : 0;
+    return fx_to_double((int64_t)((uint64_t)hi << (32 - r)) + ((int64_t)(uint32_t)s.lo >> r), x + r);
 }
 
 #ifdef __CUDACC__

@@ -121,8 +121,11 @@ struct fem_solid_s {
     // the assembled stiffness (MeshView::bsr_*): pattern, per-slot
     // contributions and blocks; bsr_use: the solvers take it (set_bsr_use)
     DevBuf<uint32_t> bsr_row, bsr_col, bsr_cptr, bsr_contrib;
-    DevBuf<double> bsr_val;
-    uint32_t bsr_nnzb = 0;
+    DevBuf<int2> bsr_val;
+    DevBuf<int32_t> bsr_x, bsr_ex;
+    DevBuf<longlong2> bsr_u;
+    DevBuf<long long> bsr_eblk;
+    uint32_t bsr_groups = 0;  // of four blocks
     bool bsr_want = false, bsr_use = false;  // fem_solid_set_assembled; the solvers take it now
     // node vectors
     DevBuf<double> rest, x, v, y, b, r, d, q, tmp;
@@ -175,6 +178,20 @@ struct fem_solid_s {
         graph = nullptr;
     }
 
+    void release_bsr()
+    {
+        bsr_row.release();
+        bsr_col.release();
+        bsr_cptr.release();
+        bsr_contrib.release();
+        bsr_val.release();
+        bsr_x.release();
+        bsr_ex.release();
+        bsr_u.release();
+        bsr_eblk.release();
+        bsr_groups = 0;
+    }
+
     MeshView<double> view()
     {
         MeshView<double> m;
@@ -198,13 +215,15 @@ struct fem_solid_s {
             m.bsr_row = bsr_row.p;
             m.bsr_col = bsr_col.p;
             m.bsr_val = bsr_val.p;
+            m.bsr_x = bsr_x.p;
+            m.bsr_u = bsr_u.p;
         }
         return m;
     }
 
     void release()
     {
-        DevBuf<double>* dbl[] = {&Dinv, &mat, &vol, &R, &detF, &eout, &bsr_val, &rest, &x, &v, &y, &b, &r, &d, &q, &tmp,
+        DevBuf<double>* dbl[] = {&Dinv, &mat, &vol, &R, &detF, &eout, &rest, &x, &v, &y, &b, &r, &d, &q, &tmp,
                                  &xn, &vn, &prev_x, &mr_p, &mr_p0, &Fe, &knc_targets, &partials, &partials2,
                                  &lk_x, &lk_v};
         for (auto* p : dbl) p->release();
@@ -215,10 +234,7 @@ struct fem_solid_s {
         csr_ptr.release();
         csr_idx.release();
         cl_ent.release();
-        bsr_row.release();
-        bsr_col.release();
-        bsr_cptr.release();
-        bsr_contrib.release();
+        release_bsr();
         fixed.release();
         knc_nodes.release();
         st.release();
@@ -325,6 +341,16 @@ void set_consts(fem_solid s)
     s->dapd.eNL = (double)(float)params->dapd_nl_exponent;
 }
 
+// The assembled stiffness on the last rotations.
+void assemble(fem_solid s)
+{
+    MeshView<double> m = s->view();
+    m.bsr_row = s->bsr_row.p;  // also before the solvers take it (bsr_use)
+    m.bsr_col = s->bsr_col.p;
+    launch_bsr_assemble_fp64(m, BsrBuild{s->bsr_groups, s->bsr_cptr.p, s->bsr_contrib.p, s->bsr_eblk.p, s->bsr_ex.p,
+                                         s->bsr_val.p, s->bsr_x.p}, s->stream);
+}
+
 // The fixed-point product matrices of a C_WRP solid on its last rotations.
 void bake_products(fem_solid s)
 {
@@ -345,8 +371,7 @@ void begin_eval(fem_solid s, const double* xprev, const double* x)
         launch_begin_eval_fp64(m, x, F_out, s->st.p, s->stream);
     // the solvers' operator on the new rotations
     s->kfx_fresh = false;
-    if (s->bsr_use)
-        launch_bsr_assemble_fp64(m, s->bsr_nnzb, s->bsr_cptr.p, s->bsr_contrib.p, s->bsr_val.p, s->stream);
+    if (s->bsr_use) assemble(s);
     else
         bake_products(s);
 }
@@ -372,11 +397,12 @@ void elem_spmv(fem_solid s, const MeshView<double>& m, const double* d, int chec
     }
 }
 
-// The solvers' product ahead of their node kernels: nothing when those take
-// K u from the assembled stiffness (m.bsr_val), else the element outputs.
+// The solvers' product ahead of their node kernels: the vector's records when
+// those take K u from the assembled stiffness, else the element outputs.
 void solve_product(fem_solid s, const MeshView<double>& m, const double* d, int check_done)
 {
-    if (!m.bsr_val) elem_spmv(s, m, d, check_done);
+    if (m.bsr_val) launch_bsr_vector_fp64(m, d, s->st.p, check_done, s->stream);
+    else elem_spmv(s, m, d, check_done);
 }
 
 // FixedStep's opening: BeginEvaluation(m_vecPos0, x), then m_vecPos0 = x
@@ -400,27 +426,26 @@ bool cg_on_cluster(const fem_solid s)
 
 // Whether the solvers take K u from the assembled stiffness (asked for by
 // fem_solid_set_assembled and built): a C_WRP solid whose solve is not the
-// one-cluster CG. GB300's
-// FP64 element product is bound by the FP64 pipe at about 140 instructions
-// per tet per iteration; the assembled rows take 9 FMAs per block, about
-// 27 per tet, at the price of one assembly per evaluation (about 90 per
-// element corner pair, 16 pairs per tet).
+// one-cluster CG. The assembled rows read 81 bytes per block and iteration,
+// about 230 per tet on grid meshes, where the element product reads and
+// writes 580 per tet; an assembly costs about as much as five products.
 void set_bsr_use(fem_solid s)
 {
-    s->bsr_use = s->bsr_want && s->bsr_nnzb > 0 && s->params.material == FEM_MATERIAL_C_WRP &&
+    s->bsr_use = s->bsr_want && s->bsr_groups > 0 && s->params.material == FEM_MATERIAL_C_WRP &&
                  !(s->params.ls_solver != FEM_LS_MINRES && cg_on_cluster(s));
 }
 
-// The assembled stiffness's pattern and contributions (MeshView::bsr_*):
-// row n holds n's neighbours through its elements and n itself, ascending;
-// slot (n, j) sums the corner pairs (li of n, lj of j) of the elements
-// holding both, in element order. ptr/idx: the node CSR of element corners.
+// The assembled stiffness's pattern and contributions (MeshView::bsr_*): row n
+// holds n's neighbours through its elements and n itself, ascending, padded
+// with n to a multiple of four; slot (n, j), j other than n, sums the corner
+// pairs (li of n, lj of j) of the elements holding both, in element order.
+// ptr/idx: the node CSR of element corners.
 int build_bsr(fem_solid s, const uint32_t* tets, const std::vector<uint32_t>& ptr, const std::vector<uint32_t>& idx)
 {
     const uint32_t N = s->N, T = s->T;
     if ((uint64_t)T >= (1ull << 28)) return FEM_OK;  // contributions pack the element in 28 bits
-    std::vector<uint32_t> brow(N + 1, 0), bcol, nb;
-    bcol.reserve(16 * (size_t)N);
+    std::vector<uint32_t> brow(N + 1, 0), used(N), bcol, nb;
+    bcol.reserve(18 * (size_t)N);
     for (uint32_t n = 0; n < N; n++) {
         nb.clear();
         nb.push_back(n);
@@ -430,41 +455,53 @@ int build_bsr(fem_solid s, const uint32_t* tets, const std::vector<uint32_t>& pt
         }
         std::sort(nb.begin(), nb.end());
         nb.erase(std::unique(nb.begin(), nb.end()), nb.end());
+        used[n] = (uint32_t)nb.size();
+        while (nb.size() % 4) nb.push_back(n);
         bcol.insert(bcol.end(), nb.begin(), nb.end());
-        if (bcol.size() >= (1ull << 32)) return FEM_OK;
-        brow[n + 1] = (uint32_t)bcol.size();
+        if (bcol.size() >= (1ull << 28)) return FEM_OK;
+        brow[n + 1] = (uint32_t)(bcol.size() / 4);
     }
-    const size_t nnzb = bcol.size();
+    const size_t slots = bcol.size();
     auto slot_of = [&](uint32_t n, uint32_t col) {
-        return (size_t)(std::lower_bound(bcol.begin() + brow[n], bcol.begin() + brow[n + 1], col) - bcol.begin());
+        const auto b = bcol.begin() + 4 * (size_t)brow[n];
+        return (size_t)(std::lower_bound(b, b + used[n], col) - bcol.begin());
     };
-    std::vector<uint32_t> bcptr(nnzb + 1, 0), bcon(16 * (size_t)T);
+    std::vector<uint32_t> bcptr(slots + 1, 0), bcon(12 * (size_t)T), at(12 * (size_t)T);
+    size_t k = 0;
     for (uint32_t n = 0; n < N; n++)
         for (uint32_t j = ptr[n]; j < ptr[n + 1]; j++)
-            for (int lj = 0; lj < 4; lj++) bcptr[slot_of(n, tets[4 * (size_t)(idx[j] >> 2) + lj]) + 1]++;
-    for (size_t k = 0; k < nnzb; k++) bcptr[k + 1] += bcptr[k];
+            for (uint32_t lj = 0; lj < 4; lj++) {
+                if (lj == (idx[j] & 3u)) continue;
+                at[k] = (uint32_t)slot_of(n, tets[4 * (size_t)(idx[j] >> 2) + lj]);
+                bcptr[at[k++] + 1]++;
+            }
+    for (size_t i = 0; i < slots; i++) bcptr[i + 1] += bcptr[i];
     {
         std::vector<uint32_t> fill(bcptr.begin(), bcptr.end() - 1);
+        k = 0;
         for (uint32_t n = 0; n < N; n++)
             for (uint32_t j = ptr[n]; j < ptr[n + 1]; j++) {
                 const uint32_t e = idx[j] >> 2, li = idx[j] & 3u;
                 for (uint32_t lj = 0; lj < 4; lj++)
-                    bcon[fill[slot_of(n, tets[4 * (size_t)e + lj])]++] = (e << 4) | (li << 2) | lj;
+                    if (lj != li) bcon[fill[at[k++]]++] = (e << 4) | (li << 2) | lj;
             }
     }
     cudaStream_t st = s->stream;
     CK(s->bsr_row.alloc(N + 1));
-    CK(s->bsr_col.alloc(nnzb));
-    CK(s->bsr_cptr.alloc(nnzb + 1));
+    CK(s->bsr_col.alloc(slots));
+    CK(s->bsr_cptr.alloc(slots + 1));
     CK(s->bsr_contrib.alloc(bcon.size()));
-    CK(s->bsr_val.alloc(9 * nnzb));
+    CK(s->bsr_val.alloc(9 * slots));
+    CK(s->bsr_x.alloc(N));
+    CK(s->bsr_u.alloc(2 * (size_t)N));
+    CK(s->bsr_ex.alloc(T));
+    CK(s->bsr_eblk.alloc((size_t)kBsrElemWords * T));
     CK(cudaMemcpyAsync(s->bsr_row.p, brow.data(), sizeof(uint32_t) * brow.size(), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(s->bsr_col.p, bcol.data(), sizeof(uint32_t) * nnzb, cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(s->bsr_col.p, bcol.data(), sizeof(uint32_t) * slots, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(s->bsr_cptr.p, bcptr.data(), sizeof(uint32_t) * bcptr.size(), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(s->bsr_contrib.p, bcon.data(), sizeof(uint32_t) * bcon.size(), cudaMemcpyHostToDevice, st));
-    CK(cudaMemsetAsync(s->bsr_val.p, 0, sizeof(double) * 9 * nnzb, st));
     CK(cudaStreamSynchronize(st));
-    s->bsr_nnzb = (uint32_t)nnzb;
+    s->bsr_groups = (uint32_t)(slots / 4);
     return FEM_OK;
 }
 
@@ -518,16 +555,17 @@ int cg_solve(fem_solid s, const StepConsts& c, int chunk)
         CK(cudaGetLastError());
         return FEM_OK;
     }
-    const uint32_t gN = node_grid(s->N), gV = vec_grid(3 * s->N);
+    const uint32_t gN = node_grid(s->N, m.bsr_val != nullptr), gV = vec_grid(3 * s->N);
     solve_product(s, m, s->y.p, 0);
     launch_node_residual_fp64(m, c, s->b.p, s->y.p, s->r.p, s->d.p, s->partials.p, st);
     launch_finalize(FIN_INIT, s->partials.p, gN, c, s->st.p, st);
+    if (m.bsr_val) solve_product(s, m, s->d.p, 0);  // then node_d keeps d's records
     for (;;) {
         for (int i = 0; i < chunk; i++) {
-            solve_product(s, m, s->d.p, 1);
+            if (!m.bsr_val) solve_product(s, m, s->d.p, 1);
             launch_node_q_fp64(m, c, s->d.p, s->q.p, s->partials.p, s->st.p, st);
-            launch_node_xr_fp64(s->N, s->y.p, s->r.p, s->d.p, s->q.p, s->partials.p, s->partials2.p, s->st.p, st);
-            launch_node_d_fp64(s->N, s->fixed.p, s->d.p, s->r.p, s->partials2.p, s->st.p, st);
+            launch_node_xr_fp64(m, s->y.p, s->r.p, s->d.p, s->q.p, s->partials.p, s->partials2.p, s->st.p, st);
+            launch_node_d_fp64(m, s->d.p, s->r.p, s->partials2.p, s->st.p, st);
         }
         CK(cudaMemcpyAsync(s->st_host, s->st.p, sizeof(StepScalars), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
@@ -546,7 +584,7 @@ int minres_solve(fem_solid s, const StepConsts& c, int chunk)
 {
     cudaStream_t st = s->stream;
     MeshView<double> m = s->view();
-    const uint32_t gN = node_grid(s->N), gV = vec_grid(3 * s->N);
+    const uint32_t gN = node_grid(s->N, m.bsr_val != nullptr), gV = vec_grid(3 * s->N);
     double *v = s->r.p, *v0 = s->d.p, *v1 = s->q.p, *p = s->mr_p.p, *p0 = s->mr_p0.p;
     launch_sq_norm_fp64(3 * s->N, s->b.p, s->partials.p, st);
     launch_finalize(FIN_SUM, s->partials.p, gV, c, s->st.p, st);  // |b|^2
@@ -562,7 +600,7 @@ int minres_solve(fem_solid s, const StepConsts& c, int chunk)
             v1 = t;
             solve_product(s, m, v, 1);
             launch_mr_q_fp64(m, c, v, v0, v1, s->partials.p, s->st.p, st);
-            launch_mr_v1_fp64(s->N, v1, v, s->partials.p, s->partials2.p, s->st.p, st);
+            launch_mr_v1_fp64(m, v1, v, s->partials.p, s->partials2.p, s->st.p, st);
             launch_mr_update_fp64(s->N, v1, v, p, p0, s->y.p, s->partials2.p, s->st.p, st);
             t = p;  // the new p was written into p0's buffer
             p = p0;
@@ -592,7 +630,7 @@ cudaError_t ls_solve_capture(fem_solid s, const StepConsts& c, cudaGraph_t top)
 {
     cudaStream_t st = s->stream;
     MeshView<double> m = s->view();
-    const uint32_t gN = node_grid(s->N), gV = vec_grid(3 * s->N);
+    const uint32_t gN = node_grid(s->N, m.bsr_val != nullptr), gV = vec_grid(3 * s->N);
     if (s->params.ls_solver != FEM_LS_MINRES && cg_on_cluster(s))
         return launch_cg_cluster_fp64(m, c, s->cl_plan, s->cl_ent.p, s->b.p, s->y.p, s->st.p, st);
     cudaGraphConditionalHandle cond = 0;
@@ -602,12 +640,13 @@ cudaError_t ls_solve_capture(fem_solid s, const StepConsts& c, cudaGraph_t top)
         solve_product(s, m, s->y.p, 0);
         launch_node_residual_fp64(m, c, s->b.p, s->y.p, s->r.p, s->d.p, s->partials.p, st);
         launch_finalize(FIN_INIT, s->partials.p, gN, c, s->st.p, st, cond, 1);
+        if (m.bsr_val) solve_product(s, m, s->d.p, 0);  // then node_d keeps d's records
         e = capture_conditional(st, cond, cudaGraphCondTypeWhile, [&](cudaStream_t bs, cudaGraph_t) {
             s->stream = bs;
-            solve_product(s, m, s->d.p, 1);
+            if (!m.bsr_val) solve_product(s, m, s->d.p, 1);
             launch_node_q_fp64(m, c, s->d.p, s->q.p, s->partials.p, s->st.p, bs);
-            launch_node_xr_fp64(s->N, s->y.p, s->r.p, s->d.p, s->q.p, s->partials.p, s->partials2.p, s->st.p, bs);
-            launch_node_d_fp64(s->N, s->fixed.p, s->d.p, s->r.p, s->partials2.p, s->st.p, bs, cond, 1);
+            launch_node_xr_fp64(m, s->y.p, s->r.p, s->d.p, s->q.p, s->partials.p, s->partials2.p, s->st.p, bs);
+            launch_node_d_fp64(m, s->d.p, s->r.p, s->partials2.p, s->st.p, bs, cond, 1);
             s->stream = st;
             return cudaGetLastError();
         });
@@ -634,7 +673,7 @@ cudaError_t ls_solve_capture(fem_solid s, const StepConsts& c, cudaGraph_t top)
             v1 = t;
             solve_product(s, m, v, 1);
             launch_mr_q_fp64(m, c, v, v0, v1, s->partials.p, s->st.p, bs);
-            launch_mr_v1_fp64(s->N, v1, v, s->partials.p, s->partials2.p, s->st.p, bs);
+            launch_mr_v1_fp64(m, v1, v, s->partials.p, s->partials2.p, s->st.p, bs);
             launch_mr_update_fp64(s->N, v1, v, p, p0, s->y.p, s->partials2.p, s->st.p, bs, cond, 1);
             t = p;  // the new p was written into p0's buffer
             p = p0;
@@ -1065,14 +1104,9 @@ int fem_solid_create(const double* rest_xyz, uint32_t N, const uint32_t* tets, u
     CKC(cudaMemsetAsync(s->v.p, 0, sizeof(double) * n3, st));
     CKC(cudaMemsetAsync(s->y.p, 0, sizeof(double) * n3, st));
     CKC(cudaMemsetAsync(s->st.p, 0, sizeof(StepScalars), st));
-    // R = I, det F = 1 until the first evaluation (CreateCache, TetrahedronElementSet3.cpp:190-209)
-    {
-        std::vector<double> Rh(9 * (size_t)T, 0.0), dh(T, 1.0);
-        for (uint32_t e = 0; e < T; e++) Rh[e] = Rh[4 * (size_t)T + e] = Rh[8 * (size_t)T + e] = 1.0;
-        CKC(cudaMemcpyAsync(s->R.p, Rh.data(), sizeof(double) * Rh.size(), cudaMemcpyHostToDevice, st));
-        CKC(cudaMemcpyAsync(s->detF.p, dh.data(), sizeof(double) * T, cudaMemcpyHostToDevice, st));
-        CKC(cudaStreamSynchronize(st));
-    }
+    launch_rest_rotations_fp64(T, s->R.p, s->detF.p, st);
+    CKC(cudaGetLastError());
+    CKC(cudaStreamSynchronize(st));
 #undef CKC
     // the static scratch of fem_solid_apply_A_noalloc: its address is looked
     // up here, where allocating is expected, so that the no-alloc call never
@@ -1099,7 +1133,7 @@ int fem_solid_set_assembled(fem_solid s, int on)
 {
     if (int e = check_handle(s)) return e;
     s->drop_graph();  // the step graph holds the operator's launches
-    if (on && !s->bsr_nnzb) {
+    if (on && !s->bsr_groups) {
         const uint32_t N = s->N, T = s->T;
         std::vector<int4> t4(T);
         std::vector<uint32_t> tets(4 * (size_t)T), ptr(N + 1), idx(4 * (size_t)T);
@@ -1115,17 +1149,11 @@ int fem_solid_set_assembled(fem_solid s, int on)
             tets[4 * (size_t)e + 3] = (uint32_t)t4[e].w;
         }
         if (int e = build_bsr(s, tets.data(), ptr, idx)) {
-            s->bsr_row.release();
-            s->bsr_col.release();
-            s->bsr_cptr.release();
-            s->bsr_contrib.release();
-            s->bsr_val.release();
-            s->bsr_nnzb = 0;
+            s->release_bsr();
             return e;
         }
         // the current rotations' blocks, for a solve before the next evaluation
-        MeshView<double> m = s->view();
-        launch_bsr_assemble_fp64(m, s->bsr_nnzb, s->bsr_cptr.p, s->bsr_contrib.p, s->bsr_val.p, s->stream);
+        if (s->bsr_groups) assemble(s);
         CK(cudaStreamSynchronize(s->stream));
     }
     s->bsr_want = on != 0;

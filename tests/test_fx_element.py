@@ -37,7 +37,7 @@ int one(const double* R, const double* Di, double kl, double km, double grade, c
     int64_t out[12];
     int32_t x;
     if (!fx_grade_ok((float)grade, kl, km)) return 1;
-    const int32_t scale = fx_bake(R, Di, kl, km, [&](int k, FxL v) { K[k] = v; });
+    const int32_t scale = fx_bake(R, Di, kl, km, [&](int k, int64_t v) { K[k] = fx_split(v); });
     if (scale == kFxFp64) return 1;
     if (!fx_differences(d, D, x)) return 2;
     x += scale + fx_product([&](int k) { return K[k]; }, D, out);
