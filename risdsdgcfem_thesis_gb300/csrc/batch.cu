@@ -138,6 +138,8 @@ struct fem_batch_s {
     Dev<int4> gtets;
     Dev<unsigned char> Dinv_s, mat_s, R_s;  // S-typed, raw bytes
     Dev<double> Dinv64, vol, detF;
+    Dev<int4> Kfx;     // FP64 (BatchView::Kfx)
+    Dev<float> grade;
     Dev<uint32_t> tile_nodes, lptr0, ov_ptr, ov_map, knc_node, knc_mesh;
     std::vector<uint32_t> perm_h, inv_h;  // batch node -> caller's node, and back (global ids)
     std::vector<uint32_t> eperm_h;        // batch element -> the caller's element index in its mesh
@@ -212,7 +214,9 @@ struct fem_batch_s {
         b.Dinv = reinterpret_cast<const S*>(Dinv_s.p);
         b.mat = reinterpret_cast<const S*>(mat_s.p);
         b.R = reinterpret_cast<S*>(R_s.p);
-        b.Dinv64 = Dinv64.p;
+        b.Dinv64 = sizeof(S) == 8 ? reinterpret_cast<const double*>(Dinv_s.p) : Dinv64.p;
+        b.Kfx = Kfx.p;
+        b.grade = grade.p;
         b.vol = vol.p;
         b.detF = detF.p;
         b.tile_nodes = tile_nodes.p;
@@ -262,7 +266,7 @@ struct fem_batch_s {
         exec = nullptr;
         graph = nullptr;
         tiles.release(); chunks.release(); mc.release(); st.release(); active.release(); gtets.release();
-        Dinv_s.release(); mat_s.release(); R_s.release(); Dinv64.release(); vol.release(); detF.release();
+        Dinv_s.release(); mat_s.release(); R_s.release(); Dinv64.release(); Kfx.release(); grade.release(); vol.release(); detF.release();
         tile_nodes.release(); lptr0.release(); ov_ptr.release(); ov_map.release(); knc_node.release();
         perm.release(); stage_x.release(); stage_v.release();
         knc_mesh.release(); lconn.release(); lptr.release(); lidx.release(); fixed.release(); rest.release();
@@ -771,6 +775,7 @@ int fem_batch_finalize(fem_batch b)
     std::vector<uint32_t> perm_h;    // batch node id -> caller's node id (both global)
     // element data collected AoS then transposed
     std::vector<double> Dinv_aos, mat_aos;
+    std::vector<float> grade;  // FP64 (BatchView::grade)
 
     uint64_t node0 = 0, elem0 = 0;
     for (uint32_t mi = 0; mi < b->M; mi++) {
@@ -843,6 +848,14 @@ int fem_batch_finalize(fem_batch b)
             const double nu = (hm.nu.empty() || scalar_mat) ? p.poisson_ratio : hm.nu[e];
             const double a = E / ((1.0 + nu) * (1.0 - 2.0 * nu));
             for (int c = 0; c < 9; c++) Dinv_aos.push_back(Di[c]);
+            if (fp64) {
+                double edge = 0.0, slope = 0.0;
+                for (int c = 0; c < 9; c++) {
+                    edge = std::max(edge, std::fabs(D[c]));
+                    slope = std::max(slope, std::fabs(Di[c]));
+                }
+                grade.push_back((float)(edge * slope));
+            }
             mat_aos.push_back(V * (a * (1.0 - nu)));
             mat_aos.push_back(V * (a * nu));
             mat_aos.push_back(V * (a * (0.5 - nu)));
@@ -1079,8 +1092,6 @@ int fem_batch_finalize(fem_batch b)
             for (uint32_t i = tm.nown; i < tm.nn; i++) hdr[3 + i - tm.nown] = ov_map[tm.ov0 + i - tm.nown];
         }
     }
-    std::vector<double> Rinit(9 * T, 0.0);
-    for (size_t e = 0; e < T; e++) Rinit[e] = Rinit[4 * T + e] = Rinit[8 * T + e] = 1.0;
 
     // ---- device ----
     auto cleanup = [&](int code) {
@@ -1107,7 +1118,12 @@ int fem_batch_finalize(fem_batch b)
     BCKC(b->Dinv_s.alloc(9 * T * SB));
     BCKC(b->mat_s.alloc(3 * T * SB));
     BCKC(b->R_s.alloc(9 * T * SB));
-    BCKC(b->Dinv64.alloc(9 * T));
+    if (fp64) {
+        BCKC(b->Kfx.alloc(kFxGroups * ((T + 31) / 32 * 32)));
+        BCKC(b->grade.alloc(T));
+    } else {
+        BCKC(b->Dinv64.alloc(9 * T));
+    }
     BCKC(b->vol.alloc(T));
     BCKC(b->detF.alloc(T));
     BCKC(b->tile_nodes.alloc(tile_nodes.size()));
@@ -1132,8 +1148,10 @@ int fem_batch_finalize(fem_batch b)
     BCKC(b->q_s.alloc(N3 * SB));
     BCKC(b->part_s.alloc(3 * b->nslots * SB));
     BCKC(cudaMemsetAsync(b->part_s.p, 0, 3 * b->nslots * SB, s));  // slots of nodes no tet names stay zero
-    BCKC(b->ydelta_s.alloc(N3 * SB));
-    BCKC(cudaMemsetAsync(b->ydelta_s.p, 0, N3 * SB, s));
+    if (!fp64) {
+        BCKC(b->ydelta_s.alloc(N3 * SB));
+        BCKC(cudaMemsetAsync(b->ydelta_s.p, 0, N3 * SB, s));
+    }
     BCKC(b->part64.alloc(3 * b->nslots));
     BCKC(cudaMemsetAsync(b->part64.p, 0, 3 * b->nslots * sizeof(double), s));
     BCKC(b->cpart.alloc(b->nchunks));
@@ -1183,18 +1201,26 @@ int fem_batch_finalize(fem_batch b)
     BCKC(cudaMemsetAsync(b->st.p, 0, sizeof(StepScalars) * b->M, s));
     BCKC(cudaMemsetAsync(b->active.p, 1, b->M, s));
     BCKC(b->gtets.upload(gtets, s));
-    {
-        std::vector<unsigned char> tmp = fp64 ? as_bytes<double>(Dinv_soa) : as_bytes<float>(Dinv_soa);
+    if (fp64) {
+        BCKC(cudaMemcpyAsync(b->Dinv_s.p, Dinv_soa.data(), sizeof(double) * Dinv_soa.size(), cudaMemcpyHostToDevice, s));
+        BCKC(cudaMemcpyAsync(b->mat_s.p, mat_soa.data(), sizeof(double) * mat_soa.size(), cudaMemcpyHostToDevice, s));
+        launch_rest_rotations_fp64((uint32_t)T, reinterpret_cast<double*>(b->R_s.p), b->detF.p, s);
+        BCKC(cudaGetLastError());
+    } else {
+        std::vector<unsigned char> tmp = as_bytes<float>(Dinv_soa);
         BCKC(b->Dinv_s.upload(tmp, s));
         BCKC(cudaStreamSynchronize(s));
-        tmp = fp64 ? as_bytes<double>(mat_soa) : as_bytes<float>(mat_soa);
+        tmp = as_bytes<float>(mat_soa);
         BCKC(b->mat_s.upload(tmp, s));
         BCKC(cudaStreamSynchronize(s));
-        tmp = fp64 ? as_bytes<double>(Rinit) : as_bytes<float>(Rinit);
+        std::vector<double> Rinit(9 * T, 0.0);
+        for (size_t e = 0; e < T; e++) Rinit[e] = Rinit[4 * T + e] = Rinit[8 * T + e] = 1.0;
+        tmp = as_bytes<float>(Rinit);
         BCKC(b->R_s.upload(tmp, s));
         BCKC(cudaStreamSynchronize(s));
     }
-    BCKC(b->Dinv64.upload(Dinv_soa, s));
+    if (fp64) BCKC(b->grade.upload(grade, s));
+    else BCKC(b->Dinv64.upload(Dinv_soa, s));
     BCKC(b->vol.upload(vol, s));
     BCKC(b->tile_nodes.upload(tile_nodes, s));
     BCKC(b->lptr0.upload(lptr0, s));
@@ -1250,7 +1276,7 @@ int fem_batch_finalize(fem_batch b)
 #undef BCKC
     b->device_bytes = b->tiles.bytes() + b->chunks.bytes() + b->mc.bytes() + b->st.bytes() + b->active.bytes() +
                       b->gtets.bytes() + b->Dinv_s.bytes() + b->mat_s.bytes() + b->R_s.bytes() +
-                      b->Dinv64.bytes() + b->vol.bytes() + b->detF.bytes() + b->tile_nodes.bytes() +
+                      b->Dinv64.bytes() + b->Kfx.bytes() + b->grade.bytes() + b->vol.bytes() + b->detF.bytes() + b->tile_nodes.bytes() +
                       b->lptr0.bytes() + b->ov_ptr.bytes() + b->ov_map.bytes() + b->knc_node.bytes() +
                       b->perm.bytes() + b->prev_x.bytes() + b->doc.bytes() + b->Fe.bytes() + b->lcmh_w.bytes() + b->mr_p_s.bytes() +
                       b->mr_p0_s.bytes() + b->cpart_b.bytes() + b->xn.bytes() + b->vn.bytes() +

@@ -186,7 +186,10 @@ struct BatchView {
     const S* Dinv;                 // [9][Ttot]
     const S* mat;                  // [3][Ttot]
     S* R;                          // [9][Ttot]
-    const double* Dinv64;          // [9][Ttot]
+    const double* Dinv64;          // [9][Ttot] (FP64: Dinv itself)
+    int4* Kfx;                     // FP64: the elements' fixed-point product matrices (fx_device.cuh), baked
+                                   // after each evaluation of a C_WRP mesh; null on the mixed path
+    const float* grade;            // FP64: [Ttot] max|Dm| max|Dm^-1| of each rest shape
     const double* vol;             // [Ttot]
     double* detF;                  // [Ttot]
     // tile structure
@@ -230,6 +233,14 @@ template <typename S>
 __device__ __forceinline__ bool mesh_starts(const BatchView<S>& b, uint32_t m)
 {
     return b.st[m].nr_go != 0;
+}
+
+// Whether BeginEvaluation takes mesh m: the start section's meshes, or
+// (newton) those whose Newton solve has just updated x_k.
+template <typename S>
+__device__ __forceinline__ bool mesh_evaluates(const BatchView<S>& b, uint32_t m, int newton)
+{
+    return newton ? (b.lock || b.mc[m].integrator != kMeshQie) && b.st[m].finished : mesh_starts(b, m);
 }
 
 }  // namespace femgb

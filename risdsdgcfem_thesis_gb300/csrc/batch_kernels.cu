@@ -32,6 +32,7 @@
 #include "bounds.cuh"
 #include "df.cuh"
 #include "elem_math.cuh"
+#include "fx_device.cuh"
 #include "msvd.cuh"
 #include "lcm.cuh"
 #include "refresh_product.cuh"
@@ -116,81 +117,156 @@ __device__ __forceinline__ float dir_update<float>(float beta, float d, float r)
 template <>
 __device__ __forceinline__ double dir_update<double>(double beta, double d, double r) { return __fma_rn(beta, d, r); }
 
-template <typename S>
-__global__ void __launch_bounds__(256) k_tile_spmv(BatchView<S> b, const S* __restrict__ dvec,
-                                                   const S* __restrict__ rvec, S* __restrict__ part,
-                                                   cudaGraphConditionalHandle if_refresh, int set_if,
-                                                   const unsigned* __restrict__ refresh_flag)
+// FP64 batch: the product matrices (fx.cuh) of the elements of the C_WRP
+// meshes just evaluated. Integer-bound, once per evaluation (125 us for
+// 554,475 tets).
+constexpr int kFxTileThreads = 128;  // two elements of a tile per thread
+__global__ void __launch_bounds__(kFxTileThreads, 3) k_bake_batch(BatchView<double> b, int newton)
 {
-    __shared__ S sd[3 * kTileNodes];
-    __shared__ S so[12 * kTileElems];
-    // the graph's IF node after this kernel runs the FP64 refresh product
-    // only on iterations where some mesh refreshes its residual
-    if (set_if && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(if_refresh, *refresh_flag ? 1u : 0u);
-    const uint32_t t = blockIdx.x;
-    if (t >= b.ntiles) return;
-    const TileMeta tm = b.tiles[t];
-    if (!mesh_running(b, tm.mesh)) return;
-    const S beta = (S)b.st[tm.mesh].beta;
-    const uint16_t* lp = b.lptr + b.lptr0[t];
-    const uint16_t* li = b.lidx + tm.c0;
-    // element data first: these loads are in flight while the tile stages
-    // its node values
-    const bool has_elem = threadIdx.x < tm.ne;
-    const size_t e = tm.e0 + (has_elem ? threadIdx.x : 0);
+    const uint32_t n = b.list_count[0];
+    for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
+        const TileMeta tm = b.tiles[b.start_tiles[i]];
+        if (tm.material != kTileMaterialWrp || !mesh_evaluates(b, tm.mesh, newton)) continue;
+        for (uint32_t k = threadIdx.x; k < tm.ne; k += blockDim.x) {
+            const size_t e = tm.e0 + k, T = b.Ttot;
+            double R[9], Di[9];
+#pragma unroll
+            for (int c = 0; c < 9; c++) R[c] = b.R[c * T + e];
+#pragma unroll
+            for (int c = 0; c < 9; c++) Di[c] = b.Dinv[c * T + e];
+            fx_store_matrix(b.Kfx, e, R, Di, b.mat[T + e], b.mat[2 * T + e], b.grade[e]);
+        }
+    }
+}
+
+// The FP64 product of an element that is not in fixed point: a P-K material's
+// (as doubles in so), or a C_WRP element fx.cuh leaves out (as integers; the
+// exponent returned). Out of line, so that the fixed-point path keeps its
+// values in registers. d: the element's nodes in the tile's staged vector.
+__device__ __noinline__ int32_t tile_elem_fp64(const BatchView<double>& b, uint32_t material, uint32_t mesh, size_t e,
+                                               const double* sd, uchar4 lc, double* so)
+{
     const size_t T = b.Ttot;
-    S R[9], Di[9], k1 = 0, knu = 0, k2 = 0;
-    uchar4 lc = make_uchar4(0, 0, 0, 0);
-    if (has_elem) {
+    double R[9], Di[9], dl[12], out[12];
 #pragma unroll
-        for (int c = 0; c < 9; c++) R[c] = b.R[c * T + e];
-#pragma unroll
-        for (int c = 0; c < 9; c++) Di[c] = b.Dinv[c * T + e];
-        k1 = b.mat[e];
-        knu = b.mat[T + e];
-        k2 = b.mat[2 * T + e];
-        lc = b.lconn[e];
+    for (int c = 0; c < 9; c++) {
+        R[c] = b.R[c * T + e];
+        Di[c] = b.Dinv[c * T + e];
     }
-    for (int i = threadIdx.x; i < tm.nn; i += blockDim.x) {
-        const size_t g = bounds_idx(b.tile_nodes[tm.n0 + i], b.Ntot, kSiteBatchNode);
-        sd[i] = dir_update<S>(beta, dvec[3 * g], rvec[3 * g]);
-        sd[kTileNodes + i] = dir_update<S>(beta, dvec[3 * g + 1], rvec[3 * g + 1]);
-        sd[2 * kTileNodes + i] = dir_update<S>(beta, dvec[3 * g + 2], rvec[3 * g + 2]);
-    }
-    __syncthreads();
-    if (has_elem) {
-        const int ids[4] = {(int)bounds_idx((uint32_t)lc.x, tm.nn, kSiteLocalNode),
-                            (int)bounds_idx((uint32_t)lc.y, tm.nn, kSiteLocalNode),
-                            (int)bounds_idx((uint32_t)lc.z, tm.nn, kSiteLocalNode),
-                            (int)bounds_idx((uint32_t)lc.w, tm.nn, kSiteLocalNode)};
-        S dl[12];
+    const int ids[4] = {lc.x, lc.y, lc.z, lc.w};
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            dl[3 * i] = sd[ids[i]];
-            dl[3 * i + 1] = sd[kTileNodes + ids[i]];
-            dl[3 * i + 2] = sd[2 * kTileNodes + ids[i]];
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int a = 0; a < 3; a++) dl[3 * i + a] = sd[a * kTileNodes + ids[i]];
+    if (material != kTileMaterialWrp) {
+        elem_pk(b, material, mesh, e, R, Di, 0.0, 0.0, dl, out);
+#pragma unroll
+        for (int c = 0; c < 12; c++) so[c * kTileElems] = out[c];
+        return 0;
+    }
+    elem_RKRt<double>(R, Di, b.mat[e], b.mat[T + e], b.mat[2 * T + e], dl, out);
+    int64_t v[12];
+    const int32_t x = fx_from_doubles(out, v);
+#pragma unroll
+    for (int c = 0; c < 12; c++) so[c * kTileElems] = __longlong_as_double(v[c]);
+    return x;
+}
+
+// FP64 batch: one tile per block and turn. kDir: the product of the new search
+// direction d = S(r + beta d), formed while the tile's node values are staged,
+// for every running mesh (one tile per block); else that of the iterate y for
+// the residual of the meshes that start. Element outputs are block
+// fixed-point integers with one exponent per element; a node's thread adds
+// its entries in integers (fx.cuh) and leaves an FP64 partial.
+// The 138 FP64 operations per element and three adds per entry of the FP64
+// form held that pipe at 64 clocks each: 210 us for 554,475 tets. The integer
+// multiplies take 71 us, about as long as the 204 MB of matrices need.
+template <bool kDir>
+__global__ void __launch_bounds__(kFxTileThreads, 3)
+    k_tile_product_fp64(BatchView<double> b, const double* __restrict__ vec, const double* __restrict__ rvec,
+                        double* __restrict__ part)
+{
+    __shared__ double sd[3 * kTileNodes];
+    __shared__ double so[12 * kTileElems];
+    __shared__ int32_t sx[kTileElems];
+    const uint32_t n = kDir ? b.ntiles : b.list_count[0];
+    for (uint32_t it = blockIdx.x; it < n; it += gridDim.x) {
+        const uint32_t t = kDir ? it : b.start_tiles[it];
+        const TileMeta tm = b.tiles[t];
+        if (kDir ? !mesh_running(b, tm.mesh) : !mesh_starts(b, tm.mesh)) continue;
+        const double beta = kDir ? b.st[tm.mesh].beta : 0.0;
+        const bool fixed_point = tm.material == kTileMaterialWrp;
+        for (int i = threadIdx.x; i < tm.nn; i += blockDim.x) {
+            const size_t g = bounds_idx(b.tile_nodes[tm.n0 + i], b.Ntot, kSiteBatchNode);
+#pragma unroll
+            for (int a = 0; a < 3; a++)
+                sd[a * kTileNodes + i] = kDir ? dir_update<double>(beta, vec[3 * g + a], rvec[3 * g + a]) : vec[3 * g + a];
         }
-        S out[12];
-        if (tm.material != kTileMaterialWrp)
-            elem_pk(b, tm.material, tm.mesh, e, R, Di, knu, k2, dl, out);
-        else
-            elem_RKRt<S>(R, Di, k1, knu, k2, dl, out);
+        __syncthreads();
+        for (uint32_t k = threadIdx.x; k < tm.ne; k += blockDim.x) {
+            const size_t e = tm.e0 + k;
+            uchar4 lc = b.lconn[e];
+            lc.x = (unsigned char)bounds_idx((uint32_t)lc.x, tm.nn, kSiteLocalNode);
+            lc.y = (unsigned char)bounds_idx((uint32_t)lc.y, tm.nn, kSiteLocalNode);
+            lc.z = (unsigned char)bounds_idx((uint32_t)lc.z, tm.nn, kSiteLocalNode);
+            lc.w = (unsigned char)bounds_idx((uint32_t)lc.w, tm.nn, kSiteLocalNode);
+            const int ids[4] = {lc.x, lc.y, lc.z, lc.w};
+            bool ok = fixed_point;
+            if (ok) {
+                const int4 last = fx_matrix(b.Kfx, e)[32 * (kFxGroups - 1)];
+                double dl[12];
 #pragma unroll
-        for (int c = 0; c < 12; c++) so[c * kTileElems + threadIdx.x] = out[c];
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < tm.nn; i += blockDim.x) {
-        S a0 = 0, a1 = 0, a2 = 0;
-        for (int j = lp[i]; j < lp[i + 1]; j++) {
-            const int v = li[j], el = v >> 2, sl = v & 3;
-            a0 += so[(3 * sl) * kTileElems + el];
-            a1 += so[(3 * sl + 1) * kTileElems + el];
-            a2 += so[(3 * sl + 2) * kTileElems + el];
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int a = 0; a < 3; a++) dl[3 * i + a] = sd[a * kTileNodes + ids[i]];
+                FxL D[9];
+                int64_t out[12];
+                int32_t x;
+                ok = fx_differences(dl, D, x) && last.z != kFxFp64;
+                fx_load_product(b.Kfx, e, last, D, out, x);
+                x += 2048;
+                ok = ok && x < kFxNan;
+                if (ok) {
+                    const bool flush = x < 0;  // below every normal double
+                    sx[k] = flush ? 0 : x;
+#pragma unroll
+                    for (int c = 0; c < 12; c++) so[c * kTileElems + k] = __longlong_as_double(flush ? 0ll : out[c]);
+                }
+            }
+            if (!ok) sx[k] = tile_elem_fp64(b, tm.material, tm.mesh, e, sd, lc, so + k);
         }
-        const size_t o = 3 * tile_slot(b.ov_map, tm.own0, tm.ov0, tm.nown, i);
-        part[o] = a0;
-        part[o + 1] = a1;
-        part[o + 2] = a2;
+        __syncthreads();
+        const uint16_t* lp = b.lptr + b.lptr0[t];
+        const uint16_t* li = b.lidx + tm.c0;
+        for (int i = threadIdx.x; i < tm.nn; i += blockDim.x) {
+            const int beg = lp[i], end = lp[i + 1];
+            double a0 = 0, a1 = 0, a2 = 0;
+            if (fixed_point) {
+                const int32_t guard = end - beg > 1 ? 32 - __clz(end - beg - 1) : 0;
+                FxSum s{{0, 0, 0}, 0};
+                for (int j = beg; j < end; j++) {
+                    const int v = li[j], el = v >> 2, sl = v & 3;
+                    const double* o = so + 3 * sl * kTileElems + el;
+                    fx_add(s, __double_as_longlong(o[0]), __double_as_longlong(o[kTileElems]),
+                           __double_as_longlong(o[2 * kTileElems]), sx[el], guard);
+                }
+                a0 = fx_sum_value(s.acc[0], s.E, guard);
+                a1 = fx_sum_value(s.acc[1], s.E, guard);
+                a2 = fx_sum_value(s.acc[2], s.E, guard);
+            } else {
+                for (int j = beg; j < end; j++) {
+                    const int v = li[j], el = v >> 2, sl = v & 3;
+                    a0 += so[(3 * sl) * kTileElems + el];
+                    a1 += so[(3 * sl + 1) * kTileElems + el];
+                    a2 += so[(3 * sl + 2) * kTileElems + el];
+                }
+            }
+            const size_t o = 3 * tile_slot(b.ov_map, tm.own0, tm.ov0, tm.nown, i);
+            part[o] = a0;
+            part[o + 1] = a1;
+            part[o + 2] = a2;
+        }
+        __syncthreads();
     }
 }
 
@@ -1201,13 +1277,22 @@ __global__ void k_fin_energy(BatchView<S> b, int kind, const double* __restrict_
 // ---------------------------------------------------------------------------
 // launchers
 
+template <>
+void BatchLaunch<double>::bake(const BatchView<double>& b, int newton, cudaStream_t s)
+{
+    k_bake_batch<<<b.ntiles ? b.ntiles : 1, kFxTileThreads, 0, s>>>(b, newton);
+    launch_counter()++;
+}
+
 template <typename S>
 void BatchLaunch<S>::tile_spmv(const BatchView<S>& b, const S* d, const S* r, S* part,
                                cudaGraphConditionalHandle if_refresh, int set_if, const unsigned* refresh_flag,
                                cudaStream_t s)
 {
     prof_begin(sizeof(S) == 8 ? "tile_spmv_fp64" : "tile_spmv_mixed", s);
-    k_tile_spmv<S><<<b.ntiles ? b.ntiles : 1, kTileElems, 0, s>>>(b, d, r, part, if_refresh, set_if, refresh_flag);
+    // FP64 only: the mixed path's product is launch_tile_spmv_pipe
+    if constexpr (sizeof(S) == 8)
+        k_tile_product_fp64<true><<<b.ntiles ? b.ntiles : 1, kFxTileThreads, 0, s>>>(b, d, r, part);
     prof_end(sizeof(S) == 8 ? "tile_spmv_fp64" : "tile_spmv_mixed", s);
     launch_counter()++;
 }
@@ -1218,8 +1303,11 @@ void BatchLaunch<S>::tile_spmv_y64(const BatchView<S>& b, const double* y, doubl
 {
     const char* name = sizeof(S) == 8 ? "y_product_fp64" : "y_product_mixed";
     prof_begin(name, s);
-    k_tile_spmv_y64<S><<<grid_tiles(b.ntiles), kTileElems, 0, s>>>(b, y, part64,
-                                                                   refresh ? SPMV_Y64_REFRESH : SPMV_Y64_ALL, flag);
+    if constexpr (sizeof(S) == 8)  // FP64: the start's product only (no refreshes)
+        k_tile_product_fp64<false><<<b.ntiles ? b.ntiles : 1, kFxTileThreads, 0, s>>>(b, y, nullptr, part64);
+    else
+        k_tile_spmv_y64<S><<<grid_tiles(b.ntiles), kTileElems, 0, s>>>(
+            b, y, part64, refresh ? SPMV_Y64_REFRESH : SPMV_Y64_ALL, flag);
     prof_end(name, s);
     launch_counter()++;
 }

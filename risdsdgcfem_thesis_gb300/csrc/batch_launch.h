@@ -77,6 +77,9 @@ struct BatchLaunch {
     // rotation.cu; newton: the re-evaluation at x_k of the FIE meshes that
     // have just updated (otherwise the meshes of the start section)
     static void begin_eval(const BatchView<S>& b, const double* x, int newton, cudaStream_t s);
+    // FP64, part of begin_eval: the product matrices of the evaluated C_WRP
+    // meshes (batch_kernels.cu)
+    static void bake(const BatchView<S>& b, int newton, cudaStream_t s);
     // newton: the Newton loop's while condition, set when newton_form (the
     // step has a Newton level: some mesh integrates with FIE)
     static void reset_counts(const BatchView<S>& b, const LoopSync& ls, cudaGraphConditionalHandle if_start,

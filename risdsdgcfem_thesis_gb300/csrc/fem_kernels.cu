@@ -17,7 +17,7 @@
 #include "fem_device.cuh"
 #include "msvd.cuh"
 #include "elem_math.cuh"
-#include "fx.cuh"
+#include "fx_device.cuh"
 
 #include <cooperative_groups.h>
 
@@ -236,13 +236,6 @@ __global__ void k_elem_lcm_spmv_fp64(MeshView<double> m, const double* __restric
 
 // ---- element kernels ----
 
-// Element e's groups: 32 apart.
-template <typename P>
-__device__ __forceinline__ P* fx_matrix(P* K, uint32_t e)
-{
-    return K + (size_t)kFxGroups * (e & ~31u) + (e & 31u);
-}
-
 // Element e's fixed-point product matrix (fx.cuh) from R, Dm^-1 and the
 // material scalars: 45 entries and the scale, 368 bytes, written once per
 // evaluation. Integer-bound: about 250 products of three multiplies (224 us
@@ -252,15 +245,7 @@ __global__ void __launch_bounds__(128, 3) k_elem_bake_fp64(MeshView<double> m)
     for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < m.T; e += gridDim.x * blockDim.x) {
         double R[9], Di[9], k1, knu, k2;
         load_elem(m, e, R, Di, k1, knu, k2);
-        FxL even{0, 0};
-        int4* Kp = fx_matrix(m.Kfx, e);
-        auto put = [&](int k, int64_t w) {  // two entries per 16-byte group
-            const FxL v = fx_split(w);
-            if ((k & 1) == 0) even = v;
-            else Kp[32 * (k >> 1)] = make_int4(even.l, even.h, v.l, v.h);
-        };
-        const int32_t scale = fx_grade_ok(m.grade[e], knu, k2) ? fx_bake(R, Di, knu, k2, put) : kFxFp64;
-        Kp[32 * (kFxGroups - 1)] = make_int4(even.l, even.h, scale, 0);
+        fx_store_matrix(m.Kfx, e, R, Di, knu, k2, m.grade[e]);
     }
 }
 
@@ -441,23 +426,22 @@ __device__ __forceinline__ double gather_fp64(const MeshView<double>& m, uint32_
     return s;
 }
 
-// The four lanes' record sums of a node (three components with one exponent
-// each) brought to the largest exponent and added: lane a's component.
-__device__ __forceinline__ double fx_quad_sum(const FxSum* s, uint32_t a, int32_t guard)
+// The four lanes' record sums of a node brought to the largest exponent and added: lane a's component.
+__device__ __forceinline__ double fx_quad_sum(const FxSum& s, uint32_t a, int32_t guard)
 {
-    int32_t E = s[0].E;
+    int32_t E = s.E;
     E = max(E, __shfl_xor_sync(0xffffffffu, E, 1));
     E = max(E, __shfl_xor_sync(0xffffffffu, E, 2));
-    const int32_t sh = fx_min63(E - s[0].E);
-    FxSum t{0, E};
+    const int32_t sh = fx_min63(E - s.E);
+    int64_t t = 0;
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-        long long v = s[c].acc >> sh;
+        long long v = s.acc[c] >> sh;
         v += __shfl_xor_sync(0xffffffffu, v, 1);
         v += __shfl_xor_sync(0xffffffffu, v, 2);
-        if ((int)a == c) t.acc = v;
+        if ((int)a == c) t = v;
     }
-    return fx_sum_value(t, guard);
+    return fx_sum_value(t, E, guard);
 }
 
 // Fixed-point records: lane l adds the corners beg + l, beg + l + 4, ... in
@@ -466,29 +450,28 @@ __device__ __forceinline__ double gather_fx(const MeshView<double>& m, uint32_t 
 {
     constexpr int kBatch = 3;  // records in flight per lane
     const int32_t guard = (int32_t)m.fx_guard;
-    FxSum s[3] = {{0, 0}, {0, 0}, {0, 0}};
+    FxSum s{{0, 0, 0}, 0};
     if (on) {
         const uint32_t beg = m.csr_ptr[n], end = m.csr_ptr[n + 1];
         const long long* rec = reinterpret_cast<const long long*>(m.eout);
         for (uint32_t j = beg + a; j < end; j += 4 * kBatch) {
+            // loaded without a branch, past the end the last one again
             int64_t v[kBatch][3];
+            uint32_t at[kBatch];
+#pragma unroll
+            for (int k = 0; k < kBatch; k++)
+                at[k] = bounds_idx(m.csr_idx[min(j + 4 * k, end - 1)], 4ull * m.T, kSiteCsrEntry);
 #pragma unroll
             for (int k = 0; k < kBatch; k++) {
-                v[k][0] = v[k][1] = v[k][2] = 0;  // an empty record: the lowest exponent
-                if (j + 4 * k < end) {
-                    const long long* r = rec + 3 * (size_t)bounds_idx(m.csr_idx[j + 4 * k], 4ull * m.T, kSiteCsrEntry);
-                    v[k][0] = r[0];
-                    v[k][1] = r[1];
-                    v[k][2] = r[2];
-                }
+                const long long* r = rec + 3 * (size_t)at[k];
+                const bool in = j + 4 * k < end;
+                v[k][0] = r[0];
+                v[k][1] = r[1];
+                v[k][2] = r[2];
+                if (!in) v[k][0] = v[k][1] = v[k][2] = 0;  // an empty record: the lowest exponent
             }
 #pragma unroll
-            for (int k = 0; k < kBatch; k++) {
-                const int32_t x = fx_record_exp(v[k][0], v[k][1], v[k][2]);
-                fx_add(s[0], v[k][0], x, guard);
-                fx_add(s[1], v[k][1], x, guard);
-                fx_add(s[2], v[k][2], x, guard);
-            }
+            for (int k = 0; k < kBatch; k++) fx_add(s, v[k][0], v[k][1], v[k][2], guard);
         }
     }
     return fx_quad_sum(s, a, guard);
@@ -1413,16 +1396,12 @@ __global__ void __launch_bounds__(kReg ? kCgClusterRegThreads : kCgClusterMaxThr
     };
     // the lane's component of node k's sum (gather_fx over the CTAs)
     auto gather = [&](int k) {
-        FxSum s[3] = {{0, 0}, {0, 0}, {0, 0}};
+        FxSum s{{0, 0, 0}, 0};
 #pragma unroll 2
         for (uint32_t j = cb[k]; j < ce[k]; j += 4) {
             const uint32_t w = cent[j];
             const long long* r = reinterpret_cast<const long long*>(cl.map_shared_rank(eo, w >> 24)) + 3 * (w & 0xffffffu);
-            const int64_t v0 = r[0], v1 = r[1], v2 = r[2];
-            const int32_t x = fx_record_exp(v0, v1, v2);
-            fx_add(s[0], v0, x, guard);
-            fx_add(s[1], v1, x, guard);
-            fx_add(s[2], v2, x, guard);
+            fx_add(s, r[0], r[1], r[2], guard);
         }
         return fx_quad_sum(s, a, guard);
     };

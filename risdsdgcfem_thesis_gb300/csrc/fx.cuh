@@ -172,8 +172,9 @@ FX_HD bool fx_stamp(int64_t* out, int32_t x)
     return true;
 }
 
-// The record of 12 FP64 outputs.
-FX_HD void fx_stamp_doubles(const double* v, int64_t* out)
+// 12 FP64 outputs as integers; returns their units' exponent + 2048 (kFxNan
+// with zeros when one is not finite).
+FX_HD int32_t fx_from_doubles(const double* v, int64_t* out)
 {
     int32_t E = 0;
 #pragma unroll
@@ -181,32 +182,41 @@ FX_HD void fx_stamp_doubles(const double* v, int64_t* out)
         const int32_t e = fx_exp(v[k]);
         E = e > E ? e : E;
     }
-    if (E == 2047) {
 #pragma unroll
-        for (int k = 0; k < 12; k++) out[k] = 15;
-        return;
-    }
-#pragma unroll
-    for (int k = 0; k < 12; k++) out[k] = fx_align<61>(v[k], E);
-    fx_stamp(out, E - 1022 - 61);
+    for (int k = 0; k < 12; k++) out[k] = E == 2047 ? 0 : fx_align<61>(v[k], E);
+    return E == 2047 ? kFxNan : E - 1022 - 61 + 2048;
 }
 
-// The running sum of one component's records: acc in units of 2^(E - 2048 +
-// guard), the guard bits sized so that a node's entries cannot overflow.
+// The record of 12 FP64 outputs.
+FX_HD void fx_stamp_doubles(const double* v, int64_t* out)
+{
+    const int32_t b = fx_from_doubles(v, out);
+#pragma unroll
+    for (int k = 0; k < 12; k++) out[k] = (out[k] & ~15ll) | ((b >> (4 * (k % 3))) & 15);
+}
+
+// The running sum of a node's records: acc in units of 2^(E - 2048 + guard),
+// the guard bits sized so that a node's records cannot overflow.
 struct FxSum {
-    int64_t acc;
+    int64_t acc[3];
     int32_t E;
 };
 FX_HD int32_t fx_min63(int32_t s) { return s > 63 ? 63 : s; }
-FX_HD void fx_add(FxSum& s, int64_t m, int32_t e, int32_t guard)
+FX_HD void fx_add(FxSum& s, int64_t v0, int64_t v1, int64_t v2, int32_t e, int32_t guard)
 {
-    const int32_t up = e > s.E ? e - s.E : 0, down = (e < s.E ? s.E - e : 0) + guard;
-    s.acc = (s.acc >> fx_min63(up)) + (m >> fx_min63(down));
+    const int32_t up = fx_min63(e > s.E ? e - s.E : 0), down = fx_min63((e < s.E ? s.E - e : 0) + guard);
+    s.acc[0] = (s.acc[0] >> up) + (v0 >> down);
+    s.acc[1] = (s.acc[1] >> up) + (v1 >> down);
+    s.acc[2] = (s.acc[2] >> up) + (v2 >> down);
     s.E = e > s.E ? e : s.E;
 }
-FX_HD double fx_sum_value(const FxSum& s, int32_t guard)
+FX_HD void fx_add(FxSum& s, int64_t v0, int64_t v1, int64_t v2, int32_t guard)
 {
-    return s.E == kFxNan ? fx_from_bits(0x7ff8000000000000ull) : fx_to_double(s.acc, s.E - 2048 + guard);
+    fx_add(s, v0, v1, v2, fx_record_exp(v0, v1, v2), guard);
+}
+FX_HD double fx_sum_value(int64_t acc, int32_t E, int32_t guard)
+{
+    return E == kFxNan ? fx_from_bits(0x7ff8000000000000ull) : fx_to_double(acc, E - 2048 + guard);
 }
 
 // K9's packed upper triangle: entry (r, c), r <= c, of the 9 x 9 matrix whose

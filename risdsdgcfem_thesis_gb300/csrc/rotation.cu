@@ -175,9 +175,7 @@ __global__ void __launch_bounds__(256, 3) k_begin_eval_batch(BatchView<S> b, con
         // newton: the FIE meshes whose solve has just updated x_k
         // (BeginEvaluation(x^n, x_k), LeafDSH_Solid3D_FEM.cpp:1529; their
         // DAPD previous positions are x^n); otherwise the start section's
-        if (newton ? ((!b.lock && b.mc[tm.mesh].integrator == kMeshQie) || !b.st[tm.mesh].finished)
-                   : !mesh_starts(b, tm.mesh))
-            continue;
+        if (!mesh_evaluates(b, tm.mesh, newton)) continue;
         if (threadIdx.x == 0) { s_inv = 0; s_res = 0; s_cause[0] = s_cause[1] = s_cause[2] = s_cause[3] = 0; }
         __syncthreads();
         if (threadIdx.x < tm.ne) {
@@ -313,6 +311,7 @@ void BatchLaunch<S>::begin_eval(const BatchView<S>& b, const double* x, int newt
     k_begin_eval_batch<S><<<grid_tiles(b.ntiles), kTileElems, 0, s>>>(b, x, newton);
     prof_end("begin_eval_batch", s);
     launch_counter()++;
+    if constexpr (sizeof(S) == 8) bake(b, newton, s);
 }
 
 template void BatchLaunch<double>::begin_eval(const BatchView<double>&, const double*, int, cudaStream_t);

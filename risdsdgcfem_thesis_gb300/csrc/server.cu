@@ -102,7 +102,7 @@ struct Shard {
 uint64_t estimate_bytes(uint32_t precision, uint64_t T, uint64_t N, uint64_t M)
 {
     const bool fp64 = precision == FEM_PRECISION_FP64;
-    const uint64_t per_tet = fp64 ? 300 : 310;
+    const uint64_t per_tet = fp64 ? 600 : 310;
     const uint64_t per_node = fp64 ? 400 : 330;
     return per_tet * T + per_node * N + 512 * M + (1u << 20);
 }
