@@ -273,9 +273,11 @@ int fem_solid_get_params(fem_solid s, fem_params* params);
  * blocks per node on grid meshes, rows padded to a multiple of four), 628 B
  * per tet for the assembly and one assembly per evaluation (about five
  * iterations' time); the sums run in another order, so other bits, within
- * the same parity tolerances. Other materials keep the element product, and so does the
- * one-cluster CG of solids of at most 8,192 tets. FEM_E_OOM when the blocks
- * do not fit. */
+ * the same parity tolerances. Other materials keep the element product. The
+ * CG of a C_WRP solid whose rows fit the GPU's shared memory (about 130,000
+ * tets on grid meshes) keeps them there in either setting, in memory it takes
+ * at its first solve; without that memory it runs as above. FEM_E_OOM when
+ * the blocks asked for do not fit. */
 int fem_solid_set_assembled(fem_solid s, int on);
 
 /* Replaces: the multi-solid Newton lock-step phases of the Leaf,

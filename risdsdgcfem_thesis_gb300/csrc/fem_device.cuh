@@ -21,6 +21,7 @@
 #include <stdint.h>
 
 #include "lcm.cuh"
+#include "rows_plan.h"
 
 namespace femgb {
 
@@ -267,25 +268,20 @@ void launch_bsr_assemble_fp64(const MeshView<double>& m, const BsrBuild& a, cuda
 void launch_bsr_vector_fp64(const MeshView<double>& m, const double* u, const StepScalars* st, int check_done,
                             cudaStream_t s);
 
-// The whole CG solve of a small C_WRP solid on one thread-block cluster
-// (fem_kernels.cu): CTA r of `ctas` owns the elements [r ept, (r+1) ept) and
-// the nodes [r npt, (r+1) npt); ent_max bounds a CTA's CSR entries; smem is
-// its dynamic shared memory (cg_cluster_smem_bytes).
-constexpr uint32_t kCgClusterMaxCtas = 16, kCgClusterMaxThreads = 512, kCgClusterRegThreads = 256;
-constexpr size_t kCgClusterMaxSmem = 200 * 1024;
-// nodes: per four lanes (1, 2 or 4; npt <= nodes threads / 4).
-struct CgClusterPlan {
-    uint32_t ctas, threads, ept, npt, ent_max, nodes;
-    size_t smem;
+// The CG solve on resident rows (cg_rows.cu): the layout's tables (rows_plan.h).
+struct CgRowsView {
+    const CgRowsBlock* blk;
+    const uint32_t *node, *group, *slot, *halo, *owner;
+    const uint16_t* col;
+    ulonglong2* words;  // [3 N]: r for other clusters
+    ulonglong2* parts;  // [2][blocks][clusters]: the clusters' sums
+    uint32_t cluster, warps, npb, units, records;  // CgRowsPlan's
+    uint32_t* seq;  // the last number used
 };
-size_t cg_cluster_smem_bytes(uint32_t ept, uint32_t npt, uint32_t ent_max);
-// The plan launches on this device (its cluster size, threads and shared
-// memory give at least one resident cluster).
-bool cg_cluster_fits(const CgClusterPlan& p);
-// ent: per CSR entry, (CTA owning the corner's element) << 24 | (local
-// element index * 4 + corner).
-cudaError_t launch_cg_cluster_fp64(const MeshView<double>& m, const StepConsts& c, const CgClusterPlan& p,
-                                   const uint32_t* ent, const double* b, double* y, StepScalars* st, cudaStream_t s);
+// The blocks of the plan's shape that are resident together; 0 when it does not launch.
+uint32_t cg_rows_max_blocks(const CgRowsPlan& p);
+cudaError_t launch_cg_rows_fp64(const MeshView<double>& m, const StepConsts& c, const CgRowsPlan& plan,
+                                const CgRowsView& p, const double* b, double* y, StepScalars* st, cudaStream_t s);
 
 // Launch shapes of the grid-stride kernels. One FP64 instruction of a warp
 // holds its sub-partition for 64 clocks, so small launches spread one warp

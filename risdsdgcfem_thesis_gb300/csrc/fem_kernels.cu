@@ -19,8 +19,6 @@
 #include "elem_math.cuh"
 #include "fx_device.cuh"
 
-#include <cooperative_groups.h>
-
 #include <map>
 #include <mutex>
 #include <string>
@@ -672,8 +670,7 @@ __global__ void __launch_bounds__(128) k_bsr_slots_fp64(MeshView<double> m, BsrB
 // Each row to one exponent, in place, and its diagonal block as minus the sum
 // of the others (an element's blocks sum to zero along a row), exactly as the
 // row now holds them: rigid translations have no force. Entries below 2^60,
-// less a bit per doubling of the row beyond 16 blocks (the product's
-// headroom).
+// their magnitudes along a matrix row below 2^62 (the products' headroom).
 __global__ void k_bsr_rows_fp64(MeshView<double> m, BsrBuild b)
 {
     const uint32_t a = threadIdx.x & 3u, step = (gridDim.x * blockDim.x) >> 2;
@@ -688,43 +685,60 @@ __global__ void k_bsr_rows_fp64(MeshView<double> m, BsrBuild b)
 #pragma unroll
             for (int k = 0; k < 9; k++) E = max(E, fx_exp(val[36 * (size_t)g + 4 * k + a]));
         }
-        int32_t room = 0, guard = 0;  // bits for the diagonal's sum, and for the product
+        int32_t room = 0;  // bits for the sums of a row
         while ((2u << room) < end - beg) room++;
-        while ((4u << guard) < end - beg) guard++;
 #pragma unroll
         for (int o = 1; o <= 2; o <<= 1) {
             E = max(E, __shfl_xor_sync(0xffffffffu, E, o));
             diag = min(diag, __shfl_xor_sync(0xffffffffu, diag, o));
         }
         long long sum[9];
+        unsigned long long mag[3] = {0, 0, 0};  // eighths
 #pragma unroll
         for (int k = 0; k < 9; k++) sum[k] = 0;
-        uint64_t top = 1;
         for (uint32_t g = beg; g < end; g++)
 #pragma unroll
             for (int k = 0; k < 9; k++) {
                 const int64_t v = fx_align<60>(val[36 * (size_t)g + 4 * k + a], E) >> room;
                 sum[k] += v;
-                top |= fx_mag(v);
+                mag[k / 3] += fx_mag(v) >> 3;
             }
+        uint64_t top = 1;
 #pragma unroll
         for (int k = 0; k < 9; k++) {
             sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], 1);
             sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], 2);
             top |= fx_mag(sum[k]);
         }
-        uint32_t bits = 64 - fx_clz(top);
-        bits = max(bits, __shfl_xor_sync(0xffffffffu, bits, 1));
-        bits = max(bits, __shfl_xor_sync(0xffffffffu, bits, 2));
-        const int32_t down = max(0, (int32_t)bits - (60 - guard));
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+            mag[r] += __shfl_xor_sync(0xffffffffu, mag[r], 1);
+            mag[r] += __shfl_xor_sync(0xffffffffu, mag[r], 2);
+#pragma unroll
+            for (int c = 0; c < 3; c++) mag[r] += fx_mag(sum[3 * r + c]) >> 3;
+        }
+        const int32_t bits = 64 - fx_clz(top), bits3 = 67 - fx_clz((mag[0] | mag[1] | mag[2]) + 1);
+        const int32_t down = max(0, max(bits - 60, bits3 - 62));
+#pragma unroll
+        for (int k = 0; k < 9; k++) sum[k] = 0;
         for (uint32_t g = beg; g < end; g++)
 #pragma unroll
             for (int k = 0; k < 9; k++) {
                 const size_t i = 36 * (size_t)g + 4 * k + a;
-                const int64_t v = 4 * g + a == diag ? -sum[k] : fx_align<60>(val[i], E) >> room;
-                const FxL l = fx_split(v >> down);
+                const int64_t v = (fx_align<60>(val[i], E) >> room) >> down;
+                sum[k] += v;
+                const FxL l = fx_split(v);
                 b.val[i] = make_int2(l.l, l.h);
             }
+#pragma unroll
+        for (int k = 0; k < 9; k++) {
+            sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], 1);
+            sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], 2);
+            if (on && (diag & 3u) == a) {
+                const FxL l = fx_split(-sum[k]);
+                b.val[36 * (size_t)(diag >> 2) + 4 * k + a] = make_int2(l.l, l.h);
+            }
+        }
         if (on && a == 0) b.x[n] = E < 2047 ? E - 1082 + room + down : kFxFp64;
     }
 }
@@ -1297,258 +1311,6 @@ __global__ void k_finalize(int kind, const double* __restrict__ partials, uint32
     }
     if (set_cond && (kind == FIN_INIT || kind == FIN_MR_INIT))
         cudaGraphSetConditional(cond, st->done ? 0u : 1u);
-}
-
-// The whole of ILSS_CG::Solve (ILSS_CG.h:38-151) for a C_WRP solid of up to
-// kCgClusterMaxCtas x kCgClusterMaxThreads tets on one thread-block cluster,
-// on chip. CTA r owns the elements [r ept, (r+1) ept), one per thread, and the
-// nodes [r npt, (r+1) npt), kNodes per four lanes, whose y, r, d, q and b
-// components stay in the lanes' registers. An element product (fx.cuh; kReg:
-// the matrix in registers, else read from L2 each time) reads its four nodes'
-// d from the owning CTAs' shared memory (distributed shared memory) and
-// leaves its records in its own; a node's lanes add its corners' records the
-// same way (ent: per CSR entry, the owning CTA << 24 | its local corner). A
-// reduction leaves each CTA's block total in a slot of every CTA, and every
-// warp adds the slots, so all CTAs take the same scalar steps and leave the
-// loop together. Four cluster barriers per iteration: element records
-// complete, d.q, |r|^2, the new d. y and the statistics are written back at
-// the end; the loop ends on the solver's own tests (at most max_iter
-// iterations).
-template <bool kReg, int kNodes>
-__global__ void __launch_bounds__(kReg ? kCgClusterRegThreads : kCgClusterMaxThreads, 1)
-    k_cg_cluster_fp64(MeshView<double> m, StepConsts c, CgClusterPlan p, const uint32_t* __restrict__ ent,
-                      const double* __restrict__ b, double* y, StepScalars* st)
-{
-    namespace cgr = cooperative_groups;
-    cgr::cluster_group cl = cgr::this_cluster();
-    extern __shared__ __align__(16) unsigned char cl_smem[];
-    const uint32_t tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, rank = cl.block_rank(), C = p.ctas;
-    const uint32_t N = m.N, T = m.T;
-    const uint32_t e0 = rank * p.ept, n0 = rank * p.npt;
-    const uint32_t ne = e0 < T ? min(p.ept, T - e0) : 0u, nn = n0 < N ? min(p.npt, N - n0) : 0u;
-    longlong2* eo = reinterpret_cast<longlong2*>(cl_smem);                 // [6 ept]
-    double* vd = reinterpret_cast<double*>(eo + 6 * (size_t)p.ept);          // [3 npt]
-    double* part = vd + 3 * (size_t)p.npt;                                  // [3][kCgClusterMaxCtas]
-    uint32_t* cent = reinterpret_cast<uint32_t*>(part + 3 * kCgClusterMaxCtas);  // [ent_max]
-    __shared__ StepScalars sst;
-    __shared__ double wsum[kCgClusterMaxThreads / 32];
-    const double mfm = c.mass * c.factor_M;
-    const int32_t guard = (int32_t)m.fx_guard;
-    const uint32_t base = nn ? m.csr_ptr[n0] : 0u;
-    const uint32_t ne_ent = nn ? min(m.csr_ptr[n0 + nn] - base, p.ent_max) : 0u;
-    for (uint32_t i = tid; i < ne_ent; i += nt) cent[i] = ent[base + i];
-    if (tid == 0) sst = *st;
-    auto sync = [&] {
-        if (C == 1) __syncthreads();
-        else cl.sync();
-    };
-    // this lane's components: node tid / 4 + k nt / 4, component a
-    const uint32_t a = tid & 3u;
-    double ny[kNodes], nr[kNodes], nd[kNodes], nq[kNodes];
-    uint32_t cb[kNodes], ce[kNodes];
-    bool live[kNodes];  // the component exists and is not constrained
-#pragma unroll
-    for (int k = 0; k < kNodes; k++) {
-        const uint32_t ln = (tid >> 2) + k * (nt >> 2);
-        const bool on = ln < nn;
-        cb[k] = on ? m.csr_ptr[n0 + ln] - base + a : 0u;
-        ce[k] = on ? min(m.csr_ptr[n0 + ln + 1] - base, ne_ent) : 0u;
-        live[k] = on && a < 3 && !m.fixed[n0 + ln];
-        ny[k] = on && a < 3 ? y[3 * (size_t)(n0 + ln) + a] : 0.0;
-        nr[k] = nd[k] = nq[k] = 0.0;
-        if (on && a < 3) vd[3 * ln + a] = ny[k];
-    }
-    // this thread's element
-    const bool has_elem = tid < ne;
-    const uint32_t e = has_elem ? e0 + tid : 0u;
-    const int4* Kp = fx_matrix(m.Kfx, e);
-    const int32_t scale = has_elem ? Kp[32 * (kFxGroups - 1)].z : kFxFp64;
-    FxL K[kReg ? kFxK : 1];
-    if constexpr (kReg) {
-#pragma unroll
-        for (int g = 0; g < (int)kFxGroups; g++) {
-            const int4 v = has_elem ? Kp[32 * g] : make_int4(0, 0, 0, 0);
-            K[2 * g] = FxL{v.x, v.y};
-            if (2 * g + 1 < kFxK) K[2 * g + 1] = FxL{v.z, v.w};
-        }
-    }
-    const double* pd[4] = {vd, vd, vd, vd};
-    if (has_elem) {
-        const int4 t = m.tets[e];
-        const uint32_t ids[4] = {bounds_idx((uint32_t)t.x, N, kSiteElemNode), bounds_idx((uint32_t)t.y, N, kSiteElemNode),
-                                 bounds_idx((uint32_t)t.z, N, kSiteElemNode), bounds_idx((uint32_t)t.w, N, kSiteElemNode)};
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const uint32_t nrk = ids[k] / p.npt;
-            pd[k] = cl.map_shared_rank(vd, nrk) + 3 * (ids[k] - nrk * p.npt);
-        }
-    }
-    auto product = [&] {
-        if (has_elem) {
-            int4 cur;
-            elem_records(m, e, scale, [&](int k) {
-                if constexpr (kReg) return K[k];
-                if ((k & 1) == 0) cur = __ldg(Kp + 32 * (k >> 1));
-                return (k & 1) ? FxL{cur.z, cur.w} : FxL{cur.x, cur.y};
-            }, pd, eo + 6 * tid);
-        }
-        sync();  // all element records complete
-    };
-    // the lane's component of node k's sum (gather_fx over the CTAs)
-    auto gather = [&](int k) {
-        FxSum s{{0, 0, 0}, 0};
-#pragma unroll 2
-        for (uint32_t j = cb[k]; j < ce[k]; j += 4) {
-            const uint32_t w = cent[j];
-            const long long* r = reinterpret_cast<const long long*>(cl.map_shared_rank(eo, w >> 24)) + 3 * (w & 0xffffffu);
-            fx_add(s, r[0], r[1], r[2], guard);
-        }
-        return fx_quad_sum(s, a, guard);
-    };
-    // the cluster's total of every thread's acc, in every thread
-    auto cluster_total = [&](double acc, int slot) -> double {
-        double v = fx_warp_sum(acc);
-        if (nt > 32) {
-            if (lane == 0) wsum[tid >> 5] = v;
-            __syncthreads();
-            if (tid < 32) v = fx_warp_sum(lane < (nt >> 5) ? wsum[lane] : 0.0);
-        }
-        if (tid < C) cl.map_shared_rank(part, tid)[slot * kCgClusterMaxCtas + rank] = v;
-        sync();
-        return fx_warp_sum(lane < C ? part[slot * kCgClusterMaxCtas + lane] : 0.0);
-    };
-    sync();  // every CTA's y is in place
-    for (bool start = true;; start = false) {
-        // the start: r = S(b - A y), d = r, |r|^2; then q = S A d, d.q, alpha
-        product();
-        double acc = 0.0;
-#pragma unroll
-        for (int k = 0; k < kNodes; k++) {
-            const double s = gather(k);
-            const uint32_t ln = (tid >> 2) + k * (nt >> 2);
-            if (start) {
-                if (live[k]) nr[k] = nd[k] = b[3 * (size_t)(n0 + ln) + a] - (c.factor_K * s + mfm * ny[k]);
-                if (ln < nn && a < 3) vd[3 * ln + a] = nd[k];
-                acc += nr[k] * nr[k];
-            } else {
-                if (live[k]) nq[k] = c.factor_K * s + mfm * nd[k];
-                acc += nd[k] * nq[k];
-            }
-        }
-        double total = cluster_total(acc, start ? 0 : 1);  // at the start its barrier completes d too
-        if (tid == 0) {
-            if (start) fin_init(&sst, c, total);
-            else fin_alpha(&sst, total);
-        }
-        __syncthreads();
-        if (sst.done) break;
-        if (start) continue;
-        // y += alpha d, r -= alpha q, |r|^2, beta and the loop test
-        const double alpha = sst.alpha, na = -alpha;
-        acc = 0.0;
-#pragma unroll
-        for (int k = 0; k < kNodes; k++) {
-            ny[k] += alpha * nd[k];
-            nr[k] += na * nq[k];
-            acc += nr[k] * nr[k];
-        }
-        total = cluster_total(acc, 2);
-        if (tid == 0) fin_beta(&sst, total);
-        __syncthreads();
-        if (sst.done) break;
-        // d = S (beta d + r)
-        const double beta = sst.beta;
-#pragma unroll
-        for (int k = 0; k < kNodes; k++) {
-            const uint32_t ln = (tid >> 2) + k * (nt >> 2);
-            nd[k] = beta * nd[k] + nr[k];
-            if (ln < nn && a < 3) vd[3 * ln + a] = nd[k];
-        }
-        sync();  // the new d is complete
-    }
-#pragma unroll
-    for (int k = 0; k < kNodes; k++) {
-        const uint32_t ln = (tid >> 2) + k * (nt >> 2);
-        if (ln < nn && a < 3) y[3 * (size_t)(n0 + ln) + a] = ny[k];
-    }
-    if (rank == 0 && tid == 0) {
-        fin_stats(&sst);
-        *st = sst;
-    }
-    sync();  // no CTA leaves while another may still read its shared memory
-}
-
-size_t cg_cluster_smem_bytes(uint32_t ept, uint32_t npt, uint32_t ent_max)
-{
-    return sizeof(double) * (12 * (size_t)ept + 3 * (size_t)npt + 3 * kCgClusterMaxCtas) + sizeof(uint32_t) * (size_t)ent_max;
-}
-
-namespace {
-using CgClusterKernel = void (*)(MeshView<double>, StepConsts, CgClusterPlan, const uint32_t*, const double*, double*,
-                                 StepScalars*);
-// The instance for a plan: matrices in registers while the threads leave room
-// for them, else one, two or four nodes per four lanes.
-CgClusterKernel cg_cluster_kernel(const CgClusterPlan& p)
-{
-    if (p.nodes == 1) return p.threads <= kCgClusterRegThreads ? k_cg_cluster_fp64<true, 1> : k_cg_cluster_fp64<false, 1>;
-    return p.nodes == 2 ? k_cg_cluster_fp64<false, 2> : k_cg_cluster_fp64<false, 4>;
-}
-cudaError_t cg_cluster_attrs()
-{
-    static const cudaError_t e = [] {
-        for (auto* k : {k_cg_cluster_fp64<true, 1>, k_cg_cluster_fp64<false, 1>, k_cg_cluster_fp64<false, 2>,
-                        k_cg_cluster_fp64<false, 4>}) {
-            cudaError_t r = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCgClusterMaxSmem);
-            if (r == cudaSuccess) r = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-            if (r != cudaSuccess) return r;
-        }
-        return cudaSuccess;
-    }();
-    return e;
-}
-void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& at, const CgClusterPlan& p, cudaStream_t s)
-{
-    cfg = cudaLaunchConfig_t{};
-    cfg.gridDim = dim3(p.ctas);
-    cfg.blockDim = dim3(p.threads);
-    cfg.dynamicSmemBytes = p.smem;
-    cfg.stream = s;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = p.ctas;
-    at.val.clusterDim.y = 1;
-    at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-}
-}  // namespace
-
-bool cg_cluster_fits(const CgClusterPlan& p)
-{
-    if (p.ctas < 1 || p.ctas > kCgClusterMaxCtas || p.threads < 32 || p.threads > kCgClusterMaxThreads ||
-        p.threads % 32 || p.smem > kCgClusterMaxSmem || p.ept > p.threads ||
-        (p.nodes != 1 && p.nodes != 2 && p.nodes != 4) || 4 * (size_t)p.npt > (size_t)p.nodes * p.threads ||
-        cg_cluster_attrs() != cudaSuccess)
-        return false;
-    cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute at;
-    cluster_config(cfg, at, p, nullptr);
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, cg_cluster_kernel(p), &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return n >= 1;
-}
-
-cudaError_t launch_cg_cluster_fp64(const MeshView<double>& m, const StepConsts& c, const CgClusterPlan& p,
-                                   const uint32_t* ent, const double* b, double* y, StepScalars* st, cudaStream_t s)
-{
-    if (const cudaError_t e = cg_cluster_attrs(); e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute at;
-    cluster_config(cfg, at, p, s);
-    launch_counter()++;
-    return cudaLaunchKernelEx(&cfg, cg_cluster_kernel(p), m, c, p, ent, b, y, st);
 }
 
 // ---- launchers ----

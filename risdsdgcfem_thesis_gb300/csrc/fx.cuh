@@ -465,16 +465,29 @@ FX_HD double fx_wide_value(const FxWide& s, int32_t x)
 // The sum of a warp's doubles, the same in every lane: aligned to the largest
 // exponent and added exactly in three limbs by integer reductions. About 150
 // clocks; five FP64 adds and ten shuffles take about 600. The result is
-// within 2^-52 of the largest term.
-__device__ __forceinline__ double fx_warp_sum(double v)
+// within 2^-52 (several terms per lane: 2^-49) of the largest term.
+template <int K>
+__device__ __forceinline__ double fx_warp_sum(const double (&v)[K])  // K terms per lane
 {
-    const int32_t E = __reduce_max_sync(0xffffffffu, fx_exp(v));
+    static_assert(K >= 1 && K <= 5, "the limbs' headroom");
+    constexpr int kBits = K == 1 ? 57 : 55;
+    int32_t E = fx_exp(v[0]);
+#pragma unroll
+    for (int k = 1; k < K; k++) E = max(E, fx_exp(v[k]));
+    E = __reduce_max_sync(0xffffffffu, E);
     if (E == 2047) return __longlong_as_double(0x7ff8000000000000ll);
-    const int64_t m = fx_align<57>(v, E);
+    int64_t m = 0;
+#pragma unroll
+    for (int k = 0; k < K; k++) m += fx_align<kBits>(v[k], E);
     const uint32_t l0 = __reduce_add_sync(0xffffffffu, (uint32_t)m & 0xffffffu);
     const uint32_t l1 = __reduce_add_sync(0xffffffffu, (uint32_t)(m >> 24) & 0xffffffu);
     const int32_t l2 = __reduce_add_sync(0xffffffffu, (int32_t)(m >> 48));
-    return fx_to_double((int64_t)l0 + ((int64_t)l1 << 24) + ((int64_t)((uint64_t)(int64_t)l2 << 48)), E - 1022 - 57);
+    return fx_to_double((int64_t)l0 + ((int64_t)l1 << 24) + ((int64_t)((uint64_t)(int64_t)l2 << 48)), E - 1022 - kBits);
+}
+__device__ __forceinline__ double fx_warp_sum(double v)
+{
+    const double t[1] = {v};
+    return fx_warp_sum(t);
 }
 #endif
 

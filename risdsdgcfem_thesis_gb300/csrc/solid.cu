@@ -114,19 +114,24 @@ struct fem_solid_s {
     bool kfx_fresh = false;
     DevBuf<uint32_t> csr_ptr, csr_idx;
     DevBuf<uint8_t> fixed;
-    // the one-cluster CG of a small solid (ctas 0: none); cl_ent as csr_idx,
-    // each entry as the owning CTA and its local corner
-    CgClusterPlan cl_plan{};
-    DevBuf<uint32_t> cl_ent;
+    // the CG solve on resident rows (blocks 0: none), over the assembled
+    // stiffness below
+    CgRowsPlan rows{};
+    bool rows_tried = false;
+    DevBuf<CgRowsBlock> rows_blk;
+    DevBuf<uint32_t> rows_node, rows_group, rows_slot, rows_halo, rows_owner, rows_seq;
+    DevBuf<uint16_t> rows_col;
+    DevBuf<ulonglong2> rows_words;
     // the assembled stiffness (MeshView::bsr_*): pattern, per-slot
-    // contributions and blocks; bsr_use: the solvers take it (set_bsr_use)
+    // contributions and blocks; bsr_fresh: the blocks are those of the last
+    // evaluation; bsr_use: the solvers' kernels take it (set_bsr_use)
     DevBuf<uint32_t> bsr_row, bsr_col, bsr_cptr, bsr_contrib;
     DevBuf<int2> bsr_val;
     DevBuf<int32_t> bsr_x, bsr_ex;
     DevBuf<longlong2> bsr_u;
     DevBuf<long long> bsr_eblk;
     uint32_t bsr_groups = 0;  // of four blocks
-    bool bsr_want = false, bsr_use = false;  // fem_solid_set_assembled; the solvers take it now
+    bool bsr_fresh = false, bsr_want = false, bsr_use = false;  // fem_solid_set_assembled; the solvers take it now
     // node vectors
     DevBuf<double> rest, x, v, y, b, r, d, q, tmp;
     DevBuf<double> xn, vn;  // FIE: x^n and v^n of the step (allocated for the FIE integrators only)
@@ -190,6 +195,21 @@ struct fem_solid_s {
         bsr_u.release();
         bsr_eblk.release();
         bsr_groups = 0;
+        bsr_fresh = false;
+        release_rows();
+    }
+    void release_rows()
+    {
+        rows_blk.release();
+        rows_node.release();
+        rows_group.release();
+        rows_slot.release();
+        rows_halo.release();
+        rows_owner.release();
+        rows_seq.release();
+        rows_col.release();
+        rows_words.release();
+        rows = CgRowsPlan{};
     }
 
     MeshView<double> view()
@@ -233,7 +253,6 @@ struct fem_solid_s {
         tets.release();
         csr_ptr.release();
         csr_idx.release();
-        cl_ent.release();
         release_bsr();
         fixed.release();
         knc_nodes.release();
@@ -341,17 +360,18 @@ void set_consts(fem_solid s)
     s->dapd.eNL = (double)(float)params->dapd_nl_exponent;
 }
 
-// The assembled stiffness on the last rotations.
+// The assembled stiffness and the product matrices of a C_WRP solid on its
+// last rotations, made by the first product or solve that needs them.
 void assemble(fem_solid s)
 {
+    if (s->bsr_fresh) return;
     MeshView<double> m = s->view();
-    m.bsr_row = s->bsr_row.p;  // also before the solvers take it (bsr_use)
+    m.bsr_row = s->bsr_row.p;  // also when the solvers' kernels do not take it (bsr_use)
     m.bsr_col = s->bsr_col.p;
     launch_bsr_assemble_fp64(m, BsrBuild{s->bsr_groups, s->bsr_cptr.p, s->bsr_contrib.p, s->bsr_eblk.p, s->bsr_ex.p,
                                          s->bsr_val.p, s->bsr_x.p}, s->stream);
+    s->bsr_fresh = true;
 }
-
-// The fixed-point product matrices of a C_WRP solid on its last rotations.
 void bake_products(fem_solid s)
 {
     if (uses_lcm(s) || s->kfx_fresh) return;
@@ -369,11 +389,7 @@ void begin_eval(fem_solid s, const double* xprev, const double* x)
         launch_begin_eval_dapd_fp64(m, xprev, x, s->doc.p, s->dapd, F_out, s->st.p, s->stream);
     else
         launch_begin_eval_fp64(m, x, F_out, s->st.p, s->stream);
-    // the solvers' operator on the new rotations
-    s->kfx_fresh = false;
-    if (s->bsr_use) assemble(s);
-    else
-        bake_products(s);
+    s->kfx_fresh = s->bsr_fresh = false;
 }
 
 // The material's element force at x (C_f_e / C_LCM_f_e) into m.eout and/or
@@ -401,8 +417,9 @@ void elem_spmv(fem_solid s, const MeshView<double>& m, const double* d, int chec
 // those take K u from the assembled stiffness, else the element outputs.
 void solve_product(fem_solid s, const MeshView<double>& m, const double* d, int check_done)
 {
-    if (m.bsr_val) launch_bsr_vector_fp64(m, d, s->st.p, check_done, s->stream);
-    else elem_spmv(s, m, d, check_done);
+    if (!m.bsr_val) return elem_spmv(s, m, d, check_done);
+    assemble(s);
+    launch_bsr_vector_fp64(m, d, s->st.p, check_done, s->stream);
 }
 
 // FixedStep's opening: BeginEvaluation(m_vecPos0, x), then m_vecPos0 = x
@@ -417,127 +434,146 @@ int open_step(fem_solid s)
     return FEM_OK;
 }
 
-// A C_WRP solid with a one-cluster CG plan: its iteration is four cluster
-// barriers instead of four launches.
-bool cg_on_cluster(const fem_solid s)
+// A solid whose CG solve runs on resident rows (cg_rows.cu).
+bool wants_rows(const fem_params& p) { return p.material == FEM_MATERIAL_C_WRP && p.ls_solver != FEM_LS_MINRES; }
+bool cg_on_rows(const fem_solid s)
 {
-    return s->params.material == FEM_MATERIAL_C_WRP && s->cl_plan.ctas > 0;
+    return wants_rows(s->params) && s->rows.blocks > 0;
 }
 
-// Whether the solvers take K u from the assembled stiffness (asked for by
-// fem_solid_set_assembled and built): a C_WRP solid whose solve is not the
-// one-cluster CG. The assembled rows read 81 bytes per block and iteration,
-// about 230 per tet on grid meshes, where the element product reads and
-// writes 580 per tet; an assembly costs about as much as five products.
+// Whether the solvers' kernels take K u from the assembled stiffness (asked
+// for by fem_solid_set_assembled and built): a C_WRP solid whose solve is not
+// on resident rows, which are assembled anyway. The assembled rows read 81
+// bytes per block and iteration, about 230 per tet on grid meshes, where the
+// element product reads and writes 580 per tet; an assembly costs about as
+// much as five products.
 void set_bsr_use(fem_solid s)
 {
-    s->bsr_use = s->bsr_want && s->bsr_groups > 0 && s->params.material == FEM_MATERIAL_C_WRP &&
-                 !(s->params.ls_solver != FEM_LS_MINRES && cg_on_cluster(s));
+    s->bsr_use = s->bsr_want && s->bsr_groups > 0 && s->params.material == FEM_MATERIAL_C_WRP && !cg_on_rows(s);
 }
 
-// The assembled stiffness's pattern and contributions (MeshView::bsr_*): row n
-// holds n's neighbours through its elements and n itself, ascending, padded
-// with n to a multiple of four; slot (n, j), j other than n, sums the corner
-// pairs (li of n, lj of j) of the elements holding both, in element order.
-// ptr/idx: the node CSR of element corners.
-int build_bsr(fem_solid s, const uint32_t* tets, const std::vector<uint32_t>& ptr, const std::vector<uint32_t>& idx)
+template <typename V>
+cudaError_t put(DevBuf<V>& d, const std::vector<V>& h, cudaStream_t st)
 {
-    const uint32_t N = s->N, T = s->T;
-    if ((uint64_t)T >= (1ull << 28)) return FEM_OK;  // contributions pack the element in 28 bits
-    std::vector<uint32_t> brow(N + 1, 0), used(N), bcol, nb;
-    bcol.reserve(18 * (size_t)N);
-    for (uint32_t n = 0; n < N; n++) {
-        nb.clear();
-        nb.push_back(n);
-        for (uint32_t j = ptr[n]; j < ptr[n + 1]; j++) {
-            const size_t e = idx[j] >> 2;
-            for (int k = 0; k < 4; k++) nb.push_back(tets[4 * e + k]);
-        }
-        std::sort(nb.begin(), nb.end());
-        nb.erase(std::unique(nb.begin(), nb.end()), nb.end());
-        used[n] = (uint32_t)nb.size();
-        while (nb.size() % 4) nb.push_back(n);
-        bcol.insert(bcol.end(), nb.begin(), nb.end());
-        if (bcol.size() >= (1ull << 28)) return FEM_OK;
-        brow[n + 1] = (uint32_t)(bcol.size() / 4);
-    }
-    const size_t slots = bcol.size();
-    auto slot_of = [&](uint32_t n, uint32_t col) {
-        const auto b = bcol.begin() + 4 * (size_t)brow[n];
-        return (size_t)(std::lower_bound(b, b + used[n], col) - bcol.begin());
-    };
-    std::vector<uint32_t> bcptr(slots + 1, 0), bcon(12 * (size_t)T), at(12 * (size_t)T);
-    size_t k = 0;
-    for (uint32_t n = 0; n < N; n++)
-        for (uint32_t j = ptr[n]; j < ptr[n + 1]; j++)
-            for (uint32_t lj = 0; lj < 4; lj++) {
-                if (lj == (idx[j] & 3u)) continue;
-                at[k] = (uint32_t)slot_of(n, tets[4 * (size_t)(idx[j] >> 2) + lj]);
-                bcptr[at[k++] + 1]++;
-            }
-    for (size_t i = 0; i < slots; i++) bcptr[i + 1] += bcptr[i];
-    {
-        std::vector<uint32_t> fill(bcptr.begin(), bcptr.end() - 1);
-        k = 0;
-        for (uint32_t n = 0; n < N; n++)
-            for (uint32_t j = ptr[n]; j < ptr[n + 1]; j++) {
-                const uint32_t e = idx[j] >> 2, li = idx[j] & 3u;
-                for (uint32_t lj = 0; lj < 4; lj++)
-                    if (lj != li) bcon[fill[at[k++]]++] = (e << 4) | (li << 2) | lj;
-            }
-    }
+    if (cudaError_t e = d.alloc(h.size()); e != cudaSuccess) return e;
+    return cudaMemcpyAsync(d.p, h.data(), sizeof(V) * h.size(), cudaMemcpyHostToDevice, st);
+}
+
+// Uploads the pattern and allocates the blocks.
+int upload_bsr(fem_solid s, const BsrPattern& p)
+{
+    const size_t slots = p.col.size();
     cudaStream_t st = s->stream;
-    CK(s->bsr_row.alloc(N + 1));
-    CK(s->bsr_col.alloc(slots));
-    CK(s->bsr_cptr.alloc(slots + 1));
-    CK(s->bsr_contrib.alloc(bcon.size()));
+    CK(put(s->bsr_row, p.row, st));
+    CK(put(s->bsr_col, p.col, st));
+    CK(put(s->bsr_cptr, p.cptr, st));
+    CK(put(s->bsr_contrib, p.contrib, st));
     CK(s->bsr_val.alloc(9 * slots));
-    CK(s->bsr_x.alloc(N));
-    CK(s->bsr_u.alloc(2 * (size_t)N));
-    CK(s->bsr_ex.alloc(T));
-    CK(s->bsr_eblk.alloc((size_t)kBsrElemWords * T));
-    CK(cudaMemcpyAsync(s->bsr_row.p, brow.data(), sizeof(uint32_t) * brow.size(), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(s->bsr_col.p, bcol.data(), sizeof(uint32_t) * slots, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(s->bsr_cptr.p, bcptr.data(), sizeof(uint32_t) * bcptr.size(), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(s->bsr_contrib.p, bcon.data(), sizeof(uint32_t) * bcon.size(), cudaMemcpyHostToDevice, st));
+    CK(s->bsr_x.alloc(s->N));
+    CK(s->bsr_u.alloc(2 * (size_t)s->N));
+    CK(s->bsr_ex.alloc(s->T));
+    CK(s->bsr_eblk.alloc((size_t)kBsrElemWords * s->T));
     CK(cudaStreamSynchronize(st));
     s->bsr_groups = (uint32_t)(slots / 4);
     return FEM_OK;
 }
 
-// The one-cluster CG plan of a solid (see cg_on_cluster): one element per
-// thread and one node per four lanes, one CTA up to 192 tets (160 tets: 545 us
-// per step against 617 on two to sixteen, whose barriers cost more than the
-// spread saves), then 96 tets per CTA (1,080: 691 us; 256 per CTA: 750). When
-// a cluster of that size does not fit, the fewest CTAs below it that do; none
-// when the solid is too large. ptr: the node CSR's row starts.
-CgClusterPlan plan_cg_cluster(uint32_t N, uint32_t T, const std::vector<uint32_t>& ptr)
+// The CG solve on resident rows of a C_WRP solid that can have it: the
+// pattern, its blocks and the layout.
+int build_rows(fem_solid s, const uint32_t* tets, const std::vector<uint32_t>& ptr, const std::vector<uint32_t>& idx)
 {
-    if (T == 0 || N == 0) return CgClusterPlan{};
-    auto try_plan = [&](uint32_t C, CgClusterPlan& p) {
-        p = CgClusterPlan{};
-        p.ctas = C;
-        p.ept = (T + C - 1) / C;
-        p.npt = (N + C - 1) / C;
-        uint32_t emax = 0;
-        for (uint32_t r = 0; r < C; r++) {
-            const uint32_t a = std::min(N, r * p.npt), b = std::min(N, (r + 1) * p.npt);
-            emax = std::max(emax, ptr[b] - ptr[a]);
-        }
-        p.ent_max = emax;
-        const uint32_t lanes = 4 * p.npt;
-        p.nodes = lanes <= kCgClusterMaxThreads ? 1 : (lanes <= 2 * kCgClusterMaxThreads ? 2 : 4);
-        p.threads = (std::max(p.ept, (lanes + p.nodes - 1) / p.nodes) + 31) / 32 * 32;
-        p.smem = cg_cluster_smem_bytes(p.ept, p.npt, p.ent_max);
-        return p.threads <= kCgClusterMaxThreads && cg_cluster_fits(p);
-    };
-    CgClusterPlan p{};
-    const uint32_t want = T <= 192 ? 1u : std::min<uint32_t>(kCgClusterMaxCtas, (T + 95) / 96);
-    for (uint32_t C = want; C >= 1; C--) {
-        if ((T + C - 1) / C > kCgClusterMaxThreads) break;  // fewer CTAs only take more
-        if (try_plan(C, p)) return p;
+    BsrPattern p;
+    CgRowsLayout l;
+    if (!bsr_pattern(s->N, s->T, tets, ptr, idx, p) || !cg_rows_layout(s->N, p, cg_rows_max_blocks, l)) return FEM_OK;
+    if (!s->bsr_groups)
+        if (int e = upload_bsr(s, p)) return e;
+    cudaStream_t st = s->stream;
+    CK(put(s->rows_blk, l.blk, st));
+    CK(put(s->rows_node, l.node, st));
+    CK(put(s->rows_group, l.group, st));
+    CK(put(s->rows_slot, l.slot, st));
+    CK(put(s->rows_col, l.col, st));
+    CK(put(s->rows_halo, l.halo, st));
+    CK(put(s->rows_owner, l.owner, st));
+    const size_t words = 3 * (size_t)s->N + 2 * (size_t)l.plan.blocks * (l.plan.blocks / l.plan.cluster);
+    CK(s->rows_words.alloc(words));
+    CK(s->rows_seq.alloc(1));
+    CK(cudaMemsetAsync(s->rows_words.p, 0, sizeof(ulonglong2) * words, st));
+    CK(cudaMemsetAsync(s->rows_seq.p, 0, sizeof(uint32_t), st));
+    CK(cudaStreamSynchronize(st));
+    s->rows = l.plan;
+    return FEM_OK;
+}
+
+// The mesh's tables, back from the device.
+int read_tables(fem_solid s, std::vector<uint32_t>& tets, std::vector<uint32_t>& ptr, std::vector<uint32_t>& idx)
+{
+    const uint32_t N = s->N, T = s->T;
+    std::vector<int4> t4(T);
+    tets.resize(4 * (size_t)T);
+    ptr.resize(N + 1);
+    idx.resize(4 * (size_t)T);
+    CK(cudaMemcpyAsync(t4.data(), s->tets.p, sizeof(int4) * T, cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaMemcpyAsync(ptr.data(), s->csr_ptr.p, sizeof(uint32_t) * (N + 1), cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaMemcpyAsync(idx.data(), s->csr_idx.p, sizeof(uint32_t) * idx.size(), cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaStreamSynchronize(s->stream));
+    for (uint32_t e = 0; e < T; e++) {
+        tets[4 * (size_t)e] = (uint32_t)t4[e].x;
+        tets[4 * (size_t)e + 1] = (uint32_t)t4[e].y;
+        tets[4 * (size_t)e + 2] = (uint32_t)t4[e].z;
+        tets[4 * (size_t)e + 3] = (uint32_t)t4[e].w;
     }
-    return CgClusterPlan{};
+    return FEM_OK;
+}
+
+// build_rows ahead of the first solve that wants it (a solid used for its
+// products only does not pay for it); without the device memory for them the
+// solve stays on the loop of kernels. Meshes far above the GPU's shared memory
+// (a closed tetrahedral mesh has about N + T edges) are not looked at.
+int try_rows(fem_solid s)
+{
+    if (s->rows_tried || !wants_rows(s->params)) return FEM_OK;
+    s->rows_tried = true;
+    if (72.0 * (3.0 * s->N + 2.0 * s->T) > 1.2 * kCgRowsMaxBlocks * kCgRowsMaxSmem) return FEM_OK;
+    const std::string keep = g_err;
+    const bool had_bsr = s->bsr_groups > 0;
+    int rc = FEM_E_OOM;
+    try {
+        std::vector<uint32_t> tets, ptr, idx;
+        if (int e = read_tables(s, tets, ptr, idx)) return e;
+        rc = build_rows(s, tets.data(), ptr, idx);
+    } catch (const std::bad_alloc&) {
+    }
+    if (rc != FEM_OK) {
+        cudaGetLastError();
+        if (had_bsr) s->release_rows();
+        else s->release_bsr();
+        g_err = keep;
+    }
+    set_bsr_use(s);
+    return FEM_OK;
+}
+
+// The CG solve on resident rows, enqueued.
+cudaError_t solve_on_rows(fem_solid s, const StepConsts& c)
+{
+    assemble(s);
+    MeshView<double> m = s->view();
+    m.bsr_val = s->bsr_val.p;
+    m.bsr_x = s->bsr_x.p;
+    const CgRowsPlan& p = s->rows;
+    const CgRowsView v{s->rows_blk.p, s->rows_node.p, s->rows_group.p, s->rows_slot.p, s->rows_halo.p, s->rows_owner.p,
+                       s->rows_col.p, s->rows_words.p, s->rows_words.p + 3 * (size_t)s->N, p.cluster, p.warps, p.npb,
+                       p.units, p.records, s->rows_seq.p};
+    return launch_cg_rows_fp64(m, c, s->rows, v, s->b.p, s->y.p, s->st.p, s->stream);
+}
+
+// The solve's status as an error of the call.
+int solve_status(const StepScalars& h)
+{
+    if (h.status == FEM_E_NAN) return fail(FEM_E_NAN, "NaN or Inf in the CG residual");
+    if (h.status == FEM_E_TIMEOUT) return fail(FEM_E_TIMEOUT, "a device-side wait of the linear solve gave up");
+    return FEM_OK;
 }
 
 // ILSS_CG::Solve (ILSS_CG.h:38-151) of A y = b from the warm start in y,
@@ -546,14 +582,15 @@ CgClusterPlan plan_cg_cluster(uint32_t N, uint32_t T, const std::vector<uint32_t
 // chunk of iterations).
 int cg_solve(fem_solid s, const StepConsts& c, int chunk)
 {
+    if (int e = try_rows(s)) return e;
     cudaStream_t st = s->stream;
     MeshView<double> m = s->view();
-    if (cg_on_cluster(s)) {
-        CK(launch_cg_cluster_fp64(m, c, s->cl_plan, s->cl_ent.p, s->b.p, s->y.p, s->st.p, st));
+    if (cg_on_rows(s)) {
+        CK(solve_on_rows(s, c));
         CK(cudaMemcpyAsync(s->st_host, s->st.p, sizeof(StepScalars), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         CK(cudaGetLastError());
-        return FEM_OK;
+        return s->st_host->status == FEM_E_TIMEOUT ? solve_status(*s->st_host) : FEM_OK;
     }
     const uint32_t gN = node_grid(s->N, m.bsr_val != nullptr), gV = vec_grid(3 * s->N);
     solve_product(s, m, s->y.p, 0);
@@ -631,8 +668,7 @@ cudaError_t ls_solve_capture(fem_solid s, const StepConsts& c, cudaGraph_t top)
     cudaStream_t st = s->stream;
     MeshView<double> m = s->view();
     const uint32_t gN = node_grid(s->N, m.bsr_val != nullptr), gV = vec_grid(3 * s->N);
-    if (s->params.ls_solver != FEM_LS_MINRES && cg_on_cluster(s))
-        return launch_cg_cluster_fp64(m, c, s->cl_plan, s->cl_ent.p, s->b.p, s->y.p, s->st.p, st);
+    if (cg_on_rows(s)) return solve_on_rows(s, c);
     cudaGraphConditionalHandle cond = 0;
     cudaError_t e = cudaGraphConditionalHandleCreate(&cond, top, 0, cudaGraphCondAssignDefault);
     if (e != cudaSuccess) return e;
@@ -793,6 +829,7 @@ void qie_tail(fem_solid s)
 int capture_step(fem_solid s)
 {
     s->drop_graph();
+    if (int e = try_rows(s)) return e;
     cudaStream_t st = s->stream;
     CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
     cudaGraph_t top = nullptr;
@@ -807,6 +844,7 @@ int capture_step(fem_solid s)
     cudaGraph_t g = nullptr;
     const cudaError_t e2 = cudaStreamEndCapture(st, &g);
     if (e == cudaSuccess) e = e2;
+    s->kfx_fresh = s->bsr_fresh = false;  // captured, not run
     if (rc != FEM_OK || e != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
         if (rc != FEM_OK) return rc;
@@ -826,7 +864,9 @@ int step_once(fem_solid s, int chunk)
     if (!s->exec)
         if (int e = capture_step(s)) return e;
     CK(cudaGraphLaunch(s->exec, s->stream));
-    s->kfx_fresh = !uses_lcm(s) && !s->bsr_use;  // baked by the graph's evaluation
+    // made by the graph's solve on its evaluation
+    s->bsr_fresh = s->bsr_use || cg_on_rows(s);
+    s->kfx_fresh = !uses_lcm(s) && !s->bsr_fresh;
     return FEM_OK;
 }
 void fill_stats(fem_solid s, const StepScalars& h, fem_step_stats* out)
@@ -891,7 +931,7 @@ int fem_bounds_check_status(int* enabled, uint32_t* failures, uint32_t* site, ui
 #else
     const int on = 0;
 #endif
-    int (*const units[])(unsigned*) = {bounds_read_fem_kernels, bounds_read_rotation, bounds_read_batch_kernels,
+    int (*const units[])(unsigned*) = {bounds_read_fem_kernels, bounds_read_cg_rows, bounds_read_rotation, bounds_read_batch_kernels,
                                        bounds_read_tile_pipe};
     unsigned total = 0, first[3] = {0u, 0u, 0u};
     for (auto rd : units) {
@@ -1080,17 +1120,6 @@ int fem_solid_create(const double* rest_xyz, uint32_t N, const uint32_t* tets, u
     CKC(cudaMemcpyAsync(s->grade.p, grade.data(), sizeof(float) * T, cudaMemcpyHostToDevice, st));
     CKC(cudaMemcpyAsync(s->csr_ptr.p, ptr.data(), sizeof(uint32_t) * (N + 1), cudaMemcpyHostToDevice, st));
     CKC(cudaMemcpyAsync(s->csr_idx.p, idx.data(), sizeof(uint32_t) * idx.size(), cudaMemcpyHostToDevice, st));
-    s->cl_plan = plan_cg_cluster(N, T, ptr);
-    if (s->cl_plan.ctas) {
-        std::vector<uint32_t> ent(idx.size());
-        for (size_t j = 0; j < idx.size(); j++) {
-            const uint32_t e = idx[j] >> 2, r = e / s->cl_plan.ept;
-            ent[j] = (r << 24) | (4 * (e - r * s->cl_plan.ept) + (idx[j] & 3));
-        }
-        CKC(s->cl_ent.alloc(ent.size()));
-        CKC(cudaMemcpyAsync(s->cl_ent.p, ent.data(), sizeof(uint32_t) * ent.size(), cudaMemcpyHostToDevice, st));
-        CKC(cudaStreamSynchronize(st));
-    }
     set_bsr_use(s);
     CKC(cudaMemsetAsync(s->fixed.p, 0, N, st));
     CKC(cudaMemcpyAsync(s->rest.p, rest_xyz, sizeof(double) * n3, cudaMemcpyHostToDevice, st));
@@ -1134,27 +1163,14 @@ int fem_solid_set_assembled(fem_solid s, int on)
     if (int e = check_handle(s)) return e;
     s->drop_graph();  // the step graph holds the operator's launches
     if (on && !s->bsr_groups) {
-        const uint32_t N = s->N, T = s->T;
-        std::vector<int4> t4(T);
-        std::vector<uint32_t> tets(4 * (size_t)T), ptr(N + 1), idx(4 * (size_t)T);
-        CK(cudaMemcpyAsync(t4.data(), s->tets.p, sizeof(int4) * T, cudaMemcpyDeviceToHost, s->stream));
-        CK(cudaMemcpyAsync(ptr.data(), s->csr_ptr.p, sizeof(uint32_t) * (N + 1), cudaMemcpyDeviceToHost, s->stream));
-        CK(cudaMemcpyAsync(idx.data(), s->csr_idx.p, sizeof(uint32_t) * idx.size(), cudaMemcpyDeviceToHost,
-                           s->stream));
-        CK(cudaStreamSynchronize(s->stream));
-        for (uint32_t e = 0; e < T; e++) {
-            tets[4 * (size_t)e] = (uint32_t)t4[e].x;
-            tets[4 * (size_t)e + 1] = (uint32_t)t4[e].y;
-            tets[4 * (size_t)e + 2] = (uint32_t)t4[e].z;
-            tets[4 * (size_t)e + 3] = (uint32_t)t4[e].w;
-        }
-        if (int e = build_bsr(s, tets.data(), ptr, idx)) {
-            s->release_bsr();
-            return e;
-        }
-        // the current rotations' blocks, for a solve before the next evaluation
-        if (s->bsr_groups) assemble(s);
-        CK(cudaStreamSynchronize(s->stream));
+        std::vector<uint32_t> tets, ptr, idx;
+        if (int e = read_tables(s, tets, ptr, idx)) return e;
+        BsrPattern p;
+        if (bsr_pattern(s->N, s->T, tets.data(), ptr, idx, p))
+            if (int e = upload_bsr(s, p)) {
+                s->release_bsr();
+                return e;
+            }
     }
     s->bsr_want = on != 0;
     set_bsr_use(s);
@@ -1261,7 +1277,7 @@ int fem_solid_set_params(fem_solid s, const fem_params* params)
         const double E = params->young_modulus, nu = params->poisson_ratio;
         const double a = E / ((1.0 + nu) * (1.0 - 2.0 * nu));  // Compute_E (TetrahedronElement3.h:141-156)
         launch_rebake_material_fp64(s->T, s->vol.p, a * (1.0 - nu), a * nu, a * (0.5 - nu), s->mat.p, s->stream);
-        s->kfx_fresh = false;
+        s->kfx_fresh = s->bsr_fresh = false;
         CK(cudaGetLastError());
     }
     CK(cudaStreamSynchronize(s->stream));
@@ -1342,7 +1358,7 @@ int fem_solid_nr_midstep(fem_solid s, double dt)
     if (int e = ls_solve(s, c, 8)) return e;
     s->lock_ls_iters += s->st_host->k;
     CK(cudaGetLastError());
-    if (s->st_host->status == FEM_E_NAN) return fail(FEM_E_NAN, "NaN or Inf in the CG residual");
+    if (int e = solve_status(*s->st_host)) return e;
     return FEM_OK;
 }
 
@@ -1469,7 +1485,7 @@ int fem_solid_synchronize(fem_solid s, fem_step_stats* stats)
     CK(cudaMemcpyAsync(s->st_host, s->st.p, sizeof(StepScalars), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     if (stats) fill_stats(s, *s->st_host, stats);
-    if (s->st_host->status == FEM_E_NAN) return fail(FEM_E_NAN, "NaN or Inf in the CG residual");
+    if (int e = solve_status(*s->st_host)) return e;
     return FEM_OK;
 }
 

@@ -1,0 +1,140 @@
+"""Host tables of the CG solve on resident rows (rows_plan.h) on the CPU: a
+product through them against the mesh's own adjacency, every index in range."""
+import ctypes as C
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+from risdsdgcfem_thesis_gb300 import scenes
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "risdsdgcfem_thesis_gb300", "csrc")
+SHIM = r"""
+#include "rows_plan.h"
+using namespace femgb;
+// y = A d with A(n, c) = a[n] b[c] for neighbours c, n itself included;
+// returns 0, -1 without a layout, else the line of a failed check.
+#define CHECK(x) do { if (!(x)) return __LINE__; } while (0)
+extern "C" int rows(uint32_t N, uint32_t T, const uint32_t* tets, uint32_t sms, const double* a, const double* d,
+                    double* y, uint32_t* contribs, uint32_t* blocks)
+{
+    std::vector<uint32_t> ptr(N + 1, 0), idx(4 * (size_t)T);
+    for (size_t i = 0; i < 4 * (size_t)T; i++) ptr[tets[i] + 1]++;
+    for (uint32_t n = 0; n < N; n++) ptr[n + 1] += ptr[n];
+    std::vector<uint32_t> fill(ptr.begin(), ptr.end() - 1);
+    for (size_t i = 0; i < 4 * (size_t)T; i++) idx[fill[tets[i]]++] = (uint32_t)i;
+    BsrPattern p;
+    CHECK(bsr_pattern(N, T, tets, ptr, idx, p));
+    const size_t slots = p.col.size();
+    CHECK(p.row[N] * (size_t)4 == slots && p.cptr[slots] == 12 * (size_t)T && p.contrib.size() == 12 * (size_t)T);
+    for (uint32_t n = 0; n < N; n++)
+        for (uint32_t s = 4 * p.row[n]; s < 4 * p.row[n + 1]; s++) {
+            CHECK(p.col[s] < N);
+            for (uint32_t k = p.cptr[s]; k < p.cptr[s + 1]; k++) {
+                const uint32_t e = p.contrib[k] >> 4, li = (p.contrib[k] >> 2) & 3, lj = p.contrib[k] & 3;
+                CHECK(e < T && li != lj && tets[4 * e + li] == n && tets[4 * e + lj] == p.col[s]);
+                contribs[0]++;
+            }
+        }
+    CgRowsLayout l;
+    if (!cg_rows_layout(N, p, [&](const CgRowsPlan& q) {
+            return q.threads > kCgRowsMaxThreads || q.smem > kCgRowsMaxSmem || q.cluster > sms ? 0u : sms;
+        }, l)) return -1;
+    const uint32_t L = l.plan.lanes, rows = 32 / L;
+    CHECK(l.plan.blocks == l.blk.size() && l.plan.blocks <= sms && l.node.size() == N);
+    CHECK(l.plan.threads % 32 == 0 && l.plan.threads <= kCgRowsMaxThreads);
+    const uint32_t G = l.plan.blocks, K = l.plan.cluster;
+    CHECK(G % K == 0 && K * l.plan.warps <= 160 && G / K <= 96 && l.owner.size() == l.halo.size());
+    std::vector<int> used(slots, 0), seen(N, 0);
+    std::vector<uint32_t> in_rim(N, 0);
+    for (size_t g = 0; g < l.blk.size(); g++) {
+        const CgRowsBlock b = l.blk[g];
+        CHECK(3 * b.nn <= 32 * l.plan.warps && 32 * l.plan.warps + (b.nhalo ? 32 : 0) <= l.plan.threads);
+        CHECK(cg_rows_smem_bytes(l.plan, b) <= l.plan.smem && b.nn <= l.plan.npb && b.units <= l.plan.units);
+        CHECK(b.nn + b.nhalo <= l.plan.records);
+        CHECK(l.group.size() >= b.group0 + b.ngroups + 1 && l.group[b.group0] == 0 && l.group[b.group0 + b.ngroups] == b.units);
+        CHECK(rows * b.ngroups >= b.nn && 32 * (size_t)(b.unit0 + b.units) <= l.slot.size() && l.slot.size() == l.col.size());
+        for (uint32_t w = 0; w < b.ngroups; w++)
+            for (uint32_t lane = 0; lane < 32; lane++) {
+                const uint32_t row = rows * w + lane / L;
+                for (uint32_t u = l.group[b.group0 + w]; u < l.group[b.group0 + w + 1]; u++) {
+                    const size_t at = 32 * (size_t)(b.unit0 + u) + lane;
+                    const uint32_t s = l.slot[at], c = l.col[at];
+                    CHECK(c < b.nn + b.nhalo);
+                    if (s == kCgRowsPad) continue;
+                    CHECK(row < b.nn && s < slots);
+                    const uint32_t n = l.node[b.node0 + row] & kCgRowsNode;
+                    const uint32_t gc = c < b.nn ? l.node[b.node0 + c] & kCgRowsNode : l.halo[b.halo0 + c - b.nn];
+                    CHECK(n < N && gc < N && p.col[s] == gc && s >= 4 * p.row[n] && s < 4 * p.row[n + 1]);
+                    used[s]++;
+                    if (c >= b.nn) {
+                        const uint32_t o = l.owner[b.halo0 + c - b.nn], near = g / K * K + (o >> 16);
+                        in_rim[gc] |= o == kCgRowsFar ? kCgRowsFarShared : kCgRowsNearShared;
+                        CHECK(o == kCgRowsFar || (near < G && (o & 0xffff) < l.blk[near].nn &&
+                                                  (l.node[l.blk[near].node0 + (o & 0xffff)] & kCgRowsNode) == gc));
+                    }
+                    y[n] += a[n] * a[gc] * d[gc];
+                }
+            }
+        for (uint32_t i = 0; i < b.nn; i++) seen[l.node[b.node0 + i] & kCgRowsNode]++;
+    }
+    for (uint32_t n = 0; n < N; n++) CHECK(seen[n] == 1);
+    for (uint32_t w : l.node) CHECK((w & ~kCgRowsNode) == in_rim[w & kCgRowsNode]);
+    for (uint32_t n = 0; n < N; n++)
+        for (uint32_t k = 0; k < 4 * (p.row[n + 1] - p.row[n]); k++) CHECK(used[4 * p.row[n] + k] == (k < p.used[n]));
+    *blocks = l.plan.blocks;
+    return 0;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def shim(tmp_path_factory):
+    if shutil.which("g++") is None:
+        pytest.skip("no host compiler")
+    d = tmp_path_factory.mktemp("rows")
+    src, lib = d / "rows.cpp", d / "rows.so"
+    src.write_text(SHIM)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", CSRC, str(src), "-o", str(lib)], check=True)
+    return C.CDLL(str(lib))
+
+
+def _star(k):
+    """k tets around one node, which every other node neighbours."""
+    t = np.arange(3 * k, dtype=np.uint32).reshape(k, 3) + 1
+    return 3 * k + 1, np.concatenate([np.zeros((k, 1), np.uint32), t], 1)
+
+
+def _grid(*dims):
+    rest, tets, _ = scenes.grid_mesh(*dims, 0.1, 0.01, 5)
+    return len(rest), tets
+
+
+@pytest.mark.parametrize("sms", [2, 16, 152])
+@pytest.mark.parametrize("mesh,shuffle", [(_grid(1, 1, 1), False), (_grid(5, 5, 5), False), (_grid(6, 6, 5), True),
+                                          (_grid(17, 16, 15), False), (_grid(17, 16, 15), True), (_star(150), False),
+                                          ((9, _grid(1, 1, 1)[1]), False), (_grid(45, 40, 40), False)],
+                         ids=["cell", "216", "294shuffled", "20400", "20400shuffled", "star", "lone", "360000"])
+def test_layout_covers_the_rows(shim, mesh, shuffle, sms):
+    n, tets = mesh
+    rng = np.random.default_rng(2)
+    if shuffle:
+        tets = rng.permutation(n).astype(np.uint32)[tets]
+    tets = np.ascontiguousarray(tets, np.uint32)
+    a, d, y = rng.integers(-9, 10, n).astype(float), rng.integers(-9, 10, n).astype(float), np.zeros(n)
+    contribs, blocks = C.c_uint32(0), C.c_uint32(0)
+    dp = lambda v: v.ctypes.data_as(C.POINTER(C.c_double))
+    rc = shim.rows(n, len(tets), tets.ctypes.data_as(C.POINTER(C.c_uint32)), sms, dp(a), dp(d), dp(y),
+                   C.byref(contribs), C.byref(blocks))
+    assert contribs.value == 12 * len(tets)
+    if rc == -1:
+        assert n > 200 * sms  # about 1,000 bytes a row
+        return
+    assert rc == 0
+    pairs = np.unique(np.concatenate([np.stack([tets[:, i], tets[:, j]], 1) for i in range(4) for j in range(4)] +
+                                     [np.stack([np.arange(n)] * 2, 1)]), axis=0)
+    ref = np.zeros(n)
+    np.add.at(ref, pairs[:, 0], a[pairs[:, 0]] * a[pairs[:, 1]] * d[pairs[:, 1]])
+    assert np.array_equal(y, ref)
