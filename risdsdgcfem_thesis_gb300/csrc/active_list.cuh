@@ -48,33 +48,52 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* sh, ui
 
 // Tiles and chunks of the meshes m with pred(m), in mesh order, into
 // tiles[] / chunks[] and their counts into count2[0..1]. Called by every
-// thread of one block.
+// thread of one block: a thread per mesh finds where the mesh's entries go and
+// writes them, or, when some mesh of its warp has more than kListOwn, the warp
+// does, mesh by mesh (a 27,000-tet mesh's 107 tiles one after the other: 92 us
+// for the two lists of 192 such meshes, 25 us by warps; 24 meshes of 5 tiles:
+// 6 us against 16 by warps).
+constexpr uint32_t kListOwn = 16;
 template <typename S, typename P>
 __device__ void build_mesh_lists(const BatchView<S>& b, P pred, uint32_t* tiles, uint32_t* chunks,
                                  uint32_t* count2)
 {
     __shared__ uint32_t sh[32];
-    const uint32_t per = (b.M + blockDim.x - 1) / blockDim.x;
-    const uint32_t m0 = threadIdx.x * per, m1 = min(b.M, m0 + per);
-    uint32_t nt = 0, nc = 0;
-    for (uint32_t m = m0; m < m1; m++) {
-        if (pred(m)) {
-            nt += b.mc[m].ntiles;
-            nc += b.mc[m].nchunks;
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t done_t = 0, done_c = 0;
+    for (uint32_t base = 0; base < b.M; base += blockDim.x) {
+        const uint32_t m = base + threadIdx.x;
+        uint32_t t0 = 0, nt = 0, c0 = 0, nc = 0;
+        if (m < b.M) {
+            const MeshConsts& c = b.mc[m];
+            const bool in = pred(m);
+            t0 = c.tile0;
+            c0 = c.chunk0;
+            nt = in ? c.ntiles : 0u;
+            nc = in ? c.nchunks : 0u;
         }
-    }
-    uint32_t tot_t, tot_c;
-    uint32_t pt = block_excl_scan(nt, sh, &tot_t);
-    uint32_t pc = block_excl_scan(nc, sh, &tot_c);
-    for (uint32_t m = m0; m < m1; m++) {
-        if (!pred(m)) continue;
-        const MeshConsts& c = b.mc[m];
-        for (uint32_t k = 0; k < c.ntiles; k++) tiles[pt++] = c.tile0 + k;
-        for (uint32_t k = 0; k < c.nchunks; k++) chunks[pc++] = c.chunk0 + k;
+        uint32_t tot_t, tot_c;
+        const uint32_t pt = done_t + block_excl_scan(nt, sh, &tot_t);
+        const uint32_t pc = done_c + block_excl_scan(nc, sh, &tot_c);
+        if (__all_sync(0xffffffffu, nt <= kListOwn && nc <= kListOwn)) {
+            for (uint32_t k = 0; k < nt; k++) tiles[pt + k] = t0 + k;
+            for (uint32_t k = 0; k < nc; k++) chunks[pc + k] = c0 + k;
+            nt = nc = 0;
+        }
+        for (unsigned left = __ballot_sync(0xffffffffu, nt | nc); left; left &= left - 1) {
+            const int l = __ffs(left) - 1;
+            const uint32_t wt0 = __shfl_sync(0xffffffffu, t0, l), wnt = __shfl_sync(0xffffffffu, nt, l);
+            const uint32_t wc0 = __shfl_sync(0xffffffffu, c0, l), wnc = __shfl_sync(0xffffffffu, nc, l);
+            const uint32_t wpt = __shfl_sync(0xffffffffu, pt, l), wpc = __shfl_sync(0xffffffffu, pc, l);
+            for (uint32_t k = lane; k < wnt; k += 32) tiles[wpt + k] = wt0 + k;
+            for (uint32_t k = lane; k < wnc; k += 32) chunks[wpc + k] = wc0 + k;
+        }
+        done_t += tot_t;
+        done_c += tot_c;
     }
     if (threadIdx.x == 0) {
-        count2[0] = tot_t;
-        count2[1] = tot_c;
+        count2[0] = done_t;
+        count2[1] = done_c;
     }
     __syncthreads();
 }

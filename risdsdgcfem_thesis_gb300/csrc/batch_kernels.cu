@@ -1010,7 +1010,9 @@ __global__ void k_node_update(BatchView<S> b, double* __restrict__ y, S* __restr
 //   mr_pending 1 (an iteration): p_new = (v - r2 p - r3 p0) / r1,
 //     y += beta_one c eta p_new, p0 = p, p = p_new, v0 = v,
 //     v = v1 / beta_new (ILSS_MINRES.h:131-156).
-// The last block of the mesh clears the flag.
+// The last block of the mesh clears the flag. gridDim.y blocks share a chunk: a
+// chunk's 3,000 FP64 updates of y hold an SM's pipe for 3 us (24 small meshes:
+// 8.0 us with a block per chunk, 4.4 us with four).
 template <typename S>
 __global__ void k_node_mr_finish(BatchView<S> b, double* __restrict__ y, S* __restrict__ r, S* __restrict__ d,
                                  const S* __restrict__ q, LoopSync ls)
@@ -1029,9 +1031,10 @@ __global__ void k_node_mr_finish(BatchView<S> b, double* __restrict__ y, S* __re
         // the next entries go ahead of this entry's stores
         S* __restrict__ p = b.mr_p;
         S* __restrict__ p0 = b.mr_p0;
+        const size_t first = 3 * (size_t)ch.n0 + blockIdx.y * blockDim.x + threadIdx.x, step = gridDim.y * blockDim.x;
         if (pending == 2u) {
             const S inv = (S)mr.inv_beta;
-            for (size_t i = 3 * (size_t)ch.n0 + threadIdx.x; i < 3 * (size_t)ch.n1; i += blockDim.x) {
+            for (size_t i = first; i < 3 * (size_t)ch.n1; i += step) {
                 r[i] *= inv;
                 d[i] = 0;
                 p[i] = 0;
@@ -1040,7 +1043,7 @@ __global__ void k_node_mr_finish(BatchView<S> b, double* __restrict__ y, S* __re
         } else {
             const S inv = (S)mr.inv_beta, nr2 = (S)mr.neg_r2, nr3 = (S)mr.neg_r3, ir1 = (S)mr.inv_r1;
 #pragma unroll 4
-            for (size_t i = 3 * (size_t)ch.n0 + threadIdx.x; i < 3 * (size_t)ch.n1; i += blockDim.x) {
+            for (size_t i = first; i < 3 * (size_t)ch.n1; i += step) {
                 const S v = r[i];
                 const S pi = p[i];
                 S pn = nr2 * pi + v;
@@ -1053,7 +1056,7 @@ __global__ void k_node_mr_finish(BatchView<S> b, double* __restrict__ y, S* __re
                 r[i] = q[i] * inv;
             }
         }
-        if (arrive_last(ls.mcount + ch.mesh, c.nchunks) && threadIdx.x == 0) b.st[ch.mesh].mr_pending = 0u;
+        if (arrive_last(ls.mcount + ch.mesh, c.nchunks * gridDim.y) && threadIdx.x == 0) b.st[ch.mesh].mr_pending = 0u;
     }
 }
 
@@ -1376,7 +1379,8 @@ template <typename S>
 void BatchLaunch<S>::node_mr_finish(const BatchView<S>& b, double* y, S* r, S* d, const S* q, const LoopSync& ls,
                                     cudaStream_t s)
 {
-    k_node_mr_finish<S><<<grid_chunks(b.nchunks), kNodeThreads, 0, s>>>(b, y, r, d, q, ls);
+    const uint32_t g = grid_chunks(b.nchunks);
+    k_node_mr_finish<S><<<dim3(g, std::max(1u, std::min(4u, 608u / g))), kNodeThreads, 0, s>>>(b, y, r, d, q, ls);
     launch_counter()++;
 }
 
