@@ -178,7 +178,7 @@ struct fem_batch_s {
     Dev<uint32_t> blob_off16;
     Dev<uint32_t> act_tiles, act_chunks, act_count;
     Dev<unsigned> list_dirty;
-    Dev<unsigned> slice;                // [iteration budget of a launch (0 = none), iterations run]
+    Dev<unsigned> slice;                // [iteration budget of a launch (0 = none), iterations run, the loop goes on]
     Dev<uint32_t> start_tiles, start_chunks, launch_tiles, launch_chunks, refresh_tiles, refresh_chunks, list_count;
     uint32_t slice_budget = 0;
     std::vector<uint8_t> mask_host;     // last active mask (empty = all start)
@@ -199,6 +199,7 @@ struct fem_batch_s {
         b.ntiles = ntiles;
         b.nchunks = nchunks;
         b.pipe_tile = opt.tile_elems <= (uint32_t)kPipeSmallTile ? kPipeSmallTile : kTileElems;
+        b.loop_go = slice.p + 2;
         b.fuse_alpha = opt.fuse_alpha ? 1u : 0u;
         b.has_lcm = any_lcmh ? 2u : any_lcm ? 1u : 0u;
         b.lock = lock ? 1u : 0u;
@@ -480,21 +481,23 @@ int enqueue_step(fem_batch B, cudaStream_t s, bool capture, int lock_phase = 0)
     // the CG loop as a WHILE node after the capture point of `cs`
     auto capture_cg = [&](cudaStream_t cs) {
         return capture_conditional(cs, ls.cond, cudaGraphCondTypeWhile, [&](cudaStream_t bs, cudaGraph_t bodyg) {
-            cudaGraphConditionalHandle ifh = 0;
-            if (mixed) {
-                const cudaError_t e = cudaGraphConditionalHandleCreate(&ifh, bodyg, 0, 0);
-                if (e != cudaSuccess) return e;
+            for (unsigned i = 0; i < kLoopUnroll; i++) {
+                cudaGraphConditionalHandle ifh = 0;
+                if (mixed) {
+                    const cudaError_t e = cudaGraphConditionalHandleCreate(&ifh, bodyg, 0, 0);
+                    if (e != cudaSuccess) return e;
+                }
+                body_head(bs, ifh, mixed ? 1 : 0);
+                if (mixed) {
+                    // IF (some mesh refreshes this iteration) { FP64 product of y }
+                    const cudaError_t e = capture_conditional(bs, ifh, cudaGraphCondTypeIf, [&](cudaStream_t is, cudaGraph_t) {
+                        L::tile_spmv_y64(b, B->y.p, B->part64.p, 1, nullptr, is);
+                        return cudaGetLastError();
+                    });
+                    if (e != cudaSuccess) return e;
+                }
+                body_tail(bs);
             }
-            body_head(bs, ifh, mixed ? 1 : 0);
-            if (mixed) {
-                // IF (some mesh refreshes this iteration) { FP64 product of y }
-                const cudaError_t e = capture_conditional(bs, ifh, cudaGraphCondTypeIf, [&](cudaStream_t is, cudaGraph_t) {
-                    L::tile_spmv_y64(b, B->y.p, B->part64.p, 1, nullptr, is);
-                    return cudaGetLastError();
-                });
-                if (e != cudaSuccess) return e;
-            }
-            body_tail(bs);
             return cudaGetLastError();
         });
     };
@@ -1171,8 +1174,8 @@ int fem_batch_finalize(fem_batch b)
     BCKC(b->blob.upload(blob_h, s));
     BCKC(b->blob_off16.alloc(blob_off16_h.size()));
     BCKC(b->blob_off16.upload(blob_off16_h, s));
-    BCKC(b->slice.alloc(2));
-    BCKC(cudaMemsetAsync(b->slice.p, 0, 2 * sizeof(unsigned), s));
+    BCKC(b->slice.alloc(3));
+    BCKC(cudaMemsetAsync(b->slice.p, 0, 3 * sizeof(unsigned), s));
     BCKC(b->start_tiles.alloc(b->ntiles));
     BCKC(b->start_chunks.alloc(b->nchunks));
     BCKC(b->launch_tiles.alloc(b->ntiles));

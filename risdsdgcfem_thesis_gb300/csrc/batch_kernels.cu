@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(kFxTileThreads, 3)
     for (uint32_t it = blockIdx.x; it < n; it += gridDim.x) {
         const uint32_t t = kDir ? it : b.start_tiles[it];
         const TileMeta tm = b.tiles[t];
-        if (kDir ? !mesh_running(b, tm.mesh) : !mesh_starts(b, tm.mesh)) continue;
+        if (kDir ? !loop_on(b) || !mesh_running(b, tm.mesh) : !mesh_starts(b, tm.mesh)) continue;
         const double beta = kDir ? b.st[tm.mesh].beta : 0.0;
         const bool fixed_point = tm.material == kTileMaterialWrp;
         for (int i = threadIdx.x; i < tm.nn; i += blockDim.x) {
@@ -660,6 +660,7 @@ __device__ void grid_tail(const BatchView<S>& b, const LoopSync& ls, bool iterat
         if (ls.slice) {
             if (iteration) ls.slice[1] += 1u;
             budget_left = ls.slice[0] == 0u || ls.slice[1] < ls.slice[0];
+            ls.slice[2] = any && !stop && budget_left ? 1u : 0u;
         }
         if (ls.set_cond) cudaGraphSetConditional(ls.cond, (any && !stop && budget_left) ? 1u : 0u);
     }
@@ -891,7 +892,7 @@ __global__ void k_node_q(BatchView<S> b, const S* __restrict__ part, S* __restri
         const uint32_t ci = blockIdx.x;
         if (ci >= b.nchunks) return;
         const ChunkMeta ch = b.chunks[ci];
-        if (!mesh_running(b, ch.mesh)) return;
+        if (!loop_on(b) || !mesh_running(b, ch.mesh)) return;
         const MeshConsts& c = b.mc[ch.mesh];
         const StepScalars& sm = b.st[ch.mesh];
         if (c.solver == kMeshSolverMinres) {
@@ -960,6 +961,7 @@ __global__ void k_node_update(BatchView<S> b, double* __restrict__ y, S* __restr
 {
     const uint32_t ci = blockIdx.x;
     const ChunkMeta ch = b.chunks[ci < b.nchunks ? ci : 0];
+    if (!loop_on(b)) return;  // every block: the loop's arrivals too
     if (ci < b.nchunks && mesh_running(b, ch.mesh) && b.mc[ch.mesh].solver == kMeshSolverMinres) {
         node_update_minres(b, b.mc[ch.mesh], b.st[ch.mesh], ci, ch, r, q, cpart, ls);
     } else if (ci < b.nchunks && mesh_running(b, ch.mesh)) {
@@ -1246,7 +1248,10 @@ __global__ void k_reset_counts(BatchView<S> b, LoopSync ls, cudaGraphConditional
     build_mesh_lists(
         b, [&](uint32_t m) { return b.active[m] != 0; }, b.launch_tiles, b.launch_chunks, b.list_count + 2);
     if (threadIdx.x == 0) {
-        if (ls.slice) ls.slice[1] = 0u;
+        if (ls.slice) {
+            ls.slice[1] = 0u;
+            ls.slice[2] = cont ? 1u : 0u;
+        }
         if (ls.set_cond) {
             cudaGraphSetConditional(if_start, start ? 1u : 0u);
             // with a Newton level, the CG loop's condition belongs to the

@@ -21,7 +21,7 @@ struct LoopSync {
     unsigned* refresh_flag;  // raised when a mesh refreshes its residual next iteration
     unsigned* body_runs;     // CG-loop body executions (launch accounting)
     const unsigned* err;     // batch error word: the loop stops once it is set
-    unsigned* slice;         // [budget (0 = none), iterations run in this launch]
+    unsigned* slice;         // [budget (0 = none), iterations run in this launch, the loop goes on]
     cudaGraphConditionalHandle cond;
     int set_cond;
 };

@@ -25,6 +25,13 @@ __device__ __forceinline__ double y_full(const BatchView<S>& b, const double* y,
     return b.ydelta ? y[i] + (double)b.ydelta[i] : y[i];
 }
 
+// Whether the solver's loop goes on (BatchView::loop_go).
+template <typename S>
+__device__ __forceinline__ bool loop_on(const BatchView<S>& b)
+{
+    return *(volatile const unsigned*)b.loop_go != 0u;
+}
+
 // Whether the mesh's next iteration recomputes its residual in FP64 (set by
 // the last block of the mesh in the node pass, see refresh_decide).
 __device__ __forceinline__ bool refresh_now(const MeshConsts&, const StepScalars& s) { return s.refresh_next != 0; }

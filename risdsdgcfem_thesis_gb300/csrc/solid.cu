@@ -679,10 +679,12 @@ cudaError_t ls_solve_capture(fem_solid s, const StepConsts& c, cudaGraph_t top)
         if (m.bsr_val) solve_product(s, m, s->d.p, 0);  // then node_d keeps d's records
         e = capture_conditional(st, cond, cudaGraphCondTypeWhile, [&](cudaStream_t bs, cudaGraph_t) {
             s->stream = bs;
-            if (!m.bsr_val) solve_product(s, m, s->d.p, 1);
-            launch_node_q_fp64(m, c, s->d.p, s->q.p, s->partials.p, s->st.p, bs);
-            launch_node_xr_fp64(m, s->y.p, s->r.p, s->d.p, s->q.p, s->partials.p, s->partials2.p, s->st.p, bs);
-            launch_node_d_fp64(m, s->d.p, s->r.p, s->partials2.p, s->st.p, bs, cond, 1);
+            for (unsigned i = 0; i < kLoopUnroll; i++) {
+                if (!m.bsr_val) solve_product(s, m, s->d.p, 1);
+                launch_node_q_fp64(m, c, s->d.p, s->q.p, s->partials.p, s->st.p, bs);
+                launch_node_xr_fp64(m, s->y.p, s->r.p, s->d.p, s->q.p, s->partials.p, s->partials2.p, s->st.p, bs);
+                launch_node_d_fp64(m, s->d.p, s->r.p, s->partials2.p, s->st.p, bs, cond, 1);
+            }
             s->stream = st;
             return cudaGetLastError();
         });

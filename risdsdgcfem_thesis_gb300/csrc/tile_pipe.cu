@@ -311,6 +311,15 @@ __device__ __forceinline__ void node_sum(const float4* so4, const uint16_t* li, 
     }
 }
 
+// Tiles (0) or chunks (1) of the CG work list; none once the loop has ended
+// inside the body of its WHILE node.
+__device__ __forceinline__ uint32_t loop_count(const BatchView<float>& b, int which)
+{
+    const uint32_t n = *(volatile const uint32_t*)(b.act_count + which);
+    const unsigned go = *(volatile const unsigned*)b.loop_go;
+    return go ? n : 0u;
+}
+
 template <bool kCoherent>
 __device__ __forceinline__ float ld_dir(const float* p)
 {
@@ -372,7 +381,7 @@ __device__ __forceinline__ void tile_pipe_pass(const BatchView<float>& b, const 
     //   next is resolved and this thread's d and r of the next tile are
     //   gathered into registers | barrier B | outputs over the element data |
     //   barrier C | node sums.
-    const uint32_t n_act = *(volatile const uint32_t*)b.act_count;
+    const uint32_t n_act = loop_count(b, 0);
     uint32_t i = block;
     TileLook cur, nxt, n2;
     look_meta(b, i, n_act, cur);
@@ -556,7 +565,8 @@ __global__ void __launch_bounds__(TILE, PipeShape<TILE>::kMinBlocks) k_tile_spmv
                                                            unsigned* __restrict__ err)
 {
     extern __shared__ __align__(128) unsigned char smem[];
-    if (set_if && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(if_refresh, *refresh_flag ? 1u : 0u);
+    if (set_if && blockIdx.x == 0 && threadIdx.x == 0)
+        cudaGraphSetConditional(if_refresh, *refresh_flag && *b.loop_go ? 1u : 0u);
     tile_pipe_init<TILE>(smem);
     uint32_t phase = 0u;
     tile_pipe_pass<TILE, false, kPk>(b, dvec, rvec, part, tshare, err, smem, phase, blockIdx.x, gridDim.x,
@@ -605,7 +615,8 @@ __global__ void __launch_bounds__(256) k_mesh_alpha(BatchView<float> b, const fl
 {
     const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t m = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; m < b.M; m += nw) {
-        if (b.st[m].done) continue;
+        const unsigned go = *(volatile const unsigned*)b.loop_go;
+        if (b.st[m].done || !go) continue;
         (void)warp_mesh_alpha(b, tshare, m, true);
     }
 }
@@ -837,7 +848,7 @@ __device__ __forceinline__ void node_update_pass(const BatchView<float>& b, cons
                                                  const float2* tshare,
                                                  const uint32_t block, const uint32_t G, const bool fuse)
 {
-    const uint32_t n_act = *(volatile const uint32_t*)(b.act_count + 1);
+    const uint32_t n_act = loop_count(b, 1);
     for (uint32_t ia = block; ia < n_act; ia += G) {
         const uint32_t ci = b.act_chunks[ia];
         const ChunkMeta ch = b.chunks[ci];
@@ -1031,7 +1042,10 @@ __device__ __forceinline__ bool loop_flags(const LoopSync& ls, const LoopIn& in,
 {
     const bool go = any && !in.stop && (in.budget == 0u || in.runs + 1u < in.budget);
     if (ls.set_cond) cudaGraphSetConditional(ls.cond, go ? 1u : 0u);
-    if (ls.slice) ls.slice[1] = in.runs + 1u;
+    if (ls.slice) {
+        ls.slice[1] = in.runs + 1u;
+        ls.slice[2] = go ? 1u : 0u;
+    }
     if (ls.refresh_flag) *ls.refresh_flag = refresh ? 1u : 0u;
     if (ls.body_runs) *ls.body_runs = in.body + 1u;
     return go;
@@ -1229,6 +1243,7 @@ __global__ void __launch_bounds__(kUpdateThreads, 1) k_mesh_update(BatchView<flo
     MinresStep mi;
     LoopIn li;
     uint32_t dirty = 0, act = 0;
+    const unsigned go = *(volatile const unsigned*)b.loop_go;
     if (mine) {
         const MeshConsts& c = b.mc[m0 + own];
         const StepScalars& g = b.st[m0 + own];
@@ -1242,6 +1257,7 @@ __global__ void __launch_bounds__(kUpdateThreads, 1) k_mesh_update(BatchView<flo
         li = load_loop(ls);
     }
     if (tid == 0) s_flags = UpdateFlags{0u, 0u, 0u, 0u};
+    if (!go) return;  // the loop has ended inside the body of its WHILE node
     if (warp < n) {
         const MeshConsts& c = b.mc[m0 + warp];
         const uint32_t done = b.st[m0 + warp].done, chunk0 = c.chunk0, nchunks = c.nchunks;
