@@ -145,6 +145,8 @@ struct fem_batch_s {
     std::vector<uint32_t> eperm_h;        // batch element -> the caller's element index in its mesh
     Dev<uint32_t> perm;                   // perm_h on the device (whole-batch state transfers)
     Dev<double> stage_x, stage_v;         // caller-order staging for whole-batch transfers
+    Dev<double> stage_mesh;               // the same for one mesh's x and v (the largest's)
+    uint32_t stage_nodes = 0;
     Dev<uchar4> lconn;
     Dev<uint16_t> lptr, lidx;
     Dev<uint8_t> fixed;
@@ -269,7 +271,7 @@ struct fem_batch_s {
         tiles.release(); chunks.release(); mc.release(); st.release(); active.release(); gtets.release();
         Dinv_s.release(); mat_s.release(); R_s.release(); Dinv64.release(); Kfx.release(); grade.release(); vol.release(); detF.release();
         tile_nodes.release(); lptr0.release(); ov_ptr.release(); ov_map.release(); knc_node.release();
-        perm.release(); stage_x.release(); stage_v.release();
+        perm.release(); stage_x.release(); stage_v.release(); stage_mesh.release();
         knc_mesh.release(); lconn.release(); lptr.release(); lidx.release(); fixed.release(); rest.release();
         x.release(); v.release(); bvec.release(); y.release(); part64.release(); cpart.release(); tpart.release();
         knc_target.release(); r_s.release(); d_s.release(); q_s.release(); part_s.release(); ydelta_s.release(); counter.release();
@@ -1174,6 +1176,8 @@ int fem_batch_finalize(fem_batch b)
     BCKC(b->blob.upload(blob_h, s));
     BCKC(b->blob_off16.alloc(blob_off16_h.size()));
     BCKC(b->blob_off16.upload(blob_off16_h, s));
+    for (const MeshConsts& c : mcs) b->stage_nodes = std::max(b->stage_nodes, c.N);
+    BCKC(b->stage_mesh.alloc(6 * (size_t)b->stage_nodes));
     BCKC(b->slice.alloc(3));
     BCKC(cudaMemsetAsync(b->slice.p, 0, 3 * sizeof(unsigned), s));
     BCKC(b->start_tiles.alloc(b->ntiles));
@@ -1290,7 +1294,7 @@ int fem_batch_finalize(fem_batch b)
                       b->tpart.bytes() + b->counter.bytes() + b->any_flag.bytes() + b->refresh_flag.bytes() +
                       b->mcount.bytes() + b->err.bytes() + b->blob.bytes() + b->blob_off16.bytes() +
                       b->act_tiles.bytes() + b->act_chunks.bytes() + b->act_count.bytes() + b->list_dirty.bytes() +
-                      b->slice.bytes() + b->start_tiles.bytes() + b->start_chunks.bytes() +
+                      b->slice.bytes() + b->stage_mesh.bytes() + b->start_tiles.bytes() + b->start_chunks.bytes() +
                       b->launch_tiles.bytes() + b->launch_chunks.bytes() + b->refresh_tiles.bytes() +
                       b->refresh_chunks.bytes() + b->list_count.bytes();
     b->finalized = true;
@@ -1355,22 +1359,21 @@ int fem_batch_set_state(fem_batch b, uint32_t mesh, const double* x, const doubl
     if (mesh >= b->M) return batch_fail(FEM_E_ARG, "mesh %u out of range", mesh);
     const MeshConsts& c = b->mc_host[mesh];
     const size_t off = 3 * (size_t)c.node0, bytes = sizeof(double) * 3 * c.N;
-    std::vector<double> tmp(3 * (size_t)c.N);
     const double* src[2] = {x, v};
     double* dst[2] = {b->x.p, b->v.p};
     for (int k = 0; k < 2; k++) {
         if (!src[k]) continue;
-        for (uint32_t u = 0; u < c.N; u++) {
-            const size_t i = b->inv_h[c.node0 + u] - c.node0;
-            for (int a = 0; a < 3; a++) tmp[3 * i + a] = src[k][3 * (size_t)u + a];
-        }
-        BCK(cudaMemcpyAsync(dst[k] + off, tmp.data(), bytes, cudaMemcpyHostToDevice, b->stream));
+        // put in the batch's order on the device; the copy returns with the
+        // caller's buffer read (pageable memory), the rest is in stream order
+        double* stage = b->stage_mesh.p + k * 3 * (size_t)b->stage_nodes;
+        BCK(cudaMemcpyAsync(stage, src[k], bytes, cudaMemcpyHostToDevice, b->stream));
+        launch_permute(b->perm.p + c.node0, c.N, stage - off, dst[k] + off, true, b->stream);
         // a DAPD mesh's previous positions restart at the new x, as on the
         // solid (fem_solid_set_state); fem_batch_set_dapd_state restores them
         if (k == 0 && c.rotation == FEM_ROTATION_DAPD && b->prev_x.p)
-            BCK(cudaMemcpyAsync(b->prev_x.p + off, tmp.data(), bytes, cudaMemcpyHostToDevice, b->stream));
-        BCK(cudaStreamSynchronize(b->stream));
+            BCK(cudaMemcpyAsync(b->prev_x.p + off, dst[k] + off, bytes, cudaMemcpyDeviceToDevice, b->stream));
     }
+    BCK(cudaStreamSynchronize(b->stream));
     return FEM_OK;
 }
 
@@ -1558,18 +1561,14 @@ int fem_batch_get_state(fem_batch b, uint32_t mesh, double* x, double* v)
     if (mesh >= b->M) return batch_fail(FEM_E_ARG, "mesh %u out of range", mesh);
     const MeshConsts& c = b->mc_host[mesh];
     const size_t off = 3 * (size_t)c.node0, bytes = sizeof(double) * 3 * c.N;
-    std::vector<double> tmp(3 * (size_t)c.N);
     double* dst[2] = {x, v};
     const double* src[2] = {b->x.p, b->v.p};
-    for (int k = 0; k < 2; k++) {
-        if (!dst[k]) continue;
-        BCK(cudaMemcpyAsync(tmp.data(), src[k] + off, bytes, cudaMemcpyDeviceToHost, b->stream));
-        BCK(cudaStreamSynchronize(b->stream));
-        for (uint32_t u = 0; u < c.N; u++) {
-            const size_t i = b->inv_h[c.node0 + u] - c.node0;
-            for (int a = 0; a < 3; a++) dst[k][3 * (size_t)u + a] = tmp[3 * i + a];
-        }
-    }
+    double* stage[2] = {b->stage_mesh.p, b->stage_mesh.p + 3 * (size_t)b->stage_nodes};
+    for (int k = 0; k < 2; k++)  // to the caller's order on the device
+        if (dst[k]) launch_permute(b->perm.p + c.node0, c.N, src[k] + off, stage[k] - off, false, b->stream);
+    for (int k = 0; k < 2; k++)
+        if (dst[k]) BCK(cudaMemcpyAsync(dst[k], stage[k], bytes, cudaMemcpyDeviceToHost, b->stream));
+    BCK(cudaStreamSynchronize(b->stream));
     return FEM_OK;
 }
 
