@@ -274,7 +274,7 @@ int fem_solid_get_params(fem_solid s, fem_params* params);
  * per tet for the assembly and one assembly per evaluation (about five
  * iterations' time); the sums run in another order, so other bits, within
  * the same parity tolerances. Other materials keep the element product. The
- * CG of a C_WRP solid whose rows fit the GPU's shared memory (about 130,000
+ * solve of a C_WRP solid whose rows fit the GPU's shared memory (about 130,000
  * tets on grid meshes) keeps them there in either setting, in memory it takes
  * at its first solve; without that memory it runs as above. FEM_E_OOM when
  * the blocks asked for do not fit. */

@@ -1,5 +1,5 @@
-// cg_rows.cu -- the whole of ILSS_CG::Solve (ILSS_CG.h:38-151) for a C_WRP
-// solid in one launch, the assembled stiffness's rows resident in shared
+// cg_rows.cu -- the whole of ILSS_CG::Solve (ILSS_CG.h:38-151) or
+// ILSS_MINRES::Solve (ILSS_MINRES.h:51-168) for a C_WRP solid in one launch, the assembled stiffness's rows resident in shared
 // memory (rows_plan.h).
 //
 // Block g owns a range of nodes: their rows as fixed-point 3x3 blocks (fx.cuh),
@@ -11,7 +11,8 @@
 // polled word), and the reader polls the word itself. Two exchanges make an
 // iteration, the sums of d.q and of |r|^2; r of the nodes on a block's rim goes
 // out beside the second, and every block keeps the d of its rim by the same
-// recurrence as the owner. Sums stay integers from the lanes to the total, and
+// recurrence as the owner (MINRES: v1.v, |v1|^2 and v1, which the norm makes
+// v). Sums stay integers from the lanes to the total, and
 // every block adds them all, so all take the same scalar steps and leave
 // together. A word is overwritten only after an exchange that its reader has
 // taken part in since it read it: the two sums by each other, r by the d.q
@@ -180,14 +181,48 @@ struct __align__(16) RowRecord {
 
 }  // namespace
 
-template <int L>  // lanes per row
+// ILSS_MINRES's Givens rotation from |v1|^2 (ILSS_MINRES.h:131-144) by a warp:
+// its two roots and its four quotients each on four lanes.
+__device__ __forceinline__ void givens_by_warp(MinresScalars& s, double total)
+{
+    const uint32_t q = threadIdx.x & 3u;
+    const MinresScalars mr = s;
+    const double be = mr.beta_new;
+    const double r2 = mr.s * mr.alpha + mr.c * mr.c_old * be;
+    const double r3 = mr.s_old * be;
+    const double r1_hat = mr.c * mr.alpha - mr.c_old * mr.s * be;
+    const double root = ::sqrt(q == 0 ? total : r1_hat * r1_hat + total);
+    const double beta_new = __shfl_sync(0xffffffffu, root, 0), r1 = __shfl_sync(0xffffffffu, root, 1);
+    const double part = (q == 1 ? r1_hat : (q == 2 ? beta_new : 1.0)) / (q == 0 ? beta_new : r1);
+    const double inv_beta = __shfl_sync(0xffffffffu, part, 0), c = __shfl_sync(0xffffffffu, part, 1);
+    const double sn = __shfl_sync(0xffffffffu, part, 2), ir1 = __shfl_sync(0xffffffffu, part, 3);
+    if (threadIdx.x == 0) {
+        s.beta = be;
+        s.beta_new = beta_new;
+        s.inv_beta = inv_beta;
+        s.c_old = mr.c;
+        s.s_old = mr.s;
+        s.c = c;
+        s.s = sn;
+        s.neg_r2 = -r2;
+        s.neg_r3 = -r3;
+        s.inv_r1 = ir1;
+        s.x_coef = mr.beta_one * c * mr.eta;
+        s.norm_r_sq = mr.norm_r_sq * (sn * sn);
+        s.eta = -sn * mr.eta;
+    }
+    __syncwarp();
+}
+
+template <int L, bool kMinres>  // L: lanes per row
 __global__ void __launch_bounds__(kCgRowsMaxThreads, 1)
     k_cg_rows_fp64(MeshView<double> m, StepConsts c, CgRowsView p, const double* __restrict__ b, double* y,
                    StepScalars* st)
 {
     extern __shared__ __align__(16) unsigned char rows_smem[];
     __shared__ double s_scalar;
-    __shared__ int s_go;
+    __shared__ MinresScalars s_mr;
+    __shared__ int s_go, s_ok;  // the loop test; the first sum is there (0: breakdown)
     const uint32_t tid = threadIdx.x, nt = blockDim.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t G = gridDim.x, g = blockIdx.x, C = p.cluster, row0 = g / C * C, rank = g - row0, nrow = G / C;
     const CgRowsBlock B = p.blk[g];
@@ -375,7 +410,12 @@ __global__ void __launch_bounds__(kCgRowsMaxThreads, 1)
     };
     auto nothing = [] {};
 
-    // r = S (b - A y), d = r, |r|^2   (ILSS_CG.h:53-64)
+    double norm_b = 0.0;
+    if constexpr (kMinres) {  // |b|^2, constrained rows too
+        const double bi = mine ? b[at] : 0.0;
+        norm_b = total(vec ? bi * bi : 0.0, 0, seq, bad, nothing);
+    }
+    // r = S (b - A y), d = r, |r|^2   (ILSS_CG.h:53-64; ILSS_MINRES.h:66-95: v1 = r)
     if (mine) put(tid, ny);
     if (tid >= rim0)
         for (uint32_t i = tid - rim0; i < h3; i += nt - rim0) {
@@ -389,17 +429,82 @@ __global__ void __launch_bounds__(kCgRowsMaxThreads, 1)
         const double t = total(vec ? nr * nr : 0.0, 1, seq, bad, nothing);
         if (warp == 0) {
             delta_0 = delta = delta_old = t;
-            target = c.rel_eps_sq * t;
+            if constexpr (kMinres) delta_0 = norm_b;
+            target = c.rel_eps_sq * delta_0;
             target_bits = target == target && abs_sq == abs_sq ? max(fx_bits(target), abs_bits) : ~(uint64_t)0;
             if (lane == 0) {
                 s_scalar = 0.0;
                 s_go = bad ? -1 : proceeds();
+                if constexpr (kMinres) {
+                    s_mr = MinresScalars{};
+                    minres_start(s_mr, t);
+                    s_mr.norm_b_sq = norm_b;
+                }
             }
         }
     }
     int stop = __syncthreads_or(receive(seq));
     int go = stop ? -1 : s_go;
-    while (go > 0) {
+    bool finite = true;  // of the totals, in warp 0
+    if constexpr (kMinres) {
+        double np = 0.0, np0 = 0.0;
+        while (go > 0) {
+            // v0 <- v, v <- v1 / beta, v1 = S A v - beta v0, v1.v   (ILSS_MINRES.h:117-123)
+            const double inv = s_mr.inv_beta, nb = -s_mr.beta_new;
+            double v0 = 0.0, t = 0.0;
+            if (vec) {
+                v0 = nd;
+                nd = nr * inv;
+            }
+            if (mine) put(tid, nd);
+            if (tid >= rim0)
+                for (uint32_t i = tid - rim0; i < h3; i += nt - rim0) put(n3 + i, rimr[i] * inv);
+            product();
+            if (vec) {
+                nq = live ? c.factor_K * ku[tid] + mfm * nd : 0.0;
+                nr = __fma_rn(nb, v0, nq);
+                t = nr * nd;
+            }
+            seq++;
+            t = total(t, 0, seq, bad, nothing);
+            if (tid == 0) {
+                s_scalar = s_mr.alpha = t;
+                s_ok = bad ? -1 : 1;
+            }
+            __syncthreads();
+            if (s_ok < 0) {
+                go = -1;
+                break;
+            }
+            // v1 -= alpha v, |v1|^2, the rotation and the loop test, p and y   (:123-156)
+            if (vec) {
+                nr = __fma_rn(-s_scalar, nd, nr);
+                send(seq);
+                t = nr * nr;
+            }
+            t = total(t, 1, seq, bad, nothing);
+            if (warp == 0) {
+                givens_by_warp(s_mr, t);
+                delta_old = delta;
+                delta = s_mr.norm_r_sq;
+                finite = isfinite(t) && isfinite(delta);
+                k++;
+                if (lane == 0) s_go = bad ? -1 : proceeds();
+            }
+            stop = __syncthreads_or(receive(seq));
+            go = stop ? -1 : s_go;
+            if (vec) {
+                double pn = s_mr.neg_r2 * np + nd;
+                pn += s_mr.neg_r3 * np0;
+                pn *= s_mr.inv_r1;
+                np0 = np;
+                np = pn;
+                ny += s_mr.x_coef * pn;
+            }
+            __syncthreads();  // before warp 0 writes the scalars again
+        }
+    }
+    while (!kMinres && go > 0) {
         // d = S (beta d + r), q = S A d, d.q   (ILSS_CG.h:90-96,137)
         const double be = s_scalar;
         if (vec) nd = __fma_rn(be, nd, nr);
@@ -427,11 +532,11 @@ __global__ void __launch_bounds__(kCgRowsMaxThreads, 1)
             if (!brk) alpha = delta / t;
             if (lane == 0) {
                 s_scalar = alpha;
-                s_go = bad ? -1 : !brk;
+                s_ok = bad ? -1 : !brk;
             }
         }
         __syncthreads();
-        go = s_go;
+        go = s_ok;
         if (go <= 0) break;
         // y += alpha d, r -= alpha q, |r|^2, beta and the loop test   (ILSS_CG.h:96-137)
         if (vec) {
@@ -472,11 +577,12 @@ __global__ void __launch_bounds__(kCgRowsMaxThreads, 1)
         st->dot_dq = dq;
         st->alpha = alpha;
         st->beta = beta;
-        st->status = go < 0 ? 6u : (isfinite(delta) ? 0u : 3u);  // FEM_E_TIMEOUT, FEM_E_NAN
+        st->status = go < 0 ? 6u : (isfinite(delta) && finite ? 0u : 3u);  // FEM_E_TIMEOUT, FEM_E_NAN
+        if constexpr (kMinres) st->mr = st->mr_pend = s_mr;
         st->done = 1;
         st->delta_pend = delta;
         st->done_pend = 1;
-        st->rel_residual = delta_0 > 0 ? ::sqrt(delta / delta_0) : 0.0;
+        st->rel_residual = kMinres || delta_0 > 0 ? ::sqrt(delta / delta_0) : 0.0;
         st->abs_residual = ::sqrt(delta);
         *p.seq = go < 0 ? seq + 4 : seq;  // past the numbers of blocks that were ahead
     }
@@ -484,9 +590,10 @@ __global__ void __launch_bounds__(kCgRowsMaxThreads, 1)
 
 namespace {
 using CgRowsKernel = void (*)(MeshView<double>, StepConsts, CgRowsView, const double*, double*, StepScalars*);
-CgRowsKernel cg_rows_kernel(uint32_t lanes)
+CgRowsKernel cg_rows_kernel(uint32_t lanes, bool minres)
 {
-    return lanes == 4 ? k_cg_rows_fp64<4> : (lanes == 8 ? k_cg_rows_fp64<8> : k_cg_rows_fp64<16>);
+    if (minres) return lanes == 4 ? k_cg_rows_fp64<4, true> : (lanes == 8 ? k_cg_rows_fp64<8, true> : k_cg_rows_fp64<16, true>);
+    return lanes == 4 ? k_cg_rows_fp64<4, false> : (lanes == 8 ? k_cg_rows_fp64<8, false> : k_cg_rows_fp64<16, false>);
 }
 }  // namespace
 
@@ -512,30 +619,35 @@ void rows_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, const CgRowsP
 uint32_t cg_rows_max_blocks(const CgRowsPlan& p)
 {
     if (p.smem > kCgRowsMaxSmem || p.threads > kCgRowsMaxThreads || p.cluster < 1 || p.cluster > 16) return 0;
-    auto* k = cg_rows_kernel(p.lanes);
-    int n = 0;
-    cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute at[2];
-    rows_config(cfg, at, p, nullptr);
-    cfg.gridDim = dim3(p.cluster);
-    cfg.numAttrs = 1;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCgRowsMaxSmem) != cudaSuccess ||
-        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
+    int least = 0x7fffffff;
+    for (bool minres : {false, true}) {
+        auto* k = cg_rows_kernel(p.lanes, minres);
+        int n = 0;
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute at[2];
+        rows_config(cfg, at, p, nullptr);
+        cfg.gridDim = dim3(p.cluster);
+        cfg.numAttrs = 1;
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCgRowsMaxSmem) != cudaSuccess ||
+            cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        least = std::min(least, n);
     }
-    return std::min((uint32_t)n * p.cluster, kCgRowsMaxBlocks);
+    return std::min((uint32_t)least * p.cluster, kCgRowsMaxBlocks);
 }
 
 cudaError_t launch_cg_rows_fp64(const MeshView<double>& m, const StepConsts& c, const CgRowsPlan& plan,
-                                const CgRowsView& p, const double* b, double* y, StepScalars* st, cudaStream_t s)
+                                const CgRowsView& p, bool minres, const double* b, double* y, StepScalars* st,
+                                cudaStream_t s)
 {
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at[2];
     rows_config(cfg, at, plan, s);
     prof_begin("cg_rows_fp64", s);
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, cg_rows_kernel(plan.lanes), m, c, p, b, y, st);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, cg_rows_kernel(plan.lanes, minres), m, c, p, b, y, st);
     prof_end("cg_rows_fp64", s);
     launch_counter()++;
     return e;

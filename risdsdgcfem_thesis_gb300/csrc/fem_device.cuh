@@ -268,7 +268,7 @@ void launch_bsr_assemble_fp64(const MeshView<double>& m, const BsrBuild& a, cuda
 void launch_bsr_vector_fp64(const MeshView<double>& m, const double* u, const StepScalars* st, int check_done,
                             cudaStream_t s);
 
-// The CG solve on resident rows (cg_rows.cu): the layout's tables (rows_plan.h).
+// The solve on resident rows (cg_rows.cu): the layout's tables (rows_plan.h).
 struct CgRowsView {
     const CgRowsBlock* blk;
     const uint32_t *node, *group, *slot, *halo, *owner;
@@ -281,7 +281,8 @@ struct CgRowsView {
 // The blocks of the plan's shape that are resident together; 0 when it does not launch.
 uint32_t cg_rows_max_blocks(const CgRowsPlan& p);
 cudaError_t launch_cg_rows_fp64(const MeshView<double>& m, const StepConsts& c, const CgRowsPlan& plan,
-                                const CgRowsView& p, const double* b, double* y, StepScalars* st, cudaStream_t s);
+                                const CgRowsView& p, bool minres, const double* b, double* y, StepScalars* st,
+                                cudaStream_t s);
 
 // Launch shapes of the grid-stride kernels. One FP64 instruction of a warp
 // holds its sub-partition for 64 clocks, so small launches spread one warp

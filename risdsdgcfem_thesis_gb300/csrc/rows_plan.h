@@ -1,5 +1,5 @@
 // rows_plan.h -- host tables of the assembled stiffness (MeshView::bsr_*) and
-// of the CG solve on resident rows (cg_rows.cu).
+// of the solve on resident rows (cg_rows.cu).
 #pragma once
 #include <stddef.h>
 #include <stdint.h>
@@ -70,7 +70,7 @@ inline bool bsr_pattern(uint32_t N, uint32_t T, const uint32_t* tets, const std:
     return true;
 }
 
-// The CG solve of a C_WRP solid in one launch, the assembled rows in shared
+// The CG or MINRES solve of a C_WRP solid in one launch, its rows in shared
 // memory (cg_rows.cu). Block g owns node[node0 .. node0 + nn), rows of `lanes`
 // lanes, 32 / lanes rows per group; a group's units [group[group0 + w],
 // group[group0 + w + 1]) hold one 3x3 block per lane: its bsr slot (kCgRowsPad:
@@ -99,7 +99,7 @@ inline size_t cg_rows_smem_bytes(const CgRowsPlan& p, const CgRowsBlock& b)
            (24 + 4) * (size_t)b.nn + (48 + 8) * (size_t)b.nhalo + 4 * (size_t)(b.ngroups + 1) + 32 * sizeof(uint16_t) * (size_t)b.units;
 }
 
-// The layout of the CG solve on resident rows (CgRowsBlock).
+// The layout of the solve on resident rows (CgRowsBlock).
 struct CgRowsLayout {
     CgRowsPlan plan;
     std::vector<CgRowsBlock> blk;

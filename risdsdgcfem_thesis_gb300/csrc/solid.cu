@@ -114,7 +114,7 @@ struct fem_solid_s {
     bool kfx_fresh = false;
     DevBuf<uint32_t> csr_ptr, csr_idx;
     DevBuf<uint8_t> fixed;
-    // the CG solve on resident rows (blocks 0: none), over the assembled
+    // the solve on resident rows (blocks 0: none), over the assembled
     // stiffness below
     CgRowsPlan rows{};
     bool rows_tried = false;
@@ -434,9 +434,9 @@ int open_step(fem_solid s)
     return FEM_OK;
 }
 
-// A solid whose CG solve runs on resident rows (cg_rows.cu).
-bool wants_rows(const fem_params& p) { return p.material == FEM_MATERIAL_C_WRP && p.ls_solver != FEM_LS_MINRES; }
-bool cg_on_rows(const fem_solid s)
+// A solid whose solve runs on resident rows (cg_rows.cu).
+bool wants_rows(const fem_params& p) { return p.material == FEM_MATERIAL_C_WRP; }
+bool on_rows(const fem_solid s)
 {
     return wants_rows(s->params) && s->rows.blocks > 0;
 }
@@ -449,7 +449,7 @@ bool cg_on_rows(const fem_solid s)
 // much as five products.
 void set_bsr_use(fem_solid s)
 {
-    s->bsr_use = s->bsr_want && s->bsr_groups > 0 && s->params.material == FEM_MATERIAL_C_WRP && !cg_on_rows(s);
+    s->bsr_use = s->bsr_want && s->bsr_groups > 0 && s->params.material == FEM_MATERIAL_C_WRP && !on_rows(s);
 }
 
 template <typename V>
@@ -478,7 +478,7 @@ int upload_bsr(fem_solid s, const BsrPattern& p)
     return FEM_OK;
 }
 
-// The CG solve on resident rows of a C_WRP solid that can have it: the
+// The solve on resident rows of a C_WRP solid that can have it: the
 // pattern, its blocks and the layout.
 int build_rows(fem_solid s, const uint32_t* tets, const std::vector<uint32_t>& ptr, const std::vector<uint32_t>& idx)
 {
@@ -554,7 +554,7 @@ int try_rows(fem_solid s)
     return FEM_OK;
 }
 
-// The CG solve on resident rows, enqueued.
+// The solve on resident rows, enqueued.
 cudaError_t solve_on_rows(fem_solid s, const StepConsts& c)
 {
     assemble(s);
@@ -565,7 +565,7 @@ cudaError_t solve_on_rows(fem_solid s, const StepConsts& c)
     const CgRowsView v{s->rows_blk.p, s->rows_node.p, s->rows_group.p, s->rows_slot.p, s->rows_halo.p, s->rows_owner.p,
                        s->rows_col.p, s->rows_words.p, s->rows_words.p + 3 * (size_t)s->N, p.cluster, p.warps, p.npb,
                        p.units, p.records, s->rows_seq.p};
-    return launch_cg_rows_fp64(m, c, s->rows, v, s->b.p, s->y.p, s->st.p, s->stream);
+    return launch_cg_rows_fp64(m, c, s->rows, v, s->params.ls_solver == FEM_LS_MINRES, s->b.p, s->y.p, s->st.p, s->stream);
 }
 
 // The solve's status as an error of the call.
@@ -582,16 +582,8 @@ int solve_status(const StepScalars& h)
 // chunk of iterations).
 int cg_solve(fem_solid s, const StepConsts& c, int chunk)
 {
-    if (int e = try_rows(s)) return e;
     cudaStream_t st = s->stream;
     MeshView<double> m = s->view();
-    if (cg_on_rows(s)) {
-        CK(solve_on_rows(s, c));
-        CK(cudaMemcpyAsync(s->st_host, s->st.p, sizeof(StepScalars), cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        CK(cudaGetLastError());
-        return s->st_host->status == FEM_E_TIMEOUT ? solve_status(*s->st_host) : FEM_OK;
-    }
     const uint32_t gN = node_grid(s->N, m.bsr_val != nullptr), gV = vec_grid(3 * s->N);
     solve_product(s, m, s->y.p, 0);
     launch_node_residual_fp64(m, c, s->b.p, s->y.p, s->r.p, s->d.p, s->partials.p, st);
@@ -655,6 +647,14 @@ int minres_solve(fem_solid s, const StepConsts& c, int chunk)
 // LS_Solve's solver choice (LeafDSH_Solid3D_FEM.cpp:1136-1154)
 int ls_solve(fem_solid s, const StepConsts& c, int chunk)
 {
+    if (int e = try_rows(s)) return e;
+    if (on_rows(s)) {
+        CK(solve_on_rows(s, c));
+        CK(cudaMemcpyAsync(s->st_host, s->st.p, sizeof(StepScalars), cudaMemcpyDeviceToHost, s->stream));
+        CK(cudaStreamSynchronize(s->stream));
+        CK(cudaGetLastError());
+        return s->st_host->status == FEM_E_TIMEOUT ? solve_status(*s->st_host) : FEM_OK;
+    }
     return s->params.ls_solver == FEM_LS_MINRES ? minres_solve(s, c, chunk) : cg_solve(s, c, chunk);
 }
 
@@ -668,7 +668,7 @@ cudaError_t ls_solve_capture(fem_solid s, const StepConsts& c, cudaGraph_t top)
     cudaStream_t st = s->stream;
     MeshView<double> m = s->view();
     const uint32_t gN = node_grid(s->N, m.bsr_val != nullptr), gV = vec_grid(3 * s->N);
-    if (cg_on_rows(s)) return solve_on_rows(s, c);
+    if (on_rows(s)) return solve_on_rows(s, c);
     cudaGraphConditionalHandle cond = 0;
     cudaError_t e = cudaGraphConditionalHandleCreate(&cond, top, 0, cudaGraphCondAssignDefault);
     if (e != cudaSuccess) return e;
@@ -867,7 +867,7 @@ int step_once(fem_solid s, int chunk)
         if (int e = capture_step(s)) return e;
     CK(cudaGraphLaunch(s->exec, s->stream));
     // made by the graph's solve on its evaluation
-    s->bsr_fresh = s->bsr_use || cg_on_rows(s);
+    s->bsr_fresh = s->bsr_use || on_rows(s);
     s->kfx_fresh = !uses_lcm(s) && !s->bsr_fresh;
     return FEM_OK;
 }

@@ -220,10 +220,12 @@ def test_batch_products_match_the_oracle(fem_lib, oracle):
                                    _block((4, 4, 4), (1, 1, 0.1)), _block((4, 3, 4), (1, 1, 0.4)),
                                    _block((4, 4, 4), poisson=0.499), _fan(5), _fan(100)],
                          ids=["5", "20", "625", "7260", "graded", "part-graded", "stiff", "fan5", "fan100"])
-def test_solve_on_resident_rows_matches_the_oracle(fem_lib, oracle, scene):
+@pytest.mark.parametrize("solver", ["cg", "minres"])
+def test_solve_on_resident_rows_matches_the_oracle(fem_lib, oracle, scene, solver):
     """The solid's solve from one block of nodes to all clusters, with fixed
-    nodes: as the batch above, 1e-12 after two CG iterations."""
+    nodes: as the batch above, 1e-12 after two CG or MINRES iterations."""
     rng = np.random.default_rng(4)
+    scene.ls_solver = fem_lib.FEM_LS_MINRES if solver == "minres" else fem_lib.FEM_LS_CG
     scene.init_vel = 0.1 * rng.standard_normal(scene.rest.shape)
     scene.knc_nodes = np.array([0, len(scene.rest) - 1], np.uint32)
     scene.knc_targets = scene.rest[scene.knc_nodes].copy()
