@@ -45,6 +45,12 @@ constexpr int kChunkNodes = 1024;  // default node chunk (one work item of a nod
 constexpr int kPipeSmallTile = 128;
 constexpr int kPipeSmallNodes = 120;
 constexpr int kNodeThreads = 256;  // threads per node-kernel block
+// FP64 batch's solver loop: a node per thread of a chunk of 1,024. A node's
+// twenty FP64 instructions hold a sub-partition 64 clocks each per warp, and
+// four nodes one after the other on 256 threads left the pipe idle between
+// (140,802 nodes in 64 meshes: the two node kernels 26.7 and 21.3 us, now 22.9
+// and 20.2; what is left is the chain of per-mesh and grid arrivals).
+constexpr int kNodeThreads64 = 1024;
 // Default poll limit of the tile product's waits for a tile copy (each poll
 // suspends for a hardware time slice: far above any copy's latency).
 constexpr unsigned kDefaultWaitPolls = 1u << 22;

@@ -103,7 +103,17 @@ __device__ __forceinline__ double chunk_sum(S v);
 template <>
 __device__ __forceinline__ double chunk_sum<float>(float v) { return bblock_sum_f(v); }
 template <>
-__device__ __forceinline__ double chunk_sum<double>(double v) { return bblock_sum(v); }
+__device__ __forceinline__ double chunk_sum<double>(double v)  // by integer reductions; in warp 0
+{
+    __shared__ double sh[32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    v = fx_warp_sum(v);
+    __syncthreads();
+    if (lane == 0) sh[wid] = v;
+    __syncthreads();
+    if (wid != 0) return 0.0;
+    return fx_warp_sum(lane < (int)((blockDim.x + 31) >> 5) ? sh[lane] : 0.0);
+}
 
 // ---------------------------------------------------------------------------
 // Element tile product of the new search direction: for each local node the
@@ -618,6 +628,15 @@ __device__ __forceinline__ double mesh_partial_sum(const double* cpart, uint32_t
     return bblock_sum(acc);
 }
 
+// The same by the block's first warp, in integers.
+__device__ __forceinline__ double mesh_partial_sum_warp(const double* cpart, uint32_t c0, uint32_t n)
+{
+    if (threadIdx.x >= 32) return 0.0;
+    double acc = 0.0;
+    for (uint32_t i = threadIdx.x; i < n; i += 32) acc += __ldcg(cpart + c0 + i);
+    return fx_warp_sum(acc);
+}
+
 __device__ __forceinline__ bool cg_cont(const StepScalars& s)
 {
     return s.delta_new > s.abs_eps_sq && s.delta_new > s.delta_target && s.k < s.max_iter;
@@ -832,7 +851,7 @@ __device__ void node_q_minres(const BatchView<S>& b, const MeshConsts& c, const 
     const double sum = chunk_sum<S>(acc);
     if (threadIdx.x == 0) cpart[ci] = sum;
     if (arrive_last(ls.mcount + ch.mesh, c.nchunks)) {
-        const double total = mesh_partial_sum(cpart, c.chunk0, c.nchunks);
+        const double total = mesh_partial_sum_warp(cpart, c.chunk0, c.nchunks);
         if (threadIdx.x == 0) {
             StepScalars& s = b.st[ch.mesh];
             s.mr.beta = s.mr.beta_new;
@@ -862,7 +881,7 @@ __device__ void node_update_minres(const BatchView<S>& b, const MeshConsts& c, c
     const double sum = chunk_sum<S>(acc);
     if (threadIdx.x == 0) cpart[ci] = sum;
     if (arrive_last(ls.mcount + ch.mesh, c.nchunks)) {
-        const double total = mesh_partial_sum(cpart, c.chunk0, c.nchunks);
+        const double total = mesh_partial_sum_warp(cpart, c.chunk0, c.nchunks);
         if (threadIdx.x == 0) {
             StepScalars& s = b.st[ch.mesh];
             minres_givens(s.mr, total);
@@ -884,7 +903,7 @@ __device__ void node_update_minres(const BatchView<S>& b, const MeshConsts& c, c
 // d = S(r + beta d) written back ; q = S A d ; d.q ; last block of a mesh:
 // alpha (ILSS_CG.h:90-98). On refresh iterations r becomes S(b - A y).
 template <typename S>
-__global__ void k_node_q(BatchView<S> b, const S* __restrict__ part, S* __restrict__ d, S* __restrict__ q,
+__global__ void __launch_bounds__(kNodeThreads64) k_node_q(BatchView<S> b, const S* __restrict__ part, S* __restrict__ d, S* __restrict__ q,
                          const double* __restrict__ part64, const double* __restrict__ bv,
                          const double* __restrict__ y, S* __restrict__ r, double* __restrict__ cpart, LoopSync ls)
 {
@@ -937,7 +956,7 @@ __global__ void k_node_q(BatchView<S> b, const S* __restrict__ part, S* __restri
         const double sum = chunk_sum<S>(acc);
         if (threadIdx.x == 0) cpart[ci] = sum;
         if (arrive_last(ls.mcount + ch.mesh, c.nchunks)) {
-            const double total = mesh_partial_sum(cpart, c.chunk0, c.nchunks);
+            const double total = mesh_partial_sum_warp(cpart, c.chunk0, c.nchunks);
             if (threadIdx.x == 0) {
                 StepScalars& s = b.st[ch.mesh];
                 s.dot_dq = total;
@@ -956,7 +975,7 @@ __global__ void k_node_q(BatchView<S> b, const S* __restrict__ part, S* __restri
 // y += alpha d (FP64) ; r -= alpha q (in S) ; |r|^2 ; last block of a mesh:
 // beta, k += 1 and the loop test (ILSS_CG.h:100-144).
 template <typename S>
-__global__ void k_node_update(BatchView<S> b, double* __restrict__ y, S* __restrict__ r, const S* __restrict__ d,
+__global__ void __launch_bounds__(kNodeThreads64) k_node_update(BatchView<S> b, double* __restrict__ y, S* __restrict__ r, const S* __restrict__ d,
                               S* __restrict__ q, double* __restrict__ cpart, LoopSync ls)
 {
     const uint32_t ci = blockIdx.x;
@@ -985,7 +1004,7 @@ __global__ void k_node_update(BatchView<S> b, double* __restrict__ y, S* __restr
         const double sum = chunk_sum<S>(acc);
         if (threadIdx.x == 0) cpart[ci] = sum;
         if (arrive_last(ls.mcount + ch.mesh, c.nchunks)) {
-            const double total = mesh_partial_sum(cpart, c.chunk0, c.nchunks);
+            const double total = mesh_partial_sum_warp(cpart, c.chunk0, c.nchunks);
             if (threadIdx.x == 0) {
                 StepScalars& s = b.st[ch.mesh];
                 s.delta_old = s.delta_new;
@@ -1367,7 +1386,7 @@ void BatchLaunch<S>::node_q(const BatchView<S>& b, const S* part, S* d, S* q, co
                             cudaStream_t s)
 {
     prof_begin(sizeof(S) == 8 ? "node_q_fp64" : "node_q_mixed", s);
-    k_node_q<S><<<b.nchunks ? b.nchunks : 1, kNodeThreads, 0, s>>>(b, part, d, q, part64, bv, y, r, cpart, ls);
+    k_node_q<S><<<b.nchunks ? b.nchunks : 1, sizeof(S) == 8 ? kNodeThreads64 : kNodeThreads, 0, s>>>(b, part, d, q, part64, bv, y, r, cpart, ls);
     prof_end(sizeof(S) == 8 ? "node_q_fp64" : "node_q_mixed", s);
     launch_counter()++;
 }
@@ -1376,7 +1395,7 @@ template <typename S>
 void BatchLaunch<S>::node_update(const BatchView<S>& b, double* y, S* r, const S* d, S* q, double* cpart,
                                  const LoopSync& ls, cudaStream_t s)
 {
-    k_node_update<S><<<b.nchunks ? b.nchunks : 1, kNodeThreads, 0, s>>>(b, y, r, d, q, cpart, ls);
+    k_node_update<S><<<b.nchunks ? b.nchunks : 1, sizeof(S) == 8 ? kNodeThreads64 : kNodeThreads, 0, s>>>(b, y, r, d, q, cpart, ls);
     launch_counter()++;
 }
 
