@@ -102,6 +102,12 @@ struct fem_solid_s {
     StepConsts consts{};
     double node_mass = 0, total_volume = 0, rayleigh[2] = {0, 0};
     cudaStream_t stream = nullptr;
+    // work beside the main chain of a step (fork, join): its stream (made at
+    // the first step), the events that start and end it; forked: it has not been
+    // waited for yet
+    cudaStream_t side = nullptr;
+    cudaEvent_t side_start = nullptr, side_end = nullptr;
+    bool forked = false;
     // element data
     DevBuf<int4> tets;
     DevBuf<double> Dinv, mat, vol, R, detF, eout;
@@ -260,6 +266,11 @@ struct fem_solid_s {
         if (st_host) cudaFreeHost(st_host);
         st_host = nullptr;
         drop_graph();
+        if (side_start) cudaEventDestroy(side_start);
+        if (side_end) cudaEventDestroy(side_end);
+        if (side) cudaStreamDestroy(side);
+        side_start = side_end = nullptr;
+        side = nullptr;
         if (stream) cudaStreamDestroy(stream);
         stream = nullptr;
     }
@@ -422,10 +433,41 @@ void solve_product(fem_solid s, const MeshView<double>& m, const double* d, int 
     launch_bsr_vector_fp64(m, d, s->st.p, check_done, s->stream);
 }
 
+// Work beside the main chain from here on, and the main chain's wait for it:
+// the small kernels of a step are short of the GPU by far.
+template <typename F>
+int fork(fem_solid s, F&& work)
+{
+    cudaStream_t st = s->stream;
+    if (!s->side) CK(cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking));
+    if (!s->side_start) CK(cudaEventCreateWithFlags(&s->side_start, cudaEventDisableTiming));
+    if (!s->side_end) CK(cudaEventCreateWithFlags(&s->side_end, cudaEventDisableTiming));
+    CK(cudaEventRecord(s->side_start, st));
+    CK(cudaStreamWaitEvent(s->side, s->side_start, 0));
+    s->stream = s->side;
+    work();
+    s->stream = st;
+    CK(cudaEventRecord(s->side_end, s->side));
+    s->forked = true;
+    return FEM_OK;
+}
+int join(fem_solid s)
+{
+    if (s->forked) CK(cudaStreamWaitEvent(s->stream, s->side_end, 0));
+    s->forked = false;
+    return FEM_OK;
+}
+
+// The solver's operator on the last rotations, made beside the force and the
+// right-hand side (three dependent kernels against four: 20 us of a step of
+// 160 to 20,480 tets).
+int fork_operator(fem_solid s);
+
 // FixedStep's opening: BeginEvaluation(m_vecPos0, x), then m_vecPos0 = x
 // (LeafDSH_Solid3D_FEM.cpp:927-935).
 int open_step(fem_solid s)
 {
+    if (int e = join(s)) return e;  // an abandoned step's
     cudaStream_t st = s->stream;
     CK(cudaMemsetAsync(&s->st.p->inverted, 0, sizeof(uint32_t), st));
     begin_eval(s, s->prev_x.p, s->x.p);
@@ -568,6 +610,15 @@ cudaError_t solve_on_rows(fem_solid s, const StepConsts& c)
     return launch_cg_rows_fp64(m, c, s->rows, v, s->params.ls_solver == FEM_LS_MINRES, s->b.p, s->y.p, s->st.p, s->stream);
 }
 
+int fork_operator(fem_solid s)
+{
+    if (uses_lcm(s)) return FEM_OK;
+    return fork(s, [&] {
+        if (s->bsr_use || on_rows(s)) assemble(s);
+        else bake_products(s);
+    });
+}
+
 // The solve's status as an error of the call.
 int solve_status(const StepScalars& h)
 {
@@ -648,6 +699,7 @@ int minres_solve(fem_solid s, const StepConsts& c, int chunk)
 int ls_solve(fem_solid s, const StepConsts& c, int chunk)
 {
     if (int e = try_rows(s)) return e;
+    if (int e = join(s)) return e;
     if (on_rows(s)) {
         CK(solve_on_rows(s, c));
         CK(cudaMemcpyAsync(s->st_host, s->st.p, sizeof(StepScalars), cudaMemcpyDeviceToHost, s->stream));
@@ -738,16 +790,19 @@ int host_sum(fem_solid s, uint32_t count, double* out)
 
 // Elastic and potential energy at x with the current rotations
 // (FixedStep's m_TES.V and RecomputeEnergy, LeafDSH_Solid3D_FEM.cpp:979,1554-1584).
-void energy(fem_solid s)
+int energy(fem_solid s)
 {
-    cudaStream_t st = s->stream;
     MeshView<double> m = s->view();
     const StepConsts& c = s->consts;
     const uint32_t gE = elem_grid(s->T);
+    if (int e = fork(s, [&] {
+            launch_potential_fp64(m, c, s->x.p, s->partials.p, s->stream);
+            launch_finalize(FIN_ENERGY_P, s->partials.p, gE, c, s->st.p, s->stream);
+        }))
+        return e;
     elem_force(s, m, s->x.p, 0, s->partials2.p);
-    launch_finalize(FIN_ENERGY_E, s->partials2.p, gE, c, s->st.p, st);
-    launch_potential_fp64(m, c, s->x.p, s->partials2.p, st);
-    launch_finalize(FIN_ENERGY_P, s->partials2.p, gE, c, s->st.p, st);
+    launch_finalize(FIN_ENERGY_E, s->partials2.p, gE, c, s->st.p, s->stream);
+    return join(s);
 }
 
 // One FixedStep with Step_FullyImplicitEuler_dx (LeafDSH_Solid3D_FEM.cpp:
@@ -776,6 +831,7 @@ int step_fie(fem_solid s, int chunk)
     double delta_new = 0.0, delta_0 = -1.0, sum = 0.0;
     bool converged = false, solved = false;
     do {
+        if (int e = fork_operator(s)) return e;
         elem_force(s, m, s->x.p, 1, nullptr);
         launch_node_b_fie_fp64(m, c, s->x.p, s->xn.p, s->vn.p, nr_k == 0 ? 1 : 0, s->b.p, s->y.p, st);
         launch_knc_fie_fp64(s->N, s->knc_count, s->knc_nodes.p, s->knc_targets.p, s->x.p, s->b.p, s->y.p, st);
@@ -798,32 +854,36 @@ int step_fie(fem_solid s, int chunk)
             begin_eval(s, s->xn.p, s->x.p);
         }
     } while (!converged && nr_k < s->params.nr_max_iter);
+    if (int e = join(s)) return e;
     s->nr_iters = nr_k;
     s->fie_cg_iters = cg_iters;
     s->fie_solved = solved;
     s->nr_abs = delta_new;
     s->nr_rel = (delta_0 > 0) ? delta_new / delta_0 : 0.0;
-    if (s->params.compute_energy) energy(s);
+    if (s->params.compute_energy)
+        if (int e = energy(s)) return e;
     CK(cudaGetLastError());
     return FEM_OK;
 }
 
 // One FixedStep's QIE_V pipeline after the opening: f_e, b, constraints,
 // the solve, integration and energies.
-void qie_head(fem_solid s)
+int qie_head(fem_solid s)
 {
+    if (int e = fork_operator(s)) return e;
     cudaStream_t st = s->stream;
     MeshView<double> m = s->view();
     const StepConsts& c = s->consts;
     elem_force(s, m, s->x.p, 1, nullptr);
     launch_node_b_fp64(m, c, s->v.p, s->b.p, s->y.p, st);
     launch_knc_fp64(s->N, s->knc_count, s->knc_nodes.p, s->knc_targets.p, s->x.p, c, s->b.p, s->y.p, st);
+    return join(s);
 }
-void qie_tail(fem_solid s)
+int qie_tail(fem_solid s)
 {
     const StepConsts& c = s->consts;
     launch_integrate_fp64(s->N, c.dt, s->x.p, s->v.p, s->y.p, s->stream);
-    if (s->params.compute_energy) energy(s);
+    return s->params.compute_energy ? energy(s) : FEM_OK;
 }
 
 // The QIE_V step as one graph: the opening, the pipeline and the solver's
@@ -839,9 +899,9 @@ int capture_step(fem_solid s)
     cudaError_t e = cudaStreamGetCaptureInfo(st, &cs, nullptr, &top, nullptr, nullptr, nullptr);
     int rc = e == cudaSuccess ? open_step(s) : FEM_E_CUDA;
     if (rc == FEM_OK) {
-        qie_head(s);
-        e = ls_solve_capture(s, s->consts, top);
-        if (e == cudaSuccess) qie_tail(s);
+        rc = qie_head(s);
+        if (rc == FEM_OK) e = ls_solve_capture(s, s->consts, top);
+        if (rc == FEM_OK && e == cudaSuccess) rc = qie_tail(s);
     }
     cudaGraph_t g = nullptr;
     const cudaError_t e2 = cudaStreamEndCapture(st, &g);
