@@ -189,10 +189,12 @@ __device__ __noinline__ int32_t tile_elem_fp64(const BatchView<double>& b, uint3
 // fixed-point integers with one exponent per element; a node's thread adds
 // its entries in integers (fx.cuh) and leaves an FP64 partial.
 // The 138 FP64 operations per element and three adds per entry of the FP64
-// form held that pipe at 64 clocks each: 210 us for 554,475 tets. The integer
-// multiplies take 71 us, about as long as the 204 MB of matrices need.
+// form held that pipe at 64 clocks each: 210 us for 554,475 tets, now 67 us
+// (3.1 TB/s of matrices). Four blocks per SM, for the phases of a block that
+// wait (three: 72 us; two of 256 threads: 81 us; the matrices prefetched into
+// L2 while the nodes are gathered: 76 us).
 template <bool kDir>
-__global__ void __launch_bounds__(kFxTileThreads, 3)
+__global__ void __launch_bounds__(kFxTileThreads, 4)
     k_tile_product_fp64(BatchView<double> b, const double* __restrict__ vec, const double* __restrict__ rvec,
                         double* __restrict__ part)
 {
