@@ -6,6 +6,7 @@ import ctypes as C
 import os
 import shutil
 import subprocess
+import threading
 
 import numpy as np
 import pytest
@@ -235,3 +236,31 @@ def test_solve_on_resident_rows_matches_the_oracle(fem_lib, oracle, scene, solve
     assert o.step()["iters"] == g.stats()["cg_iterations"] == 2
     v = o.state()[1]
     assert np.linalg.norm(g.state()[1] - v) <= 1e-12 * np.linalg.norm(v)
+
+
+@pytest.mark.gpu
+def test_resident_solves_side_by_side(fem_lib):
+    """Solids of one and of several clusters stepped from threads at once give
+    the bits they give alone."""
+    shapes = [((16, 16, 12), 0), ((14, 10, 10), 1), ((10, 10, 6), 0), ((8, 2, 2), 0)]
+
+    def run(k, out):
+        dims, solver = shapes[k]
+        sc = _block(dims)
+        sc.ls_solver = solver
+        sc.init_vel = 0.1 * np.random.default_rng(k).standard_normal(sc.rest.shape)
+        s = fem_lib.Solid(sc)
+        for _ in range(20):
+            s.step(1)
+        out[k] = s.state()
+
+    alone, together = [None] * 4, [None] * 4
+    for k in range(4):
+        run(k, alone)
+    threads = [threading.Thread(target=run, args=(k, together)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for a, b in zip(alone, together):
+        assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
