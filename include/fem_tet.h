@@ -410,7 +410,8 @@ typedef struct fem_batch_options {
     uint32_t fuse_alpha;  /* mixed: 1 = every node-pass block forms its mesh's alpha from the
                              tile shares itself (one kernel fewer per CG iteration: shorter
                              iterations when few meshes run, more work when many do; the
-                             same results either way) */
+                             same results either way); 0 = so only where the batch is small
+                             enough for it to be the shorter form */
     uint32_t persistent_loop; /* mixed, tile_elems > 128: 1 = the CG iterations of a launch run
                              in one persistent cooperative kernel (the phases of an iteration
                              separated by bounded grid barriers; the fused alpha) sized to the
@@ -574,8 +575,8 @@ typedef struct fem_server_options {
                                     lone request's iterations are shorter with more,
                                     smaller chunks) */
     uint32_t fuse_alpha;         /* as fem_batch_options.fuse_alpha for the shards
-                                    (default 0: measured 3 % shorter iterations for a
-                                    lone request against 7 % less capacity) */
+                                    (default 0: by the size of the shard; always on,
+                                    large shards had 7 % less capacity) */
     uint32_t persistent_loop;    /* as fem_batch_options.persistent_loop for the shards */
 } fem_server_options;
 

@@ -125,6 +125,7 @@ struct fem_batch_s {
     std::vector<HostMesh> meshes;
     bool finalized = false;
     uint32_t M = 0, ntiles = 0, nchunks = 0, K = 0;
+    bool alpha_in_nodes = false;      // mixed: the node pass forms alpha (option, or by the sizes)
     uint64_t Ntot = 0, Ttot = 0, nslots = 0;
     std::vector<MeshConsts> mc_host;
     std::vector<uint32_t> knc_base;   // per mesh first KNC entry
@@ -202,7 +203,7 @@ struct fem_batch_s {
         b.nchunks = nchunks;
         b.pipe_tile = opt.tile_elems <= (uint32_t)kPipeSmallTile ? kPipeSmallTile : kTileElems;
         b.loop_go = slice.p + 2;
-        b.fuse_alpha = opt.fuse_alpha ? 1u : 0u;
+        b.fuse_alpha = alpha_in_nodes ? 1u : 0u;
         b.has_lcm = any_lcmh ? 2u : any_lcm ? 1u : 0u;
         b.lock = lock ? 1u : 0u;
         b.Ntot = (uint32_t)Ntot;
@@ -1198,7 +1199,12 @@ int fem_batch_finalize(fem_batch b)
         BCKC(cudaMemsetAsync(b->act_count.p, 0, 2 * sizeof(uint32_t), s));
         BCKC(cudaMemsetAsync(b->list_dirty.p, 0, sizeof(unsigned), s));
     }
-    if (!fp64) prepare_tile_pipe();
+    if (!fp64) {
+        prepare_tile_pipe();
+        uint32_t most = 0;
+        for (const MeshConsts& c : mcs) most = std::max(most, c.ntiles);
+        b->alpha_in_nodes = b->opt.fuse_alpha || node_pass_forms_alpha(b->nchunks, most);
+    }
     BCKC(cudaMallocHost(&b->st_host, sizeof(StepScalars) * b->M));
     BCKC(cudaMallocHost(&b->err_host, sizeof(unsigned)));
     *b->err_host = 0;
@@ -2024,7 +2030,7 @@ int fem_batch_kernel_launches(fem_batch b, uint32_t steps, uint64_t* launches)
     for (auto& m : b->meshes) energy |= m.p.compute_energy != 0;
     const bool mixed = b->opt.precision == FEM_PRECISION_MIXED;
     const uint64_t fixed = 8 + (b->K ? 1 : 0) + (energy ? 4 : 0);
-    const uint64_t per_iter = mixed ? (b->opt.fuse_alpha ? 5ull : 6ull) : 3ull;
+    const uint64_t per_iter = mixed ? (b->alpha_in_nodes ? 5ull : 6ull) : 3ull;
     *launches = (uint64_t)steps * fixed + per_iter * body_runs;
     return FEM_OK;
 }

@@ -8,6 +8,8 @@ namespace femgb {
 uint32_t grid_tiles(uint32_t ntiles);
 uint32_t tile_pipe_smem_bytes();
 void prepare_tile_pipe();
+// Whether the node pass of a mixed batch forms alpha itself (after prepare_tile_pipe).
+bool node_pass_forms_alpha(uint32_t nchunks, uint32_t max_mesh_tiles);
 uint32_t grid_chunks(uint32_t nchunks);
 // Node-vector permutation between the caller's order and the batch's:
 // to_batch: dst[i] = src[perm[i]]; otherwise dst[perm[i]] = src[i] (xyz each).

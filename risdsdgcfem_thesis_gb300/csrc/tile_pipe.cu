@@ -19,7 +19,9 @@
 // coalesced; shared nodes' other partials go to overflow slots).
 //
 // k_mesh_alpha: one warp per running mesh sums its tiles' shares (fixed
-// order) and forms alpha, or the breakdown flag (ILSS_CG.h:97).
+// order) and forms alpha, or the breakdown flag (ILSS_CG.h:97). Launched where
+// the meshes or their chunks are many; elsewhere the node pass does the same
+// sum itself (node_pass_forms_alpha).
 //
 // k_node_update_fused: per node of the running meshes: d = S(r + beta d) (the
 // values the tiles staged), q = S(fK sum(partials) + m fM d), y += alpha d
@@ -1873,6 +1875,25 @@ void launch_node_update_fused(const BatchView<float>& b, const float* part, cons
     k_mesh_update<<<(b.M + kUpdateGroup - 1) / kUpdateGroup, kUpdateThreads, 0, s>>>(b, cshare, ls);
     prof_end("mesh_update", s);
     launch_counter()++;
+}
+
+// Which kernel forms a mesh's alpha: the same sum in the same order either
+// way. k_mesh_alpha costs every CG iteration a launch and a chain of
+// dependent loads (3.3-4.3 us, one warp per mesh); formed by the node pass,
+// each chunk's block repeats that sum before its first update (0.8-2.5 us
+// while the chunks are a few waves of the grid).
+//  - Tiles of the largest mesh: warp 0 reads the shares in rounds of 256, all
+//    of them for every chunk. Steps of one mesh, separate / in the node pass:
+//    66 tiles 6289 / 5270 us, 641 tiles 12204 / 10933, 5121 tiles 81.4 / 81.4 ms,
+//    14239 tiles 89.7 / 103.5; eight meshes of 5121 tiles 350 / 373 ms. The line
+//    is four rounds.
+//  - Chunks: each wave of blocks pays the sum again. 64 chunks 12993 / 11737 us,
+//    256 chunks 33.2 / 30.8 ms, 1280 chunks 108.4 / 107.2, 2304 chunks
+//    226.6 / 225.2; 1024 meshes of 40k tets (about 7,000 chunks) 257.5 / 257.9.
+//    The line is four waves.
+bool node_pass_forms_alpha(uint32_t nchunks, uint32_t max_mesh_tiles)
+{
+    return max_mesh_tiles <= 4u * 256u && nchunks <= 4u * (uint32_t)node_grid();
 }
 
 void prepare_tile_pipe()

@@ -377,3 +377,36 @@ def test_fused_alpha_gives_the_same_bits(fem_lib):
     finally:
         a.close()
         f.close()
+
+
+
+@pytest.mark.parametrize("n, tile, chunk, separate", [
+    (3, 256, 1024, False),   # one tile, one chunk
+    (18, 32, 1024, False),   # 29,160 tets in at most 1,024 tiles of 32
+    (20, 32, 1024, True),    # 40,000 tets: more than 1,024 tiles
+    (44, 256, 32, True),     # 91,125 nodes in 2,848 chunks of 32: more than four waves of the node pass
+])
+@pytest.mark.parametrize("solver", [0, 1])
+def test_alpha_by_batch_size_gives_the_same_bits(fem_lib, n, tile, chunk, separate, solver):
+    """Where alpha is formed follows the batch's sizes; it is the same
+    fixed-order sum in both places, so a step equals the forced form bit for
+    bit, beyond the lines as within them."""
+    rng = np.random.default_rng(31)
+    scs = [scenes.random_block(rng, dims=(n, n, n), idx=0), scenes.random_block(rng, dims=(4, 3, 3), idx=1)]
+    scs = [dataclasses.replace(sc, max_iter=12, ls_solver=solver) for sc in scs]
+    out = []
+    for fuse in (False, True):
+        b = fem_lib.Batch(scs, precision=fem_lib.FEM_PRECISION_MIXED, compute_energy=False, tile_elems=tile,
+                          chunk_nodes=chunk, fuse_alpha=fuse)
+        try:
+            b.reset_launch_count()
+            b.step(2)
+            out.append(([b.state(i) for i in range(2)], [b.stats(i)["cg_iterations"] for i in range(2)],
+                        b.kernel_launches(2)))
+        finally:
+            b.close()
+    (sa, ia, la), (sb, ib, lb) = out
+    assert ia == ib and min(ia) > 0
+    assert (la > lb) == separate, (la, lb)
+    for (xa, va), (xb, vb) in zip(sa, sb):
+        assert np.array_equal(xa, xb) and np.array_equal(va, vb)
