@@ -237,10 +237,14 @@ constexpr float kFxMaxGrade = 3.0f, kFxMaxGradeStiff = 2.0f, kFxMaxGradeRigid = 
 constexpr double kFxStiff = 2.0, kFxRigid = 9.5;  // lambda / mu
 
 // Whether an element of this rest shape and material may take fx_bake:
-// grade = max|Dm| max|Dm^-1|.
+// grade = max|Dm| max|Dm^-1|. mu > 0 and 3 lambda + 2 mu >= 0 (a Poisson ratio
+// in (-1, 0.5) with E > 0) make K9 positive semidefinite, which its scaling
+// by the diagonal needs: with a Poisson ratio of 0.55 its other entries are
+// up to several times the diagonal.
 FX_HD bool fx_grade_ok(float grade, double kl, double km)
 {
-    return grade <= (kl <= kFxStiff * km ? kFxMaxGrade : (kl <= kFxRigid * km ? kFxMaxGradeStiff : kFxMaxGradeRigid));
+    return km > 0.0 && 3.0 * kl + 2.0 * km >= 0.0 &&
+           grade <= (kl <= kFxStiff * km ? kFxMaxGrade : (kl <= kFxRigid * km ? kFxMaxGradeStiff : kFxMaxGradeRigid));
 }
 
 // Bakes K9 = V (lambda m_i m_j^T + mu m_j m_i^T + mu (g_i . g_j) R R^T) with g_i
@@ -305,8 +309,12 @@ FX_HD int32_t fx_bake(const double* R, const double* Di, double kl, double km, F
         U[k] = fx_split(fx_fin<2>(hi, mid));
     }
     // (mid stays below (2 (2^27.82 + 2^28.82) + 2^28.6 + 2^28.05) 2^31 < 2^63).
-    // K9 is positive semidefinite, so its largest entry is on the diagonal:
-    // that gives the shift that moves it to [2^59, 2^60).
+    // K9 is positive semidefinite (fx_grade_ok), so its largest entry is on the
+    // diagonal: that gives the shift that moves it to [2^59, 2^60). Another
+    // entry as large as its row's and column's diagonal belongs to a rotation
+    // that moves nodes i and j along m_j and m_i; both diagonals are then V mu
+    // |m|^2, at most 3/4 of V (lambda + 2 mu) |m|^2 elsewhere, so truncation
+    // cannot lift it above the largest.
     const int sym[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
     auto entry = [&](int r, int c) {
         const int i = r / 3, a = r % 3, j = c / 3, b = c % 3;

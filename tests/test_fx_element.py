@@ -132,6 +132,14 @@ def test_error_is_no_larger_than_fp64s(shim, nu, field):
     assert n == 300 and sfx <= s64, (np.sqrt(sfx / n), np.sqrt(s64 / n))
 
 
+@pytest.mark.parametrize("nu", [-2.0, -1.2, 0.50001, 0.51, 0.55, 0.6, 1.0])
+def test_indefinite_materials_take_fp64(shim, nu):
+    """Outside (-1, 0.5) the element matrix is not positive semidefinite, and
+    its largest entry need not be on the diagonal that scales it."""
+    rng = np.random.default_rng(7)
+    assert all(_run(shim, el, rng.standard_normal((4, 3)))[0] == 1 for el in _elements(nu, rng))
+
+
 def test_edges_of_the_number_format(shim):
     rng = np.random.default_rng(3)
     el = next(_elements(0.3, rng))
@@ -194,6 +202,33 @@ def test_products_match_the_oracle(fem_lib, oracle, scene):
             assert np.abs(a - b).max() <= 2e-13 * np.abs(b).max()
     d[scene.tets[0, 1], 2] = np.nan
     assert np.array_equal(np.isnan(g.df_x(d)).any(1), np.isnan(o.df_x(d)).any(1))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nu", [-1.2, 0.55, 1.0])
+def test_indefinite_materials_match_the_oracle(fem_lib, oracle, nu):
+    """Elements whose matrix is not semidefinite run in FP64 in every form of
+    the product: the hooks', the resident rows' and the FP64 batch's. Bars as
+    in test_products_match_the_oracle (products) and
+    test_batch_products_match_the_oracle (two CG iterations)."""
+    rng = np.random.default_rng(8)
+    scene = _block((4, 3, 4), poisson=nu)
+    scene.init_vel = 0.1 * rng.standard_normal(scene.rest.shape)
+    scene.max_iter = 2
+    g, o, b = fem_lib.Solid(scene), oracle.Solid(scene, "port"), fem_lib.Batch([scene], precision=fem_lib.FEM_PRECISION_FP64)
+    x = scene.rest + 0.005 * rng.standard_normal(scene.rest.shape)
+    g.begin_eval(x)
+    o.begin_eval(x)
+    d = rng.standard_normal(scene.rest.shape)
+    for p, q in ((g.df_x(d), o.df_x(d)), (g.apply_A(1.0, 1 / 3600, d), o.apply_A(1.0, 1 / 3600, d))):
+        assert np.abs(p - q).max() <= 2e-13 * np.abs(q).max()
+    g, o = fem_lib.Solid(scene), oracle.Solid(scene, "port")
+    g.step(1)
+    b.step(1)
+    assert o.step()["iters"] == g.stats()["cg_iterations"] == b.stats(0)["cg_iterations"] == 2
+    v = o.state()[1]
+    for w in (g.state()[1], b.state(0)[1]):
+        assert np.linalg.norm(w - v) <= 1e-12 * np.linalg.norm(v)
 
 
 @pytest.mark.gpu
