@@ -524,7 +524,8 @@ int fem_batch_finished(fem_batch b, uint8_t* flags);
  * no counterpart in the reference, which has no device waits). A wait that
  * gives up sets the batch's error word: the CG loops stop at the end of that
  * iteration, the blocks drain their copies in flight, and the next
- * fem_batch_synchronize returns FEM_E_TIMEOUT once (the word is cleared). The
+ * fem_batch_synchronize (in a lock-step: fem_batch_nr_midstep) returns
+ * FEM_E_TIMEOUT once (the word is cleared). The
  * default (FEM_WAIT_LIMIT_DEFAULT) is 2^22 polls, far above any copy's
  * latency; 0 makes every such wait give up at once, which exercises that
  * error path. */

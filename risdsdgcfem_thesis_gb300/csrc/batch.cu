@@ -400,6 +400,27 @@ void param_consts(MeshConsts& c, const fem_params& p, double acc_total_volume, u
 }
 
 
+// The meshes' scalars and the error word, to st_host and err_host.
+int read_loop(fem_batch B, cudaStream_t s)
+{
+    BCK(cudaMemcpyAsync(B->st_host, B->st.p, sizeof(StepScalars) * B->M, cudaMemcpyDeviceToHost, s));
+    BCK(cudaMemcpyAsync(B->err_host, B->err.p, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+    BCK(cudaStreamSynchronize(s));
+    return FEM_OK;
+}
+
+// The error word read_loop found set as an error of the call, once: the next
+// launches start with a clear word.
+int report_give_up(fem_batch B)
+{
+    const unsigned err = *B->err_host;
+    if (!err) return FEM_OK;
+    BCK(cudaMemsetAsync(B->err.p, 0, sizeof(unsigned), B->stream));
+    BCK(cudaStreamSynchronize(B->stream));
+    return batch_fail(FEM_E_TIMEOUT, "a bounded device wait gave up (code %u: 1 tile copy, 2 copy drain, 3 grid "
+                                     "barrier)", err);
+}
+
 // Enqueue one launch of the step on `s`:
 //   reset (one block: which meshes start, continue or are left out)
 //   IF some mesh starts: BeginEvaluation, f_e, b, constraints, A y, r0
@@ -531,11 +552,11 @@ int enqueue_step(fem_batch B, cudaStream_t s, bool capture, int lock_phase = 0)
         }
         uint32_t budget = B->slice_budget, ran = 0;
         for (; !coop;) {
-            BCK(cudaMemcpyAsync(B->st_host, B->st.p, sizeof(StepScalars) * B->M, cudaMemcpyDeviceToHost, s));
-            BCK(cudaStreamSynchronize(s));
+            if (int e = read_loop(B, s)) return e;
             bool any = false;
             for (uint32_t m = 0; m < B->M; m++) any |= !B->st_host[m].done;
-            if (!any || (budget && ran >= budget)) break;
+            // a wait that gave up ends the loop on the device with meshes not done
+            if (!any || *B->err_host || (budget && ran >= budget)) break;
             for (int i = 0; i < 8 && !(budget && ran >= budget); i++, ran++) {
                 body_head(s, 0, 0);
                 if (mixed) L::tile_spmv_y64(b, B->y.p, B->part64.p, 1, B->refresh_flag.p, s);
@@ -599,11 +620,10 @@ int enqueue_step(fem_batch B, cudaStream_t s, bool capture, int lock_phase = 0)
         after_solve(s);
         // further Newton iterations while some FIE mesh goes on
         while (newton) {
-            BCK(cudaMemcpyAsync(B->st_host, B->st.p, sizeof(StepScalars) * B->M, cudaMemcpyDeviceToHost, s));
-            BCK(cudaStreamSynchronize(s));
+            if (int e = read_loop(B, s)) return e;
             bool go = false;
             for (uint32_t m = 0; m < B->M; m++) go |= B->st_host[m].nr_go != 0;
-            if (!go) break;
+            if (!go || *B->err_host) break;
             solve_start(s);
             if (int e = host_cg()) return e;
             after_solve(s);
@@ -1870,8 +1890,8 @@ int fem_batch_nr_midstep(fem_batch b, double dt)
     if (int e = lock_consts(b, dt)) return e;
     blob_factors(b, true);
     if (int e = lock_solve_phase(b, 1)) return e;
-    BCK(cudaMemcpyAsync(b->st_host, b->st.p, sizeof(StepScalars) * b->M, cudaMemcpyDeviceToHost, b->stream));
-    BCK(cudaStreamSynchronize(b->stream));
+    if (int e = read_loop(b, b->stream)) return e;
+    if (int e = report_give_up(b)) return e;
     for (uint32_t m = 0; m < b->M; m++)
         if (b->st_host[m].status == FEM_E_NAN) return batch_fail(FEM_E_NAN, "NaN or Inf in the residual of mesh %u", m);
     return FEM_OK;
@@ -1943,17 +1963,8 @@ int fem_batch_multi_step(fem_batch b, double dt, uint32_t nsteps)
 int fem_batch_synchronize(fem_batch b)
 {
     if (int e = check_ready(b)) return e;
-    BCK(cudaMemcpyAsync(b->st_host, b->st.p, sizeof(StepScalars) * b->M, cudaMemcpyDeviceToHost, b->stream));
-    unsigned err = 0;
-    if (b->err.p) BCK(cudaMemcpyAsync(&err, b->err.p, sizeof(unsigned), cudaMemcpyDeviceToHost, b->stream));
-    BCK(cudaStreamSynchronize(b->stream));
-    if (err) {
-        // reported once: the next launches start with a clear word
-        BCK(cudaMemsetAsync(b->err.p, 0, sizeof(unsigned), b->stream));
-        BCK(cudaStreamSynchronize(b->stream));
-        return batch_fail(FEM_E_TIMEOUT, "a bounded device wait gave up (code %u: 1 tile copy, 2 copy drain, 3 grid "
-                                         "barrier)", err);
-    }
+    if (int e = read_loop(b, b->stream)) return e;
+    if (int e = report_give_up(b)) return e;
     for (uint32_t m = 0; m < b->M; m++)
         if (b->st_host[m].status == FEM_E_NAN) return batch_fail(FEM_E_NAN, "NaN or Inf in the CG residual of mesh %u", m);
     return FEM_OK;

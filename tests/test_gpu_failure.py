@@ -91,3 +91,45 @@ def test_nan_velocity_is_reported_by_the_server(fem_lib):
     done = {c["scene"]: c for c in srv.drain()}
     assert done[ids[2]]["status"] == fem_lib.FEM_E_NAN
     assert done[ids[0]]["status"] == fem_lib.FEM_OK and done[ids[1]]["status"] == fem_lib.FEM_OK
+
+
+def _same_after_recovery(fem_lib, b, fresh, x0, step):
+    b.set_wait_limit(None)
+    for i, (x, v) in enumerate(x0):
+        b.set_state(i, x, v)
+    step(b)
+    step(fresh)
+    for i in range(len(x0)):
+        for p, q in zip(b.state(i), fresh.state(i)):
+            assert np.isfinite(p).all() and np.array_equal(p, q), i
+
+
+@pytest.mark.parametrize("integrator", [0, 1])
+@pytest.mark.parametrize("solver", [0, 1])
+def test_host_driven_loops_end_when_a_wait_gives_up(fem_lib, integrator, solver):
+    """Without a step graph the host drives the solver's and the Newton loop:
+    both end when the device reports that a wait gave up."""
+    sc = _meshes()
+    for s in sc:
+        s.integrator, s.ls_solver = integrator, solver
+    b, fresh = (fem_lib.Batch(sc, fem_lib.FEM_PRECISION_MIXED, use_graph=False) for _ in range(2))
+    x0 = [b.state(i) for i in range(len(sc))]
+    b.set_wait_limit(0)
+    with pytest.raises(fem_lib.FemError) as e:
+        b.step(2)
+    assert e.value.code == fem_lib.FEM_E_TIMEOUT
+    assert fem_lib.load().fem_batch_synchronize(b.h) != fem_lib.FEM_E_TIMEOUT
+    _same_after_recovery(fem_lib, b, fresh, x0, lambda s: s.step(2))
+
+
+def test_lock_step_reports_a_wait_that_gives_up(fem_lib):
+    sc = _meshes()
+    b, fresh = (fem_lib.Batch(sc, fem_lib.FEM_PRECISION_MIXED) for _ in range(2))
+    x0 = [b.state(i) for i in range(len(sc))]
+    b.set_wait_limit(0)
+    b.nr_phase("init", 1 / 60)
+    b.nr_phase("prestep", 1 / 60)
+    with pytest.raises(fem_lib.FemError) as e:
+        b.nr_phase("midstep", 1 / 60)
+    assert e.value.code == fem_lib.FEM_E_TIMEOUT
+    _same_after_recovery(fem_lib, b, fresh, x0, lambda s: s.multi_step(1 / 60))
