@@ -410,6 +410,13 @@ __global__ void __launch_bounds__(kCgRowsMaxThreads, 1)
     };
     auto nothing = [] {};
 
+    if (!kMinres && warp == 0 && nrow > 1)
+        // a solve without iterations sends no d.q: the words are renewed, so
+        // that none is older than a solve (their numbers wrap at 2^16)
+        for (uint32_t i = lane; i < nrow; i += 32) {
+            const ulonglong2 w = word_of(Part{0, 0}, seq);
+            word_put(p.parts + (size_t)(i * C + rank) * nrow + g / C, w.x, w.y);
+        }
     double norm_b = 0.0;
     if constexpr (kMinres) {  // |b|^2, constrained rows too
         const double bi = mine ? b[at] : 0.0;

@@ -299,3 +299,30 @@ def test_resident_solves_side_by_side(fem_lib):
         t.join()
     for a, b in zip(alone, together):
         assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+
+
+@pytest.mark.gpu
+def test_solve_after_many_solves_without_iterations(fem_lib):
+    """The words between the clusters carry 16 bits of the exchange's number.
+    65,534 solves that end at their residual bring the number round to that
+    of the last d.q: the next solve takes none of its sums."""
+    sc = _block((17, 16, 15))
+    v0 = 0.1 * np.random.default_rng(6).standard_normal(sc.rest.shape)
+    fresh, s = (fem_lib.Solid(sc, compute_energy=False) for _ in range(2))
+    s.set_state(v=v0)
+    s.step(1)
+    p = s.get_params()
+    full, p.ls_max_iter = p.ls_max_iter, 0
+    s.set_params(p)
+    s.set_state(sc.rest, np.zeros_like(v0))
+    s.step(65534)
+    assert s.stats()["cg_iterations"] == 0
+    p.ls_max_iter = full
+    s.set_params(p)
+    s.set_state(sc.rest, v0)
+    fresh.set_state(v=v0)
+    s.step(1)
+    fresh.step(1)
+    assert s.stats()["cg_iterations"] == fresh.stats()["cg_iterations"] > 0
+    for a, b in zip(s.state(), fresh.state()):
+        assert np.array_equal(a, b)
