@@ -27,6 +27,7 @@
 #include "bounds.cuh"
 #include "fem_device.cuh"
 #include "fx_device.cuh"
+#include "rows_words.h"
 
 #include <algorithm>
 
@@ -64,24 +65,6 @@ __device__ __forceinline__ ulonglong2 near_get(uint32_t p)
     asm volatile("ld.relaxed.cluster.shared::cluster.v2.b64 {%0, %1}, [%2];" : "=l"(w.x), "=l"(w.y) : "r"(p) : "memory");
     return w;
 }
-__device__ __forceinline__ ulonglong2 word_of(double v, uint32_t seq)
-{
-    const unsigned long long u = (unsigned long long)__double_as_longlong(v), s = (unsigned long long)seq << 32;
-    return make_ulonglong2((u & 0xffffffffull) | s, (u >> 32) | s);
-}
-__device__ __forceinline__ bool word_is(const ulonglong2& w, double& v, uint32_t seq)
-{
-    v = __longlong_as_double((long long)((w.x & 0xffffffffull) | (w.y << 32)));
-    return (uint32_t)(w.x >> 32) == seq && (uint32_t)(w.y >> 32) == seq;
-}
-
-// A partial sum: m in units of 2^(e - 1079); kPartNan: not finite. It stays
-// in integers from the lanes to the solid's total.
-struct Part {
-    int64_t m;
-    int32_t e;
-};
-constexpr int32_t kPartNan = 0x7fff;
 // The warp's sum of m 2^e (|m| <= 2^62), in every lane: added in three limbs.
 template <int K>
 __device__ __forceinline__ Part part_sum(const Part (&v)[K])
@@ -119,17 +102,6 @@ __device__ __forceinline__ double part_value(const Part& p)
     if (p.m == 0 || e < 1 || e > 2046) return fx_to_double(p.m, p.e - 1079);
     return __hiloint2double(__double2hiint(v) + ((p.e - 1079) << 20), __double2loint(v));
 }
-__device__ __forceinline__ ulonglong2 word_of(const Part& v, uint32_t seq)
-{
-    const unsigned long long m = (unsigned long long)v.m, s = (unsigned long long)seq << 48;
-    return make_ulonglong2((m & 0xffffffffffffull) | s, (m >> 48) | ((unsigned long long)(v.e & 0xffff) << 16) | s);
-}
-__device__ __forceinline__ bool word_is(const ulonglong2& w, Part& v, uint32_t seq)
-{
-    v.m = (int64_t)((w.x & 0xffffffffffffull) | (w.y << 48));
-    v.e = (int32_t)(w.y >> 16) & 0xffff;
-    return (uint32_t)(w.x >> 48) == (seq & 0xffffu) && (uint32_t)(w.y >> 48) == (seq & 0xffffu);
-}
 // Out of line: the compiler would otherwise divide on every path.
 __device__ __noinline__ double divide(double a, double b) { return a / b; }
 
@@ -147,7 +119,7 @@ __device__ __forceinline__ Part words_sum(F&& get, uint32_t n, uint32_t seq, boo
 #pragma unroll
         for (int i = 0; i < K; i++) {  // all in flight together
             const bool on = lane + 32 * i < n;
-            const bool there = word_is(get(on ? lane + 32 * i : 0u), part[i], seq);
+            const bool there = rows_word_is(get(on ? lane + 32 * i : 0u), part[i], seq);
             ok = ok && (there || !on);
             if (!on) part[i] = Part{0, 0};
         }
@@ -262,7 +234,7 @@ __global__ void __launch_bounds__(kCgRowsMaxThreads, 1)
         const uint32_t w = p.owner[B.halo0 + i];  // CTA << 16 | its node
         rimw[i] = w == kCgRowsFar ? w : near_address(myr + 3 * (w & 0xffffu), w >> 16);
     }
-    for (uint32_t i = tid; i < 2 * C * p.warps + 3 * p.npb; i += nt) sums[i] = word_of(Part{0, 0}, seq0);
+    rows_words_start(sums, 2 * C * p.warps, 3 * p.npb, seq0, tid, nt);
     for (uint32_t i = tid; i <= B.ngroups; i += nt) group[i] = p.group[B.group0 + i];
     cluster_sync();  // every CTA's words hold an old number
 
@@ -356,7 +328,7 @@ __global__ void __launch_bounds__(kCgRowsMaxThreads, 1)
         ulonglong2* own = sums + (size_t)which * C * vwarps;
         if (vec) {
             const Part v[1] = {part_of(acc)};
-            const ulonglong2 w = word_of(part_sum(v), seq);
+            const ulonglong2 w = rows_word<ulonglong2>(part_sum(v), seq);
             if (lane < C) near_put(near_address(own + rank * vwarps + warp, lane), w.x, w.y);
         }
         if (warp != 0) return 0.0;
@@ -366,7 +338,7 @@ __global__ void __launch_bounds__(kCgRowsMaxThreads, 1)
         Part s = n <= 32 ? words_sum<1>(get, n, seq, bad) : (n <= 96 ? words_sum<3>(get, n, seq, bad) : words_sum<5>(get, n, seq, bad));
         if (nrow > 1) {
             ulonglong2* words = p.parts + (size_t)which * G * nrow;
-            const ulonglong2 w = word_of(s, seq);
+            const ulonglong2 w = rows_word<ulonglong2>(s, seq);
             for (uint32_t i = lane; i < nrow; i += 32) word_put(words + (size_t)(i * C + rank) * nrow + g / C, w.x, w.y);
             words += (size_t)g * nrow;
             auto there = [&](uint32_t i) { return word_get(words + i); };
@@ -376,7 +348,7 @@ __global__ void __launch_bounds__(kCgRowsMaxThreads, 1)
     };
     // r for the neighbours, and theirs
     auto send = [&](uint32_t seq) {
-        const ulonglong2 w = word_of(nr, seq);
+        const ulonglong2 w = rows_word<ulonglong2>(nr, seq);
         if (near) near_put(near_address(myr + tid, rank), w.x, w.y);
         if (far) word_put(p.words + at, w.x, w.y);
     };
@@ -387,7 +359,7 @@ __global__ void __launch_bounds__(kCgRowsMaxThreads, 1)
                 const uint32_t k = i / 3, a = i % 3, w = rimw[k];
                 const ulonglong2* f = p.words + 3 * (size_t)rim[k] + a;
                 uint32_t polls = 0;
-                while (!word_is(w == kCgRowsFar ? word_get(f) : near_get(w + (uint32_t)sizeof(ulonglong2) * a), rimr[i], seq))
+                while (!rows_word_is(w == kCgRowsFar ? word_get(f) : near_get(w + (uint32_t)sizeof(ulonglong2) * a), rimr[i], seq))
                     if (++polls > kWordPolls) {
                         bad = 1;
                         break;
@@ -414,7 +386,7 @@ __global__ void __launch_bounds__(kCgRowsMaxThreads, 1)
         // a solve without iterations sends no d.q: the words are renewed, so
         // that none is older than a solve (their numbers wrap at 2^16)
         for (uint32_t i = lane; i < nrow; i += 32) {
-            const ulonglong2 w = word_of(Part{0, 0}, seq);
+            const ulonglong2 w = rows_word<ulonglong2>(Part{0, 0}, seq);
             word_put(p.parts + (size_t)(i * C + rank) * nrow + g / C, w.x, w.y);
         }
     double norm_b = 0.0;

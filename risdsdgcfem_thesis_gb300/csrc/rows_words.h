@@ -1,0 +1,61 @@
+// rows_words.h -- the 128-bit words of the solve on resident rows (cg_rows.cu):
+// data, and in the top bits of each half the exchange's number, so that a
+// reader knows both halves from the one word. W: ulonglong2. Host callable.
+#pragma once
+#include "fx.cuh"
+
+namespace femgb {
+
+// A value of an exchange, with all 32 bits of its number.
+template <typename W>
+FX_HD W rows_word(double v, uint32_t seq)
+{
+    const unsigned long long u = fx_bits(v), s = (unsigned long long)seq << 32;
+    W w;
+    w.x = (u & 0xffffffffull) | s;
+    w.y = (u >> 32) | s;
+    return w;
+}
+template <typename W>
+FX_HD bool rows_word_is(const W& w, double& v, uint32_t seq)
+{
+    v = fx_from_bits((w.x & 0xffffffffull) | (w.y << 32));
+    return (uint32_t)(w.x >> 32) == seq && (uint32_t)(w.y >> 32) == seq;
+}
+
+// A partial sum: m in units of 2^(e - 1079); kPartNan: not finite. It stays
+// in integers from the lanes to the solid's total.
+struct Part {
+    int64_t m;
+    int32_t e;
+};
+constexpr int32_t kPartNan = 0x7fff;
+
+// A sum, with 16 bits of the exchange's number.
+template <typename W>
+FX_HD W rows_word(const Part& v, uint32_t seq)
+{
+    const unsigned long long m = (unsigned long long)v.m, s = (unsigned long long)seq << 48;
+    W w;
+    w.x = (m & 0xffffffffffffull) | s;
+    w.y = (m >> 48) | ((unsigned long long)(v.e & 0xffff) << 16) | s;
+    return w;
+}
+template <typename W>
+FX_HD bool rows_word_is(const W& w, Part& v, uint32_t seq)
+{
+    v.m = (int64_t)((w.x & 0xffffffffffffull) | (w.y << 48));
+    v.e = (int32_t)(w.y >> 16) & 0xffff;
+    return (uint32_t)(w.x >> 48) == (seq & 0xffffu) && (uint32_t)(w.y >> 48) == (seq & 0xffffu);
+}
+
+// What the words of a CTA hold when a solve starts after number seq: sums
+// words of sums, then values.
+template <typename W>
+FX_HD void rows_words_start(W* w, uint32_t sums, uint32_t values, uint32_t seq, uint32_t first, uint32_t step)
+{
+    for (uint32_t i = first; i < sums; i += step) w[i] = rows_word<W>(Part{0, 0}, seq);
+    for (uint32_t i = first; i < values; i += step) w[sums + i] = rows_word<W>(0.0, seq);
+}
+
+}  // namespace femgb

@@ -138,3 +138,50 @@ def test_layout_covers_the_rows(shim, mesh, shuffle, sms):
     ref = np.zeros(n)
     np.add.at(ref, pairs[:, 0], a[pairs[:, 0]] * a[pairs[:, 1]] * d[pairs[:, 1]])
     assert np.array_equal(y, ref)
+
+
+WORDS = r"""
+#include "rows_words.h"
+using namespace femgb;
+struct W { unsigned long long x, y; };
+// The words a solve starts with after number seq: 0 unless one of them reads
+// as one of the solve's first numbers.
+extern "C" int taken(uint32_t seq)
+{
+    W w[8];
+    rows_words_start(w, 3, 5, seq, 0, 1);
+    for (uint32_t ahead = 1; ahead < 5; ahead++)
+        for (int i = 0; i < 8; i++) {
+            Part p;
+            double v;
+            if (i < 3 ? rows_word_is(w[i], p, seq + ahead) : rows_word_is(w[i], v, seq + ahead)) return i + 1;
+        }
+    return 0;
+}
+extern "C" int kept(double v, int64_t m, int32_t e, uint32_t seq)
+{
+    Part p;
+    double u;
+    return rows_word_is(rows_word<W>(v, seq), u, seq) && fx_bits(u) == fx_bits(v) &&
+           rows_word_is(rows_word<W>(Part{m, e}, seq), p, seq) && p.m == m && p.e == e;
+}
+"""
+
+
+def test_words_between_blocks(tmp_path):
+    """Data survives the words, and what they hold at the start of a solve is
+    no answer to its first exchanges, whatever the number (both formats wrap)."""
+    if shutil.which("g++") is None:
+        pytest.skip("no host compiler")
+    src, so = tmp_path / "words.cpp", tmp_path / "words.so"
+    src.write_text(WORDS)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-Wno-unknown-pragmas", "-shared", "-fPIC", "-I", CSRC, str(src),
+                    "-o", str(so)], check=True)
+    lib = C.CDLL(str(so))
+    lib.taken.argtypes = [C.c_uint32]
+    lib.kept.argtypes = [C.c_double, C.c_int64, C.c_int32, C.c_uint32]
+    edges = [k + d for k in (0, 0xffff, 0x10000, 0xfffeffff, 0xffff0000, 0xffffffff, 0x7fffffff) for d in (-1, 0, 1)]
+    for seq in [e & 0xffffffff for e in edges] + [0x10001 * k for k in range(0, 0x10000, 257)]:
+        assert lib.taken(seq) == 0, hex(seq)
+        for v, m, e in ((0.0, 0, 0), (-1.5, -(1 << 62), 2046), (np.inf, (1 << 62), 0x7fff), (5e-324, -1, 1)):
+            assert lib.kept(v, m, e, seq), hex(seq)
