@@ -280,6 +280,17 @@ int fem_solid_get_params(fem_solid s, fem_params* params);
  * the blocks asked for do not fit. */
 int fem_solid_set_assembled(fem_solid s, int on);
 
+/* Poll limit of the device-side waits of the solve in shared memory (as
+ * fem_batch_set_wait_limit; no counterpart in the reference). When a wait
+ * gives up, no step is integrated until the host has been told: the positions
+ * and velocities stay those of the last step whose solve was whole, and the
+ * next fem_solid_synchronize (also as part of fem_solid_step and
+ * fem_solid_step_host, whatever their number of steps; with the FIE integrators and in a lock-step
+ * the call that solves) returns FEM_E_TIMEOUT once. The default
+ * (FEM_WAIT_LIMIT_DEFAULT) is 2^20 polls, about a second; with 0 a wait gives
+ * up unless what it waits for is there. */
+int fem_solid_set_wait_limit(fem_solid s, uint32_t polls);
+
 /* Replaces: the multi-solid Newton lock-step phases of the Leaf,
  * NR_Init / NR_PreStep / NR_MidStep / NR_PostStep / NR_End
  * (LeafDSH_Solid3D_FEM.cpp:2824-3039), which the aggregate scheme

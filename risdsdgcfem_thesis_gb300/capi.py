@@ -137,6 +137,7 @@ SIGNATURES = {
     "fem_solid_apply_A_noalloc": (C.c_int, [C.c_void_p, C.c_double, C.c_double, _dp, _dp]),
     "fem_solid_set_params": (C.c_int, [C.c_void_p, C.POINTER(FemParams)]),
     "fem_solid_set_assembled": (C.c_int, [C.c_void_p, C.c_int]),
+    "fem_solid_set_wait_limit": (C.c_int, [C.c_void_p, C.c_uint32]),
     "fem_solid_nr_init": (C.c_int, [C.c_void_p, C.c_double]),
     "fem_solid_nr_prestep": (C.c_int, [C.c_void_p, C.c_double]),
     "fem_solid_nr_midstep": (C.c_int, [C.c_void_p, C.c_double]),
@@ -292,6 +293,10 @@ class Solid:
         3x3-block stiffness (on) or from the element products (off, the
         default)."""
         check(self.lib.fem_solid_set_assembled(self.h, 1 if on else 0))
+
+    def set_wait_limit(self, polls=None):
+        """Poll limit of the resident solve's device waits (None: default)."""
+        check(self.lib.fem_solid_set_wait_limit(self.h, FEM_WAIT_LIMIT_DEFAULT if polls is None else int(polls)))
 
     def nr_phase(self, phase, dt):
         """One multi-solid Newton lock-step phase (init, prestep, midstep,

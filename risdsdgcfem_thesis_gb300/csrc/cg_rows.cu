@@ -35,8 +35,6 @@ namespace femgb {
 
 namespace {
 
-constexpr uint32_t kWordPolls = 1u << 20;  // each an L2 round trip
-
 // A 128-bit word, each half with the exchange's number in its top bits.
 __device__ __forceinline__ void word_put(ulonglong2* p, unsigned long long a, unsigned long long b)
 {
@@ -108,7 +106,7 @@ __device__ __noinline__ double divide(double a, double b) { return a / b; }
 // Polls n words (get(i), one per lane and turn) and adds them, in every lane
 // of the warp; bad when the wait gave up.
 template <int K, typename F>
-__device__ __forceinline__ Part words_sum(F&& get, uint32_t n, uint32_t seq, bool& bad)
+__device__ __forceinline__ Part words_sum(F&& get, uint32_t n, uint32_t seq, uint32_t limit, bool& bad)
 {
     const uint32_t lane = threadIdx.x & 31u;
     Part part[K];
@@ -124,7 +122,7 @@ __device__ __forceinline__ Part words_sum(F&& get, uint32_t n, uint32_t seq, boo
             if (!on) part[i] = Part{0, 0};
         }
         ok = __all_sync(0xffffffffu, ok);
-    } while (!ok && ++polls <= kWordPolls);
+    } while (!ok && ++polls <= limit);
     bad = bad || !ok;
     return part_sum(part);
 }
@@ -335,14 +333,14 @@ __global__ void __launch_bounds__(kCgRowsMaxThreads, 1)
         meanwhile();
         const uint32_t n = C * vwarps, at = near_address(own, rank);
         auto get = [&](uint32_t i) { return near_get(at + (uint32_t)sizeof(ulonglong2) * i); };
-        Part s = n <= 32 ? words_sum<1>(get, n, seq, bad) : (n <= 96 ? words_sum<3>(get, n, seq, bad) : words_sum<5>(get, n, seq, bad));
+        Part s = n <= 32 ? words_sum<1>(get, n, seq, p.polls, bad) : (n <= 96 ? words_sum<3>(get, n, seq, p.polls, bad) : words_sum<5>(get, n, seq, p.polls, bad));
         if (nrow > 1) {
             ulonglong2* words = p.parts + (size_t)which * G * nrow;
             const ulonglong2 w = rows_word<ulonglong2>(s, seq);
             for (uint32_t i = lane; i < nrow; i += 32) word_put(words + (size_t)(i * C + rank) * nrow + g / C, w.x, w.y);
             words += (size_t)g * nrow;
             auto there = [&](uint32_t i) { return word_get(words + i); };
-            s = nrow <= 32 ? words_sum<1>(there, nrow, seq, bad) : words_sum<3>(there, nrow, seq, bad);
+            s = nrow <= 32 ? words_sum<1>(there, nrow, seq, p.polls, bad) : words_sum<3>(there, nrow, seq, p.polls, bad);
         }
         return part_value(s);
     };
@@ -360,7 +358,7 @@ __global__ void __launch_bounds__(kCgRowsMaxThreads, 1)
                 const ulonglong2* f = p.words + 3 * (size_t)rim[k] + a;
                 uint32_t polls = 0;
                 while (!rows_word_is(w == kCgRowsFar ? word_get(f) : near_get(w + (uint32_t)sizeof(ulonglong2) * a), rimr[i], seq))
-                    if (++polls > kWordPolls) {
+                    if (++polls > p.polls) {
                         bad = 1;
                         break;
                     }
@@ -544,6 +542,7 @@ __global__ void __launch_bounds__(kCgRowsMaxThreads, 1)
     }
     cluster_sync();  // no CTA leaves while another may still use its shared memory
     if (mine) y[at] = ny;
+    if (go < 0 && tid == 0) st->gave_up = 1;  // any block's wait: another one may have seen the loop end
     if (g == 0 && tid == 0) {
         st->delta_0 = delta_0;
         st->delta_new = delta;

@@ -76,6 +76,9 @@ struct StepScalars {
     double delta_pend;
     MinresScalars mr_pend;
     uint32_t done_pend;
+    // FP64 solid: a wait of the resident solve gave up; stays until the host
+    // has read it, and no step is integrated in the meantime
+    uint32_t gave_up;
 };
 
 // One MINRES iteration's Givens rotation and update coefficients from
@@ -196,7 +199,9 @@ void launch_node_xr_fp64(const MeshView<double>& m, double* y, double* r, const 
 // (with the assembled stiffness also the records of d)
 void launch_node_d_fp64(const MeshView<double>& m, double* d, const double* r, const double* pr, StepScalars* st,
                         cudaStream_t s, cudaGraphConditionalHandle cond = 0, int set_cond = 0);
-void launch_integrate_fp64(uint32_t N, double dt, double* x, double* v, const double* y, cudaStream_t s);
+// (nothing once a solve has given up)
+void launch_integrate_fp64(uint32_t N, double dt, double* x, double* v, const double* y, const StepScalars* st,
+                           cudaStream_t s);
 // Fully-implicit Euler (Newton on Delta x) pieces, FP64 solid path.
 void launch_node_b_fie_fp64(const MeshView<double>& m, const StepConsts& c, const double* x, const double* xn,
                             const double* vn, int warm, double* b, double* y, cudaStream_t s);
@@ -277,6 +282,7 @@ struct CgRowsView {
     ulonglong2* parts;  // [2][blocks][clusters]: the clusters' sums
     uint32_t cluster, warps, npb, units, records;  // CgRowsPlan's
     uint32_t* seq;  // the last number used
+    uint32_t polls;  // of a word that is not there yet, before the wait gives up
 };
 // The blocks of the plan's shape that are resident together; 0 when it does not launch.
 uint32_t cg_rows_max_blocks(const CgRowsPlan& p);

@@ -934,8 +934,10 @@ __global__ void k_node_d_fp64(MeshView<double> m, double* d, const double* __res
 }
 
 // v = y ; x += dt y   (Step_QuasiImplicitEuler_v, :1322-1327)
-__global__ void k_integrate_fp64(uint32_t N, double dt, double* x, double* v, const double* __restrict__ y)
+__global__ void k_integrate_fp64(uint32_t N, double dt, double* x, double* v, const double* __restrict__ y,
+                                 const StepScalars* st)
 {
+    if (st->gave_up) return;
     const uint32_t n3 = 3 * N;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n3; i += gridDim.x * blockDim.x) {
         const double yi = y[i];
@@ -1385,9 +1387,10 @@ void launch_node_d_fp64(const MeshView<double>& m, double* d, const double* r, c
     else
         FEMGB_LAUNCH(k_node_d_fp64<false>, npr, row_block(3 * m.N), m, d, r, pr, npr, st, cond, set_cond);
 }
-void launch_integrate_fp64(uint32_t N, double dt, double* x, double* v, const double* y, cudaStream_t s)
+void launch_integrate_fp64(uint32_t N, double dt, double* x, double* v, const double* y, const StepScalars* st,
+                           cudaStream_t s)
 {
-    FEMGB_LAUNCH(k_integrate_fp64, vec_grid(3 * N), row_block(3 * N), N, dt, x, v, y);
+    FEMGB_LAUNCH(k_integrate_fp64, vec_grid(3 * N), row_block(3 * N), N, dt, x, v, y, st);
 }
 void launch_node_b_fie_fp64(const MeshView<double>& m, const StepConsts& c, const double* x, const double* xn,
                             const double* vn, int warm, double* b, double* y, cudaStream_t s)

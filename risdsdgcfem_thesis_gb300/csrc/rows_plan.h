@@ -83,6 +83,7 @@ constexpr uint32_t kCgRowsPad = 0xffffffffu, kCgRowsFar = 0xffffffffu;
 constexpr uint32_t kCgRowsFarShared = 0x80000000u, kCgRowsNearShared = 0x40000000u, kCgRowsNode = 0x3fffffffu;
 constexpr uint32_t kCgRowsMaxThreads = 768, kCgRowsMaxBlocks = 160, kCgRowsMaxWords = 160;  // words: five per lane of a warp
 constexpr size_t kCgRowsMaxSmem = 226 * 1024;
+constexpr uint32_t kCgRowsPolls = 1u << 20;  // default poll limit of a wait, each an L2 round trip
 struct CgRowsBlock {
     uint32_t node0, nn, group0, ngroups, unit0, units, halo0, nhalo;
 };

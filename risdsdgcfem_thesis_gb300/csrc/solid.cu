@@ -124,6 +124,7 @@ struct fem_solid_s {
     // stiffness below
     CgRowsPlan rows{};
     bool rows_tried = false;
+    uint32_t wait_polls = kCgRowsPolls;
     DevBuf<CgRowsBlock> rows_blk;
     DevBuf<uint32_t> rows_node, rows_group, rows_slot, rows_halo, rows_owner, rows_seq;
     DevBuf<uint16_t> rows_col;
@@ -606,7 +607,7 @@ cudaError_t solve_on_rows(fem_solid s, const StepConsts& c)
     const CgRowsPlan& p = s->rows;
     const CgRowsView v{s->rows_blk.p, s->rows_node.p, s->rows_group.p, s->rows_slot.p, s->rows_halo.p, s->rows_owner.p,
                        s->rows_col.p, s->rows_words.p, s->rows_words.p + 3 * (size_t)s->N, p.cluster, p.warps, p.npb,
-                       p.units, p.records, s->rows_seq.p};
+                       p.units, p.records, s->rows_seq.p, s->wait_polls};
     return launch_cg_rows_fp64(m, c, s->rows, v, s->params.ls_solver == FEM_LS_MINRES, s->b.p, s->y.p, s->st.p, s->stream);
 }
 
@@ -619,11 +620,18 @@ int fork_operator(fem_solid s)
     });
 }
 
-// The solve's status as an error of the call.
-int solve_status(const StepScalars& h)
+// What the scalars in st_host say of the solves as an error of the call: a
+// wait that gave up, reported once, or the last solve's NaN.
+int report_give_up(fem_solid s)
 {
-    if (h.status == FEM_E_NAN) return fail(FEM_E_NAN, "NaN or Inf in the CG residual");
-    if (h.status == FEM_E_TIMEOUT) return fail(FEM_E_TIMEOUT, "a device-side wait of the linear solve gave up");
+    if (!s->st_host->gave_up) return FEM_OK;
+    CK(cudaMemsetAsync(&s->st.p->gave_up, 0, sizeof(uint32_t), s->stream));
+    return fail(FEM_E_TIMEOUT, "a device-side wait of the linear solve gave up");
+}
+int solve_status(fem_solid s)
+{
+    if (int e = report_give_up(s)) return e;
+    if (s->st_host->status == FEM_E_NAN) return fail(FEM_E_NAN, "NaN or Inf in the CG residual");
     return FEM_OK;
 }
 
@@ -705,7 +713,7 @@ int ls_solve(fem_solid s, const StepConsts& c, int chunk)
         CK(cudaMemcpyAsync(s->st_host, s->st.p, sizeof(StepScalars), cudaMemcpyDeviceToHost, s->stream));
         CK(cudaStreamSynchronize(s->stream));
         CK(cudaGetLastError());
-        return s->st_host->status == FEM_E_TIMEOUT ? solve_status(*s->st_host) : FEM_OK;
+        return report_give_up(s);
     }
     return s->params.ls_solver == FEM_LS_MINRES ? minres_solve(s, c, chunk) : cg_solve(s, c, chunk);
 }
@@ -842,7 +850,13 @@ int step_fie(fem_solid s, int chunk)
         if (!std::isfinite(delta_new)) return fail(FEM_E_NAN, "NaN or Inf in the Newton right-hand side");
         converged = delta_new < s->params.nr_abs_epsilon;
         if (!converged) {
-            if (int e = ls_solve(s, c, chunk)) return e;
+            if (int e = ls_solve(s, c, chunk)) {
+                if (e == FEM_E_TIMEOUT) {  // the step is not made
+                    CK(cudaMemcpyAsync(s->x.p, s->xn.p, bytes, cudaMemcpyDeviceToDevice, st));
+                    CK(cudaMemcpyAsync(s->v.p, s->vn.p, bytes, cudaMemcpyDeviceToDevice, st));
+                }
+                return e;
+            }
             cg_iters += s->st_host->k;
             solved = true;
             launch_fie_update_fp64(s->N, c.inv_dt, s->x.p, s->v.p, s->xn.p, s->y.p, s->partials.p, st);
@@ -882,7 +896,7 @@ int qie_head(fem_solid s)
 int qie_tail(fem_solid s)
 {
     const StepConsts& c = s->consts;
-    launch_integrate_fp64(s->N, c.dt, s->x.p, s->v.p, s->y.p, s->stream);
+    launch_integrate_fp64(s->N, c.dt, s->x.p, s->v.p, s->y.p, s->st.p, s->stream);
     return s->params.compute_energy ? energy(s) : FEM_OK;
 }
 
@@ -934,7 +948,7 @@ int step_once(fem_solid s, int chunk)
 void fill_stats(fem_solid s, const StepScalars& h, fem_step_stats* out)
 {
     out->cg_iterations = h.k;
-    out->status = h.status;
+    out->status = h.gave_up ? FEM_E_TIMEOUT : h.status;
     out->rel_residual = h.rel_residual;
     out->abs_residual = h.abs_residual;
     out->elastic_energy = h.elastic_energy;
@@ -1239,6 +1253,14 @@ int fem_solid_set_assembled(fem_solid s, int on)
     return FEM_OK;
 }
 
+int fem_solid_set_wait_limit(fem_solid s, uint32_t polls)
+{
+    if (int e = check_handle(s)) return e;
+    s->drop_graph();  // the step graph holds the limit
+    s->wait_polls = polls == FEM_WAIT_LIMIT_DEFAULT ? kCgRowsPolls : polls;
+    return FEM_OK;
+}
+
 int fem_solid_get_sizes(fem_solid s, uint32_t* N, uint32_t* T)
 {
     if (int e = check_handle(s)) return e;
@@ -1420,8 +1442,7 @@ int fem_solid_nr_midstep(fem_solid s, double dt)
     if (int e = ls_solve(s, c, 8)) return e;
     s->lock_ls_iters += s->st_host->k;
     CK(cudaGetLastError());
-    if (int e = solve_status(*s->st_host)) return e;
-    return FEM_OK;
+    return solve_status(s);
 }
 
 int fem_solid_nr_poststep(fem_solid s, double dt)
@@ -1547,8 +1568,7 @@ int fem_solid_synchronize(fem_solid s, fem_step_stats* stats)
     CK(cudaMemcpyAsync(s->st_host, s->st.p, sizeof(StepScalars), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     if (stats) fill_stats(s, *s->st_host, stats);
-    if (int e = solve_status(*s->st_host)) return e;
-    return FEM_OK;
+    return solve_status(s);
 }
 
 int fem_solid_step(fem_solid s, uint32_t nsteps, fem_step_stats* stats)

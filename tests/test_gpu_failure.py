@@ -133,3 +133,55 @@ def test_lock_step_reports_a_wait_that_gives_up(fem_lib):
         b.nr_phase("midstep", 1 / 60)
     assert e.value.code == fem_lib.FEM_E_TIMEOUT
     _same_after_recovery(fem_lib, b, fresh, x0, lambda s: s.multi_step(1 / 60))
+
+
+@pytest.mark.parametrize("dims", [(10, 10, 6), (17, 16, 15)], ids=["cluster", "clusters"])
+@pytest.mark.parametrize("solver", [0, 1])
+@pytest.mark.parametrize("integrator", [0, 1])
+def test_resident_solve_gives_up_and_reports_timeout(fem_lib, dims, solver, integrator):
+    """A solve whose waits give up reports it once, however many steps the
+    call makes and whatever the later solves do, and no step is made from it;
+    then the solid steps as a fresh one."""
+    rest, tets, _ = scenes.grid_mesh(*dims, 0.1, 0.01, 5)
+    sc = scenes.Scene(name="block", rest=rest, tets=tets, ls_solver=solver, integrator=integrator)
+    sc.init_vel = 0.1 * np.random.default_rng(5).standard_normal(rest.shape)
+    s, fresh = fem_lib.Solid(sc), fem_lib.Solid(sc)
+    x0, v0 = s.state()
+    s.step(1)
+    s.set_state(x0, v0)
+    s.set_wait_limit(0)
+    with pytest.raises(fem_lib.FemError) as e:
+        s.step(3)
+    assert e.value.code == fem_lib.FEM_E_TIMEOUT
+    assert all(np.array_equal(a, b) for a, b in zip(s.state(), (x0, v0)))
+    if integrator == 0:  # unread while the later solves are whole
+        assert fem_lib.load().fem_solid_step_async(s.h, 1) == fem_lib.FEM_OK
+        s.set_wait_limit(None)
+        with pytest.raises(fem_lib.FemError) as e:
+            s.step(2)
+        assert e.value.code == fem_lib.FEM_E_TIMEOUT
+        assert all(np.array_equal(a, b) for a, b in zip(s.state(), (x0, v0)))
+    s.set_wait_limit(None)
+    s.step(2)
+    fresh.step(2)
+    assert s.stats()["cg_iterations"] == fresh.stats()["cg_iterations"]
+    for a, b in zip(s.state(), fresh.state()):
+        assert np.isfinite(a).all() and np.array_equal(a, b)
+
+
+def test_lock_step_solve_gives_up_and_reports_timeout(fem_lib):
+    rest, tets, _ = scenes.grid_mesh(10, 10, 6, 0.1, 0.01, 5)
+    sc = scenes.Scene(name="block", rest=rest, tets=tets)
+    sc.init_vel = 0.1 * np.random.default_rng(5).standard_normal(rest.shape)
+    s, fresh = fem_lib.Solid(sc), fem_lib.Solid(sc)
+    s.set_wait_limit(0)
+    s.nr_phase("init", 1 / 60)
+    s.nr_phase("prestep", 1 / 60)
+    with pytest.raises(fem_lib.FemError) as e:
+        s.nr_phase("midstep", 1 / 60)
+    assert e.value.code == fem_lib.FEM_E_TIMEOUT
+    s.set_wait_limit(None)
+    for a in (s, fresh):
+        fem_lib.multi_step([a], 1 / 60)
+    for a, b in zip(s.state(), fresh.state()):
+        assert np.array_equal(a, b)
