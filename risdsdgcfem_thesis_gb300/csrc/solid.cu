@@ -454,8 +454,9 @@ int fork(fem_solid s, F&& work)
 }
 int join(fem_solid s)
 {
-    if (s->forked) CK(cudaStreamWaitEvent(s->stream, s->side_end, 0));
+    const bool forked = s->forked;
     s->forked = false;
+    if (forked) CK(cudaStreamWaitEvent(s->stream, s->side_end, 0));
     return FEM_OK;
 }
 
@@ -468,7 +469,6 @@ int fork_operator(fem_solid s);
 // (LeafDSH_Solid3D_FEM.cpp:927-935).
 int open_step(fem_solid s)
 {
-    if (int e = join(s)) return e;  // an abandoned step's
     cudaStream_t st = s->stream;
     CK(cudaMemsetAsync(&s->st.p->inverted, 0, sizeof(uint32_t), st));
     begin_eval(s, s->prev_x.p, s->x.p);
@@ -820,7 +820,7 @@ int energy(fem_solid s)
 //   A = (1/h^2 + a0/h) M + (1 + a1/h) K(x_k),
 // x_k += y, v_k = (x_k - x^n)/h, |y|, and BeginEvaluation at the new x_k.
 // h = 0 (quasi-static) drops every 1/h term.
-int step_fie(fem_solid s, int chunk)
+int newton_step(fem_solid s, int chunk)
 {
     cudaStream_t st = s->stream;
     MeshView<double> m = s->view();
@@ -868,7 +868,7 @@ int step_fie(fem_solid s, int chunk)
             begin_eval(s, s->xn.p, s->x.p);
         }
     } while (!converged && nr_k < s->params.nr_max_iter);
-    if (int e = join(s)) return e;
+    if (int e = join(s)) return e;  // the operator of a step that needed no solve
     s->nr_iters = nr_k;
     s->fie_cg_iters = cg_iters;
     s->fie_solved = solved;
@@ -878,6 +878,13 @@ int step_fie(fem_solid s, int chunk)
         if (int e = energy(s)) return e;
     CK(cudaGetLastError());
     return FEM_OK;
+}
+
+int step_fie(fem_solid s, int chunk)
+{
+    const int rc = newton_step(s, chunk);
+    const int e = join(s);  // nothing goes on beside the next call, also where the step has failed
+    return rc ? rc : e;
 }
 
 // One FixedStep's QIE_V pipeline after the opening: f_e, b, constraints,
@@ -921,6 +928,7 @@ int capture_step(fem_solid s)
     const cudaError_t e2 = cudaStreamEndCapture(st, &g);
     if (e == cudaSuccess) e = e2;
     s->kfx_fresh = s->bsr_fresh = false;  // captured, not run
+    s->forked = false;
     if (rc != FEM_OK || e != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
         if (rc != FEM_OK) return rc;

@@ -10,6 +10,8 @@
   FEM_E_NAN (ILSS_CG.h:42-46 -- the reference has no such check; its loop
   test is false for NaN and it returns silently).
 """
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -185,3 +187,25 @@ def test_lock_step_solve_gives_up_and_reports_timeout(fem_lib):
         fem_lib.multi_step([a], 1 / 60)
     for a, b in zip(s.state(), fresh.state()):
         assert np.array_equal(a, b)
+
+
+def test_step_graph_after_a_newton_step_that_failed(fem_lib):
+    """A Newton step that ends at a NaN right-hand side leaves work on the
+    solid's second stream; a step graph captured next does not wait for it."""
+    sc = scenes.cantilever_160()
+    fresh = fem_lib.Solid(sc)
+    sc = dataclasses.replace(sc, integrator=1)
+    s = fem_lib.Solid(sc)
+    x0, v0 = s.state()
+    s.set_state(v=_nan_velocity(sc))
+    with pytest.raises(fem_lib.FemError) as e:
+        s.step(1)
+    assert e.value.code == fem_lib.FEM_E_NAN
+    s.set_state(x0, v0)
+    p = s.get_params()
+    p.integrator = 0
+    s.set_params(p)
+    s.step(2)
+    fresh.step(2)
+    for a, b in zip(s.state(), fresh.state()):
+        assert np.isfinite(a).all() and np.array_equal(a, b)
