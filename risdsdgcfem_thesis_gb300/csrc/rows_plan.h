@@ -127,7 +127,6 @@ bool cg_rows_layout(uint32_t N, const BsrPattern& p, F&& max_blocks, CgRowsLayou
 {
     if (N > kCgRowsNode) return false;
     std::vector<uint32_t> order(N), seen(N, 0), place(N);
-    for (uint32_t n = 0; n < N; n++) order[n] = n;
     uint32_t sorted = 0;  // rows per block that order is sorted for
     auto build = [&](uint32_t blocks, uint32_t cluster, uint32_t lanes) {
         const uint32_t npb = (N + blocks - 1) / blocks, rows = 32 / lanes, warps = (3 * npb + 31) / 32;
@@ -135,6 +134,7 @@ bool cg_rows_layout(uint32_t N, const BsrPattern& p, F&& max_blocks, CgRowsLayou
             cluster * warps > kCgRowsMaxWords || blocks / cluster > 96)
             return false;
         if (sorted != npb) {
+            for (uint32_t n = 0; n < N; n++) order[n] = n;
             for (uint32_t a = 0; a < N; a += npb)
                 std::sort(order.begin() + a, order.begin() + std::min(N, a + npb),
                           [&](uint32_t i, uint32_t j) { return p.used[i] != p.used[j] ? p.used[i] > p.used[j] : i < j; });

@@ -140,6 +140,61 @@ def test_layout_covers_the_rows(shim, mesh, shuffle, sms):
     assert np.array_equal(y, ref)
 
 
+FITS = r"""
+#include "rows_plan.h"
+using namespace femgb;
+// Bit 0: the layout succeeds; bit 2: some block does not hold its own range of nodes.
+extern "C" int fits(uint32_t N, uint32_t T, const uint32_t* tets)
+{
+    std::vector<uint32_t> ptr(N + 1, 0), idx(4 * (size_t)T);
+    for (size_t i = 0; i < 4 * (size_t)T; i++) ptr[tets[i] + 1]++;
+    for (uint32_t n = 0; n < N; n++) ptr[n + 1] += ptr[n];
+    std::vector<uint32_t> fill(ptr.begin(), ptr.end() - 1);
+    for (size_t i = 0; i < 4 * (size_t)T; i++) idx[fill[tets[i]]++] = (uint32_t)i;
+    auto blocks = [](const CgRowsPlan& q) {
+        return q.threads > kCgRowsMaxThreads || q.smem > kCgRowsMaxSmem ? 0u : q.cluster == 2 ? 152u : 120u;
+    };
+    BsrPattern p;
+    CgRowsLayout l;
+    int r = bsr_pattern(N, T, tets, ptr, idx, p) && cg_rows_layout(N, p, blocks, l) ? 1 : 0;
+    if (r & 1)
+        for (const CgRowsBlock& b : l.blk)
+            for (uint32_t i = b.node0; i < b.node0 + b.nn; i++) {
+                const uint32_t n = l.node[i] & kCgRowsNode;
+                if (n < b.node0 || n >= b.node0 + b.nn) r |= 4;
+            }
+    return r;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def fits(tmp_path_factory):
+    if shutil.which("g++") is None:
+        pytest.skip("no host compiler")
+    d = tmp_path_factory.mktemp("fits")
+    src, so = d / "fits.cpp", d / "fits.so"
+    src.write_text(FITS)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", CSRC, str(src), "-o", str(so)], check=True)
+    return C.CDLL(str(so)).fits
+
+
+@pytest.mark.parametrize("mesh,fit", [(_grid(1, 1, 1), True), (_grid(12, 12, 12), True), (_grid(16, 16, 16), True),
+                                      (_grid(26, 26, 26), True), (_grid(28, 28, 27), True), (_grid(80, 80, 2), True),
+                                      (_grid(28, 28, 28), False), (_grid(60, 20, 18), False), (_grid(100, 30, 6), False),
+                                      (_grid(200, 11, 11), False), (_grid(1000, 5, 5), False), (_star(150), True),
+                                      (_star(3000), False)],
+                         ids=["5", "8640", "20480", "87880", "105840", "flat64000", "109760", "108000", "flat90000",
+                              "long121000", "long125000", "star", "star3000"])
+def test_layout_of_the_largest_meshes(fits, mesh, fit):
+    """Which meshes have a layout (120 SMs in clusters of 8, 152 in pairs); the
+    blocks hold ranges of nodes whatever shape was tried first."""
+    n, tets = mesh
+    tets = np.ascontiguousarray(tets, np.uint32)
+    r = fits(n, len(tets), tets.ctypes.data_as(C.POINTER(C.c_uint32)))
+    assert bool(r & 1) == fit and not r & 4
+
+
 WORDS = r"""
 #include "rows_words.h"
 using namespace femgb;
