@@ -16,57 +16,67 @@ namespace femgb {
 struct BsrPattern {
     std::vector<uint32_t> row, used, col, cptr, contrib;
 };
-// False: too large. ptr/idx: the node CSR of element corners.
+// False: too large. ptr/idx: the node CSR of element corners. One pass over
+// the corners finds a row's columns and counts its contributions, which start
+// at three per corner.
 inline bool bsr_pattern(uint32_t N, uint32_t T, const uint32_t* tets, const std::vector<uint32_t>& ptr,
                  const std::vector<uint32_t>& idx, BsrPattern& p)
 {
     if ((uint64_t)T >= (1ull << 28)) return false;  // contributions pack the element in 28 bits
-    std::vector<uint32_t> seen(N, 0xffffffffu), place(N), at(12 * (size_t)T), nb;
+    std::vector<uint32_t> seen(N, 0xffffffffu), place(N), count, which;
+    std::vector<uint64_t> nb;  // column << 32 | the order it was met in
     p.row.assign(N + 1, 0);
     p.used.resize(N);
     p.col.reserve(18 * (size_t)N);
-    std::vector<uint32_t> count;
-    count.reserve(18 * (size_t)N);
-    size_t k = 0;
+    p.cptr.reserve(18 * (size_t)N + 1);
+    p.contrib.resize(12 * (size_t)T);
     for (uint32_t n = 0; n < N; n++) {
-        nb.assign(1, n);
+        const uint32_t beg = ptr[n], end = ptr[n + 1];
+        const size_t most = 3 * (size_t)(end - beg) + 1;
+        if (nb.size() < most) {
+            nb.resize(2 * most);
+            count.resize(2 * most);
+            which.resize(2 * most);
+        }
+        uint64_t* const col = nb.data();
+        uint32_t *const at = count.data(), *w = which.data();
+        uint32_t used = 1;
+        col[0] = (uint64_t)n << 32;
+        at[0] = place[n] = 0;
         seen[n] = n;
-        for (uint32_t j = ptr[n]; j < ptr[n + 1]; j++)
-            for (int i = 0; i < 4; i++) {
-                const uint32_t c = tets[4 * (size_t)(idx[j] >> 2) + i];
+        for (uint32_t j = beg; j < end; j++)
+            for (uint32_t k = 1; k < 4; k++) {
+                const uint32_t c = tets[(size_t)(idx[j] & ~3u) + ((idx[j] + k) & 3u)];
                 if (seen[c] != n) {
                     seen[c] = n;
-                    nb.push_back(c);
+                    place[c] = used;
+                    at[used] = 0;
+                    col[used] = (uint64_t)c << 32 | used;
+                    used++;
                 }
+                at[*w++ = place[c]]++;
             }
-        std::sort(nb.begin(), nb.end());
-        p.used[n] = (uint32_t)nb.size();
-        const uint32_t base = (uint32_t)p.col.size();
-        for (uint32_t i = 0; i < nb.size(); i++) place[nb[i]] = base + i;
-        while (nb.size() % 4) nb.push_back(n);
-        p.col.insert(p.col.end(), nb.begin(), nb.end());
+        std::sort(col, col + used);
+        p.used[n] = used;
+        uint32_t next = 3 * beg;
+        for (uint32_t i = 0; i < used; i++) {
+            uint32_t& k = at[(uint32_t)col[i]];
+            p.col.push_back((uint32_t)(col[i] >> 32));
+            p.cptr.push_back(next);
+            next += k;
+            k = next - k;  // where its next contribution goes
+        }
+        while (p.col.size() % 4) {
+            p.col.push_back(n);
+            p.cptr.push_back(next);
+        }
         if (p.col.size() >= (1ull << 28)) return false;
         p.row[n + 1] = (uint32_t)(p.col.size() / 4);
-        count.resize(p.col.size(), 0);
-        for (uint32_t j = ptr[n]; j < ptr[n + 1]; j++)
-            for (uint32_t lj = 0; lj < 4; lj++) {
-                if (lj == (idx[j] & 3u)) continue;
-                at[k] = place[tets[4 * (size_t)(idx[j] >> 2) + lj]];
-                count[at[k++]]++;
-            }
+        w = which.data();
+        for (uint32_t j = beg; j < end; j++)
+            for (uint32_t k = 1; k < 4; k++) p.contrib[at[*w++]++] = idx[j] << 2 | ((idx[j] + k) & 3u);
     }
-    const size_t slots = p.col.size();
-    p.cptr.assign(slots + 1, 0);
-    for (size_t i = 0; i < slots; i++) p.cptr[i + 1] = p.cptr[i] + count[i];
-    std::copy(p.cptr.begin(), p.cptr.end() - 1, count.begin());  // where the next one goes
-    p.contrib.resize(12 * (size_t)T);
-    k = 0;
-    for (uint32_t n = 0; n < N; n++)
-        for (uint32_t j = ptr[n]; j < ptr[n + 1]; j++) {
-            const uint32_t e = idx[j] >> 2, li = idx[j] & 3u;
-            for (uint32_t lj = 0; lj < 4; lj++)
-                if (lj != li) p.contrib[count[at[k++]]++] = (e << 4) | (li << 2) | lj;
-        }
+    p.cptr.push_back(12 * T);
     return true;
 }
 
@@ -122,6 +132,79 @@ struct CgRowsLayout {
 // lanes per row while a block has up to 16 rows, else 8 (20,480 tets: 660 us
 // with 16, 658 us with 4), else 4.
 constexpr uint32_t kRowsPerBlock = 8;
+// lay(blocks, cluster) for each shape, the best one first, until one is true.
+template <typename F, typename L>
+bool cg_rows_shapes(uint32_t N, F&& max_blocks, L&& lay)
+{
+    const uint32_t near = std::max(1u, std::min(16u, (N + kRowsPerBlock - 1) / kRowsPerBlock));
+    if (lay(near, near)) return true;
+    for (uint32_t cluster : {8u, 2u}) {
+        CgRowsPlan shape;
+        shape.lanes = 4;
+        shape.threads = kCgRowsMaxThreads;
+        shape.smem = kCgRowsMaxSmem;
+        shape.cluster = cluster;
+        const uint32_t blocks = max_blocks(shape) / cluster * cluster;
+        if (blocks && lay(blocks, cluster)) return true;
+    }
+    return false;
+}
+inline bool cg_rows_shape_ok(uint32_t npb, uint32_t blocks, uint32_t cluster, uint32_t lanes)
+{
+    return 3 * npb + (blocks > 1 ? 32u : 0u) <= kCgRowsMaxThreads && (lanes <= 4 || lanes * npb <= kCgRowsMaxThreads) &&
+           cluster * ((3 * npb + 31) / 32) <= kCgRowsMaxWords && blocks / cluster <= 96;
+}
+
+// Whether cg_rows_layout can succeed, from three blocks of each shape: the
+// least their rows, vectors and rims take. Ahead of the pattern, which takes
+// far longer (109,760 tets, which do not fit: 0.1 ms against 4.3 and 3.5 for
+// pattern and layout).
+template <typename F>
+bool cg_rows_may_fit(uint32_t N, const uint32_t* tets, const std::vector<uint32_t>& ptr,
+                     const std::vector<uint32_t>& idx, F&& max_blocks)
+{
+    std::vector<uint32_t> in_row(N, 0), in_rim(N, 0), used;
+    uint32_t row = 0, mark = 0;
+    return cg_rows_shapes(N, max_blocks, [&](uint32_t blocks, uint32_t cluster) {
+        CgRowsPlan plan;
+        plan.cluster = cluster;
+        plan.npb = (N + blocks - 1) / blocks;
+        plan.warps = (3 * plan.npb + 31) / 32;
+        if (!cg_rows_shape_ok(plan.npb, blocks, cluster, 4)) return false;
+        for (uint32_t g : {blocks / 2, blocks / 4, blocks - 1 - blocks / 4}) {
+            const uint32_t a = std::min(N, g * plan.npb), e = std::min(N, a + plan.npb);
+            CgRowsBlock b{a, e - a, 0, 0, 0, 0, 0, 0};
+            used.assign(e - a, 1);
+            mark++;
+            for (uint32_t n = a; n < e; n++) {
+                in_row[n] = ++row;
+                for (uint32_t j = ptr[n]; j < ptr[n + 1]; j++)
+                    for (uint32_t k = 1; k < 4; k++) {
+                        const uint32_t c = tets[(size_t)(idx[j] & ~3u) + ((idx[j] + k) & 3u)];
+                        if (in_row[c] == row) continue;
+                        in_row[c] = row;
+                        used[n - a]++;
+                        if ((c < a || c >= e) && in_rim[c] != mark) {
+                            in_rim[c] = mark;
+                            b.nhalo++;
+                        }
+                    }
+            }
+            plan.records = b.nn + b.nhalo;
+            std::sort(used.begin(), used.end(), [](uint32_t i, uint32_t j) { return i > j; });
+            size_t least = ~(size_t)0;
+            for (uint32_t lanes : {4u, 8u, 16u}) {
+                b.units = b.ngroups = 0;
+                for (uint32_t i = 0; i < e - a; i += 32 / lanes, b.ngroups++) b.units += (used[i] + lanes - 1) / lanes;
+                plan.units = b.units;
+                least = std::min(least, cg_rows_smem_bytes(plan, b));
+            }
+            if (least > kCgRowsMaxSmem) return false;
+        }
+        return true;
+    });
+}
+
 template <typename F>
 bool cg_rows_layout(uint32_t N, const BsrPattern& p, F&& max_blocks, CgRowsLayout& o)
 {
@@ -130,9 +213,7 @@ bool cg_rows_layout(uint32_t N, const BsrPattern& p, F&& max_blocks, CgRowsLayou
     uint32_t sorted = 0;  // rows per block that order is sorted for
     auto build = [&](uint32_t blocks, uint32_t cluster, uint32_t lanes) {
         const uint32_t npb = (N + blocks - 1) / blocks, rows = 32 / lanes, warps = (3 * npb + 31) / 32;
-        if (3 * npb + (blocks > 1 ? 32u : 0u) > kCgRowsMaxThreads || (lanes > 4 && lanes * npb > kCgRowsMaxThreads) ||
-            cluster * warps > kCgRowsMaxWords || blocks / cluster > 96)
-            return false;
+        if (!cg_rows_shape_ok(npb, blocks, cluster, lanes)) return false;
         if (sorted != npb) {
             for (uint32_t n = 0; n < N; n++) order[n] = n;
             for (uint32_t a = 0; a < N; a += npb)
@@ -192,6 +273,7 @@ bool cg_rows_layout(uint32_t N, const BsrPattern& p, F&& max_blocks, CgRowsLayou
             const uint32_t rim = std::min((3 * b.nhalo + 31) / 32 * 32, 256u);
             plan.threads = std::max({plan.threads, 32 * b.ngroups, 32 * warps + rim});
             o.blk.push_back(b);
+            if (cg_rows_smem_bytes(plan, b) > kCgRowsMaxSmem) return false;
         }
         plan.threads = std::min(plan.threads, kCgRowsMaxThreads);
         for (const CgRowsBlock& b : o.blk) plan.smem = std::max(plan.smem, cg_rows_smem_bytes(plan, b));
@@ -213,18 +295,7 @@ bool cg_rows_layout(uint32_t N, const BsrPattern& p, F&& max_blocks, CgRowsLayou
     auto lay = [&](uint32_t blocks, uint32_t cluster) {
         return ((N + blocks - 1) / blocks <= 16 && build(blocks, cluster, 16)) || build(blocks, cluster, 8) || build(blocks, cluster, 4);
     };
-    const uint32_t near = std::max(1u, std::min(16u, (N + kRowsPerBlock - 1) / kRowsPerBlock));
-    if (lay(near, near)) return true;
-    for (uint32_t cluster : {8u, 2u}) {
-        CgRowsPlan shape;
-        shape.lanes = 4;
-        shape.threads = kCgRowsMaxThreads;
-        shape.smem = kCgRowsMaxSmem;
-        shape.cluster = cluster;
-        const uint32_t blocks = max_blocks(shape) / cluster * cluster;
-        if (blocks && lay(blocks, cluster)) return true;
-    }
-    return false;
+    return cg_rows_shapes(N, max_blocks, lay);
 }
 
 }  // namespace femgb

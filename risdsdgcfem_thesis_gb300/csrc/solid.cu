@@ -571,13 +571,12 @@ int read_tables(fem_solid s, std::vector<uint32_t>& tets, std::vector<uint32_t>&
 
 // build_rows ahead of the first solve that wants it (a solid used for its
 // products only does not pay for it); without the device memory for them the
-// solve stays on the loop of kernels. Meshes far above the GPU's shared memory
-// (a closed tetrahedral mesh has about N + T edges) are not looked at.
+// solve stays on the loop of kernels. Whether a large mesh's rows fit is known
+// from its creation (rows_tried).
 int try_rows(fem_solid s)
 {
     if (s->rows_tried || !wants_rows(s->params)) return FEM_OK;
     s->rows_tried = true;
-    if (72.0 * (3.0 * s->N + 2.0 * s->T) > 1.2 * kCgRowsMaxBlocks * kCgRowsMaxSmem) return FEM_OK;
     const std::string keep = g_err;
     const bool had_bsr = s->bsr_groups > 0;
     int rc = FEM_E_OOM;
@@ -1142,6 +1141,8 @@ int fem_solid_create(const double* rest_xyz, uint32_t N, const uint32_t* tets, u
     }
     for (uint32_t n = 0; n < N; n++)
         while ((1u << s->fx_guard) < ptr[n + 1] - ptr[n]) s->fx_guard++;
+    // (a mesh of up to 8,192 nodes nearly always fits)
+    s->rows_tried = N > 8192 && !cg_rows_may_fit(N, tets, ptr, idx, cg_rows_max_blocks);
     std::vector<int4> t4(T);
     for (uint32_t e = 0; e < T; e++)
         t4[e] = make_int4((int)tets[4 * (size_t)e], (int)tets[4 * (size_t)e + 1], (int)tets[4 * (size_t)e + 2],

@@ -143,7 +143,7 @@ def test_layout_covers_the_rows(shim, mesh, shuffle, sms):
 FITS = r"""
 #include "rows_plan.h"
 using namespace femgb;
-// Bit 0: the layout succeeds; bit 2: some block does not hold its own range of nodes.
+// Bit 0: the layout succeeds; bit 1: cg_rows_may_fit; bit 2: some block does not hold its own range of nodes.
 extern "C" int fits(uint32_t N, uint32_t T, const uint32_t* tets)
 {
     std::vector<uint32_t> ptr(N + 1, 0), idx(4 * (size_t)T);
@@ -157,6 +157,7 @@ extern "C" int fits(uint32_t N, uint32_t T, const uint32_t* tets)
     BsrPattern p;
     CgRowsLayout l;
     int r = bsr_pattern(N, T, tets, ptr, idx, p) && cg_rows_layout(N, p, blocks, l) ? 1 : 0;
+    if (cg_rows_may_fit(N, tets, ptr, idx, blocks)) r |= 2;
     if (r & 1)
         for (const CgRowsBlock& b : l.blk)
             for (uint32_t i = b.node0; i < b.node0 + b.nn; i++) {
@@ -186,13 +187,14 @@ def fits(tmp_path_factory):
                                       (_star(3000), False)],
                          ids=["5", "8640", "20480", "87880", "105840", "flat64000", "109760", "108000", "flat90000",
                               "long121000", "long125000", "star", "star3000"])
-def test_layout_of_the_largest_meshes(fits, mesh, fit):
-    """Which meshes have a layout (120 SMs in clusters of 8, 152 in pairs); the
-    blocks hold ranges of nodes whatever shape was tried first."""
+def test_whether_the_rows_fit_is_known_ahead(fits, mesh, fit):
+    """cg_rows_may_fit agrees with the layout (it may only err towards a try),
+    and the layout's blocks hold ranges of nodes whatever shape was tried first."""
     n, tets = mesh
     tets = np.ascontiguousarray(tets, np.uint32)
     r = fits(n, len(tets), tets.ctypes.data_as(C.POINTER(C.c_uint32)))
     assert bool(r & 1) == fit and not r & 4
+    assert bool(r & 2) == fit if len(tets) > 3000 else r & 2 or not fit
 
 
 WORDS = r"""
