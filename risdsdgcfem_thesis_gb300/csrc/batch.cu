@@ -75,6 +75,7 @@ struct Dev {
     {
         if (p) cudaFree(p);
         p = nullptr;
+        n = 0;
     }
     size_t bytes() const { return sizeof(T) * n; }
 };
@@ -140,6 +141,7 @@ struct fem_batch_s {
     Dev<unsigned char> Dinv_s, mat_s, R_s;  // S-typed, raw bytes
     Dev<double> Dinv64, vol, detF;
     Dev<int4> Kfx;     // FP64 (BatchView::Kfx)
+    bool want_matrices = true;  // false: Kfx is left out
     Dev<float> grade;
     Dev<uint32_t> tile_nodes, lptr0, ov_ptr, ov_map, knc_node, knc_mesh;
     std::vector<uint32_t> perm_h, inv_h;  // batch node -> caller's node, and back (global ids)
@@ -641,6 +643,20 @@ int enqueue_step(fem_batch B, cudaStream_t s, bool capture, int lock_phase = 0)
     return FEM_OK;
 }
 
+// The product matrices of an FP64 batch with C_WRP meshes, after everything
+// else: without the memory for them the elements run in FP64.
+void alloc_matrices(fem_batch b)
+{
+    bool wrp = false;
+    for (auto& m : b->meshes) wrp |= m.p.material == FEM_MATERIAL_C_WRP;
+    if (b->opt.precision != FEM_PRECISION_FP64 || !wrp || !b->want_matrices || b->Kfx.p) return;
+    if (b->Kfx.alloc(kFxGroups * ((b->Ttot + 31) / 32 * 32)) != cudaSuccess) {
+        cudaGetLastError();
+        b->Kfx.release();
+        b->want_matrices = false;  // the meshes' steps in progress keep their product
+    }
+}
+
 int build_graph(fem_batch B)
 {
     if (B->exec) return FEM_OK;
@@ -660,6 +676,26 @@ int build_graph(fem_batch B)
 }
 
 }  // namespace
+
+namespace femgb {
+// An FP64 batch without its product matrices (368 bytes per tet): before
+// fem_batch_finalize they are not made, later they are given back.
+int batch_leave_matrices(fem_batch b)
+{
+    b->want_matrices = false;
+    if (!b->Kfx.p) return FEM_OK;
+    BCK(cudaStreamSynchronize(b->stream));
+    b->device_bytes -= b->Kfx.bytes();
+    b->Kfx.release();
+    if (!b->exec) return FEM_OK;
+    cudaGraphExecDestroy(b->exec);  // it holds the address
+    cudaGraphDestroy(b->graph);
+    b->exec = nullptr;
+    b->graph = nullptr;
+    return build_graph(b);
+}
+bool batch_has_matrices(fem_batch b) { return b->Kfx.p != nullptr; }
+}  // namespace femgb
 
 extern "C" {
 
@@ -1144,12 +1180,8 @@ int fem_batch_finalize(fem_batch b)
     BCKC(b->Dinv_s.alloc(9 * T * SB));
     BCKC(b->mat_s.alloc(3 * T * SB));
     BCKC(b->R_s.alloc(9 * T * SB));
-    if (fp64) {
-        BCKC(b->Kfx.alloc(kFxGroups * ((T + 31) / 32 * 32)));
-        BCKC(b->grade.alloc(T));
-    } else {
-        BCKC(b->Dinv64.alloc(9 * T));
-    }
+    if (fp64) BCKC(b->grade.alloc(T));
+    else BCKC(b->Dinv64.alloc(9 * T));
     BCKC(b->vol.alloc(T));
     BCKC(b->detF.alloc(T));
     BCKC(b->tile_nodes.alloc(tile_nodes.size()));
@@ -1307,6 +1339,7 @@ int fem_batch_finalize(fem_batch b)
     BCKC(cudaMemsetAsync(b->mcount.p, 0, sizeof(unsigned) * b->M, s));
     BCKC(cudaStreamSynchronize(s));
 #undef BCKC
+    alloc_matrices(b);
     b->device_bytes = b->tiles.bytes() + b->chunks.bytes() + b->mc.bytes() + b->st.bytes() + b->active.bytes() +
                       b->gtets.bytes() + b->Dinv_s.bytes() + b->mat_s.bytes() + b->R_s.bytes() +
                       b->Dinv64.bytes() + b->Kfx.bytes() + b->grade.bytes() + b->vol.bytes() + b->detF.bytes() + b->tile_nodes.bytes() +
@@ -1560,6 +1593,9 @@ int fem_batch_set_params(fem_batch b, uint32_t mesh, const fem_params* params)
     if (en_changed) b->elem_mat[mesh] = 0;  // replaced by the scalar values
     if (!fp64) launch_blob_factors(b->view<float>(), s);
     b->meshes[mesh].p = *params;
+    const size_t had = b->Kfx.bytes();
+    alloc_matrices(b);
+    b->device_bytes += b->Kfx.bytes() - had;
     b->lock_dt = -1.0;  // the lock-step's constants are rebuilt at its next phase
     BCK(cudaGetLastError());
     BCK(cudaStreamSynchronize(s));

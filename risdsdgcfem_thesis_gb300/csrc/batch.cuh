@@ -195,7 +195,8 @@ struct BatchView {
     S* R;                          // [9][Ttot]
     const double* Dinv64;          // [9][Ttot] (FP64: Dinv itself)
     int4* Kfx;                     // FP64: the elements' fixed-point product matrices (fx_device.cuh), baked
-                                   // after each evaluation of a C_WRP mesh; null on the mixed path
+                                   // after each evaluation of a C_WRP mesh; null on the mixed path and without
+                                   // C_WRP meshes or the memory for them (the elements then run in FP64)
     const float* grade;            // FP64: [Ttot] max|Dm| max|Dm^-1| of each rest shape
     const double* vol;             // [Ttot]
     double* detF;                  // [Ttot]

@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(kFxTileThreads, 4)
             lc.z = (unsigned char)bounds_idx((uint32_t)lc.z, tm.nn, kSiteLocalNode);
             lc.w = (unsigned char)bounds_idx((uint32_t)lc.w, tm.nn, kSiteLocalNode);
             const int ids[4] = {lc.x, lc.y, lc.z, lc.w};
-            bool ok = fixed_point;
+            bool ok = fixed_point && b.Kfx != nullptr;
             if (ok) {
                 const int4 last = fx_matrix(b.Kfx, e)[32 * (kFxGroups - 1)];
                 double dl[12];
@@ -1312,6 +1312,7 @@ __global__ void k_fin_energy(BatchView<S> b, int kind, const double* __restrict_
 template <>
 void BatchLaunch<double>::bake(const BatchView<double>& b, int newton, cudaStream_t s)
 {
+    if (!b.Kfx) return;
     k_bake_batch<<<b.ntiles ? b.ntiles : 1, kFxTileThreads, 0, s>>>(b, newton);
     launch_counter()++;
 }

@@ -145,10 +145,12 @@ struct MeshView {
     // FP64 solid, C_WRP: each element's fixed-point product matrix (fx.cuh),
     // kFxGroups 16-byte groups of two entries, the last group's second half
     // the scale, [T / 32][kFxGroups][32] (a warp's groups at fixed offsets);
-    // when set, eout holds fixed-point records of the product instead of
+    // null without the memory for them (every element then runs in FP64).
+    // records: eout holds fixed-point records of the product instead of
     // doubles. fx_guard: log2 of the largest
     // number of element corners at a node, rounded up.
     int4* Kfx = nullptr;
+    uint32_t records = 0;
     uint32_t fx_guard = 0;
     const float* grade = nullptr;  // [T] max|Dm| max|Dm^-1| of the rest shape
 };

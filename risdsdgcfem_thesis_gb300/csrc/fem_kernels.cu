@@ -313,6 +313,11 @@ __global__ void __launch_bounds__(128, 3) k_elem_spmv_fp64(MeshView<double> m, c
                               d + 3 * (size_t)bounds_idx((uint32_t)t.y, m.N, kSiteElemNode),
                               d + 3 * (size_t)bounds_idx((uint32_t)t.z, m.N, kSiteElemNode),
                               d + 3 * (size_t)bounds_idx((uint32_t)t.w, m.N, kSiteElemNode)};
+        if (!m.Kfx) {
+            elem_record_fp64(m.R + e, m.Dinv + e, m.mat + e, m.T, p[0], p[1], p[2], p[3],
+                             reinterpret_cast<longlong2*>(m.eout + 12 * (size_t)e));
+            continue;
+        }
         const int4* Kp = fx_matrix(m.Kfx, e);
         const int4 last = Kp[32 * (kFxGroups - 1)];
         int4 cur;
@@ -1152,7 +1157,7 @@ __global__ void k_apply_A_fp64(MeshView<double> m, double factor_M, double facto
     const uint32_t a = threadIdx.x & 3u, step = (gridDim.x * blockDim.x) >> 2;
     for (uint32_t n = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; (n & ~7u) < m.N; n += step) {
         const bool on = n < m.N;
-        const double s = m.Kfx ? gather_fx(m, n, a, on) : gather_fp64(m, n, a, on);
+        const double s = m.records ? gather_fx(m, n, a, on) : gather_fp64(m, n, a, on);
         if (!on || a == 3) continue;
         const size_t i = 3 * (size_t)n + a;
         q[i] = m.fixed[n] ? 0.0 : factor_K * s + mfm * d[i];
@@ -1323,7 +1328,7 @@ __global__ void k_finalize(int kind, const double* __restrict__ partials, uint32
         const bool bsr_ = (m).bsr_val != nullptr;                                                                    \
         const uint32_t g_ = node_grid((m).N, bsr_), b_ = node_block((m).N, bsr_);                                    \
         if (bsr_) kernel<kKuBsr><<<g_, b_, 0, s>>>(m, __VA_ARGS__);                                                  \
-        else if ((m).Kfx) kernel<kKuRecords><<<g_, b_, 0, s>>>(m, __VA_ARGS__);                                      \
+        else if ((m).records) kernel<kKuRecords><<<g_, b_, 0, s>>>(m, __VA_ARGS__);                                      \
         else kernel<kKuFp64><<<g_, b_, 0, s>>>(m, __VA_ARGS__);                                                      \
         launch_counter()++;                                                                                          \
     } while (0)

@@ -53,6 +53,8 @@ namespace femgb {
 int batch_fail(int code, const char* fmt, ...);
 int batch_enqueue_readback(fem_batch b);
 unsigned batch_host_err(fem_batch b);
+int batch_leave_matrices(fem_batch b);
+bool batch_has_matrices(fem_batch b);
 }  // namespace femgb
 
 using femgb::batch_fail;
@@ -98,11 +100,12 @@ struct Shard {
 
 // Upper estimate of a shard's device bytes (the batch layout: per tet the
 // FP64 and element-type element data, tile CSR and mixed blob; per node the
-// FP64 state vectors, element-type CG vectors and about 2.5 partial slots).
-uint64_t estimate_bytes(uint32_t precision, uint64_t T, uint64_t N, uint64_t M)
+// FP64 state vectors, element-type CG vectors and about 2.5 partial slots;
+// matrices: an FP64 shard's product matrices too).
+uint64_t estimate_bytes(uint32_t precision, uint64_t T, uint64_t N, uint64_t M, bool matrices)
 {
     const bool fp64 = precision == FEM_PRECISION_FP64;
-    const uint64_t per_tet = fp64 ? 600 : 310;
+    const uint64_t per_tet = (fp64 ? 300 : 310) + (matrices ? 368 : 0);
     const uint64_t per_node = fp64 ? 400 : 330;
     return per_tet * T + per_node * N + 512 * M + (1u << 20);
 }
@@ -148,7 +151,7 @@ int check_server(fem_server s)
 
 // Builds one shard from the scenes in `ids` (all waiting). Returns FEM_OK and
 // fills `out`, or an error (nothing is left allocated).
-int build_shard(fem_server srv, const std::vector<uint32_t>& ids, Shard& out)
+int build_shard(fem_server srv, const std::vector<uint32_t>& ids, bool matrices, Shard& out)
 {
     fem_batch_options o;
     fem_batch_options_default(&o);
@@ -172,7 +175,8 @@ int build_shard(fem_server srv, const std::vector<uint32_t>& ids, Shard& out)
             return e;
         }
     }
-    int e = fem_batch_finalize(b);
+    int e = matrices ? FEM_OK : femgb::batch_leave_matrices(b);
+    if (!e) e = fem_batch_finalize(b);
     // FIE shards step whole (a Newton step takes no iteration budget)
     const bool newton = srv->scenes[ids[0]].params.integrator != FEM_INTEGRATOR_QIE_V;
     if (!e) e = fem_batch_set_slice(b, newton ? 0u : srv->opt.slice_iterations);
@@ -198,6 +202,25 @@ int build_shard(fem_server srv, const std::vector<uint32_t>& ids, Shard& out)
     out.flags.assign(ids.size(), 0);
     out.bytes = bytes;
     out.live = (uint32_t)ids.size();
+    return FEM_OK;
+}
+
+// Whether `bytes` more fit the budget, if need be without the product
+// matrices of the resident FP64 shards, which are given back one by one (a
+// shard's launch in flight is waited for): they make its steps faster, but
+// take no scene's place.
+int make_room(fem_server srv, uint64_t bytes, bool& fits)
+{
+    for (auto& sh : srv->shards) {
+        if (srv->used_bytes + bytes <= srv->opt.hbm_budget_bytes) break;
+        if (!sh.b || !femgb::batch_has_matrices(sh.b)) continue;
+        if (int e = femgb::batch_leave_matrices(sh.b)) return e;
+        uint64_t now = 0;
+        fem_batch_info(sh.b, nullptr, nullptr, nullptr, nullptr, &now);
+        srv->used_bytes -= sh.bytes - now;
+        sh.bytes = now;
+    }
+    fits = srv->used_bytes + bytes <= srv->opt.hbm_budget_bytes;
     return FEM_OK;
 }
 
@@ -346,10 +369,21 @@ int fem_server_admit(fem_server s, uint32_t* admitted)
             N += s->scenes[wait[k]].N;
             ids.push_back(wait[k++]);
         }
-        if (s->used_bytes + estimate_bytes(s->opt.precision, T, N, ids.size()) > s->opt.hbm_budget_bytes) break;
+        bool wrp = false, fits = true;
+        if (s->opt.precision == FEM_PRECISION_FP64)
+            for (uint32_t i : ids) wrp |= s->scenes[i].params.material == FEM_MATERIAL_C_WRP;
+        const bool matrices =
+            s->used_bytes + estimate_bytes(s->opt.precision, T, N, ids.size(), wrp) <= s->opt.hbm_budget_bytes;
+        if (int e = make_room(s, estimate_bytes(s->opt.precision, T, N, ids.size(), wrp && matrices), fits)) return e;
+        if (!fits) break;
         Shard sh;
-        if (int e = build_shard(s, ids, sh)) return e;
-        if (s->used_bytes + sh.bytes > s->opt.hbm_budget_bytes) {  // estimate was short: undo
+        if (int e = build_shard(s, ids, matrices, sh)) return e;
+        if (int e = make_room(s, sh.bytes, fits)) {
+            sh.bytes = 0;
+            s->take_down(sh);
+            return e;
+        }
+        if (!fits) {  // estimate was short: undo
             sh.bytes = 0;  // not counted yet
             s->take_down(sh);
             break;
@@ -391,7 +425,17 @@ int fem_server_set_params(fem_server s, uint32_t scene, const fem_params* params
         if (newton_old != newton_new)
             return batch_fail(FEM_E_ARG, "scene %u: an integrator change moves it between shard kinds; remove and "
                                          "add it again", scene);
-        if (int e = fem_batch_set_params(s->shards[sc.shard].b, sc.mesh, &p)) return e;
+        Shard& sh = s->shards[sc.shard];
+        if (int e = fem_batch_set_params(sh.b, sc.mesh, &p)) return e;
+        // the first C_WRP scene of an FP64 shard brings the product matrices
+        uint64_t now = 0;
+        fem_batch_info(sh.b, nullptr, nullptr, nullptr, nullptr, &now);
+        if (now > sh.bytes && s->used_bytes + (now - sh.bytes) > s->opt.hbm_budget_bytes) {
+            if (int e = femgb::batch_leave_matrices(sh.b)) return e;
+            fem_batch_info(sh.b, nullptr, nullptr, nullptr, nullptr, &now);
+        }
+        s->used_bytes += now - sh.bytes;
+        sh.bytes = now;
     }
     sc.params = p;
     return FEM_OK;

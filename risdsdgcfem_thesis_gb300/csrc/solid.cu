@@ -235,7 +235,8 @@ struct fem_solid_s {
         m.csr_idx = csr_idx.p;
         m.fixed = fixed.p;
         m.eout = eout.p;
-        if (params.material == FEM_MATERIAL_C_WRP) m.Kfx = Kfx.p;
+        m.Kfx = Kfx.p;
+        m.records = params.material == FEM_MATERIAL_C_WRP ? 1u : 0u;
         m.fx_guard = fx_guard;
         m.grade = grade.p;
         if (bsr_use) {
@@ -384,9 +385,20 @@ void assemble(fem_solid s)
                                          s->bsr_val.p, s->bsr_x.p}, s->stream);
     s->bsr_fresh = true;
 }
+// The product matrices of a C_WRP solid, after everything else: without the
+// memory for them its elements run in FP64.
+void alloc_matrices(fem_solid s)
+{
+    if (uses_lcm(s) || s->Kfx.p) return;
+    if (s->Kfx.alloc(kFxGroups * (((size_t)s->T + 31) / 32 * 32)) != cudaSuccess) {
+        cudaGetLastError();
+        s->Kfx.release();
+    }
+    s->kfx_fresh = false;
+}
 void bake_products(fem_solid s)
 {
-    if (uses_lcm(s) || s->kfx_fresh) return;
+    if (uses_lcm(s) || s->kfx_fresh || !s->Kfx.p) return;
     launch_elem_bake_fp64(s->view(), s->stream);
     s->kfx_fresh = true;
 }
@@ -1170,7 +1182,6 @@ int fem_solid_create(const double* rest_xyz, uint32_t N, const uint32_t* tets, u
     CKC(s->R.alloc(9 * (size_t)T));
     CKC(s->detF.alloc(T));
     CKC(s->eout.alloc(12 * (size_t)T));
-    CKC(s->Kfx.alloc(kFxGroups * (((size_t)T + 31) / 32 * 32)));
     CKC(s->grade.alloc(T));
     CKC(s->csr_ptr.alloc(N + 1));
     CKC(s->csr_idx.alloc(4 * (size_t)T));
@@ -1220,6 +1231,7 @@ int fem_solid_create(const double* rest_xyz, uint32_t N, const uint32_t* tets, u
     CKC(cudaMemsetAsync(s->st.p, 0, sizeof(StepScalars), st));
     launch_rest_rotations_fp64(T, s->R.p, s->detF.p, st);
     CKC(cudaGetLastError());
+    alloc_matrices(s);
     CKC(cudaStreamSynchronize(st));
 #undef CKC
     // the static scratch of fem_solid_apply_A_noalloc: its address is looked
@@ -1360,6 +1372,7 @@ int fem_solid_set_params(fem_solid s, const fem_params* params)
         CK(cudaMemcpyAsync(s->doc.p, none.data(), sizeof(uchar2) * s->T, cudaMemcpyHostToDevice, s->stream));
     }
     s->params = *params;
+    alloc_matrices(s);
     set_bsr_use(s);
     set_consts(s);
     // a new Young's modulus or Poisson ratio re-bakes every element from the

@@ -2,6 +2,8 @@
 same alone and in the mix under continuous batching (bit-identical to the
 scene stepped alone in its own batch with the server's node chunk), admission respects the device-memory
 budget, and shards overlap on the device."""
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -153,3 +155,59 @@ def test_server_scene_parameter_change_equals_the_batch(fem_lib):
     with pytest.raises(fem_lib.FemError) as e:
         srv.set_params(sid, fem_lib.params_for(dataclasses.replace(sc, integrator=1), fem_lib.FEM_PRECISION_MIXED))
     assert e.value.code == fem_lib.FEM_E_ARG
+
+
+@pytest.mark.parametrize("waves", [1, 2])
+def test_product_matrices_take_no_scenes_place(fem_lib, waves):
+    """FP64 shards keep product matrices (368 bytes per tet) where the budget
+    has room for them. A budget for the scenes without them admits them all,
+    also when the first ones came with matrices; they step as a batch does
+    (two CG iterations: 1e-12, as the FP64 products' tests)."""
+    rng = np.random.default_rng(3)
+    pool = [scenes.random_block(rng, dims=d, idx=i) for i, d in enumerate([(13, 12, 13), (14, 12, 12), (13, 13, 13)] * 2)]
+    for sc in pool:
+        sc.max_iter = 2
+        sc.init_vel = 0.1 * rng.standard_normal(sc.rest.shape)
+    budget = sum(300 * sc.num_tets + 400 * sc.num_nodes + 512 + (1 << 20) for sc in pool)
+    assert sum(368 * sc.num_tets for sc in pool) > len(pool) << 20
+    srv = fem_lib.Server(fem_lib.FEM_PRECISION_FP64, hbm_budget_bytes=budget, shard_max_scenes=1)
+    ids = []
+    for k in range(waves):
+        ids += [srv.add(sc) for sc in pool[k * len(pool) // waves:(k + 1) * len(pool) // waves]]
+        srv.admit()
+        for i in ids:
+            srv.set_state(i, pool[i].rest, pool[i].init_vel)
+            srv.submit(i)
+        srv.drain()
+    assert len(srv.resident()) == len(pool) and srv.status()["device_bytes"] <= budget
+    ref = fem_lib.Batch(pool, fem_lib.FEM_PRECISION_FP64)
+    ref.step(1)
+    for i, sc in enumerate(pool):
+        x, v = srv.state(ids[i])
+        xr, vr = ref.state(i)
+        assert np.linalg.norm(v - vr) <= 1e-12 * np.linalg.norm(vr) and np.linalg.norm(x - xr) <= 1e-12 * np.linalg.norm(xr)
+    srv.close()
+
+
+@pytest.mark.parametrize("room", [True, False])
+def test_product_matrices_come_with_the_first_elastic_scene(fem_lib, room):
+    """A scene that changes from a P-K material to C_WRP brings its shard the
+    matrices, where the budget has room for them."""
+    sc = scenes.random_block(np.random.default_rng(4), dims=(14, 14, 14), idx=0)
+    sc.material, sc.max_iter = 1, 2
+    srv = fem_lib.Server(fem_lib.FEM_PRECISION_FP64, hbm_budget_bytes=None if room else
+                         300 * sc.num_tets + 400 * sc.num_nodes + 512 + (1 << 20))
+    i = srv.add(sc)
+    assert srv.admit() == 1
+    before = srv.status()["device_bytes"]
+    p = fem_lib.params_for(sc, fem_lib.FEM_PRECISION_FP64, False)
+    p.material = 0
+    srv.set_params(i, p)
+    assert srv.status()["device_bytes"] - before == (368 * (-(-sc.num_tets // 32) * 32) if room else 0)
+    srv.submit(i)
+    srv.drain()
+    ref = fem_lib.Batch([dataclasses.replace(sc, material=0)], fem_lib.FEM_PRECISION_FP64)
+    ref.step(1)
+    for a, b in zip(srv.state(i), ref.state(0)):
+        assert np.linalg.norm(a - b) <= 1e-12 * np.linalg.norm(b)
+    srv.close()
