@@ -2069,15 +2069,17 @@ int fem_batch_kernel_launches(fem_batch b, uint32_t steps, uint64_t* launches)
     unsigned body_runs = 0;
     BCK(cudaMemcpyAsync(&body_runs, b->any_flag.p, sizeof(unsigned), cudaMemcpyDeviceToHost, b->stream));
     BCK(cudaStreamSynchronize(b->stream));
-    // kernels per step outside the CG loop, plus per executed CG iteration 3
-    // (FP64 path) or 6 (mixed path: tile product, refresh product -- counted
-    // in every iteration, an upper bound --, mesh alpha unless the node pass
-    // forms it, node pass, mesh update)
+    // kernels per step outside the solver's loop (one Newton iteration), plus
+    // per iteration, with those that find the loop ended in the body of its
+    // WHILE node or chunk, 3 (FP64 path) or 5 (mixed path: tile product,
+    // refresh product -- counted in every iteration, an upper bound for a
+    // graph --, mesh alpha unless the node pass forms it, node pass, mesh
+    // update), and the MINRES meshes' updates
     bool energy = false;
     for (auto& m : b->meshes) energy |= m.p.compute_energy != 0;
     const bool mixed = b->opt.precision == FEM_PRECISION_MIXED;
-    const uint64_t fixed = 8 + (b->K ? 1 : 0) + (energy ? 4 : 0);
-    const uint64_t per_iter = mixed ? (b->alpha_in_nodes ? 5ull : 6ull) : 3ull;
+    const uint64_t fixed = 7 + (b->K ? 1 : 0) + (energy ? 4 : 0) + (b->Kfx.p ? 1 : 0) + (b->any_minres ? 1 : 0);
+    const uint64_t per_iter = (mixed ? (b->alpha_in_nodes ? 4ull : 5ull) : 3ull) + (b->any_minres ? 1ull : 0ull);
     *launches = (uint64_t)steps * fixed + per_iter * body_runs;
     return FEM_OK;
 }

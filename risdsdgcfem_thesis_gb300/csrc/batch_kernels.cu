@@ -985,7 +985,10 @@ __global__ void __launch_bounds__(kNodeThreads64) k_node_update(BatchView<S> b, 
 {
     const uint32_t ci = blockIdx.x;
     const ChunkMeta ch = b.chunks[ci < b.nchunks ? ci : 0];
-    if (!loop_on(b)) return;  // every block: the loop's arrivals too
+    if (!loop_on(b)) {  // every block: the loop's arrivals too
+        if (ls.body_runs && blockIdx.x == 0 && threadIdx.x == 0) *ls.body_runs += 1u;
+        return;
+    }
     if (ci < b.nchunks && mesh_running(b, ch.mesh) && b.mc[ch.mesh].solver == kMeshSolverMinres) {
         node_update_minres(b, b.mc[ch.mesh], b.st[ch.mesh], ci, ch, r, q, cpart, ls);
     } else if (ci < b.nchunks && mesh_running(b, ch.mesh)) {

@@ -21,7 +21,7 @@ struct LoopSync {
     unsigned* mcount;        // [M] per-mesh chunk arrivals (FP64 path)
     unsigned* gcount;        // grid arrivals
     unsigned* refresh_flag;  // raised when a mesh refreshes its residual next iteration
-    unsigned* body_runs;     // CG-loop body executions (launch accounting)
+    unsigned* body_runs;     // iterations launched, also those after the loop's end (launch accounting)
     const unsigned* err;     // batch error word: the loop stops once it is set
     unsigned* slice;         // [budget (0 = none), iterations run in this launch, the loop goes on]
     cudaGraphConditionalHandle cond;

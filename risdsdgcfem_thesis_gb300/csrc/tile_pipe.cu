@@ -1259,7 +1259,10 @@ __global__ void __launch_bounds__(kUpdateThreads, 1) k_mesh_update(BatchView<flo
         li = load_loop(ls);
     }
     if (tid == 0) s_flags = UpdateFlags{0u, 0u, 0u, 0u};
-    if (!go) return;  // the loop has ended inside the body of its WHILE node
+    if (!go) {  // the loop has ended inside the body of its WHILE node
+        if (ls.body_runs && blockIdx.x == 0 && tid == 0) *ls.body_runs += 1u;
+        return;
+    }
     if (warp < n) {
         const MeshConsts& c = b.mc[m0 + warp];
         const uint32_t done = b.st[m0 + warp].done, chunk0 = c.chunk0, nchunks = c.nchunks;

@@ -410,3 +410,29 @@ def test_alpha_by_batch_size_gives_the_same_bits(fem_lib, n, tile, chunk, separa
     assert (la > lb) == separate, (la, lb)
     for (xa, va), (xb, vb) in zip(sa, sb):
         assert np.array_equal(xa, xb) and np.array_equal(va, vb)
+
+
+@pytest.mark.parametrize("solver", [0, 1])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("energy", [False, True])
+def test_kernel_launches_are_all_counted(fem_lib, solver, precision, energy):
+    """fem_batch_kernel_launches against the library's own count where the
+    host launches every kernel, and, per iteration, where a graph does: the
+    four iterations of its loop's body run whole."""
+    prec = fem_lib.FEM_PRECISION_FP64 if precision == "fp64" else fem_lib.FEM_PRECISION_MIXED
+    sc = dataclasses.replace(scenes.random_block(np.random.default_rng(6), dims=(5, 4, 4), idx=0), ls_solver=solver)
+    counts = []
+    for graph in (False, True):
+        b = fem_lib.Batch([sc], prec, compute_energy=energy, use_graph=graph)
+        b.step(1)
+        b.reset_launch_count()
+        before = fem_lib.kernel_launches()
+        b.step(1)
+        counts.append((b.kernel_launches(1), fem_lib.kernel_launches() - before, b.stats(0)["cg_iterations"]))
+        b.close()
+    (host, actual, k), (graph, _, kg) = counts
+    assert host == actual and k == kg
+    runs = lambda chunk: -(-k // chunk) * chunk
+    per = (3 if precision == "fp64" else 4) + solver
+    fixed = host - per * runs(8)
+    assert 7 <= fixed <= 14 and graph == fixed + per * runs(4)
