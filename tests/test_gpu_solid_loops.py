@@ -1,0 +1,87 @@
+"""The FP64 solid's solvers as loops of kernels, on the element products and
+on the assembled stiffness: solids whose rows do not fit the shared memory of
+the GPU's SMs (test_rows_plan.py), which solve there otherwise."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+from risdsdgcfem_thesis_gb300 import scenes
+from test_fx_element import _block, _fan
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = {
+    "block": (lambda: _block((30, 30, 30)), 1e-12),
+    "flat": (lambda: _block((100, 30, 6)), 1e-12),
+    "graded": (lambda: _block((30, 30, 30), (1, 1, 0.1)), 1e-12),
+    "part-graded": (lambda: _block((30, 30, 30), (1, 1, 0.4)), 1e-12),
+    "stiff": (lambda: _block((30, 30, 30), poisson=0.499), 1e-12),
+    # ten times thinner wedges and ten times longer sums than the fan of 100 in test_fx_element.py
+    "fan1000": (lambda: _fan(1000), 1e-10),
+}
+
+
+@pytest.fixture(scope="module")
+def reference(oracle):
+    """The oracle's velocities after one step of two iterations, per shape,
+    solver and integrator."""
+    made = {}
+
+    def get(shape, solver, integrator):
+        key = (shape, solver, integrator)
+        if key not in made:
+            sc = SHAPES[shape][0]()
+            rng = np.random.default_rng(4)
+            sc = dataclasses.replace(sc, ls_solver=solver, integrator=integrator, max_iter=2, nr_max_iter=1,
+                                     init_vel=0.1 * rng.standard_normal(sc.rest.shape),
+                                     knc_nodes=np.array([0, len(sc.rest) - 1], np.uint32))
+            sc.knc_targets = sc.rest[sc.knc_nodes].copy()
+            o = oracle.Solid(sc, "port")
+            o.step()
+            made[key] = sc, o.state()[1]
+        return made[key]
+
+    return get
+
+
+@pytest.mark.parametrize("integrator", [0, 1], ids=["graph", "host"])
+@pytest.mark.parametrize("assembled", [False, True], ids=["elements", "assembled"])
+@pytest.mark.parametrize("solver", [0, 1], ids=["cg", "minres"])
+@pytest.mark.parametrize("shape", list(SHAPES))
+def test_solver_loop_matches_the_oracle(fem_lib, reference, shape, solver, assembled, integrator):
+    """As test_solve_on_resident_rows_matches_the_oracle: two iterations, from
+    a step graph (QIE) and driven from the host (FIE, one Newton iteration),
+    where the kernels that ran are read back."""
+    sc, v = reference(shape, solver, integrator)
+    s = fem_lib.Solid(sc, compute_energy=False)
+    s.set_assembled(assembled)
+    if integrator:
+        fem_lib.profile_enable(True)  # from zero
+    try:
+        s.step(1)
+    finally:
+        fem_lib.profile_enable(False)
+    if integrator:
+        rows, elem, assembly, node_q = [fem_lib.profile_read(n)[1] for n in
+                                        ("cg_rows_fp64", "elem_spmv_fp64", "bsr_assemble_fp64", "node_q_fp64")]
+        assert rows == 0 and (elem == 0) == assembled and (assembly > 0) == assembled and (node_q > 0) == (solver == 0)
+    assert s.stats()["cg_iterations"] == 2
+    assert np.linalg.norm(s.state()[1] - v) <= SHAPES[shape][1] * np.linalg.norm(v)
+
+
+@pytest.mark.parametrize("solver", [0, 1], ids=["cg", "minres"])
+def test_assembled_stiffness_switched_between_steps(fem_lib, solver):
+    """Steps on the element products and on the assembled stiffness in turn,
+    which each agree with the oracle's to 1e-12, stay within ten times that
+    of steps on the element products alone over four steps."""
+    sc = _block((30, 30, 30))
+    sc = dataclasses.replace(sc, ls_solver=solver, max_iter=2,
+                             init_vel=0.1 * np.random.default_rng(4).standard_normal(sc.rest.shape))
+    a, b = (fem_lib.Solid(sc, compute_energy=False) for _ in range(2))
+    for on in (False, True, False, True):
+        b.set_assembled(on)
+        a.step(1)
+        b.step(1)
+    for p, q in zip(a.state(), b.state()):
+        assert np.linalg.norm(p - q) <= 1e-11 * np.linalg.norm(p)
