@@ -527,10 +527,7 @@ __global__ void __launch_bounds__(kCgRowsMaxThreads, 1)
         if (warp == 0) {
             delta_old = delta;
             delta = t;
-            // t / delta_old from its reciprocal, with one correction of the remainder
-            const double q = t * rdelta;
-            beta = __fma_rn(__fma_rn(-q, delta_old, t), rdelta, q);
-            if (fx_exp(rdelta) - 64u > 1900u || fx_exp(q) - 64u > 1900u) beta = divide(t, delta_old);
+            if (!rows_quotient(t, delta_old, rdelta, beta)) beta = divide(t, delta_old);
             k++;
             if (lane == 0) {
                 s_scalar = beta;

@@ -2,6 +2,8 @@
 // data, and in the top bits of each half the exchange's number, so that a
 // reader knows both halves from the one word. W: ulonglong2. Host callable.
 #pragma once
+#include <math.h>
+
 #include "fx.cuh"
 
 namespace femgb {
@@ -47,6 +49,20 @@ FX_HD bool rows_word_is(const W& w, Part& v, uint32_t seq)
     v.m = (int64_t)((w.x & 0xffffffffffffull) | (w.y << 48));
     v.e = (int32_t)(w.y >> 16) & 0xffff;
     return (uint32_t)(w.x >> 48) == (seq & 0xffffu) && (uint32_t)(w.y >> 48) == (seq & 0xffffu);
+}
+
+// t / d from r, 1 / d rounded to nearest: the product t r, corrected once by
+// its remainder t - q d, which a fused multiply-add gives exactly (P.
+// Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990): within 2^-105 of t / d before the last rounding. False
+// where a reciprocal, quotient or remainder may be subnormal or none is
+// finite: divide there.
+FX_HD bool rows_quotient(double t, double d, double r, double& q)
+{
+    const double q0 = t * r;
+    q = fma(fma(-q0, d, t), r, q0);
+    // q0 and r between 2^-959 and 2^941, t above 2^-900
+    return (uint32_t)fx_exp(r) - 64u <= 1900u && (uint32_t)fx_exp(q0) - 64u <= 1900u && fx_exp(t) > 123;
 }
 
 // What the words of a CTA hold when a solve starts after number seq: sums

@@ -242,3 +242,53 @@ def test_words_between_blocks(tmp_path):
         assert lib.taken(seq) == 0, hex(seq)
         for v, m, e in ((0.0, 0, 0), (-1.5, -(1 << 62), 2046), (np.inf, (1 << 62), 0x7fff), (5e-324, -1, 1)):
             assert lib.kept(v, m, e, seq), hex(seq)
+
+
+QUOTIENT = r"""
+#include <math.h>
+#include "rows_words.h"
+using namespace femgb;
+#include <float.h>
+#if LDBL_MANT_DIG >= 113
+typedef long double Q;
+#else
+typedef __float128 Q;
+#endif
+// The error of t / d in units of its last place; -1 where it is to be divided.
+extern "C" double ulps(double t, double d)
+{
+    double q;
+    if (!rows_quotient(t, d, 1.0 / d, q)) return -1.0;
+    int e;
+    frexp(q, &e);
+    const Q err = ((Q)q - (Q)t / (Q)d) / (Q)ldexp(1.0, e - 53);
+    return (double)(err < 0 ? -err : err);
+}
+"""
+
+
+def test_quotient_by_the_reciprocal(tmp_path):
+    """Half a unit in the last place, and 2^-50 for the corrected product's
+    own error, wherever it is taken."""
+    if shutil.which("g++") is None:
+        pytest.skip("no host compiler")
+    src, so = tmp_path / "quotient.cpp", tmp_path / "quotient.so"
+    src.write_text(QUOTIENT)
+    subprocess.run(["g++", "-std=gnu++17", "-O2", "-ffp-contract=off", "-Wno-unknown-pragmas", "-shared", "-fPIC", "-I", CSRC,
+                    str(src), "-o", str(so)], check=True)
+    lib = C.CDLL(str(so))
+    lib.ulps.argtypes, lib.ulps.restype = [C.c_double, C.c_double], C.c_double
+    rng = np.random.default_rng(9)
+    taken = 0
+    for span in (0.001, 1, 30, 280, 307):
+        t, d = (rng.uniform(1, 2, 20000) * 10.0 ** rng.uniform(-span, span, 20000) for _ in range(2))
+        for a, b in zip(t, d):
+            u = lib.ulps(a, b)
+            assert u <= 0.5 + 2.0 ** -50, (a, b, u)
+            taken += u >= 0
+    assert taken > 60000
+    edges = [0.0, 5e-324, 2.2250738585072014e-308, 1e-300, 1.0, np.nextafter(1, 2), 1.7976931348623157e308, np.inf, np.nan]
+    for a in edges:
+        for b in edges:
+            u = lib.ulps(a, b)
+            assert u <= 0.5 + 2.0 ** -50 and (u == -1.0 or np.isfinite([a, b]).all()), (a, b, u)
