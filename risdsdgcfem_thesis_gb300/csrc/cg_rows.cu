@@ -85,20 +85,7 @@ __device__ __forceinline__ Part part_sum(const Part (&v)[K])
     l2 = __reduce_add_sync(0xffffffffu, l2);
     const int64_t t = (int64_t)l1 + (int64_t)((uint64_t)(int64_t)l2 << 24);  // units of 2^24, the rest in l0
     const int32_t sh = max(0, 64 - fx_clz(fx_mag(t) | 1u) - 38);             // at most 9
-    return Part{(int64_t)((uint64_t)t << (24 - sh)) | (int64_t)((l0 & 0xffffffu) >> sh), E == kPartNan ? E : E + sh};
-}
-__device__ __forceinline__ Part part_of(double v)
-{
-    const int32_t e = fx_exp(v);
-    return Part{fx_align<57>(v, e), e == 2047 ? kPartNan : e};
-}
-__device__ __forceinline__ double part_value(const Part& p)
-{
-    if (p.e == kPartNan) return fx_from_bits(0x7ff8000000000000ull);
-    const double v = __ll2double_rn(p.m);
-    const int32_t e = fx_exp(v) + p.e - 1079;
-    if (p.m == 0 || e < 1 || e > 2046) return fx_to_double(p.m, p.e - 1079);
-    return __hiloint2double(__double2hiint(v) + ((p.e - 1079) << 20), __double2loint(v));
+    return Part{(int64_t)((uint64_t)t << (24 - sh)) | (int64_t)((l0 & 0xffffffu) >> sh), E >= kPartInf ? E : E + sh};
 }
 // Out of line: the compiler would otherwise divide on every path.
 __device__ __noinline__ double divide(double a, double b) { return a / b; }

@@ -483,7 +483,14 @@ __device__ __forceinline__ double fx_warp_sum(const double (&v)[K])  // K terms 
 #pragma unroll
     for (int k = 1; k < K; k++) E = max(E, fx_exp(v[k]));
     E = __reduce_max_sync(0xffffffffu, E);
-    if (E == 2047) return __longlong_as_double(0x7ff8000000000000ll);
+    if (E == 2047) {  // infinities and NaN add as they do
+        double s = v[0];
+#pragma unroll
+        for (int k = 1; k < K; k++) s += v[k];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        return s;
+    }
     int64_t m = 0;
 #pragma unroll
     for (int k = 0; k < K; k++) m += fx_align<kBits>(v[k], E);

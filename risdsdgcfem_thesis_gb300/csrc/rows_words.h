@@ -25,13 +25,34 @@ FX_HD bool rows_word_is(const W& w, double& v, uint32_t seq)
     return (uint32_t)(w.x >> 32) == seq && (uint32_t)(w.y >> 32) == seq;
 }
 
-// A partial sum: m in units of 2^(e - 1079); kPartNan: not finite. It stays
-// in integers from the lanes to the solid's total.
+// A partial sum: m in units of 2^(e - 1079), |m| <= 2^62; kPartNan: NaN;
+// kPartInf: m counts infinities by their sign, 2^40 each, so that what finite
+// parts leave of m when it is added in their place (-1 at most) is no
+// infinity. It stays in integers from the lanes to the solid's total.
 struct Part {
     int64_t m;
     int32_t e;
 };
-constexpr int32_t kPartNan = 0x7fff;
+constexpr int32_t kPartNan = 0x7fff, kPartInf = 0x7ffe;
+FX_HD Part part_of(double v)
+{
+    const int32_t e = fx_exp(v);
+    const uint64_t u = fx_bits(v);
+    if (e == 2047) return Part{(int64_t)u < 0 ? -(1ll << 40) : 1ll << 40, (u << 12) != 0 ? kPartNan : kPartInf};
+    return Part{fx_align<57>(v, e), e};
+}
+FX_HD double part_value(const Part& p)
+{
+    if (p.e >= kPartInf) {
+        const int64_t least = 1ll << 39;
+        if (p.e == kPartNan || (p.m < least && p.m > -least)) return fx_from_bits(0x7ff8000000000000ull);
+        return fx_from_bits(p.m < 0 ? 0xfff0000000000000ull : 0x7ff0000000000000ull);
+    }
+    const double v = (double)p.m;
+    const int32_t e = fx_exp(v) + p.e - 1079;
+    if (p.m == 0 || e < 1 || e > 2046) return fx_to_double(p.m, p.e - 1079);
+    return fx_from_bits(fx_bits(v) + ((uint64_t)(int64_t)(p.e - 1079) << 52));
+}
 
 // A sum, with 16 bits of the exchange's number.
 template <typename W>

@@ -1,6 +1,7 @@
 """The FP64 solid's solvers as loops of kernels, on the element products and
 on the assembled stiffness: solids whose rows do not fit the shared memory of
 the GPU's SMs (test_rows_plan.py), which solve there otherwise."""
+import ctypes
 import dataclasses
 
 import numpy as np
@@ -85,3 +86,38 @@ def test_assembled_stiffness_switched_between_steps(fem_lib, solver):
         b.step(1)
     for p, q in zip(a.state(), b.state()):
         assert np.linalg.norm(p - q) <= 1e-11 * np.linalg.norm(p)
+
+
+@pytest.mark.parametrize("solver", [0, 1], ids=["cg", "minres"])
+@pytest.mark.parametrize("form", ["cluster", "clusters", "elements", "assembled", "batch"])
+def test_sums_that_overflow(fem_lib, oracle, form, solver):
+    """Velocities near the square root of the largest double: where |r|^2 or
+    d.q overflows, a solve ends or goes on as the reference's does (an infinite
+    d.q makes alpha zero, not NaN). Bar as above, where the oracle is finite."""
+    sc = _block({"cluster": (3, 2, 4), "clusters": (16, 16, 12), "batch": (9, 8, 7)}.get(form, (30, 30, 30)))
+    v0 = np.random.default_rng(4).standard_normal(sc.rest.shape)
+    for scale in 10.0 ** np.arange(148, 160):
+        sc = dataclasses.replace(sc, ls_solver=solver, max_iter=3, init_vel=scale * v0)
+        o = oracle.Solid(sc, "port")
+        iters = o.step()["iters"]
+        x, v = o.state()
+        g = fem_lib.Batch([sc], fem_lib.FEM_PRECISION_FP64, compute_energy=False) if form == "batch" else \
+            fem_lib.Solid(sc, compute_energy=False)
+        if form in ("elements", "assembled"):
+            g.set_assembled(form == "assembled")
+        try:
+            g.step(1)
+        except fem_lib.FemError as e:
+            assert e.code == fem_lib.FEM_E_NAN
+        if form == "batch":
+            (xg, vg), k = g.state(0), g.stats(0)["cg_iterations"]
+        else:
+            st = fem_lib.FemStepStats()
+            fem_lib.load().fem_solid_synchronize(g.h, ctypes.byref(st))
+            (xg, vg), k = g.state(), st.cg_iterations
+        assert k == iters, (scale, k, iters)
+        ok = np.isfinite(v)
+        assert np.array_equal(np.isfinite(vg), ok) and np.array_equal(np.isfinite(xg), np.isfinite(x)), scale
+        if ok.all():
+            assert np.abs((vg - v) / scale).max() <= 1e-12 * np.abs(v / scale).max(), scale
+        g.close()

@@ -215,6 +215,8 @@ extern "C" int taken(uint32_t seq)
         }
     return 0;
 }
+extern "C" double through(double v) { return part_value(part_of(v)); }
+extern "C" double infinities(int plus, int minus) { return part_value(Part{(int64_t)(plus - minus) * (1ll << 40) - 5120, kPartInf}); }
 extern "C" int kept(double v, int64_t m, int32_t e, uint32_t seq)
 {
     Part p;
@@ -242,6 +244,12 @@ def test_words_between_blocks(tmp_path):
         assert lib.taken(seq) == 0, hex(seq)
         for v, m, e in ((0.0, 0, 0), (-1.5, -(1 << 62), 2046), (np.inf, (1 << 62), 0x7fff), (5e-324, -1, 1)):
             assert lib.kept(v, m, e, seq), hex(seq)
+
+    lib.through.argtypes, lib.through.restype, lib.infinities.restype = [C.c_double], C.c_double, C.c_double
+    for v in (0.0, 1.0, -1.5, 2.2250738585072014e-308, 1.7976931348623157e308, np.inf, -np.inf):
+        assert lib.through(v) == v
+    assert np.isnan(lib.through(np.nan))
+    assert lib.infinities(3, 1) == np.inf and lib.infinities(1, 2) == -np.inf and np.isnan(lib.infinities(2, 2))
 
 
 QUOTIENT = r"""
