@@ -274,9 +274,11 @@ int fem_solid_get_params(fem_solid s, fem_params* params);
  * per tet for the assembly and one assembly per evaluation (about five
  * iterations' time); the sums run in another order, so other bits, within
  * the same parity tolerances. Other materials keep the element product. The
- * solve of a C_WRP solid whose rows fit the GPU's shared memory (about 130,000
- * tets on grid meshes) keeps them there in either setting, in memory it takes
- * at its first solve; without that memory it runs as above. FEM_E_OOM when
+ * solve of a C_WRP solid whose rows fit the GPU's shared memory (on grid meshes
+ * up to 106,000 tets as a cube, fewer when flat or long: 64,000 of 80 x 80 x 2
+ * cells do, 90,000 of 100 x 30 x 6 do not) keeps them there in either setting,
+ * in tables and memory it takes at its first solve (2 ms more for that step at
+ * 20,480 tets, 7 at 88,000); without that memory it runs as above. FEM_E_OOM when
  * the blocks asked for do not fit. */
 int fem_solid_set_assembled(fem_solid s, int on);
 
@@ -364,7 +366,11 @@ int fem_solid_get_rotations(fem_solid s, double* R, double* detF);
 int fem_solid_get_doc(fem_solid s, uint8_t* doc);
 /* f += f_e at the evaluated positions (C_f_e, TetrahedronElementSet3.cpp:1053-1096). N*3. */
 int fem_solid_force_elastic(fem_solid s, double* f);
-/* df += df_x(dx) = -R K0 R^T dx (C_df_x, TetrahedronElementSet3.cpp:1761-1836). N*3. */
+/* df += df_x(dx) = -R K0 R^T dx (C_df_x, TetrahedronElementSet3.cpp:1761-1836). N*3.
+ * C_WRP products, here and in the solvers, are formed in 60-bit block fixed
+ * point: subnormal operands count as zero and results below 2.2e-308 become
+ * zero; where an element's output overflows or is not finite at one of its
+ * nodes, it is NaN at all four. */
 int fem_solid_df_x(fem_solid s, const double* dx, double* df);
 /* q = S (factor_M M d - factor_K df_x(d)) (LS_A_times_d + LS_ZeroKNC,
  * LeafDSH_Solid3D_FEM.cpp:1045-1079). N*3. */

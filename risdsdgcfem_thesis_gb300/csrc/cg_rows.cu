@@ -1,6 +1,6 @@
 // cg_rows.cu -- the whole of ILSS_CG::Solve (ILSS_CG.h:38-151) or
-// ILSS_MINRES::Solve (ILSS_MINRES.h:51-168) for a C_WRP solid in one launch, the assembled stiffness's rows resident in shared
-// memory (rows_plan.h).
+// ILSS_MINRES::Solve (ILSS_MINRES.h:51-168) for a C_WRP solid in one launch,
+// the assembled stiffness's rows resident in shared memory (rows_plan.h).
 //
 // Block g owns a range of nodes: their rows as fixed-point 3x3 blocks (fx.cuh),
 // and their y, r, d, q and b, one component per thread, in registers. An
@@ -16,10 +16,14 @@
 // every block adds them all, so all take the same scalar steps and leave
 // together. A word is overwritten only after an exchange that its reader has
 // taken part in since it read it: the two sums by each other, r by the d.q
-// before it. Every wait is bounded.
+// before it; every solve writes both sums' words, so that no number comes round
+// to a word that is still there. Every wait is bounded; a block that gives up
+// says so in a word of its own (StepScalars::gave_up), and the others give up
+// at their next exchange.
 //
-// Per iteration: 3.5 us at 160 tets and 4.7 us at 3,000 on one cluster, 6.5 us
-// at 20,480 on 15; the product over the rows is a fifth of it, the rest are
+// Per iteration of CG: 3.2 us at 160 tets and 4.6 us at 3,000 on one cluster,
+// 6.3 us at 20,480 on 15, 10.3 at 87,880 on 76 of two (MINRES 4.2, 7.1 at
+// 7,215, 7.6 at 20,480); the product over the rows is a fifth of it, the rest are
 // the sums (half on 15 clusters), the division, and the vector arithmetic (one
 // FP64 instruction of a warp holds its sub-partition 64 clocks). The four launches
 // per iteration it replaces took 22 us at 20,480 tets, and its predecessor on

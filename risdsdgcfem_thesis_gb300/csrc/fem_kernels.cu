@@ -10,8 +10,9 @@
 //
 // Scatter is atomics-free: each element writes its four nodal vectors to
 // eout, and four lanes per node sum its entries in a fixed order. Reductions are
-// deterministic: integer warp sums (fx_warp_sum), a fixed block tree, then
-// the last block to finish summing the block partials.
+// deterministic: integer warp sums (fx_warp_sum), one partial per block, and
+// every block of the kernel that uses the sum adds them all (grid_total); norms
+// and energies end in one block (k_finalize).
 #include "bounds.cuh"
 #include "lcm.cuh"
 #include "fem_device.cuh"
@@ -118,13 +119,6 @@ uint64_t& launch_counter()
 {
     static uint64_t n = 0;
     return n;
-}
-
-__device__ __forceinline__ double warp_sum(double v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    return v;
 }
 
 // Block sum, valid in every thread (two rounds of fx_warp_sum).
@@ -1221,10 +1215,9 @@ __device__ __forceinline__ bool cg_continue(const StepScalars* st)
     return st->delta_new > st->abs_eps_sq && st->delta_new > st->delta_target && st->k < st->max_iter;
 }
 
-// ILSS_CG::Solve's scalar steps (ILSS_CG.h:53-151) on a reduced total: the
-// start, alpha with the breakdown test, beta with the loop test, and the
-// statistics at the end. Shared by the finaliser kernel and the one-block
-// solver below.
+// ILSS_CG::Solve's scalar steps outside its loop (ILSS_CG.h:53-73,146-151) on a
+// reduced total: the start, and the statistics at the end. The loop's are in
+// the kernels that use them (k_node_xr_fp64, k_node_d_fp64).
 __device__ __forceinline__ void fin_init(StepScalars* st, const StepConsts& c, double total)
 {
     st->delta_0 = total;
@@ -1241,27 +1234,6 @@ __device__ __forceinline__ void fin_init(StepScalars* st, const StepConsts& c, d
     st->delta_pend = total;
     st->done_pend = st->done;
     if (!isfinite(total)) st->status = 3;  // FEM_E_NAN
-}
-__device__ __forceinline__ void fin_alpha(StepScalars* st, double total)
-{
-    if (st->done) return;
-    st->dot_dq = total;
-    if (::fabs(total) < st->abs_eps_sq) {  // breakdown: leave before the update (ILSS_CG.h:97)
-        st->done = 1;
-        return;
-    }
-    st->alpha = st->delta_new / total;
-}
-__device__ __forceinline__ void fin_beta(StepScalars* st, double total)
-{
-    if (st->done) return;
-    st->delta_old = st->delta_new;
-    st->delta_new = total;
-    st->beta = total / st->delta_old;
-    st->k += 1;
-    st->total_iters += 1;
-    st->done = cg_continue(st) ? 0u : 1u;
-    if (!isfinite(total)) st->status = 3;
 }
 __device__ __forceinline__ void fin_stats(StepScalars* st)
 {

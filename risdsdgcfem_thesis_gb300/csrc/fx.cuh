@@ -229,10 +229,16 @@ FX_HD constexpr int fx_at(int r, int c)  // r <= c
 
 // An element's grade max|Dm| max|Dm^-1| (1 for a cube corner): one exponent
 // for all of Dm^-1 costs bits of K9 with it, and stiff materials cost bits of
-// the shear terms. Measured against 128-bit products (random shapes,
-// rotations and fields), the error below these grades is 0.4 to 0.95 of the
-// FP64 strain form's; above them it passes it (grade 2 to 3 at nu 0.45: up to
-// 1.2 times).
+// the shear terms. Measured against 128-bit products (jittered and stretched
+// blocks, random rotations; geometric mean over the elements of the ratio to
+// the FP64 strain form's error), random fields: 0.6 to 0.8 up to grade 3;
+// smooth ones: 0.7 to 0.8 below grade 1.5, 0.9 to 1.0 up to 2, then 1.1 to 1.2
+// up to 2.5 and 1.2 to 1.5 up to 3. At nu 0.49 to 0.4999999, grade 1.2: 0.6.
+// Blocks of cubic cells jittered by a tenth hold one element in ten thousand
+// above grade 2; its FP64 product would be the longest warp of every launch
+// (20,480 tets, a step: 515 us with the line at 3, 539 with it at 2). All
+// elements in FP64 cost what the strain form did (320,000 tets, 20 iterations:
+// 3.2 ms, none 1.8, strain form 3.3).
 constexpr float kFxMaxGrade = 3.0f, kFxMaxGradeStiff = 2.0f, kFxMaxGradeRigid = 1.2f;
 constexpr double kFxStiff = 2.0, kFxRigid = 9.5;  // lambda / mu
 
@@ -243,7 +249,7 @@ constexpr double kFxStiff = 2.0, kFxRigid = 9.5;  // lambda / mu
 // up to several times the diagonal.
 FX_HD bool fx_grade_ok(float grade, double kl, double km)
 {
-    return km > 0.0 && 3.0 * kl + 2.0 * km >= 0.0 &&
+    return (int64_t)fx_bits(km) > 0 && ((int64_t)fx_bits(kl) >= 0 || 3.0 * kl + 2.0 * km >= 0.0) &&
            grade <= (kl <= kFxStiff * km ? kFxMaxGrade : (kl <= kFxRigid * km ? kFxMaxGradeStiff : kFxMaxGradeRigid));
 }
 

@@ -72,8 +72,8 @@ __device__ __forceinline__ void elem_pk(const BatchView<S>& b, uint32_t material
 // mode SPMV_Y64_ALL for every active mesh (initial residual of a step);
 // mode SPMV_Y64_REFRESH for meshes refreshing their residual this iteration,
 // and only when the finaliser raised the batch's refresh flag (otherwise the
-// launch returns at once). The FP64 path evaluates it in FP64. The mixed
-// path, whose element data is FP32, evaluates it in double-float arithmetic
+// launch returns at once). The mixed path only (the FP64 path's is
+// k_tile_product_fp64): its element data is FP32, and it evaluates the product in double-float arithmetic
 // (about 48 bits; FP64 would cost about 60 times the FP32 rate on this GPU)
 // and writes FP64 partial sums, so its residual is accurate to about 1e-14
 // of the magnitudes of the terms of A y.

@@ -123,14 +123,14 @@ struct CgRowsLayout {
 // shared memory. max_blocks(plan): the blocks of that shape that are resident
 // together (cg_rows_max_blocks).
 // One cluster of up to 16 blocks, kRowsPerBlock rows in each before there are
-// 16 (160 tets, a step: 399 us; 12 rows 417, 24 rows 424, 48 rows 485), as long
-// as its blocks' sums fit the words a warp polls; a mesh of 3,000 tets takes
-// 512 us on it, 575 us on all clusters, whose sums go through L2 (1.3 us more
-// each). Above that clusters of 8, all that are resident together with one
-// block per SM (20,480 tets: 637 us on 15 clusters; 727 us on 36 of 4, 746 us
-// on 76 of 2, 648 us on 7 of 16), of 2 for the last of the SMs' memory. 16
-// lanes per row while a block has up to 16 rows, else 8 (20,480 tets: 660 us
-// with 16, 658 us with 4), else 4.
+// 16, as long as its blocks' sums fit the words a warp polls. Above that
+// clusters of 8, all that are resident together with one block per SM, of 2 for
+// the last of the SMs' memory. 16 lanes per row while a block has up to 16
+// rows, else 8, else 4. Measured side by side, whole steps in early forms of
+// the kernel (now 300, 421 and 515 us): 160 tets, rows in each 8 / 12 / 24 / 48:
+// 399 / 417 / 424 / 485 us; 3,000 tets on one cluster 512, on all clusters, whose
+// sums go through L2 (1.3 us more each), 575; 20,480 tets on clusters of 8 / 4 /
+// 2 / 16: 637 / 727 / 746 / 648, with 8 / 16 / 4 lanes 637 / 660 / 658.
 constexpr uint32_t kRowsPerBlock = 8;
 // lay(blocks, cluster) for each shape, the best one first, until one is true.
 template <typename F, typename L>
