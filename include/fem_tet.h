@@ -277,8 +277,8 @@ int fem_solid_get_params(fem_solid s, fem_params* params);
  * solve of a C_WRP solid whose rows fit the GPU's shared memory (on grid meshes
  * up to 106,000 tets as a cube, fewer when flat or long: 64,000 of 80 x 80 x 2
  * cells do, 90,000 of 100 x 30 x 6 do not) keeps them there in either setting,
- * in tables and memory it takes at its first solve (2 ms more for that step at
- * 20,480 tets, 7 at 88,000); without that memory it runs as above. FEM_E_OOM when
+ * in tables and memory it takes at its first solve (0.1 to 0.4 ms more for that
+ * step); without that memory it runs as above. FEM_E_OOM when
  * the blocks asked for do not fit. */
 int fem_solid_set_assembled(fem_solid s, int on);
 

@@ -72,10 +72,11 @@ __device__ __forceinline__ I bounds_idx(I idx, uint64_t, uint32_t)
     }
 #endif
 
-// the per-unit accessors (fem_kernels.cu, cg_rows.cu, rotation.cu,
+// the per-unit accessors (fem_kernels.cu, cg_rows.cu, rows_build.cu, rotation.cu,
 // batch_kernels.cu, tile_pipe.cu)
 int bounds_read_fem_kernels(unsigned* out);
 int bounds_read_cg_rows(unsigned* out);
+int bounds_read_rows_build(unsigned* out);
 int bounds_read_rotation(unsigned* out);
 int bounds_read_batch_kernels(unsigned* out);
 int bounds_read_tile_pipe(unsigned* out);

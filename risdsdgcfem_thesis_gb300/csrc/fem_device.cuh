@@ -275,6 +275,18 @@ void launch_bsr_assemble_fp64(const MeshView<double>& m, const BsrBuild& a, cuda
 void launch_bsr_vector_fp64(const MeshView<double>& m, const double* u, const StepScalars* st, int check_done,
                             cudaStream_t s);
 
+// The tables of both made on the device (rows_build.cu). most: entries of the
+// longest row (kRowEntries at most); launch_row_lengths gives each row's columns
+// and, in groups of four, the row starts.
+struct LayoutShape;
+struct LayoutRows;
+struct LayoutOut;
+void launch_row_lengths(const MeshView<double>& m, uint32_t most, uint32_t* used, uint32_t* row, cudaStream_t s);
+void launch_row_write(const MeshView<double>& m, uint32_t most, const uint32_t* used, const uint32_t* row, uint32_t* col,
+                      uint32_t* cptr, uint32_t* contrib, cudaStream_t s);
+void launch_layout_count(const LayoutShape& s, uint32_t blocks, const LayoutRows& m, CgRowsCount* count, cudaStream_t st);
+void launch_layout_write(const LayoutShape& s, uint32_t blocks, const LayoutRows& m, const LayoutOut& o, cudaStream_t st);
+
 // The solve on resident rows (cg_rows.cu): the layout's tables (rows_plan.h).
 struct CgRowsView {
     const CgRowsBlock* blk;

@@ -110,6 +110,45 @@ inline size_t cg_rows_smem_bytes(const CgRowsPlan& p, const CgRowsBlock& b)
            (24 + 4) * (size_t)b.nn + (48 + 8) * (size_t)b.nhalo + 4 * (size_t)(b.ngroups + 1) + 32 * sizeof(uint16_t) * (size_t)b.units;
 }
 
+// The plan of a shape and its blocks from each block's units and rim; false when
+// they do not fit the shared memory.
+struct CgRowsCount {
+    uint32_t units, halo;
+};
+inline bool cg_rows_plan(uint32_t N, uint32_t blocks, uint32_t cluster, uint32_t lanes, const CgRowsCount* count,
+                         CgRowsPlan& plan, std::vector<CgRowsBlock>& blk)
+{
+    plan = CgRowsPlan{};
+    plan.blocks = blocks;
+    plan.cluster = cluster;
+    plan.lanes = lanes;
+    plan.npb = (N + blocks - 1) / blocks;
+    plan.warps = (3 * plan.npb + 31) / 32;
+    plan.threads = 64;
+    blk.clear();
+    CgRowsBlock b{};
+    for (uint32_t g = 0; g < blocks; g++) {
+        b.node0 = std::min(N, g * plan.npb);
+        b.nn = std::min(N, b.node0 + plan.npb) - b.node0;
+        b.ngroups = (b.nn + 32 / lanes - 1) / (32 / lanes);
+        b.units = count[g].units;
+        b.nhalo = count[g].halo;
+        blk.push_back(b);
+        plan.units = std::max(plan.units, b.units);
+        plan.records = std::max(plan.records, b.nn + b.nhalo);
+        const uint32_t rim = std::min((3 * b.nhalo + 31) / 32 * 32, 256u);
+        plan.threads = std::max({plan.threads, 32 * b.ngroups, 32 * plan.warps + rim});
+        b.group0 += b.ngroups + 1;
+        b.unit0 += b.units;
+        b.halo0 += b.nhalo;
+    }
+    plan.threads = std::min(plan.threads, kCgRowsMaxThreads);
+    for (const CgRowsBlock& c : blk) plan.smem = std::max(plan.smem, cg_rows_smem_bytes(plan, c));
+    if (plan.smem > kCgRowsMaxSmem) return false;
+    if (blocks > 1) plan.smem = std::max(plan.smem, kCgRowsMaxSmem / 2 + 4096);  // one block per SM
+    return true;
+}
+
 // The layout of the solve on resident rows (CgRowsBlock).
 struct CgRowsLayout {
     CgRowsPlan plan;
@@ -148,6 +187,12 @@ bool cg_rows_shapes(uint32_t N, F&& max_blocks, L&& lay)
         if (blocks && lay(blocks, cluster)) return true;
     }
     return false;
+}
+// build(lanes) for each number of lanes per row, the best one first, until one is true.
+template <typename B>
+bool cg_rows_lanes(uint32_t N, uint32_t blocks, B&& build)
+{
+    return ((N + blocks - 1) / blocks <= 16 && build(16)) || build(8) || build(4);
 }
 inline bool cg_rows_shape_ok(uint32_t npb, uint32_t blocks, uint32_t cluster, uint32_t lanes)
 {
@@ -205,6 +250,7 @@ bool cg_rows_may_fit(uint32_t N, const uint32_t* tets, const std::vector<uint32_
     });
 }
 
+// The layout on the host: what the device's (rows_build.h) is checked against.
 template <typename F>
 bool cg_rows_layout(uint32_t N, const BsrPattern& p, F&& max_blocks, CgRowsLayout& o)
 {
@@ -212,7 +258,7 @@ bool cg_rows_layout(uint32_t N, const BsrPattern& p, F&& max_blocks, CgRowsLayou
     std::vector<uint32_t> order(N), seen(N, 0), place(N);
     uint32_t sorted = 0;  // rows per block that order is sorted for
     auto build = [&](uint32_t blocks, uint32_t cluster, uint32_t lanes) {
-        const uint32_t npb = (N + blocks - 1) / blocks, rows = 32 / lanes, warps = (3 * npb + 31) / 32;
+        const uint32_t npb = (N + blocks - 1) / blocks, rows = 32 / lanes;
         if (!cg_rows_shape_ok(npb, blocks, cluster, lanes)) return false;
         if (sorted != npb) {
             for (uint32_t n = 0; n < N; n++) order[n] = n;
@@ -222,80 +268,60 @@ bool cg_rows_layout(uint32_t N, const BsrPattern& p, F&& max_blocks, CgRowsLayou
             sorted = npb;
         }
         o = CgRowsLayout{};
-        CgRowsPlan& plan = o.plan;
-        plan.blocks = blocks;
-        plan.cluster = cluster;
-        plan.lanes = lanes;
-        plan.warps = warps;
-        plan.npb = npb;
-        plan.threads = 64;
-        // the shared memory without the rims first
-        for (uint32_t a = 0; a < N; a += npb) {
-            uint32_t units = 0;
-            for (uint32_t n = a; n < std::min(N, a + npb); n += rows) units += (p.used[order[n]] + lanes - 1) / lanes;
-            plan.units = std::max(plan.units, units);
-        }
-        if (cg_rows_smem_bytes(plan, CgRowsBlock{}) > kCgRowsMaxSmem) return false;
-        o.node = order;
+        std::vector<CgRowsCount> count(blocks);
+        std::vector<uint32_t> rim;
         std::fill(seen.begin(), seen.end(), 0u);
         for (uint32_t g = 0; g < blocks; g++) {
             const uint32_t a = std::min(N, g * npb), e = std::min(N, a + npb), mark = g + 1;
-            CgRowsBlock b{a, e - a, (uint32_t)o.group.size(), 0, (uint32_t)(o.slot.size() / 32), 0, (uint32_t)o.halo.size(), 0};
             for (uint32_t i = a; i < e; i++) {
                 seen[order[i]] = mark;
                 place[order[i]] = i - a;
             }
+            rim.clear();
+            for (uint32_t i = a; i < e; i++)
+                for (uint32_t k = 0; k < p.used[i]; k++) {
+                    const uint32_t c = p.col[4 * p.row[i] + k];
+                    if (seen[c] != mark) {
+                        seen[c] = mark;
+                        rim.push_back(c);
+                    }
+                }
+            std::sort(rim.begin(), rim.end());
+            for (uint32_t i = 0; i < rim.size(); i++) place[rim[i]] = e - a + i;
+            o.halo.insert(o.halo.end(), rim.begin(), rim.end());
+            uint32_t units = 0;
             for (uint32_t g0 = a; g0 < e; g0 += rows) {
-                o.group.push_back(b.units);
-                const uint32_t units = (p.used[order[g0]] + lanes - 1) / lanes;
-                for (uint32_t u = 0; u < units; u++)
+                o.group.push_back(units);
+                const uint32_t most = (p.used[order[g0]] + lanes - 1) / lanes;
+                for (uint32_t u = 0; u < most; u++)
                     for (uint32_t l = 0; l < 32; l++) {
                         const uint32_t i = g0 + l / lanes, k = lanes * u + l % lanes;
-                        if (i >= e || k >= p.used[order[i]]) {
-                            o.slot.push_back(kCgRowsPad);
-                            o.col.push_back((uint16_t)(std::min(i, e - 1) - a));
-                            continue;
-                        }
-                        const uint32_t s = 4 * p.row[order[i]] + k, c = p.col[s];
-                        if (seen[c] != mark) {
-                            seen[c] = mark;
-                            place[c] = b.nn + b.nhalo++;
-                            o.halo.push_back(c);
-                        }
+                        const bool pad = i >= e || k >= p.used[order[i]];
+                        const uint32_t s = pad ? kCgRowsPad : 4 * p.row[order[i]] + k;
                         o.slot.push_back(s);
-                        o.col.push_back((uint16_t)place[c]);
+                        o.col.push_back((uint16_t)(pad ? std::min(i, e - 1) - a : place[p.col[s]]));
                     }
-                b.units += units;
-                b.ngroups++;
+                units += most;
             }
-            o.group.push_back(b.units);
-            plan.records = std::max(plan.records, b.nn + b.nhalo);
-            const uint32_t rim = std::min((3 * b.nhalo + 31) / 32 * 32, 256u);
-            plan.threads = std::max({plan.threads, 32 * b.ngroups, 32 * warps + rim});
-            o.blk.push_back(b);
-            if (cg_rows_smem_bytes(plan, b) > kCgRowsMaxSmem) return false;
+            o.group.push_back(units);
+            count[g] = CgRowsCount{units, (uint32_t)rim.size()};
         }
-        plan.threads = std::min(plan.threads, kCgRowsMaxThreads);
-        for (const CgRowsBlock& b : o.blk) plan.smem = std::max(plan.smem, cg_rows_smem_bytes(plan, b));
-        if (plan.smem > kCgRowsMaxSmem) return false;
-        if (blocks > 1) plan.smem = std::max(plan.smem, kCgRowsMaxSmem / 2 + 4096);  // one block per SM
+        if (!cg_rows_plan(N, blocks, cluster, lanes, count.data(), o.plan, o.blk)) return false;
+        o.node = order;
         for (uint32_t i = 0; i < N; i++) place[order[i]] = i;
-        std::vector<uint32_t> shared(N, 0);
         o.owner.resize(o.halo.size());
         for (uint32_t g = 0; g < blocks; g++)
             for (uint32_t i = o.blk[g].halo0; i < o.blk[g].halo0 + o.blk[g].nhalo; i++) {
                 const uint32_t at = place[o.halo[i]], from = at / npb;
                 const bool near = from / cluster == g / cluster;
-                shared[at] |= near ? kCgRowsNearShared : kCgRowsFarShared;
+                o.node[at] |= near ? kCgRowsNearShared : kCgRowsFarShared;
                 o.owner[i] = near ? (from % cluster) << 16 | (at - from * npb) : kCgRowsFar;
             }
-        for (uint32_t i = 0; i < N; i++) o.node[i] |= shared[i];
-        return blocks <= max_blocks(plan);
+        return blocks <= max_blocks(o.plan);
     };
-    auto lay = [&](uint32_t blocks, uint32_t cluster) {
-        return ((N + blocks - 1) / blocks <= 16 && build(blocks, cluster, 16)) || build(blocks, cluster, 8) || build(blocks, cluster, 4);
-    };
-    return cg_rows_shapes(N, max_blocks, lay);
+    return cg_rows_shapes(N, max_blocks, [&](uint32_t blocks, uint32_t cluster) {
+        return cg_rows_lanes(N, blocks, [&](uint32_t lanes) { return build(blocks, cluster, lanes); });
+    });
 }
 
 }  // namespace femgb

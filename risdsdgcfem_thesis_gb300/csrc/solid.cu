@@ -18,6 +18,7 @@
 #include "dapd.cuh"
 #include "fem_device.cuh"
 #include "graph_capture.h"
+#include "rows_build.h"
 
 #include <algorithm>
 #include <cmath>
@@ -116,7 +117,7 @@ struct fem_solid_s {
     // evaluation
     DevBuf<int4> Kfx;
     DevBuf<float> grade;
-    uint32_t fx_guard = 0;
+    uint32_t fx_guard = 0, max_corners = 0;  // of elements at a node: log2, rounded up, and itself
     bool kfx_fresh = false;
     DevBuf<uint32_t> csr_ptr, csr_idx;
     DevBuf<uint8_t> fixed;
@@ -125,18 +126,22 @@ struct fem_solid_s {
     CgRowsPlan rows{};
     bool rows_tried = false;
     uint32_t wait_polls = kCgRowsPolls;
-    DevBuf<CgRowsBlock> rows_blk;
-    DevBuf<uint32_t> rows_node, rows_group, rows_slot, rows_halo, rows_owner, rows_seq;
-    DevBuf<uint16_t> rows_col;
-    DevBuf<ulonglong2> rows_words;
+    DevBuf<unsigned char> rows_mem;  // the tables and words below
+    CgRowsBlock* rows_blk = nullptr;
+    uint32_t *rows_node = nullptr, *rows_place = nullptr, *rows_group = nullptr, *rows_slot = nullptr, *rows_halo = nullptr,
+             *rows_owner = nullptr, *rows_seq = nullptr;
+    uint16_t* rows_col = nullptr;
+    ulonglong2* rows_words = nullptr;
     // the assembled stiffness (MeshView::bsr_*): pattern, per-slot
     // contributions and blocks; bsr_fresh: the blocks are those of the last
     // evaluation; bsr_use: the solvers' kernels take it (set_bsr_use)
-    DevBuf<uint32_t> bsr_row, bsr_col, bsr_cptr, bsr_contrib;
-    DevBuf<int2> bsr_val;
-    DevBuf<int32_t> bsr_x, bsr_ex;
-    DevBuf<longlong2> bsr_u;
-    DevBuf<long long> bsr_eblk;
+    DevBuf<unsigned char> bsr_lengths, bsr_pattern, bsr_blocks;  // used, row and count; col, cptr and contrib; the rest
+    uint32_t *bsr_used = nullptr, *bsr_row = nullptr, *bsr_col = nullptr, *bsr_cptr = nullptr, *bsr_contrib = nullptr;
+    CgRowsCount* bsr_count = nullptr;
+    int2* bsr_val = nullptr;
+    int32_t *bsr_x = nullptr, *bsr_ex = nullptr;
+    longlong2* bsr_u = nullptr;
+    long long* bsr_eblk = nullptr;
     uint32_t bsr_groups = 0;  // of four blocks
     bool bsr_fresh = false, bsr_want = false, bsr_use = false;  // fem_solid_set_assembled; the solvers take it now
     // node vectors
@@ -192,30 +197,16 @@ struct fem_solid_s {
 
     void release_bsr()
     {
-        bsr_row.release();
-        bsr_col.release();
-        bsr_cptr.release();
-        bsr_contrib.release();
-        bsr_val.release();
-        bsr_x.release();
-        bsr_ex.release();
-        bsr_u.release();
-        bsr_eblk.release();
+        bsr_lengths.release();
+        bsr_pattern.release();
+        bsr_blocks.release();
         bsr_groups = 0;
         bsr_fresh = false;
         release_rows();
     }
     void release_rows()
     {
-        rows_blk.release();
-        rows_node.release();
-        rows_group.release();
-        rows_slot.release();
-        rows_halo.release();
-        rows_owner.release();
-        rows_seq.release();
-        rows_col.release();
-        rows_words.release();
+        rows_mem.release();
         rows = CgRowsPlan{};
     }
 
@@ -240,11 +231,11 @@ struct fem_solid_s {
         m.fx_guard = fx_guard;
         m.grade = grade.p;
         if (bsr_use) {
-            m.bsr_row = bsr_row.p;
-            m.bsr_col = bsr_col.p;
-            m.bsr_val = bsr_val.p;
-            m.bsr_x = bsr_x.p;
-            m.bsr_u = bsr_u.p;
+            m.bsr_row = bsr_row;
+            m.bsr_col = bsr_col;
+            m.bsr_val = bsr_val;
+            m.bsr_x = bsr_x;
+            m.bsr_u = bsr_u;
         }
         return m;
     }
@@ -379,10 +370,10 @@ void assemble(fem_solid s)
 {
     if (s->bsr_fresh) return;
     MeshView<double> m = s->view();
-    m.bsr_row = s->bsr_row.p;  // also when the solvers' kernels do not take it (bsr_use)
-    m.bsr_col = s->bsr_col.p;
-    launch_bsr_assemble_fp64(m, BsrBuild{s->bsr_groups, s->bsr_cptr.p, s->bsr_contrib.p, s->bsr_eblk.p, s->bsr_ex.p,
-                                         s->bsr_val.p, s->bsr_x.p}, s->stream);
+    m.bsr_row = s->bsr_row;  // also when the solvers' kernels do not take it (bsr_use)
+    m.bsr_col = s->bsr_col;
+    launch_bsr_assemble_fp64(m, BsrBuild{s->bsr_groups, s->bsr_cptr, s->bsr_contrib, s->bsr_eblk, s->bsr_ex, s->bsr_val,
+                                         s->bsr_x}, s->stream);
     s->bsr_fresh = true;
 }
 // The product matrices of a C_WRP solid, after everything else: without the
@@ -507,57 +498,29 @@ void set_bsr_use(fem_solid s)
     s->bsr_use = s->bsr_want && s->bsr_groups > 0 && s->params.material == FEM_MATERIAL_C_WRP && !on_rows(s);
 }
 
+// One allocation for several arrays: place(at, base) sets their pointers from
+// base on (null: for the size only) and leaves the size in at.
+template <typename T>
+void take(T*& p, size_t count, size_t& at, unsigned char* base)
+{
+    at = (at + 255) & ~(size_t)255;
+    p = base ? reinterpret_cast<T*>(base + at) : nullptr;
+    at += sizeof(T) * count;
+}
+template <typename F>
+cudaError_t alloc_all(DevBuf<unsigned char>& mem, F&& place)
+{
+    size_t at = 0;
+    place(at, nullptr);
+    if (cudaError_t e = mem.alloc(at); e != cudaSuccess) return e;
+    at = 0;
+    place(at, mem.p);
+    return cudaSuccess;
+}
 template <typename V>
-cudaError_t put(DevBuf<V>& d, const std::vector<V>& h, cudaStream_t st)
+cudaError_t put(V* d, const std::vector<V>& h, cudaStream_t st)
 {
-    if (cudaError_t e = d.alloc(h.size()); e != cudaSuccess) return e;
-    return cudaMemcpyAsync(d.p, h.data(), sizeof(V) * h.size(), cudaMemcpyHostToDevice, st);
-}
-
-// Uploads the pattern and allocates the blocks.
-int upload_bsr(fem_solid s, const BsrPattern& p)
-{
-    const size_t slots = p.col.size();
-    cudaStream_t st = s->stream;
-    CK(put(s->bsr_row, p.row, st));
-    CK(put(s->bsr_col, p.col, st));
-    CK(put(s->bsr_cptr, p.cptr, st));
-    CK(put(s->bsr_contrib, p.contrib, st));
-    CK(s->bsr_val.alloc(9 * slots));
-    CK(s->bsr_x.alloc(s->N));
-    CK(s->bsr_u.alloc(2 * (size_t)s->N));
-    CK(s->bsr_ex.alloc(s->T));
-    CK(s->bsr_eblk.alloc((size_t)kBsrElemWords * s->T));
-    CK(cudaStreamSynchronize(st));
-    s->bsr_groups = (uint32_t)(slots / 4);
-    return FEM_OK;
-}
-
-// The solve on resident rows of a C_WRP solid that can have it: the
-// pattern, its blocks and the layout.
-int build_rows(fem_solid s, const uint32_t* tets, const std::vector<uint32_t>& ptr, const std::vector<uint32_t>& idx)
-{
-    BsrPattern p;
-    CgRowsLayout l;
-    if (!bsr_pattern(s->N, s->T, tets, ptr, idx, p) || !cg_rows_layout(s->N, p, cg_rows_max_blocks, l)) return FEM_OK;
-    if (!s->bsr_groups)
-        if (int e = upload_bsr(s, p)) return e;
-    cudaStream_t st = s->stream;
-    CK(put(s->rows_blk, l.blk, st));
-    CK(put(s->rows_node, l.node, st));
-    CK(put(s->rows_group, l.group, st));
-    CK(put(s->rows_slot, l.slot, st));
-    CK(put(s->rows_col, l.col, st));
-    CK(put(s->rows_halo, l.halo, st));
-    CK(put(s->rows_owner, l.owner, st));
-    const size_t words = 3 * (size_t)s->N + 2 * (size_t)l.plan.blocks * (l.plan.blocks / l.plan.cluster);
-    CK(s->rows_words.alloc(words));
-    CK(s->rows_seq.alloc(1));
-    CK(cudaMemsetAsync(s->rows_words.p, 0, sizeof(ulonglong2) * words, st));
-    CK(cudaMemsetAsync(s->rows_seq.p, 0, sizeof(uint32_t), st));
-    CK(cudaStreamSynchronize(st));
-    s->rows = l.plan;
-    return FEM_OK;
+    return cudaMemcpyAsync(d, h.data(), sizeof(V) * h.size(), cudaMemcpyHostToDevice, st);
 }
 
 // The mesh's tables, back from the device.
@@ -581,7 +544,122 @@ int read_tables(fem_solid s, std::vector<uint32_t>& tets, std::vector<uint32_t>&
     return FEM_OK;
 }
 
-// build_rows ahead of the first solve that wants it (a solid used for its
+// The assembled stiffness's pattern (bsr_groups stays 0 where it is too large),
+// made on the device unless some node is a hub (kRowEntries).
+int make_pattern(fem_solid s)
+{
+    const uint32_t N = s->N, T = s->T, most = 3 * s->max_corners + 1;
+    if ((uint64_t)T >= (1ull << 28)) return FEM_OK;
+    cudaStream_t st = s->stream;
+    BsrPattern p;
+    const bool hub = most > kRowEntries;
+    if (hub) {
+        std::vector<uint32_t> tets, ptr, idx;
+        if (int e = read_tables(s, tets, ptr, idx)) return e;
+        if (!bsr_pattern(N, T, tets.data(), ptr, idx, p)) return FEM_OK;
+    }
+    CK(alloc_all(s->bsr_lengths, [&](size_t& at, unsigned char* base) {
+        take(s->bsr_used, N, at, base);
+        take(s->bsr_row, (size_t)N + 1, at, base);
+        take(s->bsr_count, kCgRowsMaxBlocks, at, base);
+    }));
+    uint32_t groups = 0;
+    if (hub) {
+        CK(put(s->bsr_used, p.used, st));
+        CK(put(s->bsr_row, p.row, st));
+        groups = p.row[N];
+    } else {
+        launch_row_lengths(s->view(), most, s->bsr_used, s->bsr_row, st);
+        CK(cudaMemcpyAsync(&groups, s->bsr_row + N, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    }
+    CK(cudaStreamSynchronize(st));
+    if (groups >= (1u << 26)) return FEM_OK;  // slots in 28 bits
+    CK(alloc_all(s->bsr_pattern, [&](size_t& at, unsigned char* base) {
+        take(s->bsr_col, 4 * (size_t)groups, at, base);
+        take(s->bsr_cptr, 4 * (size_t)groups + 1, at, base);
+        take(s->bsr_contrib, 12 * (size_t)T, at, base);
+    }));
+    if (hub) {
+        CK(put(s->bsr_col, p.col, st));
+        CK(put(s->bsr_cptr, p.cptr, st));
+        CK(put(s->bsr_contrib, p.contrib, st));
+        CK(cudaStreamSynchronize(st));
+    } else {
+        launch_row_write(s->view(), most, s->bsr_used, s->bsr_row, s->bsr_col, s->bsr_cptr, s->bsr_contrib, st);
+    }
+    CK(cudaGetLastError());
+    s->bsr_groups = groups;
+    return FEM_OK;
+}
+
+// The blocks of a pattern, and what an assembly needs.
+int alloc_blocks(fem_solid s)
+{
+    if (s->bsr_blocks.p) return FEM_OK;
+    CK(alloc_all(s->bsr_blocks, [&](size_t& at, unsigned char* base) {
+        take(s->bsr_val, 36 * (size_t)s->bsr_groups, at, base);
+        take(s->bsr_x, s->N, at, base);
+        take(s->bsr_u, 2 * (size_t)s->N, at, base);
+        take(s->bsr_ex, s->T, at, base);
+        take(s->bsr_eblk, (size_t)kBsrElemWords * s->T, at, base);
+    }));
+    return FEM_OK;
+}
+
+// The solve on resident rows of a C_WRP solid that can have it: the pattern, the
+// layout and the blocks.
+int make_rows(fem_solid s)
+{
+    if (!s->bsr_groups)
+        if (int e = make_pattern(s)) return e;
+    if (!s->bsr_groups) return FEM_OK;
+    const uint32_t N = s->N;
+    cudaStream_t st = s->stream;
+    const LayoutRows rows{s->bsr_used, s->bsr_row, s->bsr_col};
+    LayoutShape shape{};
+    CgRowsPlan plan;
+    std::vector<CgRowsBlock> blk;
+    std::vector<CgRowsCount> count(kCgRowsMaxBlocks);
+    cudaError_t err = cudaSuccess;
+    const bool laid = cg_rows_shapes(N, cg_rows_max_blocks, [&](uint32_t blocks, uint32_t cluster) {
+        return cg_rows_lanes(N, blocks, [&](uint32_t lanes) {
+            shape = LayoutShape{N, (N + blocks - 1) / blocks, lanes, cluster};
+            if (err != cudaSuccess || !cg_rows_shape_ok(shape.npb, blocks, cluster, lanes)) return false;
+            launch_layout_count(shape, blocks, rows, s->bsr_count, st);
+            err = cudaMemcpyAsync(count.data(), s->bsr_count, sizeof(CgRowsCount) * blocks, cudaMemcpyDeviceToHost, st);
+            if (err == cudaSuccess) err = cudaStreamSynchronize(st);
+            return err == cudaSuccess && cg_rows_plan(N, blocks, cluster, lanes, count.data(), plan, blk) &&
+                   blocks <= cg_rows_max_blocks(plan);
+        });
+    });
+    CK(err);
+    if (!laid) return FEM_OK;
+    const CgRowsBlock& last = blk.back();
+    const size_t units = (size_t)last.unit0 + last.units, halo = (size_t)last.halo0 + last.nhalo;
+    const size_t words = 3 * (size_t)N + 2 * (size_t)plan.blocks * (plan.blocks / plan.cluster);
+    CK(alloc_all(s->rows_mem, [&](size_t& at, unsigned char* base) {
+        take(s->rows_words, words, at, base);
+        take(s->rows_seq, 1, at, base);  // after the words: cleared with them
+        take(s->rows_blk, blk.size(), at, base);
+        take(s->rows_node, N, at, base);
+        take(s->rows_place, N, at, base);
+        take(s->rows_group, (size_t)last.group0 + last.ngroups + 1, at, base);
+        take(s->rows_slot, 32 * units, at, base);
+        take(s->rows_halo, halo, at, base);
+        take(s->rows_owner, halo, at, base);
+        take(s->rows_col, 32 * units, at, base);
+    }));
+    if (int e = alloc_blocks(s)) return e;
+    CK(cudaMemsetAsync(s->rows_words, 0, (size_t)((unsigned char*)(s->rows_seq + 1) - (unsigned char*)s->rows_words), st));
+    CK(put(s->rows_blk, blk, st));
+    launch_layout_write(shape, plan.blocks, rows, LayoutOut{s->rows_blk, s->rows_node, s->rows_place, s->rows_group,
+                                                            s->rows_slot, s->rows_halo, s->rows_owner, s->rows_col}, st);
+    CK(cudaGetLastError());
+    s->rows = plan;
+    return FEM_OK;
+}
+
+// make_rows ahead of the first solve that wants it (a solid used for its
 // products only does not pay for it); without the device memory for them the
 // solve stays on the loop of kernels. Whether a large mesh's rows fit is known
 // from its creation (rows_tried).
@@ -590,16 +668,14 @@ int try_rows(fem_solid s)
     if (s->rows_tried || !wants_rows(s->params)) return FEM_OK;
     s->rows_tried = true;
     const std::string keep = g_err;
-    const bool had_bsr = s->bsr_groups > 0;
+    const bool had_bsr = s->bsr_blocks.p != nullptr;
     int rc = FEM_E_OOM;
     try {
-        std::vector<uint32_t> tets, ptr, idx;
-        if (int e = read_tables(s, tets, ptr, idx)) return e;
-        rc = build_rows(s, tets.data(), ptr, idx);
+        rc = make_rows(s);
     } catch (const std::bad_alloc&) {
     }
-    if (rc != FEM_OK) {
-        cudaGetLastError();
+    if (rc != FEM_OK || !on_rows(s)) {
+        if (rc != FEM_OK) cudaGetLastError();
         if (had_bsr) s->release_rows();
         else s->release_bsr();
         g_err = keep;
@@ -613,12 +689,12 @@ cudaError_t solve_on_rows(fem_solid s, const StepConsts& c)
 {
     assemble(s);
     MeshView<double> m = s->view();
-    m.bsr_val = s->bsr_val.p;
-    m.bsr_x = s->bsr_x.p;
+    m.bsr_val = s->bsr_val;
+    m.bsr_x = s->bsr_x;
     const CgRowsPlan& p = s->rows;
-    const CgRowsView v{s->rows_blk.p, s->rows_node.p, s->rows_group.p, s->rows_slot.p, s->rows_halo.p, s->rows_owner.p,
-                       s->rows_col.p, s->rows_words.p, s->rows_words.p + 3 * (size_t)s->N, p.cluster, p.warps, p.npb,
-                       p.units, p.records, s->rows_seq.p, s->wait_polls};
+    const CgRowsView v{s->rows_blk, s->rows_node, s->rows_group, s->rows_slot, s->rows_halo, s->rows_owner,
+                       s->rows_col, s->rows_words, s->rows_words + 3 * (size_t)s->N, p.cluster, p.warps, p.npb,
+                       p.units, p.records, s->rows_seq, s->wait_polls};
     return launch_cg_rows_fp64(m, c, s->rows, v, s->params.ls_solver == FEM_LS_MINRES, s->b.p, s->y.p, s->st.p, s->stream);
 }
 
@@ -843,6 +919,7 @@ int newton_step(fem_solid s, int chunk)
     c.factor_K = 1.0 + c.inv_dt * s->rayleigh[1];
     const size_t bytes = sizeof(double) * 3 * (size_t)s->N;
     const uint32_t gV = vec_grid(3 * s->N);
+    if (int e = try_rows(s)) return e;
     if (int e = open_step(s)) return e;
     CK(cudaMemcpyAsync(s->xn.p, s->x.p, bytes, cudaMemcpyDeviceToDevice, st));
     CK(cudaMemcpyAsync(s->vn.p, s->v.p, bytes, cudaMemcpyDeviceToDevice, st));
@@ -1026,7 +1103,7 @@ int fem_bounds_check_status(int* enabled, uint32_t* failures, uint32_t* site, ui
 #else
     const int on = 0;
 #endif
-    int (*const units[])(unsigned*) = {bounds_read_fem_kernels, bounds_read_cg_rows, bounds_read_rotation, bounds_read_batch_kernels,
+    int (*const units[])(unsigned*) = {bounds_read_fem_kernels, bounds_read_cg_rows, bounds_read_rows_build, bounds_read_rotation, bounds_read_batch_kernels,
                                        bounds_read_tile_pipe};
     unsigned total = 0, first[3] = {0u, 0u, 0u};
     for (auto rd : units) {
@@ -1152,7 +1229,8 @@ int fem_solid_create(const double* rest_xyz, uint32_t N, const uint32_t* tets, u
         for (size_t i = 0; i < 4 * (size_t)T; i++) idx[fill[tets[i]]++] = (uint32_t)i;
     }
     for (uint32_t n = 0; n < N; n++)
-        while ((1u << s->fx_guard) < ptr[n + 1] - ptr[n]) s->fx_guard++;
+        s->max_corners = std::max(s->max_corners, ptr[n + 1] - ptr[n]);
+    while ((1u << s->fx_guard) < s->max_corners) s->fx_guard++;
     // (a mesh of up to 8,192 nodes nearly always fits)
     s->rows_tried = N > 8192 && !cg_rows_may_fit(N, tets, ptr, idx, cg_rows_max_blocks);
     std::vector<int4> t4(T);
@@ -1259,15 +1337,16 @@ int fem_solid_set_assembled(fem_solid s, int on)
 {
     if (int e = check_handle(s)) return e;
     s->drop_graph();  // the step graph holds the operator's launches
-    if (on && !s->bsr_groups) {
-        std::vector<uint32_t> tets, ptr, idx;
-        if (int e = read_tables(s, tets, ptr, idx)) return e;
-        BsrPattern p;
-        if (bsr_pattern(s->N, s->T, tets.data(), ptr, idx, p))
-            if (int e = upload_bsr(s, p)) {
-                s->release_bsr();
-                return e;
-            }
+    if (on && !s->bsr_blocks.p) {
+        int e = FEM_E_OOM;
+        try {
+            e = make_pattern(s);
+            if (!e && s->bsr_groups) e = alloc_blocks(s);
+        } catch (const std::bad_alloc&) {
+            e = fail(FEM_E_OOM, "host memory for the assembled stiffness's pattern");
+        }
+        if (e || !s->bsr_groups) s->release_bsr();
+        if (e) return e;
     }
     s->bsr_want = on != 0;
     set_bsr_use(s);

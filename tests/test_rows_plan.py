@@ -300,3 +300,123 @@ def test_quotient_by_the_reciprocal(tmp_path):
         for b in edges:
             u = lib.ulps(a, b)
             assert u <= 0.5 + 2.0 ** -50 and (u == -1.0 or np.isfinite([a, b]).all()), (a, b, u)
+
+
+BUILD = r"""
+#include <memory>
+#include "rows_build.h"
+using namespace femgb;
+// The device's pattern and layout, every thread of a step in turn, against the
+// host's; returns 0, or the line of the first difference (-1: no layout, both).
+#define CHECK(x) do { if (!(x)) return __LINE__; } while (0)
+extern "C" int build(uint32_t N, uint32_t T, const uint32_t* tets, uint32_t sms)
+{
+    std::vector<uint32_t> ptr(N + 1, 0), idx(4 * (size_t)T);
+    for (size_t i = 0; i < 4 * (size_t)T; i++) ptr[tets[i] + 1]++;
+    for (uint32_t n = 0; n < N; n++) ptr[n + 1] += ptr[n];
+    std::vector<uint32_t> fill(ptr.begin(), ptr.end() - 1);
+    for (size_t i = 0; i < 4 * (size_t)T; i++) idx[fill[tets[i]]++] = (uint32_t)i;
+    BsrPattern p;
+    CHECK(bsr_pattern(N, T, tets, ptr, idx, p));
+    const size_t slots = p.col.size();
+    std::vector<uint32_t> e(kRowEntries), before(kRowEntries), col(slots, ~0u), cptr(slots + 1, ~0u), contrib(12 * (size_t)T, ~0u);
+    cptr[slots] = 12 * T;
+    for (uint32_t n = 0; n < N; n++) {
+        const uint32_t entries = 3 * (ptr[n + 1] - ptr[n]) + 1;
+        CHECK(entries <= kRowEntries);
+        uint32_t used = 0;
+        for (uint32_t t = 0; t < 32; t++) row_entries(n, ptr[n], entries, tets, idx.data(), e.data(), t, 32);
+        for (uint32_t t = 0; t < 32; t++) used += row_columns(e.data(), entries, before.data(), t, 32);
+        CHECK(used == p.used[n]);
+        for (uint32_t t = 0; t < 32; t++)
+            row_write(e.data(), before.data(), entries, ptr[n], used, 4 * p.row[n], idx.data(), col.data(), cptr.data(),
+                      contrib.data(), t, 32);
+    }
+    CHECK(col == p.col && cptr == p.cptr && contrib == p.contrib);
+    auto most = [&](const CgRowsPlan& q) {
+        return q.threads > kCgRowsMaxThreads || q.smem > kCgRowsMaxSmem || q.cluster > sms ? 0u : sms;
+    };
+    CgRowsLayout l;
+    const bool laid = cg_rows_layout(N, p, most, l);
+    CgRowsPlan plan;
+    std::vector<CgRowsBlock> blk;
+    const LayoutRows rows{p.used.data(), p.row.data(), p.col.data()};
+    std::unique_ptr<LayoutWork> w(new LayoutWork);
+    const uint32_t K = kLayoutThreads;
+    LayoutShape shape{};
+    auto count = [&](const LayoutShape& s, uint32_t g) {
+        const LayoutSpan b = layout_span(s, g);
+        for (uint32_t t = 0; t < K; t++) layout_begin(b, rows, *w, t, K);
+        for (uint32_t t = 0; t < K; t++) layout_rim(b, rows, *w, t, K);
+        for (uint32_t t = 0; t < K; t++) layout_parts(s, b, *w, t, K);
+        for (uint32_t t = 0; t < K; t++) layout_sum(*w, t, K);
+    };
+    const bool built = cg_rows_shapes(N, most, [&](uint32_t blocks, uint32_t cluster) {
+        return cg_rows_lanes(N, blocks, [&](uint32_t lanes) {
+            shape = LayoutShape{N, (N + blocks - 1) / blocks, lanes, cluster};
+            if (!cg_rows_shape_ok(shape.npb, blocks, cluster, lanes)) return false;
+            if (shape.npb > kLayoutRows || (N + 31) / 32 > kLayoutWords) __builtin_trap();
+            std::vector<CgRowsCount> c(blocks);
+            for (uint32_t g = 0; g < blocks; g++) {
+                count(shape, g);
+                c[g] = CgRowsCount{w->units, w->halo};
+            }
+            return cg_rows_plan(N, blocks, cluster, lanes, c.data(), plan, blk) && blocks <= most(plan);
+        });
+    });
+    CHECK(built == laid);
+    if (!laid) return -1;
+    CHECK(plan.blocks == l.plan.blocks && plan.threads == l.plan.threads && plan.smem == l.plan.smem);
+    const CgRowsBlock& z = blk.back();
+    std::vector<uint32_t> node(N, ~0u), place(N, ~0u), group(z.group0 + z.ngroups + 1, ~0u), slot(32 * (size_t)(z.unit0 + z.units), ~1u),
+        halo(z.halo0 + z.nhalo, ~0u), owner(halo.size(), ~1u);
+    std::vector<uint16_t> lcol(slot.size(), 0xffff);
+    const LayoutOut o{blk.data(), node.data(), place.data(), group.data(), slot.data(), halo.data(), owner.data(), lcol.data()};
+    for (uint32_t g = 0; g < plan.blocks; g++) {
+        count(shape, g);
+        const LayoutSpan b = layout_span(shape, g);
+        for (uint32_t t = 0; t < K; t++) layout_ahead(b, *w, t, K);
+        for (uint32_t t = 0; t < K; t++) layout_write(shape, b, g, rows, *w, o, t, K);
+    }
+    for (uint32_t g = 0; g < plan.blocks; g++)
+        for (uint32_t t = 0; t < K; t++) layout_owners(shape, g, o, t, K);
+    CHECK(node == l.node && group == l.group && slot == l.slot && halo == l.halo && owner == l.owner && lcol == l.col);
+    for (uint32_t g = 0; g < plan.blocks; g++) CHECK(memcmp(&blk[g], &l.blk[g], sizeof(CgRowsBlock)) == 0);
+    return 0;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def build(tmp_path_factory):
+    if shutil.which("g++") is None:
+        pytest.skip("no host compiler")
+    d = tmp_path_factory.mktemp("build")
+    src, so = d / "build.cpp", d / "build.so"
+    src.write_text(BUILD)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-D_GLIBCXX_ASSERTIONS", "-fsanitize=undefined", "-fno-sanitize-recover",
+                    "-Wno-unknown-pragmas", "-shared", "-fPIC", "-I", CSRC, str(src), "-o", str(so)], check=True)
+    return C.CDLL(str(so)).build
+
+
+@pytest.mark.parametrize("sms", [2, 16, 152])
+@pytest.mark.parametrize("mesh,shuffle", [(_grid(1, 1, 1), False), (_grid(2, 2, 1), False), (_grid(5, 5, 5), False),
+                                          (_grid(6, 6, 5), True), (_grid(12, 12, 11), False), (_grid(17, 16, 15), True),
+                                          (_grid(24, 24, 24), False), (_grid(26, 26, 26), False), (_star(100), False),
+                                          ((9, _grid(1, 1, 1)[1]), False), ((45, _grid(1, 1, 1)[1] + 20), False)],
+                         ids=["cell", "20", "625", "900shuffled", "7920", "20400shuffled", "69120", "87880", "star", "lone",
+                              "apart"])
+def test_tables_made_on_the_device(build, mesh, shuffle, sms):
+    """The device's steps (rows_build.h) give the host's tables, whatever the
+    mesh, entry for entry."""
+    n, tets = mesh
+    if shuffle:
+        tets = np.random.default_rng(2).permutation(n).astype(np.uint32)[tets]
+    tets = np.ascontiguousarray(tets, np.uint32)
+    assert build(n, len(tets), tets.ctypes.data_as(C.POINTER(C.c_uint32)), sms) in ((0,) if sms == 152 else (0, -1))
+
+
+def test_tables_of_a_degenerate_mesh(build):
+    """Elements that name a node twice, and twice the same element."""
+    tets = np.array([[0, 1, 2, 3], [1, 1, 2, 4], [3, 2, 1, 0], [4, 5, 5, 5], [0, 1, 2, 3]], np.uint32)
+    assert build(7, len(tets), tets.ctypes.data_as(C.POINTER(C.c_uint32)), 152) == 0
