@@ -22,8 +22,8 @@
 // at their next exchange.
 //
 // Per iteration of CG: 3.2 us at 160 tets and 4.6 us at 3,000 on one cluster,
-// 6.3 us at 20,480 on 15, 10.3 at 87,880 on 76 of two (MINRES 4.2, 7.1 at
-// 7,215, 7.6 at 20,480); the product over the rows is a fifth of it, the rest are
+// 6.3 us at 20,480 on 15, 10.3 at 87,880 on 76 of two (MINRES 4.2, 7.0 at
+// 7,215, 7.5 at 20,480); the product over the rows is a fifth of it, the rest are
 // the sums (half on 15 clusters), the division, and the vector arithmetic (one
 // FP64 instruction of a warp holds its sub-partition 64 clocks). The four launches
 // per iteration it replaces took 22 us at 20,480 tets, and its predecessor on

@@ -26,8 +26,9 @@ FX_HD bool rows_word_is(const W& w, double& v, uint32_t seq)
 }
 
 // A partial sum: m in units of 2^(e - 1079), |m| <= 2^62; kPartNan: NaN;
-// kPartInf: m counts infinities by their sign, 2^40 each, so that what finite
-// parts leave of m when it is added in their place (-1 at most) is no
+// kPartInf: m counts infinities by their sign, 2^56 each (their fraction as
+// fx_align leaves it), 2^42 at least after the sums' scaling, so that what
+// finite parts leave of m when it is added in their place (-1 at most) is no
 // infinity. It stays in integers from the lanes to the solid's total.
 struct Part {
     int64_t m;
@@ -37,20 +38,18 @@ constexpr int32_t kPartNan = 0x7fff, kPartInf = 0x7ffe;
 FX_HD Part part_of(double v)
 {
     const int32_t e = fx_exp(v);
-    const uint64_t u = fx_bits(v);
-    if (e == 2047) return Part{(int64_t)u < 0 ? -(1ll << 40) : 1ll << 40, (u << 12) != 0 ? kPartNan : kPartInf};
-    return Part{fx_align<57>(v, e), e};
+    return Part{fx_align<57>(v, e), e == 2047 ? kPartNan - ((fx_bits(v) << 12) == 0 ? 1 : 0) : e};
 }
 FX_HD double part_value(const Part& p)
 {
-    if (p.e >= kPartInf) {
-        const int64_t least = 1ll << 39;
-        if (p.e == kPartNan || (p.m < least && p.m > -least)) return fx_from_bits(0x7ff8000000000000ull);
-        return fx_from_bits(p.m < 0 ? 0xfff0000000000000ull : 0x7ff0000000000000ull);
-    }
     const double v = (double)p.m;
     const int32_t e = fx_exp(v) + p.e - 1079;
-    if (p.m == 0 || e < 1 || e > 2046) return fx_to_double(p.m, p.e - 1079);
+    if (p.m == 0 || e < 1 || e > 2046) {  // (kPartInf and kPartNan are far above)
+        const int64_t least = 1ll << 39;
+        if (p.e == kPartNan || (p.e == kPartInf && p.m < least && p.m > -least)) return fx_from_bits(0x7ff8000000000000ull);
+        if (p.e == kPartInf) return fx_from_bits(p.m < 0 ? 0xfff0000000000000ull : 0x7ff0000000000000ull);
+        return fx_to_double(p.m, p.e - 1079);
+    }
     return fx_from_bits(fx_bits(v) + ((uint64_t)(int64_t)(p.e - 1079) << 52));
 }
 
@@ -82,8 +81,8 @@ FX_HD bool rows_quotient(double t, double d, double r, double& q)
 {
     const double q0 = t * r;
     q = fma(fma(-q0, d, t), r, q0);
-    // q0 and r between 2^-959 and 2^941, t above 2^-900
-    return (uint32_t)fx_exp(r) - 64u <= 1900u && (uint32_t)fx_exp(q0) - 64u <= 1900u && fx_exp(t) > 123;
+    // q0 between 2^-511 and 2^512, r between 2^-959 and 2^389: t is above 2^-900
+    return (uint32_t)fx_exp(q0) - 512u < 1024u && (uint32_t)fx_exp(r) - 64u < 1348u;
 }
 
 // What the words of a CTA hold when a solve starts after number seq: sums

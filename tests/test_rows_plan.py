@@ -216,7 +216,7 @@ extern "C" int taken(uint32_t seq)
     return 0;
 }
 extern "C" double through(double v) { return part_value(part_of(v)); }
-extern "C" double infinities(int plus, int minus) { return part_value(Part{(int64_t)(plus - minus) * (1ll << 40) - 5120, kPartInf}); }
+extern "C" double infinities(int plus, int minus) { return part_value(Part{(int64_t)(plus - minus) * (1ll << 42) - 5120, kPartInf}); }
 extern "C" int kept(double v, int64_t m, int32_t e, uint32_t seq)
 {
     Part p;
