@@ -694,7 +694,7 @@ int batch_leave_matrices(fem_batch b)
     b->graph = nullptr;
     return build_graph(b);
 }
-bool batch_has_matrices(fem_batch b) { return b->Kfx.p != nullptr; }
+uint64_t batch_matrix_bytes(fem_batch b) { return b->Kfx.bytes(); }
 }  // namespace femgb
 
 extern "C" {

@@ -54,7 +54,7 @@ int batch_fail(int code, const char* fmt, ...);
 int batch_enqueue_readback(fem_batch b);
 unsigned batch_host_err(fem_batch b);
 int batch_leave_matrices(fem_batch b);
-bool batch_has_matrices(fem_batch b);
+uint64_t batch_matrix_bytes(fem_batch b);
 }  // namespace femgb
 
 using femgb::batch_fail;
@@ -205,22 +205,31 @@ int build_shard(fem_server srv, const std::vector<uint32_t>& ids, bool matrices,
     return FEM_OK;
 }
 
+// A shard without its product matrices (its launch in flight is waited for);
+// sh.bytes follows.
+int leave_matrices(Shard& sh)
+{
+    if (int e = femgb::batch_leave_matrices(sh.b)) return e;
+    fem_batch_info(sh.b, nullptr, nullptr, nullptr, nullptr, &sh.bytes);
+    return FEM_OK;
+}
+
 // Whether `bytes` more fit the budget, if need be without the product
-// matrices of the resident FP64 shards, which are given back one by one (a
-// shard's launch in flight is waited for): they make its steps faster, but
-// take no scene's place.
+// matrices of the resident FP64 shards, which are then given back one by one:
+// they make its steps faster, but take no scene's place.
 int make_room(fem_server srv, uint64_t bytes, bool& fits)
 {
+    uint64_t least = srv->used_bytes + bytes;
+    for (auto& sh : srv->shards)
+        if (sh.b) least -= femgb::batch_matrix_bytes(sh.b);
+    fits = least <= srv->opt.hbm_budget_bytes;
     for (auto& sh : srv->shards) {
-        if (srv->used_bytes + bytes <= srv->opt.hbm_budget_bytes) break;
-        if (!sh.b || !femgb::batch_has_matrices(sh.b)) continue;
-        if (int e = femgb::batch_leave_matrices(sh.b)) return e;
-        uint64_t now = 0;
-        fem_batch_info(sh.b, nullptr, nullptr, nullptr, nullptr, &now);
-        srv->used_bytes -= sh.bytes - now;
-        sh.bytes = now;
+        if (!fits || srv->used_bytes + bytes <= srv->opt.hbm_budget_bytes) break;
+        if (!sh.b || !femgb::batch_matrix_bytes(sh.b)) continue;
+        const uint64_t had = sh.bytes;
+        if (int e = leave_matrices(sh)) return e;
+        srv->used_bytes -= had - sh.bytes;
     }
-    fits = srv->used_bytes + bytes <= srv->opt.hbm_budget_bytes;
     return FEM_OK;
 }
 
@@ -378,12 +387,17 @@ int fem_server_admit(fem_server s, uint32_t* admitted)
         if (!fits) break;
         Shard sh;
         if (int e = build_shard(s, ids, matrices, sh)) return e;
-        if (int e = make_room(s, sh.bytes, fits)) {
+        int e = FEM_OK;
+        if (s->used_bytes + sh.bytes > s->opt.hbm_budget_bytes) {  // the estimate was short
+            e = leave_matrices(sh);
+            if (!e) e = make_room(s, sh.bytes, fits);
+        }
+        if (e) {
             sh.bytes = 0;
             s->take_down(sh);
             return e;
         }
-        if (!fits) {  // estimate was short: undo
+        if (!fits) {  // undo
             sh.bytes = 0;  // not counted yet
             s->take_down(sh);
             break;
@@ -430,12 +444,11 @@ int fem_server_set_params(fem_server s, uint32_t scene, const fem_params* params
         // the first C_WRP scene of an FP64 shard brings the product matrices
         uint64_t now = 0;
         fem_batch_info(sh.b, nullptr, nullptr, nullptr, nullptr, &now);
-        if (now > sh.bytes && s->used_bytes + (now - sh.bytes) > s->opt.hbm_budget_bytes) {
-            if (int e = femgb::batch_leave_matrices(sh.b)) return e;
-            fem_batch_info(sh.b, nullptr, nullptr, nullptr, nullptr, &now);
-        }
-        s->used_bytes += now - sh.bytes;
+        const uint64_t had = sh.bytes;
         sh.bytes = now;
+        if (now > had && s->used_bytes + (now - had) > s->opt.hbm_budget_bytes)
+            if (int e = leave_matrices(sh)) return e;
+        s->used_bytes += sh.bytes - had;
     }
     sc.params = p;
     return FEM_OK;

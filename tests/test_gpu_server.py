@@ -189,6 +189,17 @@ def test_product_matrices_take_no_scenes_place(fem_lib, waves):
     srv.close()
 
 
+def test_matrices_are_kept_where_giving_them_back_admits_nothing(fem_lib):
+    small, large = (scenes.random_block(np.random.default_rng(5), dims=d, idx=0) for d in ((13, 13, 13), (30, 30, 30)))
+    srv = fem_lib.Server(fem_lib.FEM_PRECISION_FP64, hbm_budget_bytes=20 << 20, shard_max_scenes=1)
+    srv.add(small)
+    assert srv.admit() == 1
+    before = srv.status()["device_bytes"]
+    srv.add(large)  # 40 MB and more
+    assert srv.admit() == 0 and srv.status()["device_bytes"] == before > 600 * small.num_tets
+    srv.close()
+
+
 @pytest.mark.parametrize("room", [True, False])
 def test_product_matrices_come_with_the_first_elastic_scene(fem_lib, room):
     """A scene that changes from a P-K material to C_WRP brings its shard the
